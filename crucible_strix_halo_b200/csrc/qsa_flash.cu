@@ -7,10 +7,10 @@
 // exact, and the causal rule (key position <= row position) cuts the tail block.
 //
 // qsa_union_build_kernel (one CTA per tile): every row contributes its selected blocks (or all complete blocks when
-// dense) plus its open tail block as keys (block, row); sorting the keys puts the rows of a block side by side, and
-// the first key of every run emits (block, OR of the row bits).  No array over the context is needed, so the context
-// length does not limit it (the reference keeps a byte per block in 64 KB of LDS and falls back to row-wise
-// attention past about 196K positions, engine/layers/qsa_union_lds.h:7-11).
+// dense) plus its open tail block to a bitmap over the block ids; ranks in the bitmap are places in the list, where the
+// rows OR their bits.  The bitmap is walked in windows, so the context length does not limit it (the reference keeps a
+// byte per block in 64 KB of LDS and falls back to row-wise attention past about 196K positions,
+// engine/layers/qsa_union_lds.h:7-11).
 //
 // qsa_flash_tc_kernel (one CTA per (tile, KV head), 15 warps, 64 keys per step):
 //   loader warps (6)   gather the K and V rows of 16 blocks per step with 16-byte cp.async into three stages, two
@@ -49,7 +49,6 @@ constexpr int kFlPBytes = 128 * kFlKeys * 2;        // [8 key pieces][128 rows][
 constexpr size_t kFlashSmem = 2 * kFlStages * kFlKBytes + 2 * kFlPBytes + 128;
 // TMEM columns: O 0-255, S of step j at 256 + 64 (j & 1), the query tile (two fp16 channels per column) at 384-511
 constexpr uint32_t kColO = 0, kColS = 256, kColQ = 384;
-constexpr int kUbThreads = 1024;
 
 struct FlashParams {
   cr_qsa_args a;          // the output rows (pos0 = position of row 0)
@@ -69,77 +68,95 @@ int qsa_union_rows(const cr_geometry* g) {
 int qsa_union_cap(int RT) { return (RT * 513 + 15) / 16 * 16; }
 
 // ---- union lists -------------------------------------------------------------------------------------------
-// One CTA per tile.  Every (block, row) pair of the tile becomes a 32-bit key block * 16 + row; the keys are sorted
-// in shared memory (bitonic network), which puts the rows of one block side by side.  The first key of every block
-// gathers the row bits of its run (at most 16 keys) and takes its place in the output from a prefix sum over the
-// run heads.
-__global__ void __launch_bounds__(kUbThreads) qsa_union_build_kernel(cr_qsa_args a, int2* list, int* count, int cap, int RT, int n_pad) {
-  extern __shared__ __align__(16) unsigned ukeys[];      // n_pad keys (a power of two >= RT * 513)
-  __shared__ unsigned red[33];
+// One CTA per tile, a warp per row.  The attended blocks of all rows set bits of a shared-memory bitmap over the block
+// ids; a prefix sum of the word popcounts gives every block its rank in the ascending union, and the rows then OR their
+// bit into the mask of that rank.  Contexts past kUbWindow blocks (1 M positions) are walked in windows of that many.
+// Bound: latency of four short shared-memory passes.  2,048 rows at 262,144 positions: 113 us as a bitonic sort of 8,208
+// (block, row) keys (105 barrier-separated passes over 64 KB), 8 us as bitmap + rank.
+constexpr int kUbThreads = 512;
+constexpr int kUbWindow = 262144;                      // blocks per window: 32 KB of bitmap, 32 KB of word ranks
+
+static size_t union_smem_bytes(int words, int cap) { return ((size_t)2 * words + 2 * (size_t)cap) * sizeof(unsigned); }
+
+__global__ void __launch_bounds__(kUbThreads) qsa_union_build_kernel(const __grid_constant__ cr_qsa_args a, int2* list, int* count, int cap, int RT,
+                                                                     int words) {
+  extern __shared__ __align__(16) unsigned ub[];
+  unsigned* bits = ub;                                   // words: which blocks of the window any row attends
+  unsigned* rank = bits + words;                         // words: blocks of the window below this word
+  unsigned* mask = rank + words;                         // cap: row bits of the union's entries
+  unsigned* ids = mask + cap;                            // cap: their block ids
+  __shared__ unsigned red[kUbThreads / 32 + 1];
   const int t = threadIdx.x, w = t >> 5, l = t & 31;
-  const int tile = blockIdx.x, row0 = tile * RT;
-  constexpr unsigned kNone = 0xFFFFFFFFu;                // padding: sorts last
-  for (int i = t; i < n_pad; i += kUbThreads) ukeys[i] = kNone;
-  __syncthreads();
-  if (w < RT && row0 + w < a.R) {                         // one warp per row: slots [513 w, 513 w + 513)
-    const int gr = row0 + w, p = a.pos0 + gr, nb = (p + 1) / 4, ns = a.nsel[gr];
-    const int n = ns < 0 ? nb : CR_SEL_BLOCKS;           // dense rows attend every complete block (at most 512 of them)
-    const int* sel = a.sel + (size_t)gr * CR_SEL_BLOCKS;
-    unsigned* mine = ukeys + w * 513;
-    for (int i = l; i < n; i += 32) mine[i] = ((unsigned)(ns < 0 ? i : sel[i]) << 4) | (unsigned)w;
-    if ((p + 1) % 4 != 0 && l == 0) mine[n] = ((unsigned)nb << 4) | (unsigned)w;   // the open block holds the tail tokens
-  }
-  // ascending bitonic sort
-  for (int k = 2; k <= n_pad; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      __syncthreads();
-      for (int q = t; q < (n_pad >> 1); q += kUbThreads) {
-        const int i = ((q & ~(j - 1)) << 1) | (q & (j - 1));
-        const unsigned x = ukeys[i], y = ukeys[i + j];
-        const bool up = (i & k) == 0;
-        if ((x > y) == up) { ukeys[i] = y; ukeys[i + j] = x; }
-      }
-    }
-  }
-  __syncthreads();
-  // run heads: thread t owns the keys [t * per, (t + 1) * per)
-  const int per = n_pad / kUbThreads;
-  int heads = 0;
-  for (int i = t * per; i < (t + 1) * per; ++i) {
-    const unsigned k = ukeys[i];
-    heads += k != kNone && (i == 0 || (ukeys[i - 1] >> 4) != (k >> 4));
-  }
-  // exclusive prefix sum of `heads` over the block
-  unsigned inc = (unsigned)heads;
+  const int tile = blockIdx.x, row0 = tile * RT, rows = min(RT, a.R - row0);
+  const int total = (a.pos0 + row0 + rows - 1) / 4 + 1;  // blocks up to the one of the tile's last row
+  // this warp's row (16 warps, at most 16 rows)
+  const bool have = w < rows;
+  const int gr = row0 + w, p = a.pos0 + gr, nb = (p + 1) / 4;
+  const int ns = have ? a.nsel[gr] : 0;
+  const int n = have ? (ns < 0 ? nb : CR_SEL_BLOCKS) : 0;   // dense rows attend every complete block (at most 512 of them)
+  const int* sel = a.sel + (size_t)gr * CR_SEL_BLOCKS;
+  constexpr int kPer = CR_SEL_BLOCKS / 32;
+  int blk[kPer];
 #pragma unroll
-  for (int s = 1; s < 32; s <<= 1) {
-    const unsigned o = __shfl_up_sync(0xffffffffu, inc, s);
-    if (l >= s) inc += o;
+  for (int k = 0; k < kPer; ++k) {
+    const int i = l + 32 * k;
+    blk[k] = i < n ? (ns < 0 ? i : sel[i]) : -1;
   }
-  if (l == 31) red[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    const unsigned mine = red[l];
-    unsigned winc = mine;
+  const int open = have && (p + 1) % 4 != 0 ? nb : -1;     // the open block holds the tail tokens
+  for (int i = t; i < 2 * cap; i += kUbThreads) mask[i] = 0u;
+  unsigned base = 0;                                       // entries of the windows before this one
+  for (int w0 = 0; w0 < total; w0 += kUbWindow) {
+    const int span = min(kUbWindow, total - w0), nw = (span + 31) >> 5;
+    auto in_window = [&](int b) { return b >= w0 && b - w0 < span; };
+    for (int i = t; i < nw; i += kUbThreads) bits[i] = 0u;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (in_window(blk[k])) atomicOr(&bits[(blk[k] - w0) >> 5], 1u << (blk[k] & 31));
+    if (l == 0 && in_window(open)) atomicOr(&bits[(open - w0) >> 5], 1u << (open & 31));
+    __syncthreads();
+    const int per = (nw + kUbThreads - 1) / kUbThreads, i0 = min(t * per, nw), i1 = min(i0 + per, nw);
+    unsigned mine = 0;
+    for (int i = i0; i < i1; ++i) mine += __popc(bits[i]);
+    unsigned inc = mine;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
-      const unsigned o = __shfl_up_sync(0xffffffffu, winc, s);
-      if (l >= s) winc += o;
+      const unsigned o = __shfl_up_sync(0xffffffffu, inc, s);
+      if (l >= s) inc += o;
     }
-    red[l] = winc - mine;
-    if (l == 31) red[32] = winc;
+    if (l == 31) red[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+      const unsigned v = l < kUbThreads / 32 ? red[l] : 0u;
+      unsigned winc = v;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const unsigned o = __shfl_up_sync(0xffffffffu, winc, s);
+        if (l >= s) winc += o;
+      }
+      if (l < kUbThreads / 32) red[l] = winc - v;
+      if (l == 31) red[kUbThreads / 32] = winc;
+    }
+    __syncthreads();
+    unsigned at = base + red[w] + inc - mine;
+    for (int i = i0; i < i1; ++i) { rank[i] = at; at += __popc(bits[i]); }
+    base += red[kUbThreads / 32];
+    __syncthreads();
+    auto place = [&](int b) {
+      const int word = (b - w0) >> 5;
+      const unsigned r = rank[word] + __popc(bits[word] & ((1u << (b & 31)) - 1u));
+      atomicOr(&mask[r], 1u << w);
+      ids[r] = (unsigned)b;
+    };
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (in_window(blk[k])) place(blk[k]);
+    if (l == 0 && in_window(open)) place(open);
+    __syncthreads();
   }
-  __syncthreads();
-  int at = (int)(red[w] + inc) - heads;
   int2* out = list + (size_t)tile * cap;
-  for (int i = t * per; i < (t + 1) * per; ++i) {
-    const unsigned k = ukeys[i];
-    if (k == kNone || (i != 0 && (ukeys[i - 1] >> 4) == (k >> 4))) continue;
-    int mask = 0;
-    for (int e = i; e < n_pad && (ukeys[e] >> 4) == (k >> 4); ++e) mask |= 1 << (ukeys[e] & 15u);
-    out[at++] = make_int2((int)(k >> 4), mask);
-  }
-  if (t == 0) count[tile] = (int)red[32];
+  for (int i = t; i < (int)base; i += kUbThreads) out[i] = make_int2((int)ids[i], (int)mask[i]);
+  if (t == 0) count[tile] = (int)base;
 }
 
 // ---- flash ---------------------------------------------------------------------------------------------------
@@ -461,14 +478,13 @@ __global__ void __launch_bounds__(64) qsa_out_transform_kernel(cr_qsa_args a, co
 cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int2* list, int* count, cudaStream_t stream) {
   static PerDeviceOnce configured;
   if (cr_status st = once_per_device(configured, [] {
-        CR_CUDA(cudaFuncSetAttribute(qsa_union_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * (int)sizeof(unsigned)));
+        CR_CUDA(cudaFuncSetAttribute(qsa_union_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)union_smem_bytes(kUbWindow / 32, qsa_union_cap(16))));
         return CR_OK;
       })) return st;
-  const int RT = qsa_union_rows(g), tiles = (a.R + RT - 1) / RT;
-  int n_pad = kUbThreads;
-  while (n_pad < RT * 513) n_pad <<= 1;
+  const int RT = qsa_union_rows(g), tiles = (a.R + RT - 1) / RT, cap = qsa_union_cap(RT);
+  const int blocks = (a.pos0 + a.R - 1) / 4 + 1, words = ((blocks < kUbWindow ? blocks : kUbWindow) + 31) / 32;
   use_stream(stream);
-  qsa_union_build_kernel<<<tiles, kUbThreads, (size_t)n_pad * sizeof(unsigned), stream>>>(a, list, count, qsa_union_cap(RT), RT, n_pad);
+  qsa_union_build_kernel<<<tiles, kUbThreads, union_smem_bytes(words, cap), stream>>>(a, list, count, cap, RT, words);
   CR_LAUNCH_CHECK("qsa_union_build_kernel");
   return CR_OK;
 }
