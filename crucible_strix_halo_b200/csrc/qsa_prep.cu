@@ -12,131 +12,180 @@ __global__ void rope_table_kernel(float* table) {
   else if (j < CR_ROPE_TABLE_FLOATS) table[j] = j == 32 ? 1.f : 0.f;
 }
 
-// Split-half RoPE of x[0..63] (shared memory) at cache position p by threads 0..31; two barriers.  With a table of
-// multimodal positions (mrope [capacity][4]: t, h, w of every cache position; engine/layers/ops.h:515-541) frequency j
-// turns with the h position when j % 3 == 1, with the w position when j % 3 == 2 and j < 30, else with t (interleaved
-// sections [11, 11, 10]); equal axes give the text rotation exactly.
-__device__ __forceinline__ void rope64_smem(float* x, const float* rope, const int* mrope, int p) {
-  const int j = threadIdx.x;
-  float c = 0.f, s = 0.f, a = 0.f, b = 0.f;
-  if (j < 32) {
-    int pj = p;
-    if (mrope) pj = j % 3 == 1 ? mrope[4 * (size_t)p + 1] : (j % 3 == 2 && j < 30 ? mrope[4 * (size_t)p + 2] : mrope[4 * (size_t)p]);
-    rope_cs(rope, j, pj, c, s);
-    a = x[j];
-    b = x[j + 32];
-  }
-  __syncthreads();
-  if (j < 32) {
-    x[j] = a * c - b * s;
-    x[j + 32] = b * c + a * s;
-  }
-  __syncthreads();
+// Cosine and sine of frequency j (< 32) of the row at cache position p.  With a table of multimodal positions (mrope
+// [capacity][4]: t, h, w of every cache position; engine/layers/ops.h:515-541) frequency j turns with the h position when
+// j % 3 == 1, with the w position when j % 3 == 2 and j < 30, else with t (interleaved sections [11, 11, 10]); equal axes
+// give the text rotation exactly.
+__device__ __forceinline__ void rope_terms(const cr_qsa_args& a, int j, int p, float& c, float& s) {
+  int pj = p;
+  if (a.mrope) pj = j % 3 == 1 ? a.mrope[4 * (size_t)p + 1] : (j % 3 == 2 && j < 30 ? a.mrope[4 * (size_t)p + 2] : a.mrope[4 * (size_t)p]);
+  rope_cs(a.rope, j, pj, c, s);
 }
 
-// CN-RMSNorm of n (128 or 256) values in shared memory, one per thread.
-__device__ __forceinline__ void cnorm_smem(float* x, int n, const float* w1, float* red) {
-  const int j = threadIdx.x;
-  const float v = j < n ? x[j] : 0.f;
-  const float ss = block_sum<256>(v * v, red);
-  if (j < n) x[j] = v * rsqrtf(ss / n + kEps) * w1[j];
-  __syncthreads();
+// Four consecutive floats at p (16-byte aligned where VEC).
+template <bool VEC>
+__device__ __forceinline__ float4 ld4(const float* p) {
+  if constexpr (VEC) return *reinterpret_cast<const float4*>(p);
+  else return make_float4(p[0], p[1], p[2], p[3]);
+}
+template <bool VEC>
+__device__ __forceinline__ void st4(float* p, const float4 v) {
+  if constexpr (VEC) *reinterpret_cast<float4*>(p) = v;
+  else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
+}
+template <bool VEC>
+__device__ __forceinline__ void st_half4(uint16_t* p, const float4 v) {
+  const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+  const unsigned u0 = *reinterpret_cast<const unsigned*>(&lo), u1 = *reinterpret_cast<const unsigned*>(&hi);
+  if constexpr (VEC) *reinterpret_cast<uint2*>(p) = make_uint2(u0, u1);
+  else { p[0] = (uint16_t)u0; p[1] = (uint16_t)(u0 >> 16); p[2] = (uint16_t)u1; p[3] = (uint16_t)(u1 >> 16); }
 }
 
-__device__ __forceinline__ bool raw_uses_chunk(int slots, int rows) { return slots != 0 && rows > 8; }
+// A head of 128 (N4 = 1) or 256 (N4 = 2) values spread over a warp: lane l holds elements 4 l .. 4 l + 3 (and 128 + 4 l ..).
+// CN-RMSNorm, then split-half RoPE of the first 64: lanes 0-7 hold the first half of the pairs, lanes 8-15 the second.
+// c4 / s4: cosines and sines of the frequencies 4 (l % 8) .. + 3.
+template <bool VEC, int N4>
+__device__ __forceinline__ void norm_rope(float4 (&x)[N4], const float* w1, const float4 c4, const float4 s4) {
+  const int l = threadIdx.x & 31;
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < N4; ++i) ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+  const float rs = rsqrtf(warp_sum(ss) / (128.f * N4) + kEps);
+#pragma unroll
+  for (int i = 0; i < N4; ++i) {
+    const float4 w = ld4<VEC>(w1 + 128 * i + 4 * l);
+    x[i] = make_float4(x[i].x * rs * w.x, x[i].y * rs * w.y, x[i].z * rs * w.z, x[i].w * rs * w.w);
+  }
+  float4 o;                                              // the partner of every element: j and j + 32
+  o.x = __shfl_xor_sync(0xffffffffu, x[0].x, 8); o.y = __shfl_xor_sync(0xffffffffu, x[0].y, 8);
+  o.z = __shfl_xor_sync(0xffffffffu, x[0].z, 8); o.w = __shfl_xor_sync(0xffffffffu, x[0].w, 8);
+  if (l < 16) {
+    const float sg = l < 8 ? -1.f : 1.f;
+    x[0] = make_float4(x[0].x * c4.x + sg * o.x * s4.x, x[0].y * c4.y + sg * o.y * s4.y, x[0].z * c4.z + sg * o.z * s4.z,
+                       x[0].w * c4.w + sg * o.w * s4.w);
+  }
+}
 
-__device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b, float* x, float* red);
+// Rows at which a call keeps only the newest raw keys of a ring (a longer call writes the ring once, at its end).
+__device__ __forceinline__ bool raw_kept(const cr_qsa_args& a, int r) { return a.c.raw_slots == 0 || r >= a.R - a.c.raw_slots; }
+// Whether the ring slot of row r is that of one of the positions before this call that share the call's first block:
+// the warp that pools the block reads them first and writes those rows itself.
+__device__ __forceinline__ bool raw_after_pool(const cr_qsa_args& a, int r) {
+  if (a.c.raw_slots == 0 || a.pos0 % 4 == 0 || (a.pos0 + a.R) / 4 == a.pos0 / 4) return false;
+  for (int p = a.pos0 / 4 * 4; p < a.pos0; ++p)
+    if (p % a.c.raw_slots == (a.pos0 + r) % a.c.raw_slots) return true;
+  return false;
+}
 
-// grid (units + pool_units, Rmax, spans), 256 threads.  Blocks x >= units (row 0 only) pool completed blocks.  Units: [0,Hq) query heads, [Hq,Hq+Hkv) key heads,
-// [Hq+Hkv, Hq+2Hkv) value heads, then 4 indexer-query heads, then the raw indexer key.
-// u0 skips leading units (u0 = Hq runs the cache units only).  q_hi (optional): fp16 copy of the prepared
-// queries [R][Hq][256] for the prefill attention kernels; rows < q_skip are not written to q_hi.
-// queries_only: the key, value and raw-key units and the pooling do nothing (a rank of a split-KV group that does not own
-// the rows' positions still normalises the queries).
-__global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ QsaParams P, int u0, __half* q_hi, int q_skip, int units, int queries_only) {
+// Pooled key of block b (complete within rows pos0..pos0+R-1 or earlier) by one warp: mean of 4 raw keys -> fp16 round ->
+// CN-RMSNorm -> RoPE at the block start.  Raw keys of this call's rows are read from the input rows, older ones from the
+// cache, so the result does not depend on the other warps having run.
+template <bool VEC>
+__device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
+  const int l = threadIdx.x & 31;
+  float4 k4[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int pos = b * 4 + t;
+    k4[t] = ld4<VEC>(pos >= a.pos0 ? a.idx + (size_t)(pos - a.pos0) * 640 + 512 + 4 * l : a.c.ik_raw + raw_offset(a.c.raw_slots, pos, 4 * l));
+  }
+  float cj, sj;
+  rope_terms(a, l, b * 4, cj, sj);
+  float4 c4, s4;
+  const int f0 = 4 * (l & 7);
+  c4.x = __shfl_sync(0xffffffffu, cj, f0); c4.y = __shfl_sync(0xffffffffu, cj, f0 + 1); c4.z = __shfl_sync(0xffffffffu, cj, f0 + 2); c4.w = __shfl_sync(0xffffffffu, cj, f0 + 3);
+  s4.x = __shfl_sync(0xffffffffu, sj, f0); s4.y = __shfl_sync(0xffffffffu, sj, f0 + 1); s4.z = __shfl_sync(0xffffffffu, sj, f0 + 2); s4.w = __shfl_sync(0xffffffffu, sj, f0 + 3);
+  float4 x[1];
+  x[0] = make_float4(round_h((((0.f + k4[0].x) + k4[1].x) + k4[2].x + k4[3].x) * 0.25f), round_h((((0.f + k4[0].y) + k4[1].y) + k4[2].y + k4[3].y) * 0.25f),
+                     round_h((((0.f + k4[0].z) + k4[1].z) + k4[2].z + k4[3].z) * 0.25f), round_h((((0.f + k4[0].w) + k4[1].w) + k4[2].w + k4[3].w) * 0.25f));
+  norm_rope<VEC>(x, a.ik_norm1, c4, s4);
+  float* dst = a.c.ik_pool + pool_offset(b, 4 * l);
+  dst[0] = x[0].x; dst[32] = x[0].y; dst[64] = x[0].z; dst[96] = x[0].w;
+  if (b == a.pos0 / 4 && a.c.raw_slots != 0) {            // the ring rows that had to wait for the reads above
+    __syncwarp();
+    for (int r = max(0, a.R - a.c.raw_slots); r < a.R; ++r)
+      if (raw_after_pool(a, r))
+        st4<VEC>(a.c.ik_raw + raw_offset(a.c.raw_slots, a.pos0 + r, 4 * l), ld4<VEC>(a.idx + (size_t)r * 640 + 512 + 4 * l));
+  }
+}
+
+// grid (unit groups, Rmax, spans), 256 threads; a warp takes the units blockIdx.x * 8 * UPW + w + 8 i, i < UPW, of one row.
+// Units: [0, Hq) query heads, [.., + Hkv) key heads, [.., + Hkv) value heads, 4 indexer-query heads, the raw indexer key, and
+// the pooled key of the block that the row completes.  u0 skips leading units (u0 = Hq runs the cache units only).
+// q_hi (optional): fp16 copy of the prepared queries [R][Hq][256] for the prefill attention kernels; rows < q_skip are
+// not written to q_hi.  queries_only: only the query and indexer-query units do anything (a rank of a split-KV group that
+// does not own the rows' positions still normalises the queries).
+//
+// Bound: HBM for a part (query rows in and out, fp16 copies, cache rows), latency for a step.  A head lives in one warp
+// (128-bit loads, shuffle reduction, no barrier but the one behind the row's 32 cosines and sines, which every unit of the
+// row shares: angles past 105,615 take cosf's long reduction).  A step gives every unit a warp of its own (UPW = 1); a part
+// takes a row per CTA with all loads of a warp issued first (UPW = 5).  2,048 rows at 262,144 positions: 98.8 us as one
+// CTA per (row, unit), 28 us now (4.9 TB/s).
+template <int UPW, bool VEC>
+__global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ QsaParams P, int u0, __half* q_hi, int q_skip, int queries_only) {
+  pdl_release();
+  pdl_wait();
   const cr_qsa_args& a = P.span[blockIdx.z];
   const int r = blockIdx.y;
   if (r >= a.R) return;
-  __shared__ float x[256], red[8];
-  if (queries_only) {
-    const int u = (int)blockIdx.x + u0;
-    if ((int)blockIdx.x >= units || (u >= P.Hq && u < P.Hq + 2 * P.Hkv) || u >= P.Hq + 2 * P.Hkv + 4) return;
-  }
-  if ((int)blockIdx.x >= units) {
-    const int b = a.pos0 / 4 + ((int)blockIdx.x - units);
-    if (r == 0 && b < (a.pos0 + a.R) / 4) pool_block(a, b, x, red);
-    return;
-  }
-  const int u = blockIdx.x + u0, j = threadIdx.x, p = a.pos0 + r;
-  const int Hq = P.Hq, Hkv = P.Hkv;
-  if (u < Hq) {
-    float* q = a.q + ((size_t)r * Hq + u) * 512;
-    x[j] = q[j];
-    __syncthreads();
-    cnorm_smem(x, 256, a.q_norm1, red);
-    rope64_smem(x, a.rope, a.mrope, p);
-    q[j] = x[j];
-    if (q_hi && r >= q_skip) q_hi[((size_t)r * Hq + u) * 256 + j] = __float2half(x[j]);
-  } else if (u < Hq + Hkv) {
-    const int g = u - Hq;
-    x[j] = a.k[(size_t)r * Hkv * 256 + g * 256 + j];
-    __syncthreads();
-    cnorm_smem(x, 256, a.k_norm1, red);
-    rope64_smem(x, a.rope, a.mrope, p);
-    reinterpret_cast<__half*>(a.c.k)[((size_t)p * Hkv + g) * 256 + j] = __float2half(x[j]);
-  } else if (u < Hq + 2 * Hkv) {
-    const int g = u - Hq - Hkv;
-    reinterpret_cast<__half*>(a.c.v)[((size_t)p * Hkv + g) * 256 + j] = __float2half(a.v[(size_t)r * Hkv * 256 + g * 256 + j]);
-  } else if (u < Hq + 2 * Hkv + 4) {
-    float* iq = a.idx + (size_t)r * 640 + (u - Hq - 2 * Hkv) * 128;
-    if (j < 128) x[j] = iq[j];
-    __syncthreads();
-    cnorm_smem(x, 128, a.iq_norm1, red);
-    rope64_smem(x, a.rope, a.mrope, p);
-    if (j < 128) iq[j] = x[j];
-  } else if (j < 128 && !raw_uses_chunk(a.c.raw_slots, a.R)) {
-    a.c.ik_raw[raw_offset(a.c.raw_slots, p, j)] = a.idx[(size_t)r * 640 + 512 + j];
-  }
-}
-
-// Pooled key of block b (complete within rows pos0..pos0+R-1 or earlier): mean of 4 raw keys -> fp16 round ->
-// CN-RMSNorm -> RoPE at the block start.  Raw keys of this call's rows are read from the input rows, older ones
-// from the cache, so the result does not depend on the prep units having run.
-__device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b, float* x, float* red) {
-  const int j = threadIdx.x;
-  if (j < 128) {
-    float m = 0.f;
+  __shared__ __align__(16) float cs[32], sn[32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, p = a.pos0 + r, Hq = P.Hq, Hkv = P.Hkv;
+  const int first = u0 + blockIdx.x * 8 * UPW + w;
+  float4 x[UPW][2];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int pos = b * 4 + t;
-      m += pos >= a.pos0 ? a.idx[(size_t)(pos - a.pos0) * 640 + 512 + j] : a.c.ik_raw[raw_offset(a.c.raw_slots, pos, j)];
+  for (int i = 0; i < UPW; ++i) {
+    const int u = first + 8 * i;
+    const float* src = nullptr;
+    bool wide = true;
+    if (u < Hq) src = a.q + ((size_t)r * Hq + u) * 512;
+    else if (u < Hq + 2 * Hkv) src = queries_only ? nullptr : (u < Hq + Hkv ? a.k + ((size_t)r * Hkv + u - Hq) * 256 : a.v + ((size_t)r * Hkv + u - Hq - Hkv) * 256);
+    else if (u < Hq + 2 * Hkv + 5) { src = u < Hq + 2 * Hkv + 4 || !queries_only ? a.idx + (size_t)r * 640 + (u - Hq - 2 * Hkv) * 128 : nullptr; wide = false; }
+    x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (src) {
+      x[i][0] = ld4<VEC>(src + 4 * l);
+      if (wide) x[i][1] = ld4<VEC>(src + 128 + 4 * l);
     }
-    x[j] = round_h(m * 0.25f);
+  }
+  if (w == 0) {
+    float c, s;
+    rope_terms(a, l, p, c, s);
+    cs[l] = c; sn[l] = s;
   }
   __syncthreads();
-  cnorm_smem(x, 128, a.ik_norm1, red);
-  rope64_smem(x, a.rope, a.mrope, b * 4);
-  if (j < 128) a.c.ik_pool[pool_offset(b, j)] = x[j];
-}
-
-// Block b = pos0/4 + blockIdx.x of span blockIdx.y, if these rows complete it (bulk rows; steps pool inside prep).
-__global__ void __launch_bounds__(256) qsa_pool_kernel(const __grid_constant__ QsaParams P) {
-  const cr_qsa_args& a = P.span[blockIdx.y];
-  __shared__ float x[256], red[8];
-  const int b = a.pos0 / 4 + blockIdx.x;
-  if (b >= (a.pos0 + a.R) / 4) return;
-  pool_block(a, b, x, red);
-}
-
-// Bulk rows with a raw ring: keep the newest min(R, slots) raw keys (after every pool has read the old tail).
-__global__ void qsa_retain_raw_kernel(const __grid_constant__ QsaParams P) {
-  const cr_qsa_args& a = P.span[blockIdx.y];
-  if (!raw_uses_chunk(a.c.raw_slots, a.R)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int keep = min(a.R, a.c.raw_slots);
-  if (i >= keep * 128) return;
-  const int row = a.R - keep + i / 128, dim = i % 128;
-  a.c.ik_raw[raw_offset(a.c.raw_slots, a.pos0 + row, dim)] = a.idx[(size_t)row * 640 + 512 + dim];
+  const float4 c4 = *reinterpret_cast<const float4*>(&cs[4 * (l & 7)]), s4 = *reinterpret_cast<const float4*>(&sn[4 * (l & 7)]);
+#pragma unroll
+  for (int i = 0; i < UPW; ++i) {
+    const int u = first + 8 * i;
+    if (u < Hq) {
+      norm_rope<VEC>(x[i], a.q_norm1, c4, s4);
+      float* q = a.q + ((size_t)r * Hq + u) * 512 + 4 * l;
+      st4<VEC>(q, x[i][0]);
+      st4<VEC>(q + 128, x[i][1]);
+      if (q_hi && r >= q_skip) {
+        uint16_t* h = reinterpret_cast<uint16_t*>(q_hi) + ((size_t)r * Hq + u) * 256 + 4 * l;
+        st_half4<VEC>(h, x[i][0]);
+        st_half4<VEC>(h + 128, x[i][1]);
+      }
+    } else if (u < Hq + 2 * Hkv) {
+      if (queries_only) continue;
+      const bool key = u < Hq + Hkv;
+      if (key) norm_rope<VEC>(x[i], a.k_norm1, c4, s4);
+      uint16_t* h = (key ? a.c.k : a.c.v) + ((size_t)p * Hkv + (u - Hq - (key ? 0 : Hkv))) * 256 + 4 * l;
+      st_half4<VEC>(h, x[i][0]);
+      st_half4<VEC>(h + 128, x[i][1]);
+    } else if (u < Hq + 2 * Hkv + 4) {
+      float4 y[1] = {x[i][0]};
+      norm_rope<VEC>(y, a.iq_norm1, c4, s4);
+      st4<VEC>(a.idx + (size_t)r * 640 + (u - Hq - 2 * Hkv) * 128 + 4 * l, y[0]);
+    } else if (queries_only) {
+      continue;
+    } else if (u == Hq + 2 * Hkv + 4) {
+      if (raw_kept(a, r) && !raw_after_pool(a, r))
+        st4<VEC>(a.c.ik_raw + raw_offset(a.c.raw_slots, p, 4 * l), x[i][0]);
+    } else if (u == Hq + 2 * Hkv + 5) {
+      if (p % 4 == 3) pool_block<VEC>(a, p / 4);
+    }
+  }
 }
 
 cr_status qsa_validate(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, int max_rows, const char* who, int score_blocks) {
@@ -179,28 +228,20 @@ cr_status qsa_prep_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     QsaParams P;
     qsa_fill_params(P, g, spans + s0, n);
     const int Rmax = qsa_max_rows(spans + s0, n);
-    const int units = g->q_heads + 2 * g->kv_heads + 5 - u0;
-    int completed = 0, keep = 0;
-    bool ring = false;
-    for (int s = 0; s < n; ++s) {
+    const int units = g->q_heads + 2 * g->kv_heads + 6 - u0;
+    bool vec = ((uintptr_t)q_hi & 7) == 0;          // buffers at 4-byte boundaries take scalar accesses
+    for (int s = 0; s < n && vec; ++s) {
       const cr_qsa_args& a = spans[s0 + s];
-      const int c = (a.pos0 + a.R) / 4 - a.pos0 / 4;
-      completed = c > completed ? c : completed;
-      ring = ring || (a.c.raw_slots != 0 && a.R > 8);
-      keep = a.c.raw_slots > keep ? a.c.raw_slots : keep;
+      for (const void* ptr : {(const void*)a.q, (const void*)a.k, (const void*)a.v, (const void*)a.idx, (const void*)a.q_norm1, (const void*)a.k_norm1,
+                              (const void*)a.iq_norm1, (const void*)a.ik_norm1, (const void*)a.c.k, (const void*)a.c.v, (const void*)a.c.ik_raw})
+        vec = vec && ((uintptr_t)ptr & 15) == 0;
     }
-    const bool fused_pool = Rmax <= 16;            // steps: pooling rides in the prep launch
-    qsa_prep_kernel<<<dim3(units + (fused_pool && !queries_only ? completed : 0), Rmax, n), 256, 0, stream>>>(P, u0, q_hi, q_skip, units, queries_only ? 1 : 0);
+    constexpr int kBulk = 5;                       // 40 units: every row of the built geometries in one CTA
+    const bool bulk = (long long)Rmax * n > 128;    // below that a CTA per row would leave SMs idle
+    auto kernel = bulk ? (vec ? qsa_prep_kernel<kBulk, true> : qsa_prep_kernel<kBulk, false>) : (vec ? qsa_prep_kernel<1, true> : qsa_prep_kernel<1, false>);
+    const int per_cta = 8 * (bulk ? kBulk : 1);
+    CR_CUDA(launch_pdl(kernel, dim3((units + per_cta - 1) / per_cta, Rmax, n), dim3(256), 0, stream, P, u0, q_hi, q_skip, queries_only ? 1 : 0));
     CR_LAUNCH_CHECK("qsa_prep_kernel");
-    if (queries_only) continue;
-    if (completed && !fused_pool) {
-      qsa_pool_kernel<<<dim3(completed, n), 256, 0, stream>>>(P);
-      CR_LAUNCH_CHECK("qsa_pool_kernel");
-    }
-    if (ring) {
-      qsa_retain_raw_kernel<<<dim3((keep * 128 + 255) / 256, n), 256, 0, stream>>>(P);
-      CR_LAUNCH_CHECK("qsa_retain_raw_kernel");
-    }
   }
   return CR_OK;
 }
