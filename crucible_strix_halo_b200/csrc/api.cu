@@ -53,6 +53,18 @@ void count_launch(const char* name) {
   if (g_profile.load(std::memory_order_relaxed)) mark(name);
 }
 
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+    known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 static cr_options g_options = {kGdnPartChunksDefault, 1, 0, 0};
 const cr_options& options() { return g_options; }
 

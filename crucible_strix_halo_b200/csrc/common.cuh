@@ -85,6 +85,7 @@ void use_stream(cudaStream_t stream);   // the stream the following launches go 
   } while (0)
 
 cr_status check_geometry(const cr_geometry* g);
+int sm_count();                          // multiprocessors of the current device (looked up once per device)
 
 // A device status word of one translation unit with its host-side reader and clearer (both synchronise).  A bounded
 // wait that gives up stores 1 in it; api.cu assembles the words of all units into cr_device_status().

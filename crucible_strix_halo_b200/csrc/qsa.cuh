@@ -34,12 +34,10 @@ cr_status qsa_score_tc_launch(const QsaParams& P, int Rmax, int n, cudaStream_t 
 cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream);
 cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream);
 cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream);
-// splits: KV splits per (row, KV head). p0/p1: position window (shard mode) or 0 / INT_MAX.
 struct QsaTileSplit { const int* count; int rows, max; };   // see QsaParams::tile_count
-cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int splits,
-                          int p0, int p1, cudaStream_t stream, const QsaTileSplit* tiles = nullptr);
-// Merges `nparts` partial records per (row, head) found at partials[((part_major ? part*rows_total+row : row) ...)].
-cr_status qsa_merge_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, const float* partials, int nparts,
-                           bool part_major, float* partial_out, cr_out_format fmt, cudaStream_t stream, const QsaTileSplit* tiles = nullptr);
+// Attention of the spans' rows over the attended positions inside [p0, p1): outputs, or with `partials` one (m, l, acc[256])
+// record per (row, head).
+cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int p0, int p1, cr_out_format fmt,
+                          cudaStream_t stream, const QsaTileSplit* tiles = nullptr);
 
 }  // namespace cr

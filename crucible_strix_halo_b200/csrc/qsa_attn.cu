@@ -1,367 +1,485 @@
-// QSA attention over the attended positions for sm_100a (decode, verify, and the row-wise prefill path).
+// QSA attention over the attended positions for sm_100a (decode, verify, and the row-wise prefill path): the job of
+// QsaGqaSplitKernel and QsaMergeKernel (engine/layers/qsa_long.h:399-499) in one kernel.
 //
-// Split-KV gather (QsaGqaSplitKernel, engine/layers/qsa_long.h:399-456): one CTA of four warps per (split, row,
-// KV head).  The query heads of the KV group are the M rows of a tensor-core tile (8..12 heads padded to 16), so
-// every K/V row fetched is used by all heads at once:
-//   S[16 x 32] = Q[16 x 256] K^T      mma.sync m16n8k16 f16, warp w owns positions 8w .. 8w+7 of the tile
-//   O[16 x 256] += P[16 x 32] V       warp w owns channels 64w .. 64w+63
-// K and V are fp16 in the cache.  Q and P are fp32 values: each is split into an fp16 head and an fp16 remainder
-// and multiplied twice, which keeps the products at fp32 accuracy (the remainder carries the bits fp16 drops).
-// Tiles of 32 positions are gathered with cp.async (zero fill for masked positions) into two shared-memory
-// stages, the next tile in flight while the current one is multiplied; row maxima and sums cross the four warps
-// through shared memory.  Each CTA writes the partial (m, l, acc[256]) of its heads; the merge kernel
-// (QsaMergeKernel, qsa_long.h:458-499) combines them by log-sum-exp, applies the sigmoid gate and the output
-// transform.  No CTA waits on another CTA.
+// A unit is a (row, KV head): up to 513 entries (selected blocks of 4 positions, then the open block), walked by one or
+// more streams.  A stream is one warp (two where the KV group has more than 8 query heads, half of the heads each) that
+// takes 16 positions at a time, with the positions as the M rows and the query heads as the N = 8 columns of mma.sync
+// m16n8k16, so no row of the product is padding:
+//   S^T[16 x 8] = K[16 x 256] Q^T        Q stays in registers as column fragments
+//   O^T[256 x 8] += V^T[256 x 16] P^T    V read transposed by ldmatrix; P turned by movmatrix, in registers
+// K and V are fp16 in the cache.  Q and P are fp32 values: each is split into an fp16 head and an fp16 remainder and
+// multiplied twice, which keeps the products at fp32 accuracy.  Every stream has a ring of three 8 KB halves (K or V of
+// 16 positions, one 512-byte row per cp.async instruction, XOR-swizzled in 16-byte pieces) of which two are in flight
+// while the third is multiplied, and nothing in the loop crosses warps: no block barrier, no shared maxima.
+// Streams of a unit are merged by log-sum-exp in shared memory and, when a unit spans several CTAs, over a thread-block
+// cluster through distributed shared memory; the sigmoid gate and the output transform follow in place, so no partial
+// sum goes through HBM.
+//
+// Bound: the gather.  Random 512-byte rows of a 512 MB cache arrive at 8.5 TB/s (16 MB: 20 TB/s).  The form before this
+// one (a CTA per (row, KV head, split), heads as M rows, Q re-read from shared memory for every tile, partials merged by
+// a second kernel) was held by shared-memory reads and barriers: 2,048 rows at 262,144 positions took 1,875 us plus
+// 180 us of merge, 849 us now (10.1 TB/s of gathers: the rows walk
+// their ascending positions side by side, so the rows in flight share a region of the cache that L2 holds); 72 verify
+// rows at 131,072 105 + 12 us, 53 us now; four decode rows at 262,144 17 + 9 us, 14 us now.
 #include <climits>
+#include <cooperative_groups.h>
 #include "qsa.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cr {
 
-constexpr int kTile = 32;            // positions per shared-memory tile
-constexpr int kRowH = 264;           // padded row of 256 halves: 528 B keeps ldmatrix conflict-free
-constexpr int kPRowH = 40;           // padded row of the 16 x 32 probability tile (80 B)
-constexpr int kMaxSplitPos = 576;    // positions listed in shared memory at a time (18 tiles); a longer split walks its list in chunks
+constexpr int kTok = 16;                       // positions per tile: four blocks
+constexpr int kHalfBytes = kTok * 512;         // K or V rows of a tile
+constexpr int kSlots = 3;                      // halves in a stream's ring
+constexpr int kRingBytes = kSlots * kHalfBytes;
+constexpr int kAccLd = 260;                    // floats per head of an accumulator image in shared memory (conflict-free writes)
+constexpr int kMaxWarps = 12;
 
-// STAGES = 2: the next tile is gathered while the current one is multiplied (a step: few CTAs, latency counts).
-// STAGES = 1: 55 KB per CTA, four CTAs per SM keep more gathers in flight (a prefill part: thousands of CTAs).
-template <int STAGES>
-struct SplitSmem {
-  __half q[2][16][kRowH];            // head and remainder of the query rows
-  __half k[STAGES][kTile][kRowH];
-  __half v[STAGES][kTile][kRowH];
-  __half p[2][16][kPRowH];           // head and remainder of the probabilities
-  float red[2][4][16];               // per-warp row maxima / row sums
-  int pos[kMaxSplitPos];             // cache position of every attended index of this split, -1 = masked
+// Streams of a CTA by head groups: 8 of one warp, or 6 of two (168 registers a thread fill the register file).
+template <int NG> constexpr int kStreams = NG == 1 ? 8 : 6;
+template <int NG> constexpr int kAttnThreads = kStreams<NG> * NG * 32;
+template <int NG> constexpr size_t kAttnSmem = (size_t)kStreams<NG> * kRingBytes;
+
+struct AttnShape {
+  int spu;                                     // streams of a CTA that share a unit; kStreams / spu units per CTA
+  int cluster;                                 // CTAs per unit (spu = all streams then)
 };
 
-__device__ __forceinline__ int qsa_position(const int* sel, int t, int ns, int nb) {
-  return ns < 0 ? t : (t < ns * 4 ? sel[t >> 2] * 4 + (t & 3) : nb * 4 + t - ns * 4);
-}
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+__device__ __forceinline__ void attn_cp16(unsigned dst, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
 }
-__device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)));
+__device__ __forceinline__ void ldsm_x4(unsigned (&r)[4], unsigned addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)));
+__device__ __forceinline__ void ldsm_x4_trans(unsigned (&r)[4], unsigned addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ unsigned transpose8(unsigned x) {   // 8 x 8 fp16 of a warp: row g, columns 2 tq, 2 tq + 1 per lane
+  unsigned y;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+  return y;
 }
 __device__ __forceinline__ void mma_f16(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-
-// grid (splits, Rmax * Hkv, spans), or (Rmax * Hkv, splits, spans) for STAGES == 1; 128 threads.
-template <int STAGES>
-__global__ void __launch_bounds__(128) qsa_attn_split_kernel(const __grid_constant__ QsaParams P, float* partials,
-                                                             int splits, int p0, int p1) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SplitSmem<STAGES>& sm = *reinterpret_cast<SplitSmem<STAGES>*>(smem_raw);
-  pdl_release();
-  pdl_wait();
-  const cr_qsa_args& a = P.span[blockIdx.z];
-  // STAGES == 1 (many rows): grid (rows x KV heads, splits), the split being the slow index.  Split s of every row
-  // covers about the s-th part of the context (attended positions ascend), so the CTAs in flight at any time read one
-  // region of the cache, which L2 can hold.  STAGES == 2 (steps): grid (splits, rows x KV heads).
-  const int rg = STAGES == 1 ? blockIdx.x : blockIdx.y;
-  const int r = rg / P.Hkv, g = rg % P.Hkv;
-  if (r >= a.R || qsa_row_is_tiled(P, r)) return;
-  const int gqa = P.Hq / P.Hkv;
-  const int t = threadIdx.x, w = t >> 5, l = t & 31;
-  const int split = STAGES == 1 ? blockIdx.y : blockIdx.x;
-  const int p = a.pos0 + r, ns = a.nsel[r], nb = (p + 1) / 4;
-  const int n = ns < 0 ? p + 1 : ns * 4 + (p + 1) % 4;
-  const int* sel = a.sel + (size_t)r * CR_SEL_BLOCKS;
-  // Attended indices run through ascending positions (selected blocks, then the tail), so the positions inside a rank's
-  // window [p0, p1) are one contiguous range [t_lo, t_hi) of them: only that range is split and visited.
-  int t_lo = 0, t_hi = n;
-  if (p0 > 0 || p1 <= p) {
-    if (ns < 0) { t_lo = min(p0, n); t_hi = min(p1, n); }
-    else {
-      auto first_block_at_least = [&](int blk) {          // index of the first selected block >= blk
-        int lo = 0, hi = ns;
-        while (lo < hi) { const int mid = (lo + hi) >> 1; if (sel[mid] < blk) lo = mid + 1; else hi = mid; }
-        return lo;
-      };
-      t_lo = 4 * first_block_at_least((p0 + 3) / 4);
-      t_hi = 4 * first_block_at_least(p1 / 4 + (p1 % 4 ? 1 : 0));
-      if (nb * 4 >= p0 && nb * 4 < p1) t_hi = n;          // the tail tokens 4 nb .. p
-      else if (nb * 4 < p0) t_lo = t_hi;                  // a window past every attended position
-    }
-  }
-  const int n_win = max(t_hi - t_lo, 0);
-  // tiles of 32 attended indices are dealt evenly: the first (tiles % splits) splits take one more
-  const int tiles = (n_win + kTile - 1) / kTile, tb = tiles / splits, trem = tiles % splits;
-  const int begin = t_lo + (split * tb + min(split, trem)) * kTile, end = min(begin + (tb + (split < trem ? 1 : 0)) * kTile, t_hi);
-  const int total = max(end - begin, 0);                  // positions of this split, walked in chunks of at most kMaxSplitPos
-  int cnt = 0, chunk0 = 0;
-  auto list_chunk = [&]() {                               // attended positions [begin + chunk0, + cnt) into shared memory
-    cnt = min(total - chunk0, kMaxSplitPos);
-    for (int i = t; i < cnt; i += 128) {
-      int pos = qsa_position(sel, begin + chunk0 + i, ns, nb);
-      if (pos < p0 || pos >= p1) pos = -1;
-      sm.pos[i] = pos;
-    }
-    __syncthreads();
-  };
-  list_chunk();
-
-  const __half* kc = reinterpret_cast<const __half*>(a.c.k);
-  const __half* vc = reinterpret_cast<const __half*>(a.c.v);
-  auto stage = [&](int tile, int buf) {   // 32 positions x (32 K + 32 V) 16-byte pieces
-    for (int piece = t; piece < kTile * 64; piece += 128) {
-      const int j = piece >> 6, c = piece & 63, idx = tile * kTile + j;
-      const int pos = idx < cnt ? sm.pos[idx] : -1;
-      const bool valid = pos >= 0;
-      const size_t off = valid ? ((size_t)pos * P.Hkv + g) * 256 + (c & 31) * 8 : 0;
-      cp_async_16(c < 32 ? &sm.k[buf][j][(c & 31) * 8] : &sm.v[buf][j][(c & 31) * 8], (c < 32 ? kc : vc) + off, valid);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-
-  int ntiles = (cnt + kTile - 1) / kTile;
-  const int row0 = l >> 2, cq = (l & 3) * 2;              // this thread's rows row0, row0 + 8; columns cq, cq + 1 of an n-tile
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-  float O[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) O[i][0] = O[i][1] = O[i][2] = O[i][3] = 0.f;
-  if (STAGES == 2 && ntiles > 0) stage(0, 0);
-  // the query rows are split into fp16 head + remainder while the first tile is in flight
-  for (int i = t; i < 16 * 64; i += 128) {
-    const int row = i >> 6, c = (i & 63) * 4;
-    float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < gqa) qv = *reinterpret_cast<const float4*>(a.q + ((size_t)r * P.Hq + g * gqa + row) * 512 + c);
-    const __half2 h0 = __floats2half2_rn(qv.x, qv.y), h1 = __floats2half2_rn(qv.z, qv.w);
-    const float2 b0 = __half22float2(h0), b1 = __half22float2(h1);
-    *reinterpret_cast<__half2*>(&sm.q[0][row][c]) = h0;
-    *reinterpret_cast<__half2*>(&sm.q[0][row][c + 2]) = h1;
-    *reinterpret_cast<__half2*>(&sm.q[1][row][c]) = __floats2half2_rn(qv.x - b0.x, qv.y - b0.y);
-    *reinterpret_cast<__half2*>(&sm.q[1][row][c + 2]) = __floats2half2_rn(qv.z - b1.x, qv.w - b1.y);
-  }
-  for (;;) {
-  for (int tile = 0; tile < ntiles; ++tile) {
-    const int buf = STAGES == 2 ? (tile & 1) : 0;
-    if (STAGES == 1) {
-      __syncthreads();                                    // every warp is done with the previous tile (and q is visible)
-      stage(tile, 0);
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();                                      // tile visible; every warp is done with the previous one
-    if (STAGES == 2 && tile + 1 < ntiles) stage(tile + 1, buf ^ 1);
-    // ---- S = Q K^T for positions 8w .. 8w+7
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int ks = 0; ks < 16; ks += 2) {                  // two k-steps of 16 channels per K fragment load
-      unsigned kb[4];
-      ldsm_x4(kb, &sm.k[buf][8 * w + (l & 7)][ks * 16 + (l >> 3) * 8]);
-#pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        unsigned ah[4], al[4];
-        ldsm_x4(ah, &sm.q[0][l & 15][(ks + kk) * 16 + (l >> 4) * 8]);
-        ldsm_x4(al, &sm.q[1][l & 15][(ks + kk) * 16 + (l >> 4) * 8]);
-        mma_f16(s, ah, kb[2 * kk], kb[2 * kk + 1]);
-        mma_f16(s, al, kb[2 * kk], kb[2 * kk + 1]);
-      }
-    }
-    const int pi = tile * kTile + 8 * w + cq;
-    const bool v0 = pi < cnt && sm.pos[pi] >= 0, v1 = pi + 1 < cnt && sm.pos[pi + 1] >= 0;
-    s[0] = v0 ? s[0] * 0.0625f : -INFINITY; s[1] = v1 ? s[1] * 0.0625f : -INFINITY;
-    s[2] = v0 ? s[2] * 0.0625f : -INFINITY; s[3] = v1 ? s[3] * 0.0625f : -INFINITY;
-    float mx0 = fmaxf(s[0], s[1]), mx1 = fmaxf(s[2], s[3]);
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    if ((l & 3) == 0) { sm.red[0][w][row0] = mx0; sm.red[0][w][row0 + 8] = mx1; }
-    __syncthreads();
-    float mn[2], corr[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int row = row0 + 8 * i;
-      const float tm = fmaxf(fmaxf(sm.red[0][0][row], sm.red[0][1][row]), fmaxf(sm.red[0][2][row], sm.red[0][3][row]));
-      mn[i] = fmaxf(m_run[i], tm);
-      corr[i] = m_run[i] > -INFINITY ? __expf(m_run[i] - mn[i]) : 0.f;   // nothing accumulated yet: factor irrelevant
-    }
-    float e[4];
-    e[0] = s[0] > -INFINITY ? __expf(s[0] - mn[0]) : 0.f; e[1] = s[1] > -INFINITY ? __expf(s[1] - mn[0]) : 0.f;
-    e[2] = s[2] > -INFINITY ? __expf(s[2] - mn[1]) : 0.f; e[3] = s[3] > -INFINITY ? __expf(s[3] - mn[1]) : 0.f;
-    float su0 = e[0] + e[1], su1 = e[2] + e[3];
-    su0 += __shfl_xor_sync(0xffffffffu, su0, 1); su1 += __shfl_xor_sync(0xffffffffu, su1, 1);
-    su0 += __shfl_xor_sync(0xffffffffu, su0, 2); su1 += __shfl_xor_sync(0xffffffffu, su1, 2);
-    if ((l & 3) == 0) { sm.red[1][w][row0] = su0; sm.red[1][w][row0 + 8] = su1; }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {                          // probabilities as fp16 head + remainder
-      const __half2 hi = __floats2half2_rn(e[2 * i], e[2 * i + 1]);
-      const float2 back = __half22float2(hi);
-      *reinterpret_cast<__half2*>(&sm.p[0][row0 + 8 * i][8 * w + cq]) = hi;
-      *reinterpret_cast<__half2*>(&sm.p[1][row0 + 8 * i][8 * w + cq]) = __floats2half2_rn(e[2 * i] - back.x, e[2 * i + 1] - back.y);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int row = row0 + 8 * i;
-      l_run[i] = l_run[i] * corr[i] + (sm.red[1][0][row] + sm.red[1][1][row]) + (sm.red[1][2][row] + sm.red[1][3][row]);
-      m_run[i] = mn[i];
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) { O[nt][0] *= corr[0]; O[nt][1] *= corr[0]; O[nt][2] *= corr[1]; O[nt][3] *= corr[1]; }
-    // ---- O += P V for channels 64w .. 64w+63
-#pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {                      // 16 positions per k-step
-      unsigned ph[4], pl[4];
-      ldsm_x4(ph, &sm.p[0][l & 15][kk * 16 + (l >> 4) * 8]);
-      ldsm_x4(pl, &sm.p[1][l & 15][kk * 16 + (l >> 4) * 8]);
-#pragma unroll
-      for (int nt = 0; nt < 8; nt += 2) {                 // two n-tiles of 8 channels per V fragment load
-        unsigned vb[4];
-        ldsm_x4_trans(vb, &sm.v[buf][kk * 16 + (l & 7) + ((l >> 3) & 1) * 8][64 * w + nt * 8 + (l >> 4) * 8]);
-        mma_f16(O[nt], ph, vb[0], vb[1]);
-        mma_f16(O[nt], pl, vb[0], vb[1]);
-        mma_f16(O[nt + 1], ph, vb[2], vb[3]);
-        mma_f16(O[nt + 1], pl, vb[2], vb[3]);
-      }
-    }
-  }
-    chunk0 += kMaxSplitPos;                               // a split longer than one chunk (few splits over a long list)
-    if (chunk0 >= total) break;
-    __syncthreads();                                      // every warp is done with the chunk's positions and tiles
-    list_chunk();
-    ntiles = (cnt + kTile - 1) / kTile;
-    if (STAGES == 2) stage(0, 0);
-  }
-  // partial records of this split: rows row0 and row0 + 8 are heads g * gqa + row
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int row = row0 + 8 * i;
-    if (row >= gqa) continue;
-    float* dst = partials + (((size_t)(P.base[blockIdx.z] + r) * P.Hq + g * gqa + row) * splits + split) * CR_QSA_PART;
-    if (w == 0 && (l & 3) == 0) { dst[0] = m_run[i]; dst[1] = l_run[i]; }
-    // records are 8-byte aligned (258 floats): store pairs
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-      *reinterpret_cast<float2*>(dst + 2 + 64 * w + nt * 8 + cq) = make_float2(O[nt][2 * i], O[nt][2 * i + 1]);
-  }
+__device__ __forceinline__ void split2(float x, float y, unsigned& hi, unsigned& lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 b = __half22float2(h);
+  const __half2 r = __floats2half2_rn(x - b.x, y - b.y);
+  hi = *reinterpret_cast<const unsigned*>(&h);
+  lo = *reinterpret_cast<const unsigned*>(&r);
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
-// grid (Hq, Rmax, spans), 256 threads: thread d = output channel.
-// Partial p of (row, head) is at partials[(part_major ? (p * rows_total + row) * Hq + h : (row * Hq + h) * nparts + p) * 258].
-__global__ void __launch_bounds__(256) qsa_merge_kernel(const __grid_constant__ QsaParams P, const float* partials, int nparts,
-                                                        int part_major, int rows_total, float* partial_out, int fmt) {
-  pdl_release();
-  pdl_wait();
-  const cr_qsa_args& a = P.span[blockIdx.z];
-  const int h = blockIdx.x, r = blockIdx.y, d = threadIdx.x;
-  if (r >= a.R || qsa_row_is_tiled(P, r)) return;
-  const int row = P.base[blockIdx.z] + r;
-  __shared__ float ob[256];
-  auto rec = [&](int p) -> const float* {
-    const size_t i = part_major ? ((size_t)p * rows_total + row) * P.Hq + h : ((size_t)row * P.Hq + h) * nparts + p;
-    return partials + i * CR_QSA_PART;
-  };
-  // (m, l) of the parts are combined by the first warp; every thread then sums its channel with the factors
-  // from shared memory, so the loads of the second pass are independent of each other.
-  __shared__ float fs[32];
-  __shared__ float ml[2];
-  if (d < 32) {
-    float pm = -INFINITY, pl = 0.f;
-    if (d < nparts) {
-      const float2 v = *reinterpret_cast<const float2*>(rec(d));
-      pl = v.y;
-      pm = pl != 0.f ? v.x : -INFINITY;
-    }
-    const float mx = warp_max(pm);
-    const float f = pl != 0.f ? __expf(pm - mx) : 0.f;
-    const float lt = warp_sum(pl * f);
-    fs[d] = f;
-    if (d == 0) { ml[0] = mx; ml[1] = lt; }
-  }
-  __syncthreads();
-  const float m = ml[0], lsum = ml[1];
-  float o = 0.f;
-  if (nparts == 32) {   // the decode case: all 32 loads in flight at once
-    float v[32];
-#pragma unroll
-    for (int p = 0; p < 32; ++p) v[p] = __ldcg(rec(p) + 2 + d);
-#pragma unroll
-    for (int p = 0; p < 32; ++p) o = fmaf(v[p], fs[p], o);
+// Channels c .. c + 3 (c = 128 half + 4 lane, a warp holds a 128-channel group) of one head of one row: un-gated context,
+// gate, output format.
+__device__ __forceinline__ void emit_group(const cr_qsa_args& a, int Hq, int r, int h, int c, float4 o, const float4 gate, int fmt) {
+  const size_t W = (size_t)Hq * 256, at = (size_t)r * W + h * 256 + c;
+  if (a.context) { float* cx = a.context + at; cx[0] = o.x; cx[1] = o.y; cx[2] = o.z; cx[3] = o.w; }
+  float v[4] = {o.x * sigmoidf_(gate.x), o.y * sigmoidf_(gate.y), o.z * sigmoidf_(gate.z), o.w * sigmoidf_(gate.w)};
+  if (fmt == CR_OUT_RAW_F32) {
+    float* dst = reinterpret_cast<float*>(a.out) + at;
+    if (((uintptr_t)dst & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else { dst[0] = v[0]; dst[1] = v[1]; dst[2] = v[2]; dst[3] = v[3]; }
+  } else if (fmt == CR_OUT_RAW_BF16) {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + at;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+    if (((uintptr_t)dst & 7) == 0) *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    else { dst[0] = lo.x; dst[1] = lo.y; dst[2] = hi.x; dst[3] = hi.y; }
   } else {
-#pragma unroll 8
-    for (int p = 0; p < nparts; ++p) o = fmaf(rec(p)[2 + d], fs[p], o);
-  }
-  if (partial_out) {      // shard mode: one merged partial per (row, head)
-    float* dst = partial_out + ((size_t)row * P.Hq + h) * CR_QSA_PART;
-    if (d == 0) { dst[0] = m; dst[1] = lsum; }
-    dst[2 + d] = o;
-    return;
-  }
-  o /= lsum;
-  const size_t W = (size_t)P.Hq * 256;
-  if (a.context) a.context[((size_t)r * P.Hq + h) * 256 + d] = o;
-  o *= sigmoidf_(a.q[((size_t)r * P.Hq + h) * 512 + 256 + d]);
-  if (fmt == CR_OUT_RAW_F32) { reinterpret_cast<float*>(a.out)[(size_t)r * W + h * 256 + d] = o; return; }
-  if (fmt == CR_OUT_RAW_BF16) { reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)r * W + h * 256 + d] = __float2bfloat16(o); return; }
-  ob[d] = round_h(round_h(o) * __half2float(reinterpret_cast<const __half*>(a.suh_o)[h * 256 + d]));
-  __syncthreads();
-  if (d < 64) {
-    const int half = d >> 5, lane = d & 31;
-    float v[4];
+    const __half* suh = reinterpret_cast<const __half*>(a.suh_o) + h * 256 + c;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = ob[half * 128 + lane * 4 + i];
+    for (int i = 0; i < 4; ++i) v[i] = round_h(round_h(v[i]) * __half2float(suh[i]));
     wht128(v);
     __half* dst = reinterpret_cast<__half*>(a.out);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      dst[out_index(r, h * 256 + half * 128 + lane * 4 + i, (int)W, a.pack_rows, a.pack_off)] = __float2half(v[i] * kHadNorm);
+    for (int i = 0; i < 4; ++i) dst[out_index(r, h * 256 + c + i, (int)W, a.pack_rows, a.pack_off)] = __float2half(v[i] * kHadNorm);
   }
 }
 
-cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int splits,
-                          int p0, int p1, cudaStream_t stream, const QsaTileSplit* tiles) {
+// grid (cluster x ceil(Rmax * Hkv / units per CTA), 1, spans).
+template <int NG>
+__global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __grid_constant__ QsaParams P, const AttnShape shape, float* partials,
+                                                                       int p0, int p1, int fmt) {
+  extern __shared__ __align__(128) unsigned char ring_raw[];
+  __shared__ float ml_s[kMaxWarps][8][2];              // (m, l) of every stream's heads
+  __shared__ float cta_ml[16][2];                      // of the CTA's merged unit, read by the cluster
+  pdl_release();
+  pdl_wait();
+  constexpr int W = kStreams<NG>;
+  const cr_qsa_args& a = P.span[blockIdx.z];
+  const int t = threadIdx.x, warp = t >> 5, l = t & 31, g8 = l >> 2, tq = l & 3;
+  const int stream = warp / NG, hg = warp % NG;
+  const int upc = W / shape.spu, crank = shape.cluster > 1 ? (int)(blockIdx.x % shape.cluster) : 0;
+  const int unit = (int)(blockIdx.x / shape.cluster) * upc + stream / shape.spu, sub = stream % shape.spu;
+  const int r = unit / P.Hkv, g = unit % P.Hkv;
+  const int gqa = P.Hq / P.Hkv, gh = (gqa + NG - 1) / NG;           // heads of a head group
+  const int heads = min(gh, gqa - hg * gh);
+  // Units past the rows, and rows of the tiled kernel: with one unit per CTA or cluster everybody leaves, else the stream idles
+  // through the CTA's barriers.
+  const bool live = r < a.R && !qsa_row_is_tiled(P, r);
+  if (upc == 1 && !live) return;
+
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  float O[16][4];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) O[i][0] = O[i][1] = O[i][2] = O[i][3] = 0.f;
+  unsigned char* ring = ring_raw + (size_t)stream * kRingBytes;
+
+  if (live) {
+    const int p = a.pos0 + r, ns = a.nsel[r], nb = (p + 1) / 4;
+    const int* sel = a.sel + (size_t)r * CR_SEL_BLOCKS;
+    // Entries: the selected blocks (all complete blocks when dense), then the open block.  They ascend, so those that reach
+    // into a rank's window [p0, p1) are one contiguous range.
+    const int full = ns < 0 ? nb : ns;
+    int e_lo = 0, e_hi = full + ((p + 1) % 4 != 0 ? 1 : 0);
+    if (p0 > 0 || p1 <= p) {
+      auto entry_at_least = [&](int blk) {               // first entry whose block is >= blk
+        if (ns < 0) return min(blk, e_hi);
+        int lo = 0, hi = full;
+        while (lo < hi) { const int mid = (lo + hi) >> 1; if (sel[mid] < blk) lo = mid + 1; else hi = mid; }
+        return lo == full && nb < blk ? e_hi : lo;
+      };
+      const int lo = entry_at_least(p0 / 4), hi = p1 > p ? e_hi : entry_at_least((p1 + 3) / 4);
+      e_lo = lo; e_hi = min(hi, e_hi);
+    }
+    const int tiles_all = max(e_hi - e_lo + 3, 0) / 4, streams = shape.spu * shape.cluster, s_idx = crank * shape.spu + sub;
+    const int tb = tiles_all / streams, trem = tiles_all % streams;
+    const int tile0 = s_idx * tb + min(s_idx, trem), tiles = tb + (s_idx < trem ? 1 : 0);
+    const int e0 = e_lo + 4 * tile0;                     // first entry of this stream
+
+    // Block ids: lane l of `ids` holds entry e0 + 32 k + l of the current group of eight tiles, `ids_next` the next group.
+    auto load_ids = [&](int k) {
+      const int e = e0 + 32 * k + l;
+      return e < e_hi ? (ns < 0 || e >= full ? (e >= full ? nb : e) : sel[e]) : -1;
+    };
+    int ids = load_ids(0), ids_next = load_ids(1);
+    const size_t row_bytes = (size_t)P.Hkv * 512;
+    const char* kc = reinterpret_cast<const char*>(a.c.k) + (size_t)g * 512 + l * 16;
+    const char* vc = reinterpret_cast<const char*>(a.c.v) + (size_t)g * 512 + l * 16;
+    const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
+    const int lo_pos = max(p0, 0), hi_pos = min(p, p1 - 1);          // visible positions
+    int blk[4];                                          // blocks of the tile whose K half was issued last
+    auto issue = [&](const char* base, int half) {       // the 16 rows of the tile in blk, into slot half % kSlots
+      const unsigned slot = ring_s + (half % kSlots) * kHalfBytes;
+#pragma unroll
+      for (int i = 0; i < kTok / NG; ++i) {
+        const int k = hg * (kTok / NG) + i;
+        const int b = NG == 1 ? blk[i >> 2] : (hg == 0 ? blk[i >> 2] : blk[2 + (i >> 2)]);
+        const int pos = 4 * b + (k & 3);
+        const bool ok = b >= 0 && pos >= lo_pos && pos <= hi_pos;
+        attn_cp16(slot + k * 512 + ((l ^ (k & 7)) << 4), base + (ok ? (size_t)pos * row_bytes : 0), ok);
+      }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+    auto visible = [&]() {                               // bit k: position k of the tile in blk is attended
+      const int b = l < kTok ? (l < 8 ? (l < 4 ? blk[0] : blk[1]) : (l < 12 ? blk[2] : blk[3])) : -1;
+      const int pos = 4 * b + (l & 3);
+      return __ballot_sync(0xffffffffu, b >= 0 && pos >= lo_pos && pos <= hi_pos);
+    };
+    auto take_blocks = [&](int tile) {                   // tile's four block ids (called for tile = 0, 1, 2, ...)
+      if ((tile & 7) == 0 && tile > 0) { ids = ids_next; ids_next = load_ids((tile >> 3) + 1); }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) blk[j] = __shfl_sync(0xffffffffu, ids, 4 * (tile & 7) + j);
+    };
+    auto pair_sync = [&] {                               // the warps of a stream
+      if constexpr (NG == 1) __syncwarp();
+      else asm volatile("bar.sync %0, 64;\n" ::"r"(1 + stream) : "memory");
+    };
+    unsigned see = 0, see_next = 0;
+    if (tiles > 0) { take_blocks(0); see = visible(); issue(kc, 0); }
+    commit();
+    if (tiles > 0) issue(vc, 1);
+    commit();
+    if (tiles > 1) { take_blocks(1); see_next = visible(); issue(kc, 2); }
+    commit();
+    // Query heads of the group as column fragments, fp16 head and remainder, while the first halves are in flight.
+    unsigned qh[16][2], ql[16][2];
+    {
+      const float* q = a.q + ((size_t)r * P.Hq + g * gqa + hg * gh + min(g8, heads - 1)) * 512 + 2 * tq;
+      const bool have = g8 < heads;
+#pragma unroll
+      for (int ks = 0; ks < 16; ++ks)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float2 v = *reinterpret_cast<const float2*>(q + 16 * ks + 8 * j);
+          if (!have) v = make_float2(0.f, 0.f);
+          split2(v.x, v.y, qh[ks][j], ql[ks][j]);
+        }
+    }
+    constexpr float kScale = 0.0625f * 1.4426950408889634f;           // logits / 16, in powers of two
+    // this lane's ldmatrix rows: K: matrices (positions 0-7 | 8-15) x (first | second 8 channels); V: the transpose of that
+    const int mi = l >> 3, k_row = (l & 7) + (mi & 1) * 8, v_row = (l & 7) + (mi >> 1) * 8;
+    const unsigned k_addr = k_row * 512, v_addr = v_row * 512;
+    for (int i = 0; i < tiles; ++i) {
+      asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+      pair_sync();
+      const unsigned ks_base = ring_s + ((2 * i) % kSlots) * kHalfBytes + k_addr;
+      float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int ks = 0; ks < 16; ++ks) {
+        unsigned ka[4];
+        ldsm_x4(ka, ks_base + (((2 * ks + (mi >> 1)) ^ (l & 7)) << 4));
+        mma_f16(s, ka, qh[ks][0], qh[ks][1]);
+        mma_f16(s2, ka, ql[ks][0], ql[ks][1]);
+      }
+      pair_sync();                                       // the K half is free
+      if (i + 1 < tiles) issue(vc, 2 * i + 3);           // blk still holds tile i + 1
+      commit();
+      const bool v0 = (see >> g8) & 1u, v1 = (see >> (g8 + 8)) & 1u;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[j] = (j < 2 ? v0 : v1) ? (s[j] + s2[j]) * kScale : -INFINITY;
+      float mx[2] = {fmaxf(s[0], s[2]), fmaxf(s[1], s[3])};
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], o));
+        mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], o));
+      }
+      if (__any_sync(0xffffffffu, mx[0] > m_run[0] || mx[1] > m_run[1])) {
+        float corr[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float mn = fmaxf(m_run[j], mx[j]);
+          corr[j] = m_run[j] > -INFINITY ? ex2(m_run[j] - mn) : 0.f;
+          l_run[j] *= corr[j];
+          m_run[j] = mn;
+        }
+#pragma unroll
+        for (int mt = 0; mt < 16; ++mt) { O[mt][0] *= corr[0]; O[mt][1] *= corr[1]; O[mt][2] *= corr[0]; O[mt][3] *= corr[1]; }
+      }
+      float e[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) e[j] = s[j] > -INFINITY ? ex2(s[j] - m_run[j & 1]) : 0.f;
+      l_run[0] += e[0] + e[2];
+      l_run[1] += e[1] + e[3];
+      unsigned ph[2], pl[2];
+      split2(e[0], e[1], ph[0], pl[0]);
+      split2(e[2], e[3], ph[1], pl[1]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) { ph[j] = transpose8(ph[j]); pl[j] = transpose8(pl[j]); }
+      asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+      pair_sync();
+      const unsigned vs_base = ring_s + ((2 * i + 1) % kSlots) * kHalfBytes + v_addr;
+#pragma unroll
+      for (int mt = 0; mt < 16; ++mt) {
+        unsigned va[4];
+        ldsm_x4_trans(va, vs_base + (((2 * mt + (mi & 1)) ^ (l & 7)) << 4));
+        mma_f16(O[mt], va, ph[0], ph[1]);
+        mma_f16(O[mt], va, pl[0], pl[1]);
+      }
+      pair_sync();                                       // the V half is free
+      see = see_next;
+      if (i + 2 < tiles) { take_blocks(i + 2); see_next = visible(); issue(kc, 2 * i + 4); }
+      commit();
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      l_run[0] += __shfl_xor_sync(0xffffffffu, l_run[0], o);
+      l_run[1] += __shfl_xor_sync(0xffffffffu, l_run[1], o);
+    }
+  }
+
+  // ---- merge: every stream leaves its accumulator as [head][channel] in its ring, (m, l) beside it
+  float* acc = reinterpret_cast<float*>(ring) + (size_t)hg * 8 * kAccLd;
+  if (NG == 2) asm volatile("bar.sync %0, 64;\n" ::"r"(1 + stream) : "memory");   // the other warp of the stream has left the ring
+  else __syncwarp();
+#pragma unroll
+  for (int mt = 0; mt < 16; ++mt) {
+    float* d = acc + 2 * tq * kAccLd + 16 * mt + g8;
+    d[0] = O[mt][0]; d[kAccLd] = O[mt][1]; d[8] = O[mt][2]; d[kAccLd + 8] = O[mt][3];
+  }
+  if (g8 == 0) {
+    ml_s[warp][2 * tq][0] = m_run[0]; ml_s[warp][2 * tq][1] = l_run[0];
+    ml_s[warp][2 * tq + 1][0] = m_run[1]; ml_s[warp][2 * tq + 1][1] = l_run[1];
+  }
+  if (shape.spu == 1) {
+    if (NG == 1) __syncwarp();
+    else asm volatile("bar.sync %0, 64;\n" ::"r"(1 + stream) : "memory");
+  } else {
+    __syncthreads();
+  }
+  if (shape.cluster == 1 && !live) return;
+  // This CTA's merged (m, l, acc) of head hd, channels c .. c + 3.
+  const int first_stream = stream - sub;
+  auto merged = [&](int hd, int c, float& m, float& lsum) {
+    const int hg_ = hd / gh, hl = hd % gh;
+    m = -INFINITY;
+    for (int s = 0; s < shape.spu; ++s) m = fmaxf(m, ml_s[(first_stream + s) * NG + hg_][hl][0]);
+    lsum = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < shape.spu; ++s) {
+      const float ms = ml_s[(first_stream + s) * NG + hg_][hl][0], f = ms > -INFINITY ? ex2(ms - m) : 0.f;
+      lsum = fmaf(ml_s[(first_stream + s) * NG + hg_][hl][1], f, lsum);
+      const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(ring_raw + (size_t)(first_stream + s) * kRingBytes) + (size_t)(hg_ * 8 + hl) * kAccLd + c);
+      o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+    }
+    return o;
+  };
+  auto finish = [&](int hd, int c, float m, float lsum, float4 o) {
+    const int h = g * gqa + hd;
+    if (partials) {                                      // a rank's partial: (m, l, acc) with m as a natural logarithm
+      float* dst = partials + ((size_t)(P.base[blockIdx.z] + r) * P.Hq + h) * CR_QSA_PART;
+      if (c == 0) { dst[0] = m * 0.6931471805599453f; dst[1] = lsum; }
+      *reinterpret_cast<float2*>(dst + 2 + c) = make_float2(o.x, o.y);
+      *reinterpret_cast<float2*>(dst + 4 + c) = make_float2(o.z, o.w);
+      return;
+    }
+    const float4 gate = *reinterpret_cast<const float4*>(a.q + ((size_t)r * P.Hq + h) * 512 + 256 + c);
+    const float inv = 1.f / lsum;
+    emit_group(a, P.Hq, r, h, c, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv), gate, fmt);
+  };
+  const int uw = sub * NG + hg, uwarps = shape.spu * NG;               // this warp among the warps of its unit in this CTA
+  if (shape.cluster == 1) {
+    for (int gi = uw; gi < 2 * gqa; gi += uwarps) {                     // groups: (head, 128 channels)
+      float m, lsum;
+      const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
+      const float4 o = merged(hd, c, m, lsum);
+      finish(hd, c, m, lsum, o);
+    }
+    return;
+  }
+  // cluster: the CTA's merged unit goes to shared memory behind the ring images of the first stream, then every CTA takes a
+  // share of the groups over all CTAs
+  cg::cluster_group cluster = cg::this_cluster();
+  float* mine = reinterpret_cast<float*>(ring_raw + (size_t)W * kRingBytes);
+  for (int gi = warp; gi < 2 * gqa; gi += W * NG) {
+    float m, lsum;
+    const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
+    const float4 o = merged(hd, c, m, lsum);
+    *reinterpret_cast<float4*>(mine + hd * 256 + c) = o;
+    if (c == 0) { cta_ml[hd][0] = m; cta_ml[hd][1] = lsum; }
+  }
+  cluster.sync();
+  for (int gi = crank + shape.cluster * warp; gi < 2 * gqa; gi += shape.cluster * W * NG) {
+    const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
+    float ms[8], m = -INFINITY, lsum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      ms[k] = k < shape.cluster ? cluster.map_shared_rank(&cta_ml[0][0], k)[2 * hd] : -INFINITY;
+      m = fmaxf(m, ms[k]);
+    }
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k >= shape.cluster) break;
+      const float f = ms[k] > -INFINITY ? ex2(ms[k] - m) : 0.f;
+      lsum = fmaf(cluster.map_shared_rank(&cta_ml[0][0], k)[2 * hd + 1], f, lsum);
+      const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(mine, k) + hd * 256 + c);
+      o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+    }
+    finish(hd, c, m, lsum, o);
+  }
+  cluster.sync();                                        // the images stay until every CTA has read them
+}
+
+// Merge of the partial records of several ranks (QsaMergeKernel, engine/layers/qsa_long.h:458-499), gate and output
+// transform.  grid (Hq, R), 64 threads: a warp per 128-channel group.  Record p of (row, head) lies at
+// partials[((p * rows + row) * Hq + h) * 258].
+__global__ void __launch_bounds__(64) qsa_merge_kernel(const __grid_constant__ QsaParams P, const float* partials, int nparts, int fmt) {
+  pdl_release();
+  pdl_wait();
+  const cr_qsa_args& a = P.span[0];
+  const int h = blockIdx.x, r = blockIdx.y, l = threadIdx.x & 31, c = (threadIdx.x >> 5) * 128 + 4 * l;
+  auto rec = [&](int p) { return partials + (((size_t)p * a.R + r) * P.Hq + h) * CR_QSA_PART; };
+  float pm = -INFINITY, pl = 0.f;                        // lane p: (m, l) of record p
+  if (l < nparts) {
+    const float2 v = *reinterpret_cast<const float2*>(rec(l));
+    pl = v.y;
+    pm = pl != 0.f ? v.x : -INFINITY;
+  }
+  const float mx = warp_max(pm);
+  const float f = pl != 0.f ? __expf(pm - mx) : 0.f;
+  const float lsum = warp_sum(pl * f);
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int p = 0; p < nparts; ++p) {
+    const float fp = __shfl_sync(0xffffffffu, f, p);
+    const float2 x = *reinterpret_cast<const float2*>(rec(p) + 2 + c), y = *reinterpret_cast<const float2*>(rec(p) + 4 + c);
+    o.x = fmaf(x.x, fp, o.x); o.y = fmaf(x.y, fp, o.y); o.z = fmaf(y.x, fp, o.z); o.w = fmaf(y.y, fp, o.w);
+  }
+  const float4 gate = *reinterpret_cast<const float4*>(a.q + ((size_t)r * P.Hq + h) * 512 + 256 + c);
+  const float inv = 1.f / lsum;
+  emit_group(a, P.Hq, r, h, c, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv), gate, fmt);
+}
+
+// Streams of a unit.  The pass holds SMs x kStreams streams at a time; with s streams per unit it takes
+// ceil(units x s / that) waves of (longest unit's tiles / s + the set-up and merge of a stream, worth about four tiles).
+// One stream per unit is the cheapest form but leaves SMs idle when units are few and ends in a ragged wave when they
+// are not many; a cluster (s above one CTA's streams) pays only while SMs would idle otherwise.
+static AttnShape attn_shape(int streams, long long units, int tiles, int sms) {
+  AttnShape best{1, 1};
+  double best_cost = 1e30;
+  for (int spu = 1; spu <= streams; ++spu) {
+    if (streams % spu) continue;
+    for (int cl = 1; cl <= 8; cl <<= 1) {
+      if (cl > 1 && (spu != streams || units * cl > sms)) break;
+      if (spu * cl > 1 && spu * cl > tiles) break;
+      const long long ctas = cl > 1 ? units * cl : (units * spu + streams - 1) / streams;
+      const long long waves = (ctas + sms - 1) / sms;
+      const double cost = (double)waves * ((tiles + spu * cl - 1) / (spu * cl) + 4);
+      if (cost < best_cost - 1e-9) { best_cost = cost; best = AttnShape{spu, cl}; }
+    }
+  }
+  return best;
+}
+
+template <int NG>
+static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long units, int tiles, float* partials, int p0, int p1, int fmt, cudaStream_t stream) {
+  static PerDeviceOnce configured;
+  constexpr size_t smem = kAttnSmem<NG> + 12 * 256 * sizeof(float);   // + the merged unit of a cluster's CTA
+  if (cr_status st = once_per_device(configured, [] {
+        CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return CR_OK;
+      })) return st;
+  const AttnShape shape = attn_shape(kStreams<NG>, units, tiles, sm_count());
+  const int upc = kStreams<NG> / shape.spu;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(shape.cluster * ((Rmax * P.Hkv + upc - 1) / upc), 1, n);
+  cfg.blockDim = dim3(kAttnThreads<NG>);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (pdl_enabled()) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na++].val.programmaticStreamSerializationAllowed = 1; }
+  if (shape.cluster > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = shape.cluster; attr[na].val.clusterDim.y = 1; attr[na++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr; cfg.numAttrs = na;
+  CR_CUDA(cudaLaunchKernelEx(&cfg, qsa_attn_kernel<NG>, P, shape, partials, p0, p1, fmt));
+  CR_LAUNCH_CHECK("qsa_attn_kernel");
+  return CR_OK;
+}
+
+cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int p0, int p1, cr_out_format fmt,
+                          cudaStream_t stream, const QsaTileSplit* tiles) {
   use_stream(stream);
-  CR_REQUIRE(splits >= 1 && splits <= 32, "qsa attention: %d KV splits unsupported (1..32)", splits);
   int row_base = 0;
   for (int s0 = 0; s0 < n_spans; s0 += kMaxSpans) {
     const int n = n_spans - s0 < kMaxSpans ? n_spans - s0 : kMaxSpans;
     QsaParams P;
     qsa_fill_params(P, g, spans + s0, n);
-    for (int s = 0; s < n; ++s) P.base[s] += row_base;
     if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; }
-    const int Rmax = qsa_max_rows(spans + s0, n);
-    static PerDeviceOnce configured;
-    if (cr_status st = once_per_device(configured, [] {
-          CR_CUDA(cudaFuncSetAttribute(qsa_attn_split_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem<1>)));
-          CR_CUDA(cudaFuncSetAttribute(qsa_attn_split_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem<2>)));
-          return CR_OK;
-        })) return st;
-    const dim3 grid(splits, Rmax * g->kv_heads, n);
-    if ((long long)grid.x * grid.y * grid.z > 600)          // more than two waves of the two-stage kernel (2 CTAs per SM)
-      CR_CUDA(launch_pdl(qsa_attn_split_kernel<1>, dim3(grid.y, grid.x, grid.z), dim3(128), sizeof(SplitSmem<1>), stream, P, partials, splits, p0, p1));
-    else
-      CR_CUDA(launch_pdl(qsa_attn_split_kernel<2>, grid, dim3(128), sizeof(SplitSmem<2>), stream, P, partials, splits, p0, p1));
-    CR_LAUNCH_CHECK("qsa_attn_split_kernel");
-    for (int s = 0; s < n; ++s) row_base += spans[s0 + s].R;
-  }
-  return CR_OK;
-}
-
-cr_status qsa_merge_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, const float* partials, int nparts,
-                           bool part_major, float* partial_out, cr_out_format fmt, cudaStream_t stream, const QsaTileSplit* tiles) {
-  use_stream(stream);
-  CR_REQUIRE(nparts >= 1 && nparts <= 32, "qsa merge: %d partial records per (row, head) unsupported (1..32)", nparts);
-  int rows_total = 0, row_base = 0;
-  for (int s = 0; s < n_spans; ++s) rows_total += spans[s].R;
-  for (int s0 = 0; s0 < n_spans; s0 += kMaxSpans) {
-    const int n = n_spans - s0 < kMaxSpans ? n_spans - s0 : kMaxSpans;
-    QsaParams P;
-    qsa_fill_params(P, g, spans + s0, n);
-    for (int s = 0; s < n; ++s) P.base[s] += row_base;
-    if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; }
-    const int Rmax = qsa_max_rows(spans + s0, n);
-    CR_CUDA(launch_pdl(qsa_merge_kernel, dim3(g->q_heads, Rmax, n), dim3(256), 0, stream, P, partials, nparts, part_major ? 1 : 0, rows_total, partial_out, (int)fmt));
-    CR_LAUNCH_CHECK("qsa_merge_kernel");
+    long long units = 0;
+    int last = 0;                                        // newest position of any row
+    for (int s = 0; s < n; ++s) {
+      P.base[s] += row_base;
+      units += (long long)spans[s0 + s].R * g->kv_heads;
+      last = max(last, spans[s0 + s].pos0 + spans[s0 + s].R - 1);
+    }
+    const int most = (min(last / 4 + 1, CR_SEL_BLOCKS + 1) + 3) / 4, Rmax = qsa_max_rows(spans + s0, n);
+    const cr_status st = g->q_heads / g->kv_heads <= 8 ? attn_launch_t<1>(P, Rmax, n, units, most, partials, p0, p1, (int)fmt, stream)
+                                                       : attn_launch_t<2>(P, Rmax, n, units, most, partials, p0, p1, (int)fmt, stream);
+    if (st) return st;
     for (int s = 0; s < n; ++s) row_base += spans[s0 + s].R;
   }
   return CR_OK;
@@ -385,17 +503,6 @@ static size_t total_rows(const cr_qsa_args* spans, int n) {
 
 }  // namespace cr
 
-// KV splits per (row, KV head) of a decode / verify pass: 32 for a few rows (latency: many short CTAs), fewer when the
-// pass holds many rows, so that the grid stays near two waves of CTAs and the per-CTA work (query staging, a partial
-// record per head) is shared by more positions.  A power of two between 4 and 32.
-constexpr long long kStepCtas = 1200;   // 600 and 2,400 measured 20 % and 6 % slower on 72 rows
-static int step_splits(const cr_geometry* g, const cr_qsa_args* spans, int n_spans) {
-  const long long units = (long long)cr::total_rows(spans, n_spans) * g->kv_heads;
-  int splits = CR_QSA_SPLITS;
-  while (splits > 4 && units * splits > kStepCtas) splits >>= 1;
-  return splits;
-}
-
 extern "C" size_t cr_qsa_scratch_bytes(const cr_geometry* g, int rows) {
   if (!g || rows < 1) return 0;
   return (size_t)rows * g->q_heads * CR_QSA_SPLITS * CR_QSA_PART * sizeof(float);
@@ -408,9 +515,7 @@ extern "C" cr_status cr_qsa_attn(const cr_geometry* g, const cr_qsa_args* spans,
   if (cr_status s = check_out(spans, n_spans, fmt, "cr_qsa_attn")) return s;
   const size_t need = cr_qsa_scratch_bytes(g, (int)total_rows(spans, n_spans));
   CR_REQUIRE(scratch && scratch_bytes >= need, "cr_qsa_attn: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
-  const int splits = step_splits(g, spans, n_spans);
-  if (cr_status s = qsa_attn_launch(g, spans, n_spans, (float*)scratch, splits, 0, INT_MAX, (cudaStream_t)stream)) return s;
-  return qsa_merge_launch(g, spans, n_spans, (const float*)scratch, splits, false, nullptr, fmt, (cudaStream_t)stream);
+  return qsa_attn_launch(g, spans, n_spans, nullptr, 0, INT_MAX, fmt, (cudaStream_t)stream);
 }
 
 extern "C" cr_status cr_qsa_step(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void* scratch, size_t scratch_bytes,
@@ -423,9 +528,7 @@ extern "C" cr_status cr_qsa_step(const cr_geometry* g, const cr_qsa_args* spans,
   cudaStream_t st = (cudaStream_t)stream;
   if (cr_status s = qsa_prep_launch(g, spans, n_spans, 0, nullptr, 0, st)) return s;
   if (cr_status s = qsa_select_launch(g, spans, n_spans, st)) return s;
-  const int splits = step_splits(g, spans, n_spans);
-  if (cr_status s = qsa_attn_launch(g, spans, n_spans, (float*)scratch, splits, 0, INT_MAX, st)) return s;
-  return qsa_merge_launch(g, spans, n_spans, (const float*)scratch, splits, false, nullptr, fmt, st);
+  return qsa_attn_launch(g, spans, n_spans, nullptr, 0, INT_MAX, fmt, st);
 }
 
 extern "C" cr_status cr_qsa_shard_attn(const cr_geometry* g, const cr_qsa_args* a, int p0, int p1, float* partials, void* scratch,
@@ -440,8 +543,7 @@ extern "C" cr_status cr_qsa_shard_attn(const cr_geometry* g, const cr_qsa_args* 
   const int splits = a->R <= CR_MAX_STEP_ROWS ? CR_QSA_SPLITS : (part_splits < 1 ? 1 : part_splits > 4 ? 4 : part_splits);
   const size_t need = (size_t)a->R * g->q_heads * splits * CR_QSA_PART * sizeof(float);
   CR_REQUIRE(scratch && scratch_bytes >= need, "cr_qsa_shard_attn: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
-  if (cr_status s = qsa_attn_launch(g, a, 1, (float*)scratch, splits, p0, p1, (cudaStream_t)stream)) return s;
-  return qsa_merge_launch(g, a, 1, (const float*)scratch, splits, false, partials, CR_OUT_RAW_F32, (cudaStream_t)stream);
+  return qsa_attn_launch(g, a, 1, partials, p0, p1, CR_OUT_RAW_F32, (cudaStream_t)stream);
 }
 
 extern "C" cr_status cr_qsa_merge_partials(const cr_geometry* g, const cr_qsa_args* a, int ranks, const float* partials,
@@ -450,5 +552,10 @@ extern "C" cr_status cr_qsa_merge_partials(const cr_geometry* g, const cr_qsa_ar
   if (cr_status s = qsa_validate(g, a, 1, CR_MAX_PREFILL_ROWS, "cr_qsa_merge_partials", 0)) return s;
   if (cr_status s = check_out(a, 1, fmt, "cr_qsa_merge_partials")) return s;
   CR_REQUIRE(partials && ranks >= 1 && ranks <= 32, "cr_qsa_merge_partials: need gathered partials of 1..32 ranks");
-  return qsa_merge_launch(g, a, 1, partials, ranks, true, nullptr, fmt, (cudaStream_t)stream);
+  QsaParams P;
+  qsa_fill_params(P, g, a, 1);
+  use_stream((cudaStream_t)stream);
+  CR_CUDA(launch_pdl(qsa_merge_kernel, dim3(g->q_heads, a->R), dim3(64), 0, (cudaStream_t)stream, P, partials, ranks, (int)fmt));
+  CR_LAUNCH_CHECK("qsa_merge_kernel");
+  return CR_OK;
 }

@@ -2,8 +2,8 @@
 // selection, attention with the fused gate.  Entry point of a part, in the role of LaunchQsaPrefillUnion /
 // LaunchQsaPrefill (engine/layers/kernels/prefill_qsa_union.h:782-807; prefill_qsa.h:274-299).
 // Attention runs over row tiles on tcgen05 tensor cores (qsa_flash.cu: union lists + masked flash attention); the
-// row-wise split-KV kernel of the decode path (qsa_attn.cu, 4 splits per row) remains as the alternative that
-// cr_options.qsa_union_rows = -1 selects.  Rows of a part are independent once the cache and the pool hold the
+// row-wise kernel of the decode path (qsa_attn.cu) serves the tiles whose rows share little, and every row with
+// cr_options.qsa_union_rows = -1.  Rows of a part are independent once the cache and the pool hold the
 // part, so causality inside the part falls out of pos0 + r.
 #include <climits>
 #include "qsa.cuh"
@@ -67,11 +67,9 @@ static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, c
                                        gated, fmt, tiles.max, stream)) return s;
     if (tiles.max == INT_MAX) return CR_OK;
     // the tiles with little sharing: row-wise split-KV attention (its CTAs of tiled rows exit at once)
-    if (cr_status s = qsa_attn_launch(g, &q, 1, (float*)scratch, kPrefillSplits, 0, INT_MAX, stream, &tiles)) return s;
-    return qsa_merge_launch(g, &q, 1, (const float*)scratch, kPrefillSplits, false, nullptr, fmt, stream, &tiles);
+    return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream, &tiles);
   }
-  if (cr_status s = qsa_attn_launch(g, &q, 1, (float*)scratch, kPrefillSplits, 0, INT_MAX, stream)) return s;
-  return qsa_merge_launch(g, &q, 1, (const float*)scratch, kPrefillSplits, false, nullptr, fmt, stream);
+  return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream);
 }
 }  // namespace cr
 

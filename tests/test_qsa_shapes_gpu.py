@@ -1,0 +1,101 @@
+"""QSA kernels at the sizes where their work split changes: stream counts, clusters and head groups of the attention,
+bitmap windows of the union lists.  References: plain torch in float64 / a dictionary merge."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _weights(Hq):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, Hq, 2, 4, 2)
+    one = [torch.ones(n) for n in (256, 256, 128, 128)]
+    return capi, layers, g, layers.QsaWeights(g, *one)
+
+
+def _selection(gen, pos):
+    """(sel, nsel) of the row at position pos: 512 of its complete blocks, or dense."""
+    nb = (pos + 1) // 4
+    if nb <= 512:
+        return torch.zeros(512, dtype=torch.int32, device="cuda"), -1
+    return torch.randperm(nb, generator=gen, device="cuda")[:512].sort().values.int(), 512
+
+
+def _attend(q, k, v, sel, nsel, pos):
+    """Gated attention of one row, float64: q [Hq, 512], k / v fp16 [ctx, 2, 256]."""
+    nb = (pos + 1) // 4
+    if nsel < 0:
+        at = torch.arange(pos + 1, device="cuda")
+    else:
+        at = torch.cat([(sel.long()[:, None] * 4 + torch.arange(4, device="cuda")).reshape(-1), torch.arange(4 * nb, pos + 1, device="cuda")])
+    gqa = q.shape[0] // 2
+    out = []
+    for g in range(2):
+        Q = q[g * gqa:(g + 1) * gqa].double()
+        p = torch.softmax(Q[:, :256] @ k[at, g].double().T / 16, dim=1)
+        out.append((p @ v[at, g].double()) * torch.sigmoid(Q[:, 256:]))
+    return torch.cat(out)
+
+
+# units = sessions x rows x 2 KV heads; 8 streams a CTA (16 heads) or 6 (18 and 24 heads): one position, fewer tiles than
+# streams, clusters of 8 / 4 / 2, one CTA per unit, several units per CTA, ragged last CTA
+@pytest.mark.parametrize("Hq,sessions,rows,ctx", [(16, 1, 1, 1), (16, 1, 1, 37), (16, 1, 1, 1501), (16, 1, 2, 2052), (16, 4, 1, 9003), (16, 7, 2, 2600),
+                                                   (16, 8, 9, 3001), (16, 17, 13, 2301), (24, 1, 4, 2051), (24, 3, 1, 700), (18, 5, 5, 2301), (24, 9, 13, 2301)])
+def test_attention_work_splits(Hq, sessions, rows, ctx):
+    capi, layers, g, w = _weights(Hq)
+    gen = torch.Generator(device="cuda").manual_seed(ctx + Hq)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    spans, outs, arr = [], [], (capi.QsaArgs * sessions)()
+    zero = torch.zeros(rows, 640, device="cuda")
+    for i in range(sessions):
+        pos0 = ctx - rows - (i % 3 if ctx > rows + 3 else 0)      # tails of different lengths
+        s = layers.QsaSession(g, ctx, max_rows=rows)
+        s.k.copy_(rn(ctx, 2, 256)); s.v.copy_(rn(ctx, 2, 256))
+        for r in range(rows):
+            s.sel[r], n = _selection(gen, pos0 + r)
+            s.nsel[r] = n
+        q = rn(rows, Hq, 512)
+        q[:, :, :256] *= 2.0
+        outs.append(torch.full((rows, Hq * 256), 7.0, device="cuda"))
+        spans.append((s, q, pos0))
+        arr[i] = layers.qsa_args(w, s, q, zero, zero, zero, outs[i], pos0)
+    scratch = torch.empty(capi.lib.cr_qsa_scratch_bytes(C.byref(g), sessions * rows), device="cuda", dtype=torch.uint8)
+    capi.check(capi.lib.cr_qsa_attn(C.byref(g), arr, sessions, capi.dptr(scratch), scratch.numel(), capi.OUT_RAW_F32, None))
+    torch.cuda.synchronize()
+    for i, (s, q, pos0) in enumerate(spans):
+        for r in range(rows):
+            ref = _attend(q[r], s.k, s.v, s.sel[r], int(s.nsel[r]), pos0 + r)
+            err = (outs[i][r].view(Hq, 256).double() - ref).abs().max().item()
+            assert err < 2e-5, "session %d row %d: %g" % (i, r, err)
+
+
+@pytest.mark.parametrize("pos0,R", [(4 * 262144 - 9, 20), (4 * 524288 + 3, 33)])
+def test_union_lists_past_one_bitmap_window(pos0, R):
+    capi, layers, g, w = _weights(16)
+    rng = np.random.default_rng(pos0)
+    ses = layers.QsaSession(g, 64, max_rows=R)
+    common = rng.choice((pos0 + 1) // 4, 300, replace=False)
+    sel = np.empty((R, 512), np.int32)
+    for r in range(R):
+        own = rng.choice((pos0 + 1) // 4, 700, replace=False)
+        sel[r] = np.sort(np.concatenate([common, np.setdiff1d(own, common)[:212]]))
+    ses.sel.copy_(torch.from_numpy(sel)); ses.nsel.fill_(512)
+    z = torch.zeros(R, 16, 512, device="cuda")
+    args = layers.qsa_args(w, ses, z, z, z, z, z, pos0)
+    args.sstride = (pos0 + R) // 4                               # nothing reads the scores or the cache here
+    ints, RT = capi.lib.cr_qsa_union_list_ints(C.byref(g), R), 16
+    tiles = (R + RT - 1) // RT
+    lst, cnt = torch.zeros(ints, dtype=torch.int32, device="cuda"), torch.zeros(tiles, dtype=torch.int32, device="cuda")
+    u = capi.QsaUnion(lst.data_ptr(), cnt.data_ptr())
+    capi.check(capi.lib.cr_qsa_union_build(C.byref(g), (capi.QsaArgs * 1)(args), C.byref(u), None))
+    got = lst.cpu().numpy().reshape(tiles, -1, 2)
+    for t in range(tiles):
+        want = {}
+        for r in range(t * RT, min(R, (t + 1) * RT)):
+            blocks = list(sel[r]) + ([(pos0 + r + 1) // 4] if (pos0 + r + 1) % 4 else [])
+            for b in blocks:
+                want[int(b)] = want.get(int(b), 0) | 1 << (r - t * RT)
+        np.testing.assert_array_equal(got[t, :int(cnt[t])], np.array(sorted(want.items()), np.int32))
