@@ -40,4 +40,9 @@ struct QsaTileSplit { const int* count; int rows, max; };   // see QsaParams::ti
 cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int p0, int p1, cr_out_format fmt,
                           cudaStream_t stream, const QsaTileSplit* tiles = nullptr);
 
+// Combines `nparts` (at most 32) records per (row, head), record p of row r at partials[(p * R + r) * Hq + h], into outputs;
+// with `tiles` only the rows of tiled tiles have records.
+cr_status qsa_merge_launch(const cr_geometry* g, const cr_qsa_args& a, int nparts, const float* partials, cr_out_format fmt, cudaStream_t stream,
+                           const QsaTileSplit* tiles = nullptr);
+
 }  // namespace cr

@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
   cluster.sync();                                        // the images stay until every CTA has read them
 }
 
-// Merge of the partial records of several ranks (QsaMergeKernel, engine/layers/qsa_long.h:458-499), gate and output
+// Merge of the partial records of several ranks or of a tile's splits (QsaMergeKernel, engine/layers/qsa_long.h:458-499), gate and output
 // transform.  grid (Hq, R), 64 threads: a warp per 128-channel group.  Record p of (row, head) lies at
 // partials[((p * rows + row) * Hq + h) * 258].
 __global__ void __launch_bounds__(64) qsa_merge_kernel(const __grid_constant__ QsaParams P, const float* partials, int nparts, int fmt) {
@@ -389,6 +389,7 @@ __global__ void __launch_bounds__(64) qsa_merge_kernel(const __grid_constant__ Q
   pdl_wait();
   const cr_qsa_args& a = P.span[0];
   const int h = blockIdx.x, r = blockIdx.y, l = threadIdx.x & 31, c = (threadIdx.x >> 5) * 128 + 4 * l;
+  if (P.tile_count && !qsa_row_is_tiled(P, r)) return;   // a row of the row-wise kernel
   auto rec = [&](int p) { return partials + (((size_t)p * a.R + r) * P.Hq + h) * CR_QSA_PART; };
   float pm = -INFINITY, pl = 0.f;                        // lane p: (m, l) of record p
   if (l < nparts) {
@@ -485,6 +486,17 @@ cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
   return CR_OK;
 }
 
+cr_status qsa_merge_launch(const cr_geometry* g, const cr_qsa_args& a, int nparts, const float* partials, cr_out_format fmt, cudaStream_t stream,
+                           const QsaTileSplit* tiles) {
+  QsaParams P;
+  qsa_fill_params(P, g, &a, 1);
+  if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; }
+  use_stream(stream);
+  CR_CUDA(launch_pdl(qsa_merge_kernel, dim3(g->q_heads, a.R), dim3(64), 0, stream, P, partials, nparts, (int)fmt));
+  CR_LAUNCH_CHECK("qsa_merge_kernel");
+  return CR_OK;
+}
+
 static cr_status check_out(const cr_qsa_args* spans, int n, cr_out_format fmt, const char* who) {
   CR_REQUIRE(fmt == CR_OUT_RAW_F32 || fmt == CR_OUT_RAW_BF16 || fmt == CR_OUT_EXL3_WHT, "%s: bad output format", who);
   for (int s = 0; s < n; ++s) {
@@ -552,10 +564,5 @@ extern "C" cr_status cr_qsa_merge_partials(const cr_geometry* g, const cr_qsa_ar
   if (cr_status s = qsa_validate(g, a, 1, CR_MAX_PREFILL_ROWS, "cr_qsa_merge_partials", 0)) return s;
   if (cr_status s = check_out(a, 1, fmt, "cr_qsa_merge_partials")) return s;
   CR_REQUIRE(partials && ranks >= 1 && ranks <= 32, "cr_qsa_merge_partials: need gathered partials of 1..32 ranks");
-  QsaParams P;
-  qsa_fill_params(P, g, a, 1);
-  use_stream((cudaStream_t)stream);
-  CR_CUDA(launch_pdl(qsa_merge_kernel, dim3(g->q_heads, a->R), dim3(64), 0, (cudaStream_t)stream, P, partials, ranks, (int)fmt));
-  CR_LAUNCH_CHECK("qsa_merge_kernel");
-  return CR_OK;
+  return qsa_merge_launch(g, *a, ranks, partials, fmt, (cudaStream_t)stream);
 }

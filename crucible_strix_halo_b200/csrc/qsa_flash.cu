@@ -14,9 +14,9 @@
 //
 // qsa_flash_tc_kernel (one CTA per (tile, KV head), 15 warps, 64 keys per step):
 //   loader warps (6)   gather the K and V rows of 16 blocks per step with 16-byte cp.async into three stages, two
-//                      warps per stage.  Both tiles land as 16-byte units at (piece * 64 + key) * 16: for K that is
-//                      the K-major operand [key][channel], for V the MN-major operand [key][channel] (channels
-//                      contiguous), so neither is transposed anywhere.
+//                      warps per stage, one key's 512 bytes per instruction.  Both tiles land as four groups of 64
+//                      channels, [64 keys][128 bytes] with the 128-byte swizzle: for K the K-major operand
+//                      [key][channel], for V the MN-major operand [key][channel], so neither is transposed anywhere.
 //   issuer warp        S = Q K^T (16 tcgen05.mma kind::f16, M 128 x N 64 x K 16, the query tile being the A operand
 //                      in tensor memory, which leaves the shared memory to the K/V stages) into one of two TMEM
 //                      accumulators, one step ahead of the softmax; O += P V (4 MMAs, N 256) once the probabilities
@@ -32,6 +32,7 @@
 // Every wait is bounded; a wait that gives up raises the status word and the CTA runs to its end.
 #include <climits>
 #include "qsa.cuh"
+#include "tma.cuh"
 #include "umma.cuh"
 
 namespace cr {
@@ -44,9 +45,10 @@ constexpr int kFlStages = 3;                        // K/V stages in flight
 constexpr int kFlSoftmax = 8;                       // softmax warps: two per TMEM lane quarter, 32 keys of a step each
 constexpr int kFlThreads = 32 * (kFlSoftmax + 2 * kFlStages + 1);   // + 2 loader warps per stage + 1 issuer warp
 constexpr int kFlIssuer = kFlSoftmax + 2 * kFlStages;
-constexpr int kFlKBytes = kFlKeys * 256 * 2;        // [32 channel pieces][64 keys][8 halves]
+constexpr int kFlKBytes = kFlKeys * 256 * 2;        // [4 channel groups][64 keys][128 bytes, 128-byte swizzle]
+constexpr int kFlGroup = kFlKeys * 128;             // one channel group of a tile
 constexpr int kFlPBytes = 128 * kFlKeys * 2;        // [8 key pieces][128 rows][8 halves]
-constexpr size_t kFlashSmem = 2 * kFlStages * kFlKBytes + 2 * kFlPBytes + 128;
+constexpr size_t kFlashSmem = 2 * kFlStages * kFlKBytes + 2 * kFlPBytes;   // + 3 KB of static arrays: all of the 227 KB
 // TMEM columns: O 0-255, S of step j at 256 + 64 (j & 1), the query tile (two fp16 channels per column) at 384-511
 constexpr uint32_t kColO = 0, kColS = 256, kColQ = 384;
 
@@ -56,6 +58,7 @@ struct FlashParams {
   const int2* list;       // [tiles][cap] (block, row mask), ascending blocks
   const int* count;       // [tiles]
   float* gated;           // gated fp32 [R][Hq * 256] when the output transform runs as a second kernel, else null
+  float* partials;        // splits > 1: records (m, l, acc[256]) [split][R][Hq][258] for the merge kernel, else null
   int cap, RT, Hq, Hkv, fmt;
   int flash_max;          // tiles whose union list is longer are left to the row-wise kernels
 };
@@ -160,8 +163,7 @@ __global__ void __launch_bounds__(kUbThreads) qsa_union_build_kernel(const __gri
 }
 
 // ---- flash ---------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void fl_cp_async16(void* dst, const void* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+__device__ __forceinline__ void fl_cp_async16(unsigned d, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes));
 }
@@ -169,9 +171,9 @@ __device__ __forceinline__ void fl_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_u32(bar)) : "memory");
 }
 
-// grid (tiles, Hkv).
+// grid (tiles, Hkv, splits).
 __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __grid_constant__ FlashParams P) {
-  extern __shared__ __align__(128) unsigned char sm[];
+  extern __shared__ __align__(1024) unsigned char sm[];
   unsigned char* Ks = sm;                                // kFlStages stages
   unsigned char* Vs = Ks + kFlStages * kFlKBytes;        // kFlStages stages
   unsigned char* Ps = Vs + kFlStages * kFlKBytes;        // two buffers
@@ -186,8 +188,13 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
   const int tile = blockIdx.x, g = blockIdx.y, row0 = tile * P.RT;
   const int gqa = P.Hq / P.Hkv;
   const int cnt = P.count[tile];
-  const int n = (cnt + kFlBlocks - 1) / kFlBlocks;
-  if (n == 0 || cnt > P.flash_max) return;               // a tile without rows, or one the row-wise kernels serve
+  const int n_all = (cnt + kFlBlocks - 1) / kFlBlocks;   // steps of the tile; this CTA's share is [step0, step0 + n)
+  if (n_all == 0 || cnt > P.flash_max) return;           // a tile without rows, or one the row-wise kernels serve
+  const int step0 = (int)((long long)n_all * blockIdx.z / gridDim.z), n = (int)((long long)n_all * (blockIdx.z + 1) / gridDim.z) - step0;
+  if ((umma::smem_u32(sm) & 1023u) != 0) {               // the swizzled tiles need their atoms on 1 KB boundaries
+    if (t == 0) g_qsa_flash_status = 1;
+    return;
+  }
   const int last_pos = a.pos0 + a.R - 1;                 // newest position the cache holds
 
   if (t == 0) {
@@ -243,10 +250,10 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
     if (l == 0) {
       constexpr uint32_t idS = umma::idesc_f16(128, kFlKeys, false, false), idO = umma::idesc_f16(128, 256, false, true);
       auto issue_S = [&](int j) {
-        const uint64_t dK = umma::smem_desc(Ks + (j % kFlStages) * kFlKBytes, kFlKeys * 16, 128);
+        const uint64_t dK = tma::desc_sw128(Ks + (j % kFlStages) * kFlKBytes, 16, 1024);
 #pragma unroll
-        for (int ks = 0; ks < 16; ++ks)                  // 16 channels per MMA: 8 columns of Q, two 16-byte pieces of every key
-          umma::mma_f16_ts(tm + kColS + 64 * (j & 1), tm + kColQ + 8 * ks, dK + (uint64_t)(ks * 2 * kFlKeys), idS, ks > 0);
+        for (int ks = 0; ks < 16; ++ks)                  // 16 channels per MMA: 8 columns of Q, 32 bytes of every key's 128-byte row
+          umma::mma_f16_ts(tm + kColS + 64 * (j & 1), tm + kColQ + 8 * ks, dK + (uint64_t)(((ks >> 2) * kFlGroup + (ks & 3) * 32) >> 4), idS, ks > 0);
         umma::commit(&sFull[j & 1]);
       };
       // Event loop: S of step ns (one step ahead of the softmax at most, its accumulator being free once the
@@ -265,10 +272,10 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
           const int st = np % kFlStages;
           umma::fence_after_sync();
           const uint64_t dP = umma::smem_desc(Ps + (np & 1) * kFlPBytes, 128 * 16, 128);
-          const uint64_t dV = umma::smem_desc(Vs + st * kFlKBytes, 128, kFlKeys * 16);   // MN-major: step along keys 128 B, along channels 1 KB
+          const uint64_t dV = tma::desc_sw128(Vs + st * kFlKBytes, kFlGroup, 1024);        // MN-major: 64-channel groups, atoms of 8 keys
 #pragma unroll
           for (int kk = 0; kk < kFlKeys / 16; ++kk)
-            umma::mma_f16_ss(tm + kColO, dP + (uint64_t)(kk * 2 * 128), dV + (uint64_t)(kk * 16), idO, (np > 0 || kk > 0) ? 1u : 0u);
+            umma::mma_f16_ss(tm + kColO, dP + (uint64_t)(kk * 2 * 128), dV + (uint64_t)(kk * 2048 >> 4), idO, (np > 0 || kk > 0) ? 1u : 0u);
           umma::commit(&pvDone[st]);
           ++np; idle = 0;
         } else if ((++idle & 63) == 0) {                  // nothing ready: look at the clock now and then
@@ -279,23 +286,43 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
       }
     }
   } else if (w >= kFlSoftmax) {
-    // ------------------------------------------------------------------ loaders: two warps per stage
+    // ------------------------------------------------------------------ loaders: two warps per stage, half of its keys each
+    // One cp.async instruction brings one key's 512 bytes: four full lines, and eight lanes write the eight pieces of a
+    // 128-byte swizzled row, so the writes are free of bank conflicts.
     const int st = (w - kFlSoftmax) >> 1, lw = (w - kFlSoftmax) & 1;
-    const __half* kc = reinterpret_cast<const __half*>(a.c.k) + (size_t)g * 256 + (l & 1) * 8;
-    const __half* vc = reinterpret_cast<const __half*>(a.c.v) + (size_t)g * 256 + (l & 1) * 8;
+    const char* kc = reinterpret_cast<const char*>(a.c.k) + (size_t)g * 512 + l * 16;
+    const char* vc = reinterpret_cast<const char*>(a.c.v) + (size_t)g * 512 + l * 16;
     const int2* lst = P.list + (size_t)tile * P.cap;
-    const size_t row_halves = (size_t)P.Hkv * 256;
-    unsigned char* kd = Ks + st * kFlKBytes;
-    unsigned char* vd = Vs + st * kFlKBytes;
+    const size_t row_bytes = (size_t)P.Hkv * 512;
+    const unsigned kd = umma::smem_u32(Ks + st * kFlKBytes) + (l >> 3) * kFlGroup, vd = umma::smem_u32(Vs + st * kFlKBytes) + (l >> 3) * kFlGroup;
+    auto entry = [&](int j) {                              // lane b (and b + 16): entry b of step j
+      const int idx = (step0 + j) * kFlBlocks + (l & 15);
+      return j < n && idx < cnt ? lst[idx] : make_int2(0, 0);
+    };
+    int2 e = entry(st);
     for (int j = st; j < n; j += kFlStages) {
+      const int2 e_next = entry(j + kFlStages);            // in flight while the stage is waited for
       if (j >= kFlStages) warp_wait(&pvDone[st], ((j - kFlStages) / kFlStages) & 1);   // the MMAs of the stage's last step are done
       if (dead) break;
+#pragma unroll
+      for (int b = 0; b < kFlBlocks / 2; ++b) {
+        const int pos0 = __shfl_sync(0xffffffffu, e.x, lw * (kFlBlocks / 2) + b) * 4;
+        const size_t src = (size_t)pos0 * row_bytes;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int key = (lw * (kFlBlocks / 2) + b) * 4 + k;
+          const bool valid = pos0 + k <= last_pos;
+          const size_t at = valid ? src + k * row_bytes : 0;
+          const unsigned dst = key * 128 + (((l ^ key) & 7) << 4);
+          fl_cp_async16(kd + dst, kc + at, valid);
+          fl_cp_async16(vd + dst, vc + at, valid);
+        }
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
       if (lw == 0) {
-        // Lane b < 16 holds entry b of the step; lane r < 16 then builds the word of row r: bit 4 b + k is set when the
-        // row's bit of block b's mask is set and token k of the block is not in the row's future (only the open tail
-        // block of a row can hold such tokens).  The softmax threads read one word per step.
-        const int idx = j * kFlBlocks + (l & 15);
-        const int2 e = idx < cnt ? lst[idx] : make_int2(0, 0);
+        // Lane r < 16 builds the word of row r: bit 4 b + k is set when the row's bit of block b's mask is set and token k
+        // of the block is not in the row's future (only the open tail block of a row can hold such tokens).  The softmax
+        // threads read one word per step.
         const int prow = a.pos0 + row0 + (l & 15);
         const bool rowok = (l & 15) < P.RT && row0 + (l & 15) < a.R;
         unsigned lo_w = 0u, hi_w = 0u;
@@ -308,26 +335,11 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
         }
         if (l < 16) { seen_s[st][l][0] = lo_w; seen_s[st][l][1] = hi_w; }
       }
-      // lane l serves key 16 kg + l / 2 (kg = 0..3) and the channel pieces 2 pp + l % 2, pp = 8 lw .. 8 lw + 7
-#pragma unroll
-      for (int kg = 0; kg < 4; ++kg) {
-        const int key = kg * 16 + (l >> 1), idx = j * kFlBlocks + (key >> 2);
-        const int pos = (idx < cnt ? lst[idx].x : 0) * 4 + (key & 3);
-        const bool valid = pos <= last_pos;
-        const size_t src = valid ? (size_t)pos * row_halves : 0;
-        const size_t dst = ((size_t)(l & 1) * kFlKeys + key) * 16;
-#pragma unroll
-        for (int p8 = 0; p8 < 8; ++p8) {
-          const int pp = lw * 8 + p8;
-          fl_cp_async16(kd + dst + (size_t)pp * (2 * kFlKeys * 16), kc + src + pp * 16, valid);
-          fl_cp_async16(vd + dst + (size_t)pp * (2 * kFlKeys * 16), vc + src + pp * 16, valid);
-        }
-      }
-      asm volatile("cp.async.commit_group;\n" ::);
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
       umma::fence_async_smem();
       __syncwarp();
       if (l == 0) fl_mbar_arrive(&kvFull[st]);
+      e = e_next;
     }
   } else {
     // ------------------------------------------------------------------ softmax warps: thread = (TMEM lane m, half of the step's keys)
@@ -406,15 +418,27 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
     if (hf == 0) { lsum += half_sum[m]; half_sum[128 + m] = lsum; }
     pair_sync();
     lsum = half_sum[128 + m];
-    warp_wait(&pvDone[(n - 1) % kFlStages], ((n - 1) / kFlStages) & 1);
+    if (n > 0) warp_wait(&pvDone[(n - 1) % kFlStages], ((n - 1) / kFlStages) & 1);
     umma::fence_after_sync();
-    const bool ok = rowok && lsum > 0.f && !dead;
+    if (P.partials) {                                                   // the tile is split: leave (m, l, acc) of this share
+      float* rec = P.partials + (((size_t)blockIdx.z * a.R + row0 + r) * P.Hq + g * gqa + hq) * CR_QSA_PART;
+      if (rowok && hf == 0) *reinterpret_cast<float2*>(rec) = make_float2(m_ref * 0.6931471805599453f, lsum);
+#pragma unroll 1
+      for (int c8 = 4 * hf; c8 < 4 * hf + 4; ++c8) {
+        float o[32];
+        umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+        if (!rowok) continue;
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) *reinterpret_cast<float2*>(rec + 2 + 32 * c8 + c) = n > 0 ? make_float2(o[c], o[c + 1]) : make_float2(0.f, 0.f);
+      }
+    }
+    const bool ok = !P.partials && rowok && lsum > 0.f && !dead;
     const float inv = ok ? 1.f / lsum : 0.f;
     const int gr = row0 + r, h = g * gqa + hq;
     const size_t W = (size_t)P.Hq * 256;
     const float* gate = a.q + ((size_t)gr * P.Hq + h) * 512 + 256;
 #pragma unroll 1
-    for (int c8 = 4 * hf; c8 < 4 * hf + 4; ++c8) {
+    for (int c8 = 4 * hf; c8 < 4 * hf + 4 && !P.partials; ++c8) {
       float o[32];
       umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);     // warp-collective: every lane takes part
       if (!ok) continue;
@@ -491,7 +515,7 @@ cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int
 
 // Attention of the rows of `a` over the union lists; `gated` (rows x Hq x 256 floats) is needed for CR_OUT_EXL3_WHT.
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* gated, cr_out_format fmt, int flash_max, cudaStream_t stream) {
+                           float* gated, float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream) {
   static PerDeviceOnce configured;
   if (cr_status st = once_per_device(configured, [] {
         CR_CUDA(cudaFuncSetAttribute(qsa_flash_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem));
@@ -501,14 +525,15 @@ cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __h
   P.a = a; P.q_hi = q_hi; P.list = list; P.count = count;
   P.RT = qsa_union_rows(g); P.cap = qsa_union_cap(P.RT);
   P.Hq = g->q_heads; P.Hkv = g->kv_heads; P.fmt = (int)fmt;
-  P.gated = fmt == CR_OUT_EXL3_WHT ? gated : nullptr;
+  P.gated = fmt == CR_OUT_EXL3_WHT && splits == 1 ? gated : nullptr;
+  P.partials = splits > 1 ? partials : nullptr;
   P.flash_max = flash_max;
   CR_REQUIRE(fmt != CR_OUT_EXL3_WHT || gated, "qsa flash: the EXL3 output needs the gated fp32 scratch");
   const int tiles = (a.R + P.RT - 1) / P.RT;
   use_stream(stream);
-  qsa_flash_tc_kernel<<<dim3(tiles, g->kv_heads), kFlThreads, kFlashSmem, stream>>>(P);
+  qsa_flash_tc_kernel<<<dim3(tiles, g->kv_heads, splits), kFlThreads, kFlashSmem, stream>>>(P);
   CR_LAUNCH_CHECK("qsa_flash_tc_kernel");
-  if (fmt == CR_OUT_EXL3_WHT) {
+  if (P.gated) {
     qsa_out_transform_kernel<<<dim3(g->q_heads, a.R), 64, 0, stream>>>(a, gated, g->q_heads, count, P.RT, flash_max);
     CR_LAUNCH_CHECK("qsa_out_transform_kernel");
   }

@@ -9,17 +9,29 @@
 #include "qsa.cuh"
 
 namespace cr {
-constexpr int kPrefillSplits = 4;
-
 int qsa_union_rows(const cr_geometry* g);
 int qsa_union_cap(int RT);
 cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int2* list, int* count, cudaStream_t stream);
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* gated, cr_out_format fmt, int flash_max, cudaStream_t stream);
+                           float* gated, float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream);
 
-// Scratch of a part: [split-KV partials of the row-wise kernels][gated fp32 rows for the EXL3 transform of the tiled
-// kernel][union lists, 2 ints per entry][union counts].  The list area is sized for tiles of 8 rows, the smallest tile.
-static size_t partial_bytes(const cr_geometry* g, int rows) { return (size_t)rows * g->q_heads * kPrefillSplits * CR_QSA_PART * sizeof(float); }
+// Scratch of a part: [partial records of split tiles][gated fp32 rows for the EXL3 transform of the tiled kernel][union
+// lists, 2 ints per entry][union counts].  The list area is sized for tiles of 8 rows, the smallest tile.
+//
+// A short part has fewer (tile, KV head) pairs than the GPU has SMs, and each walks its whole union list: its tiles are
+// then split along the list, as many ways as fill the SMs once, and a merge kernel combines the records.  117 rows at
+// 9,003 positions (16 CTAs): 221 us unsplit, 32 us in 9 splits plus 5 us of merge.
+constexpr int kMaxTileSplits = 16, kPartialRows = 16 * 160;
+static int tile_splits(const cr_geometry* g, int rows) {
+  const int RT = qsa_union_rows(g), ctas = (rows + RT - 1) / RT * g->kv_heads, s = sm_count() / ctas;
+  const int most = kPartialRows / rows < kMaxTileSplits ? kPartialRows / rows : kMaxTileSplits;
+  return s < 1 ? 1 : (s > most ? most : s);
+}
+// At most kPartialRows rows x splits; grows with the rows, so that the scratch of a long part serves every shorter one.
+static size_t partial_bytes(const cr_geometry* g, int rows) {
+  const int all = rows * kMaxTileSplits;
+  return (size_t)(all < kPartialRows ? all : kPartialRows) * g->q_heads * CR_QSA_PART * sizeof(float);
+}
 static size_t gated_bytes(const cr_geometry* g, int rows) { return (size_t)rows * g->q_heads * 256 * sizeof(float); }
 static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_cap(8) * 2; }
 // A tile goes to the tiled tensor-core kernel when its rows share enough blocks: at most this many union entries per
@@ -61,10 +73,13 @@ static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, c
     int2* list = reinterpret_cast<int2*>(scratch + partial_bytes(g, q.R) + gated_bytes(g, q.R));
     int* count = reinterpret_cast<int*>(list + list_ints(q.R) / 2);
     const int RT = qsa_union_rows(g);
+    const int splits = tile_splits(g, q.R);
     const QsaTileSplit tiles = {count, RT, options().qsa_union_rows > 0 ? INT_MAX : kFlashEntriesPerRow * RT};   // an explicit tile size forces the tiled kernel
     if (cr_status s = qsa_union_build_launch(g, q, list, count, stream)) return s;
     if (cr_status s = qsa_flash_launch(g, q, reinterpret_cast<const __half*>(args->q_hi) + (size_t)skip * g->q_heads * 256, list, count,
-                                       gated, fmt, tiles.max, stream)) return s;
+                                       gated, reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, stream)) return s;
+    if (splits > 1)
+      if (cr_status s = qsa_merge_launch(g, q, splits, reinterpret_cast<const float*>(scratch), fmt, stream, &tiles)) return s;
     if (tiles.max == INT_MAX) return CR_OK;
     // the tiles with little sharing: row-wise split-KV attention (its CTAs of tiled rows exit at once)
     return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream, &tiles);
