@@ -158,6 +158,25 @@ __host__ __device__ __forceinline__ size_t out_index(int r, int c, int width, in
   return pack_rows ? ((size_t)(c >> 4) * pack_rows + pack_off + r) * 16 + (c & 15) : (size_t)r * width + c;
 }
 
+// Four consecutive fp16 values: one 64-bit access where the address allows it.
+__device__ __forceinline__ void load_half4(const uint16_t* p, float (&v)[4]) {
+  __half2 h[2];
+  if (((uintptr_t)p & 7) == 0) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    h[0] = *reinterpret_cast<const __half2*>(&u.x); h[1] = *reinterpret_cast<const __half2*>(&u.y);
+  } else {
+    const __half* q = reinterpret_cast<const __half*>(p);
+    h[0] = __halves2half2(q[0], q[1]); h[1] = __halves2half2(q[2], q[3]);
+  }
+  const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void store_half4(uint16_t* p, const float (&v)[4], float scale) {
+  const __half2 lo = __floats2half2_rn(v[0] * scale, v[1] * scale), hi = __floats2half2_rn(v[2] * scale, v[3] * scale);
+  if (((uintptr_t)p & 7) == 0) *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+  else { __half* q = reinterpret_cast<__half*>(p); q[0] = lo.x; q[1] = lo.y; q[2] = hi.x; q[3] = hi.y; }
+}
+
 // Loads element i of a row buffer that is fp32 or bf16.
 template <bool BF16>
 __device__ __forceinline__ float load_in(const void* p, long long i) {

@@ -12,12 +12,18 @@ struct QsaParams {
   int Hq, Hkv, n;
   int b_lo, b_hi;          // scoring only: the blocks [b_lo, b_hi) are scored (a rank's own blocks; 0, INT_MAX = all)
   // Prefill parts that mix the tiled and the row-wise attention: tile_count[r / tile_rows] is the size of the union
-  // list of row r's tile; the row-wise kernels serve the rows whose tile has more than tile_max entries (null: all).
+  // list of row r's tile; the row-wise kernel serves the rows whose tile has more than tile_max entries for each of its
+  // rows (null: all).
   const int* tile_count;
   int tile_rows, tile_max;
 };
+// rows: rows of the part, of which the last tile may hold fewer than tile_rows
+__host__ __device__ __forceinline__ bool qsa_tile_shares(int entries, int tile, int tile_rows, int rows, int per_row) {
+  const int in_tile = rows - tile * tile_rows;
+  return entries <= per_row * (in_tile < tile_rows ? in_tile : tile_rows);
+}
 __device__ __forceinline__ bool qsa_row_is_tiled(const QsaParams& P, int r) {
-  return P.tile_count && P.tile_count[r / P.tile_rows] <= P.tile_max;
+  return P.tile_count && qsa_tile_shares(P.tile_count[r / P.tile_rows], r / P.tile_rows, P.tile_rows, P.span[0].R, P.tile_max);
 }
 
 // score_blocks >= 0: the score stride must cover that many blocks (a rank's own range, or 0 for entries that never touch
@@ -44,5 +50,30 @@ cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
 // with `tiles` only the rows of tiled tiles have records.
 cr_status qsa_merge_launch(const cr_geometry* g, const cr_qsa_args& a, int nparts, const float* partials, cr_out_format fmt, cudaStream_t stream,
                            const QsaTileSplit* tiles = nullptr);
+
+// Channels c .. c + 3 (c = 128 half + 4 lane, a warp holds a 128-channel group) of one head of one row: un-gated context,
+// gate, output format.
+__device__ __forceinline__ void emit_group(const cr_qsa_args& a, int Hq, int r, int h, int c, float4 o, const float4 gate, int fmt) {
+  const size_t W = (size_t)Hq * 256, at = (size_t)r * W + h * 256 + c;
+  if (a.context) { float* cx = a.context + at; cx[0] = o.x; cx[1] = o.y; cx[2] = o.z; cx[3] = o.w; }
+  float v[4] = {o.x * sigmoidf_(gate.x), o.y * sigmoidf_(gate.y), o.z * sigmoidf_(gate.z), o.w * sigmoidf_(gate.w)};
+  if (fmt == CR_OUT_RAW_F32) {
+    float* dst = reinterpret_cast<float*>(a.out) + at;
+    if (((uintptr_t)dst & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else { dst[0] = v[0]; dst[1] = v[1]; dst[2] = v[2]; dst[3] = v[3]; }
+  } else if (fmt == CR_OUT_RAW_BF16) {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + at;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+    if (((uintptr_t)dst & 7) == 0) *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    else { dst[0] = lo.x; dst[1] = lo.y; dst[2] = hi.x; dst[3] = hi.y; }
+  } else {
+    float su[4];
+    load_half4(a.suh_o + h * 256 + c, su);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = round_h(round_h(v[i]) * su[i]);
+    wht128(v);
+    store_half4(reinterpret_cast<uint16_t*>(a.out) + out_index(r, h * 256 + c, (int)W, a.pack_rows, a.pack_off), v, kHadNorm);   // c is a multiple of 4
+  }
+}
 
 }  // namespace cr

@@ -79,32 +79,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// Channels c .. c + 3 (c = 128 half + 4 lane, a warp holds a 128-channel group) of one head of one row: un-gated context,
-// gate, output format.
-__device__ __forceinline__ void emit_group(const cr_qsa_args& a, int Hq, int r, int h, int c, float4 o, const float4 gate, int fmt) {
-  const size_t W = (size_t)Hq * 256, at = (size_t)r * W + h * 256 + c;
-  if (a.context) { float* cx = a.context + at; cx[0] = o.x; cx[1] = o.y; cx[2] = o.z; cx[3] = o.w; }
-  float v[4] = {o.x * sigmoidf_(gate.x), o.y * sigmoidf_(gate.y), o.z * sigmoidf_(gate.z), o.w * sigmoidf_(gate.w)};
-  if (fmt == CR_OUT_RAW_F32) {
-    float* dst = reinterpret_cast<float*>(a.out) + at;
-    if (((uintptr_t)dst & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-    else { dst[0] = v[0]; dst[1] = v[1]; dst[2] = v[2]; dst[3] = v[3]; }
-  } else if (fmt == CR_OUT_RAW_BF16) {
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + at;
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-    if (((uintptr_t)dst & 7) == 0) *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
-    else { dst[0] = lo.x; dst[1] = lo.y; dst[2] = hi.x; dst[3] = hi.y; }
-  } else {
-    const __half* suh = reinterpret_cast<const __half*>(a.suh_o) + h * 256 + c;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = round_h(round_h(v[i]) * __half2float(suh[i]));
-    wht128(v);
-    __half* dst = reinterpret_cast<__half*>(a.out);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[out_index(r, h * 256 + c + i, (int)W, a.pack_rows, a.pack_off)] = __float2half(v[i] * kHadNorm);
-  }
-}
-
 // grid (cluster x ceil(Rmax * Hkv / units per CTA), 1, spans).
 template <int NG>
 __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __grid_constant__ QsaParams P, const AttnShape shape, float* partials,

@@ -12,22 +12,25 @@
 // byte per block in 64 KB of LDS and falls back to row-wise attention past about 196K positions,
 // engine/layers/qsa_union_lds.h:7-11).
 //
-// qsa_flash_tc_kernel (one CTA per (tile, KV head), 15 warps, 64 keys per step):
-//   loader warps (6)   gather the K and V rows of 16 blocks per step with 16-byte cp.async into three stages, two
-//                      warps per stage, one key's 512 bytes per instruction.  Both tiles land as four groups of 64
-//                      channels, [64 keys][128 bytes] with the 128-byte swizzle: for K the K-major operand
-//                      [key][channel], for V the MN-major operand [key][channel], so neither is transposed anywhere.
-//   issuer warp        S = Q K^T (16 tcgen05.mma kind::f16, M 128 x N 64 x K 16, the query tile being the A operand
+// qsa_flash_tc_kernel (one CTA per (tile, KV head, split), 16 warps, 64 keys per step):
+//   loader warps (6)   one per K stage and per V stage: gathers the rows of 16 blocks with 16-byte cp.async, one key's 512
+//                      bytes per instruction.  Tiles land as four groups of 64 channels, [64 keys][128 bytes] with the
+//                      128-byte swizzle: for K the K-major operand [key][channel], for V the MN-major operand
+//                      [key][channel], so neither is transposed anywhere.  The V loaders also build the visibility words.
+//   issuer warps (2)   S = Q K^T (16 tcgen05.mma kind::f16, M 128 x N 64 x K 16, the query tile being the A operand
 //                      in tensor memory, which leaves the shared memory to the K/V stages) into one of two TMEM
-//                      accumulators, one step ahead of the softmax; O += P V (4 MMAs, N 256) once the probabilities
-//                      are written.  An event loop issues whichever is ready.
-//   softmax warps (8)  two warps per TMEM lane quarter, thread = (row, head) x half of the step's 64 keys: reads S,
-//                      applies mask and causality (a 32-bit visibility word per step), keeps a running reference
-//                      maximum that moves only when a logit exceeds it by more than 2^8 (the accumulator is rescaled
-//                      in TMEM then, which is rare after the first steps; the two halves agree on the row maximum
-//                      through shared memory and a 64-thread named barrier), writes P as fp16 into a K-major
-//                      shared-memory tile, sums it.
-//   epilogue           O / sum, optional un-gated context, sigmoid gate, output format.
+//                      accumulators; O += P V (4 MMAs, N 256) once the probabilities are written.
+//   softmax warps (8)  two warpgroups that take the steps in turn, thread = (row, head) = TMEM lane: reads S, applies mask
+//                      and causality (two 32-bit visibility words per step), keeps a reference maximum that moves only
+//                      when a logit exceeds it by more than 2^8 (the accumulator is rescaled in TMEM then, which is rare
+//                      after the first steps), writes P as fp16 into a K-major shared-memory tile, sums it.
+//   epilogue           all warps: O through shared memory to a warp per (row, head), / sum, optional un-gated context,
+//                      sigmoid gate, output format.
+// Bound: latency around the two S accumulators (S product 1,000 cycles, softmax of a step 2,300, P V 520; the tensor pipe
+// alone would take 1,550 cycles per step, a step takes 2,350).  What it took to get there from 3,750: instruction fetches
+// were a third of all stalls while the roles had long unrolled bodies (rolled loops), the visibility words sat in the K
+// loaders' path (2,600 cycles), a thread wrote a row of its own at the end (20 us per CTA, now 12).  2,048 rows at 30,720,
+// 24 heads: 406 + 28 us of output transform before, 350 us now with it.
 // q and P are fp16 with fp32 accumulation, the reference's prefill numerics (prefill_qsa_union.h:680-684).
 // Every wait is bounded; a wait that gives up raises the status word and the CTA runs to its end.
 #include <climits>
@@ -41,12 +44,14 @@ CR_DEFINE_STATUS_WORD(qsa_flash)
 
 constexpr int kFlKeys = 64;                         // keys per step
 constexpr int kFlBlocks = kFlKeys / 4;              // union entries per step
-constexpr int kFlStages = 3;                        // K/V stages in flight
-constexpr int kFlSoftmax = 8;                       // softmax warps: two per TMEM lane quarter, 32 keys of a step each
-constexpr int kFlThreads = 32 * (kFlSoftmax + 2 * kFlStages + 1);   // + 2 loader warps per stage + 1 issuer warp
+constexpr int kFlStages = 3;                        // K tiles and V tiles in flight, each with a loader warp of its own
+constexpr int kFlSeen = 8;                          // steps whose visibility words are kept (a V loader runs at most 6 steps ahead)
+constexpr int kFlSoftmax = 8;                       // softmax warps: two warpgroups that take the steps in turn
+constexpr int kFlThreads = 32 * (kFlSoftmax + 2 * kFlStages + 2);   // + a loader warp per K and per V stage + an issuer warp per product
 constexpr int kFlIssuer = kFlSoftmax + 2 * kFlStages;
 constexpr int kFlKBytes = kFlKeys * 256 * 2;        // [4 channel groups][64 keys][128 bytes, 128-byte swizzle]
 constexpr int kFlGroup = kFlKeys * 128;             // one channel group of a tile
+constexpr int kFlOutLd = 260;                       // floats per (row, head) of the output image in shared memory
 constexpr int kFlPBytes = 128 * kFlKeys * 2;        // [8 key pieces][128 rows][8 halves]
 constexpr size_t kFlashSmem = 2 * kFlStages * kFlKBytes + 2 * kFlPBytes;   // + 3 KB of static arrays: all of the 227 KB
 // TMEM columns: O 0-255, S of step j at 256 + 64 (j & 1), the query tile (two fp16 channels per column) at 384-511
@@ -57,10 +62,9 @@ struct FlashParams {
   const __half* q_hi;     // [R][Hq][256]
   const int2* list;       // [tiles][cap] (block, row mask), ascending blocks
   const int* count;       // [tiles]
-  float* gated;           // gated fp32 [R][Hq * 256] when the output transform runs as a second kernel, else null
   float* partials;        // splits > 1: records (m, l, acc[256]) [split][R][Hq][258] for the merge kernel, else null
   int cap, RT, Hq, Hkv, fmt;
-  int flash_max;          // tiles whose union list is longer are left to the row-wise kernels
+  int flash_max;          // entries per row of a tile: longer lists are left to the row-wise kernel
 };
 
 int qsa_union_rows(const cr_geometry* g) {
@@ -171,25 +175,28 @@ __device__ __forceinline__ void fl_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_u32(bar)) : "memory");
 }
 
-// grid (tiles, Hkv, splits).
+// grid (Hkv, tiles, splits).  HKV: the cache's KV heads where they are two (row pitches become constants), else 0.
+template <int HKV>
 __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __grid_constant__ FlashParams P) {
   extern __shared__ __align__(1024) unsigned char sm[];
   unsigned char* Ks = sm;                                // kFlStages stages
   unsigned char* Vs = Ks + kFlStages * kFlKBytes;        // kFlStages stages
   unsigned char* Ps = Vs + kFlStages * kFlKBytes;        // two buffers
-  __shared__ __align__(8) uint64_t bars[2 * kFlStages + 4];
-  __shared__ unsigned seen_s[kFlStages][16][2];          // per stage and row of the tile: which of the step's 64 keys the row sees
-  __shared__ float half_max[2][2][128];                  // [step parity][half][lane]: exchange between the two warps of a TMEM lane quarter
+  __shared__ __align__(8) uint64_t bars[4 * kFlStages + kFlSeen + 6];
+  __shared__ unsigned seen_s[kFlSeen][16][2];            // per step and row of the tile: which of the step's 64 keys the row sees
+  __shared__ float ref_s[2][128];                        // [step parity][lane]: reference maximum after the step
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int dead;
-  uint64_t *kvFull = &bars[0], *pvDone = &bars[kFlStages], *sFull = &bars[2 * kFlStages], *pFull = &bars[2 * kFlStages + 2];
+  uint64_t *kFull = bars, *kEmpty = kFull + kFlStages, *vFull = kEmpty + kFlStages, *pvDone = vFull + kFlStages, *seenFull = pvDone + kFlStages;
+  uint64_t *sFull = seenFull + kFlSeen, *sEmpty = sFull + 2, *pFull = sEmpty + 2;
   const cr_qsa_args& a = P.a;
   const int t = threadIdx.x, w = t >> 5, l = t & 31;
-  const int tile = blockIdx.x, g = blockIdx.y, row0 = tile * P.RT;
+  // Newest tiles first: their lists are the longest while rows are dense, and the last wave should hold the short ones.
+  const int tile = (int)(gridDim.y - 1 - blockIdx.y), g = blockIdx.x, row0 = tile * P.RT;
   const int gqa = P.Hq / P.Hkv;
   const int cnt = P.count[tile];
   const int n_all = (cnt + kFlBlocks - 1) / kFlBlocks;   // steps of the tile; this CTA's share is [step0, step0 + n)
-  if (n_all == 0 || cnt > P.flash_max) return;           // a tile without rows, or one the row-wise kernels serve
+  if (n_all == 0 || !qsa_tile_shares(cnt, tile, P.RT, a.R, P.flash_max)) return;           // a tile without rows, or one the row-wise kernels serve
   const int step0 = (int)((long long)n_all * blockIdx.z / gridDim.z), n = (int)((long long)n_all * (blockIdx.z + 1) / gridDim.z) - step0;
   if ((umma::smem_u32(sm) & 1023u) != 0) {               // the swizzled tiles need their atoms on 1 KB boundaries
     if (t == 0) g_qsa_flash_status = 1;
@@ -199,12 +206,16 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
 
   if (t == 0) {
     for (int i = 0; i < kFlStages; ++i) {
-      umma::mbar_init(&kvFull[i], 2);                    // the two loader warps of the stage
-      umma::mbar_init(&pvDone[i], 1);                    // every MMA that read the stage has completed
+      umma::mbar_init(&kFull[i], 1);                     // the loader warp of the stage
+      umma::mbar_init(&vFull[i], 1);
+      umma::mbar_init(&kEmpty[i], 1);                    // S of the stage's step has completed
+      umma::mbar_init(&pvDone[i], 1);                    // P V of the stage's step has completed
     }
+    for (int i = 0; i < kFlSeen; ++i) umma::mbar_init(&seenFull[i], 1);
     for (int i = 0; i < 2; ++i) {
       umma::mbar_init(&sFull[i], 1);
-      umma::mbar_init(&pFull[i], kFlSoftmax);            // one arrival per softmax warp
+      umma::mbar_init(&sEmpty[i], kFlSoftmax / 2);       // one arrival per warp of the step's warpgroup
+      umma::mbar_init(&pFull[i], kFlSoftmax / 2);
     }
     umma::mbar_fence_init();
     dead = 0;
@@ -214,18 +225,37 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tm = tmem_slot;
+  // The gates of the tile's rows are asked into L2 now: the epilogue reads them with nothing else to do.
+  for (int i = t; i < min(P.RT, a.R - row0) * gqa * 8 && !P.partials; i += kFlThreads) {
+    const int m = i >> 3;
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(a.q + ((size_t)(row0 + m / gqa) * P.Hq + g * gqa + m % gqa) * 512 + 256 + (i & 7) * 32));
+  }
   // Query tile into tensor memory: M row m = (row m / gqa of the tile, head m % gqa of the group) = TMEM lane m, the
-  // 256 fp16 channels of the row as 128 columns (the A operand of S = Q K^T is read from tensor memory).
+  // 256 fp16 channels of the row as 128 columns (the A operand of S = Q K^T is read from tensor memory).  The rows come
+  // in coalesced and pass through the first K stage, swizzled so that a thread can read a row of its own.
+  {
+    constexpr int kRows = 128 * 32 / kFlThreads;           // rows per warp
+    uint4 x[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = w + i * (kFlThreads / 32), r = m / gqa, hq = m % gqa;
+      x[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < P.RT && row0 + r < a.R) x[i] = reinterpret_cast<const uint4*>(P.q_hi + ((size_t)(row0 + r) * P.Hq + g * gqa + hq) * 256)[l];
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int m = w + i * (kFlThreads / 32);
+      *reinterpret_cast<uint4*>(Ks + m * 512 + ((l ^ (m & 7)) << 4)) = x[i];
+    }
+  }
+  __syncthreads();
   if (w < 4) {
-    const int m = t, r = m / gqa, hq = m % gqa;
-    const bool have = r < P.RT && row0 + r < a.R;
-    const uint4* src = reinterpret_cast<const uint4*>(P.q_hi + ((size_t)(have ? row0 + r : 0) * P.Hq + g * gqa + hq) * 256);
 #pragma unroll 1
     for (int c8 = 0; c8 < 4; ++c8) {
       float v[32];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const uint4 x = have ? src[c8 * 8 + i] : make_uint4(0u, 0u, 0u, 0u);
+        const uint4 x = *reinterpret_cast<const uint4*>(Ks + t * 512 + (((c8 * 8 + i) ^ (t & 7)) << 4));
         v[4 * i] = __uint_as_float(x.x); v[4 * i + 1] = __uint_as_float(x.y); v[4 * i + 2] = __uint_as_float(x.z); v[4 * i + 3] = __uint_as_float(x.w);
       }
       umma::tmem_st32(umma::tmem_addr(tm, w, kColQ + 32 * c8), v);
@@ -246,55 +276,52 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
   };
 
   if (w == kFlIssuer) {
-    // ------------------------------------------------------------------ issuer
+    // ------------------------------------------------------------------ issuer of S = Q K^T
     if (l == 0) {
-      constexpr uint32_t idS = umma::idesc_f16(128, kFlKeys, false, false), idO = umma::idesc_f16(128, 256, false, true);
-      auto issue_S = [&](int j) {
-        const uint64_t dK = tma::desc_sw128(Ks + (j % kFlStages) * kFlKBytes, 16, 1024);
+      constexpr uint32_t idS = umma::idesc_f16(128, kFlKeys, false, false);
+      for (int j = 0; j < n; ++j) {
+        const int st = j % kFlStages;
+        wait(&kFull[st], (j / kFlStages) & 1);
+        if (j >= 2) wait(&sEmpty[j & 1], ((j >> 1) - 1) & 1);          // the softmax has read the accumulator's step before
+        if (gave_up || dead) break;                                    // no more tensor-core work once any wait has run out
+        umma::fence_after_sync();
+        const uint64_t dK = tma::desc_sw128(Ks + st * kFlKBytes, 16, 1024);
 #pragma unroll
         for (int ks = 0; ks < 16; ++ks)                  // 16 channels per MMA: 8 columns of Q, 32 bytes of every key's 128-byte row
           umma::mma_f16_ts(tm + kColS + 64 * (j & 1), tm + kColQ + 8 * ks, dK + (uint64_t)(((ks >> 2) * kFlGroup + (ks & 3) * 32) >> 4), idS, ks > 0);
         umma::commit(&sFull[j & 1]);
-      };
-      // Event loop: S of step ns (one step ahead of the softmax at most, its accumulator being free once the
-      // probabilities of step ns - 2 are written) as soon as its tiles have landed, O += P V of step np as soon as its
-      // probabilities are written; neither waits for the other's barrier.
-      auto ready = [&](uint64_t* bar, uint32_t parity) { return umma::mbar_try(umma::smem_u32(bar), parity); };
-      auto now_ns = [] { uint64_t v; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v)); return v; };
-      int ns = 0, np = 0, idle = 0;
-      uint64_t t_idle = 0;
-      while (np < n) {
-        if (ns < n && ns <= np + 1 && ready(&kvFull[ns % kFlStages], (ns / kFlStages) & 1)) {
-          umma::fence_after_sync();
-          issue_S(ns);
-          ++ns; idle = 0;
-        } else if (np < ns && ready(&pFull[np & 1], (np >> 1) & 1)) {
-          const int st = np % kFlStages;
-          umma::fence_after_sync();
-          const uint64_t dP = umma::smem_desc(Ps + (np & 1) * kFlPBytes, 128 * 16, 128);
-          const uint64_t dV = tma::desc_sw128(Vs + st * kFlKBytes, kFlGroup, 1024);        // MN-major: 64-channel groups, atoms of 8 keys
+        umma::commit(&kEmpty[st]);
+      }
+    }
+  } else if (w == kFlIssuer + 1) {
+    // ------------------------------------------------------------------ issuer of O += P V
+    if (l == 0) {
+      constexpr uint32_t idO = umma::idesc_f16(128, 256, false, true);
+      for (int j = 0; j < n; ++j) {
+        const int st = j % kFlStages;
+        wait(&vFull[st], (j / kFlStages) & 1);
+        wait(&pFull[j & 1], (j >> 1) & 1);
+        if (gave_up || dead) break;
+        umma::fence_after_sync();
+        const uint64_t dP = umma::smem_desc(Ps + (j & 1) * kFlPBytes, 128 * 16, 128);
+        const uint64_t dV = tma::desc_sw128(Vs + st * kFlKBytes, kFlGroup, 1024);        // MN-major: 64-channel groups, atoms of 8 keys
 #pragma unroll
-          for (int kk = 0; kk < kFlKeys / 16; ++kk)
-            umma::mma_f16_ss(tm + kColO, dP + (uint64_t)(kk * 2 * 128), dV + (uint64_t)(kk * 2048 >> 4), idO, (np > 0 || kk > 0) ? 1u : 0u);
-          umma::commit(&pvDone[st]);
-          ++np; idle = 0;
-        } else if ((++idle & 63) == 0) {                  // nothing ready: look at the clock now and then
-          const uint64_t t1 = now_ns();
-          if (idle == 64) t_idle = t1;
-          if (dead || t1 - t_idle > 2000000000ull) { dead = 1; g_qsa_flash_status = 1; break; }
-        }
+        for (int kk = 0; kk < kFlKeys / 16; ++kk)
+          umma::mma_f16_ss(tm + kColO, dP + (uint64_t)(kk * 2 * 128), dV + (uint64_t)(kk * 2048 >> 4), idO, (j > 0 || kk > 0) ? 1u : 0u);
+        umma::commit(&pvDone[st]);
       }
     }
   } else if (w >= kFlSoftmax) {
-    // ------------------------------------------------------------------ loaders: two warps per stage, half of its keys each
+    // ------------------------------------------------------------------ loaders: a warp per K stage and per V stage
     // One cp.async instruction brings one key's 512 bytes: four full lines, and eight lanes write the eight pieces of a
     // 128-byte swizzled row, so the writes are free of bank conflicts.
-    const int st = (w - kFlSoftmax) >> 1, lw = (w - kFlSoftmax) & 1;
-    const char* kc = reinterpret_cast<const char*>(a.c.k) + (size_t)g * 512 + l * 16;
-    const char* vc = reinterpret_cast<const char*>(a.c.v) + (size_t)g * 512 + l * 16;
+    const bool keys = w < kFlSoftmax + kFlStages;
+    const int st = (w - kFlSoftmax) % kFlStages;
+    const char* base = reinterpret_cast<const char*>(keys ? a.c.k : a.c.v) + (size_t)g * 512 + l * 16;
+    uint64_t *full = (keys ? kFull : vFull) + st, *empty = (keys ? kEmpty : pvDone) + st;
     const int2* lst = P.list + (size_t)tile * P.cap;
-    const size_t row_bytes = (size_t)P.Hkv * 512;
-    const unsigned kd = umma::smem_u32(Ks + st * kFlKBytes) + (l >> 3) * kFlGroup, vd = umma::smem_u32(Vs + st * kFlKBytes) + (l >> 3) * kFlGroup;
+    const size_t row_bytes = HKV ? (size_t)HKV * 512 : (size_t)P.Hkv * 512;
+    const unsigned slot = umma::smem_u32((keys ? Ks : Vs) + st * kFlKBytes) + (l >> 3) * kFlGroup + ((l & 7) << 4);
     auto entry = [&](int j) {                              // lane b (and b + 16): entry b of step j
       const int idx = (step0 + j) * kFlBlocks + (l & 15);
       return j < n && idx < cnt ? lst[idx] : make_int2(0, 0);
@@ -302,201 +329,203 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
     int2 e = entry(st);
     for (int j = st; j < n; j += kFlStages) {
       const int2 e_next = entry(j + kFlStages);            // in flight while the stage is waited for
-      if (j >= kFlStages) warp_wait(&pvDone[st], ((j - kFlStages) / kFlStages) & 1);   // the MMAs of the stage's last step are done
+      if (!keys) {
+        // Lane r + 16 h builds half h of the word pair of row r: bit 4 b + k is set when the row's bit of block b's mask is
+        // set and token k of the block is not in the row's future (only the open tail block of a row can hold such tokens).
+        // The V loaders do this, who would wait for the product before anyway: in a K loader it delayed every step.
+        const int row = l & 15, prow = a.pos0 + row0 + row;
+        const bool rowok = row < P.RT && row0 + row < a.R;
+        unsigned word = 0u;
+#pragma unroll 2
+        for (int b = 0; b < kFlBlocks / 2; ++b) {
+          const int src = (l >> 4) * (kFlBlocks / 2) + b;
+          const int blk = __shfl_sync(0xffffffffu, e.x, src), msk = __shfl_sync(0xffffffffu, e.y, src);
+          const int lim = prow - blk * 4;                             // tokens 0 .. lim of the block are visible
+          const unsigned nib = (rowok && ((msk >> row) & 1)) ? (lim >= 3 ? 0xFu : (lim < 0 ? 0u : (2u << lim) - 1u)) : 0u;
+          word |= nib << (4 * b);
+        }
+        seen_s[j % kFlSeen][row][l >> 4] = word;
+        __syncwarp();
+        if (l == 0) fl_mbar_arrive(&seenFull[j % kFlSeen]);
+      }
+      if (j >= kFlStages) warp_wait(empty, ((j - kFlStages) / kFlStages) & 1);
       if (dead) break;
+#pragma unroll 1
+      for (int b = 0; b < kFlBlocks; b += 2) {               // eight keys: one swizzle atom (small loop bodies: see the softmax)
+        const unsigned at = slot + b * 512;
 #pragma unroll
-      for (int b = 0; b < kFlBlocks / 2; ++b) {
-        const int pos0 = __shfl_sync(0xffffffffu, e.x, lw * (kFlBlocks / 2) + b) * 4;
-        const size_t src = (size_t)pos0 * row_bytes;
+        for (int h = 0; h < 2; ++h) {
+          const int blk = __shfl_sync(0xffffffffu, e.x, b + h), newest = last_pos - blk * 4;   // tokens 0 .. newest of the block are cached
+          const char* src = base + (size_t)blk * (4 * row_bytes);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int key = (lw * (kFlBlocks / 2) + b) * 4 + k;
-          const bool valid = pos0 + k <= last_pos;
-          const size_t at = valid ? src + k * row_bytes : 0;
-          const unsigned dst = key * 128 + (((l ^ key) & 7) << 4);
-          fl_cp_async16(kd + dst, kc + at, valid);
-          fl_cp_async16(vd + dst, vc + at, valid);
+          for (int k = 0; k < 4; ++k) fl_cp_async16((at ^ ((h * 4 + k) << 4)) + (h * 4 + k) * 128, k <= newest ? src + k * row_bytes : base, k <= newest);
         }
       }
       asm volatile("cp.async.commit_group;\n" ::);
-      if (lw == 0) {
-        // Lane r < 16 builds the word of row r: bit 4 b + k is set when the row's bit of block b's mask is set and token k
-        // of the block is not in the row's future (only the open tail block of a row can hold such tokens).  The softmax
-        // threads read one word per step.
-        const int prow = a.pos0 + row0 + (l & 15);
-        const bool rowok = (l & 15) < P.RT && row0 + (l & 15) < a.R;
-        unsigned lo_w = 0u, hi_w = 0u;
-#pragma unroll
-        for (int b = 0; b < kFlBlocks; ++b) {
-          const int blk = __shfl_sync(0xffffffffu, e.x, b), msk = __shfl_sync(0xffffffffu, e.y, b);
-          const int lim = prow - blk * 4;                             // tokens 0 .. lim of the block are visible
-          const unsigned nib = (rowok && ((msk >> (l & 15)) & 1)) ? (lim >= 3 ? 0xFu : (lim < 0 ? 0u : (2u << lim) - 1u)) : 0u;
-          if (b < 8) lo_w |= nib << (4 * b); else hi_w |= nib << (4 * (b - 8));
-        }
-        if (l < 16) { seen_s[st][l][0] = lo_w; seen_s[st][l][1] = hi_w; }
-      }
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
       umma::fence_async_smem();
       __syncwarp();
-      if (l == 0) fl_mbar_arrive(&kvFull[st]);
+      if (l == 0) fl_mbar_arrive(full);
       e = e_next;
     }
   } else {
-    // ------------------------------------------------------------------ softmax warps: thread = (TMEM lane m, half of the step's keys)
-    // Warps w and w + 4 share the lanes 32 (w % 4) .. +31; warp w takes the keys 0-31 of a step, warp w + 4 the keys 32-63.
-    const int m = t & 127, hf = t >> 7, r = m / gqa, hq = m % gqa;
-    const bool rowok = r < P.RT && row0 + r < a.R;
-    const int pair_bar = 1 + (w & 3);                                   // named barrier of the two warps of a lane quarter
-    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;\n" ::"r"(pair_bar) : "memory"); };
+    // ------------------------------------------------------------------ softmax warps: thread = TMEM lane m = (row, head)
+    // Warpgroup hf takes the steps hf, hf + 2, ...: while one exponentiates a step the other reads the next.  What passes
+    // from step to step is the reference maximum of the lane, through shared memory and a 64-thread named barrier per
+    // lane quarter and direction.
+    const int m = t & 127, hf = t >> 7, r = m / gqa;
+    const int give = 1 + 4 * hf + (w & 3), take = 1 + 4 * (hf ^ 1) + (w & 3);
     constexpr float kScale = 0.0625f * 1.4426950408889634f;            // logits / 16, in powers of two
-    float m_ref = -INFINITY, lsum = 0.f;
-    for (int j = 0; j < n; ++j) {
-      const int s = j & 1, st = j % kFlStages;
-      warp_wait(&kvFull[st], (j / kFlStages) & 1);                     // block ids and masks of the step are visible
-      const unsigned seen = r < 16 ? seen_s[st][r][hf] : 0u;             // which of this thread's 32 keys its row sees
+    float m_ref = -INFINITY, lsum = 0.f;                               // lsum: this warpgroup's steps, relative to m_ref
+    for (int j = hf; j < n; j += 2) {
+      const int s = j & 1;
+      warp_wait(&seenFull[j % kFlSeen], (j / kFlSeen) & 1);
+      const unsigned see0 = r < 16 ? seen_s[j % kFlSeen][r][0] : 0u, see1 = r < 16 ? seen_s[j % kFlSeen][r][1] : 0u;
       warp_wait(&sFull[s], (j >> 1) & 1);
       umma::fence_after_sync();
-      float sv[32];
-      umma::tmem_ld32(umma::tmem_addr(tm, w, kColS + 64 * s + 32 * hf), sv);
+      // S is read from tensor memory twice, 32 keys at a time in rolled loops: for the maximum, then for the exponentials.
+      // The roles of this kernel run different code on the same schedulers and evict each other's instructions; with 64
+      // keys unrolled (and unrolled loaders) a third of all stalls were instruction fetches.
       float tmax = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        sv[c] = (seen >> c) & 1u ? sv[c] * kScale : -INFINITY;
-        tmax = fmaxf(tmax, sv[c]);
-      }
-      half_max[s][hf][m] = tmax;                                        // (parity: the partner may still be reading the step before)
-      pair_sync();
-      tmax = fmaxf(tmax, half_max[s][hf ^ 1][m]);                       // the row's maximum over all 64 keys of the step
-      const bool move = tmax > m_ref + 8.f;                             // also the first visible key (m_ref = -inf)
-      if (__any_sync(0xffffffffu, move)) {
-        const float nref = move ? tmax : m_ref;
-        const float factor = move ? exp2f(m_ref - nref) : 1.f;          // 0 when nothing was accumulated yet
-        lsum *= factor;
-        m_ref = nref;
-        if (j > 0) {                                                    // O holds the steps before this one; each warp rescales half of it
-          warp_wait(&pvDone[(j - 1) % kFlStages], ((j - 1) / kFlStages) & 1);
-          umma::fence_after_sync();
 #pragma unroll 1
-          for (int c8 = 4 * hf; c8 < 4 * hf + 4; ++c8) {
-            float o[32];
-            umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+      for (int h = 0; h < 2; ++h) {
+        const unsigned see = h ? see1 : see0;
+        float sv[32], t1 = -INFINITY;
+        umma::tmem_ld32(umma::tmem_addr(tm, w, kColS + 64 * s + 32 * h), sv);
 #pragma unroll
-            for (int c = 0; c < 32; ++c) o[c] *= factor;
-            umma::tmem_st32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
-          }
-          umma::tmem_st_wait();
+        for (int c = 0; c < 32; c += 2) {
+          tmax = fmaxf(tmax, (see >> c) & 1u ? sv[c] : -INFINITY);
+          t1 = fmaxf(t1, (see >> (c + 1)) & 1u ? sv[c + 1] : -INFINITY);
         }
+        tmax = fmaxf(tmax, t1);
+      }
+      tmax *= kScale;
+      float ref = -INFINITY;                                            // the lane's reference after step j - 1
+      if (j > 0) {
+        asm volatile("bar.sync %0, 64;\n" ::"r"(take) : "memory");
+        ref = ref_s[s ^ 1][m];
+      }
+      const bool move = tmax > ref + 8.f;                               // also the first visible key (ref = -inf)
+      const float nref = move ? tmax : ref;
+      ref_s[s][m] = nref;
+      if (j + 1 < n) asm volatile("bar.arrive %0, 64;\n" ::"r"(give) : "memory");
+      if (m_ref != nref) lsum *= exp2f(m_ref - nref);                    // 0 when nothing was accumulated yet
+      m_ref = nref;
+      if (j > 0 && __any_sync(0xffffffffu, move)) {                      // O holds the steps before this one
+        const float factor = move ? exp2f(ref - nref) : 1.f;
+        warp_wait(&pvDone[(j - 1) % kFlStages], ((j - 1) / kFlStages) & 1);
+        umma::fence_after_sync();
+#pragma unroll 1
+        for (int c8 = 0; c8 < 8; ++c8) {
+          float o[32];
+          umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+#pragma unroll
+          for (int c = 0; c < 32; ++c) o[c] *= factor;
+          umma::tmem_st32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+        }
+        umma::tmem_st_wait();
       }
       if (j >= 2) warp_wait(&pvDone[(j - 2) % kFlStages], ((j - 2) / kFlStages) & 1);   // the MMAs of step j - 2 have read this P buffer
       unsigned char* pd = Ps + s * kFlPBytes;
+      const float sub = m_ref == -INFINITY ? 0.f : m_ref;               // nothing visible yet: every key drops out
       float add = 0.f;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const unsigned see = h ? see1 : see0;
+        float sv[32];
+        umma::tmem_ld32(umma::tmem_addr(tm, w, kColS + 64 * s + 32 * h), sv);
 #pragma unroll
-      for (int kc8 = 0; kc8 < 4; ++kc8) {
-        unsigned pk[4];
+        for (int kc8 = 0; kc8 < 4; ++kc8) {
+          unsigned pk[4];
 #pragma unroll
-        for (int q2 = 0; q2 < 4; ++q2) {
-          float p0, p1;                                                // 2^(-inf) = 0: keys the row does not see drop out
-          asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p0) : "f"(sv[kc8 * 8 + 2 * q2] - m_ref));
-          asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p1) : "f"(sv[kc8 * 8 + 2 * q2 + 1] - m_ref));
-          if (m_ref == -INFINITY) p0 = p1 = 0.f;                       // -inf - -inf: nothing visible yet
-          add += p0 + p1;
-          const __half2 h = __floats2half2_rn(p0, p1);
-          pk[q2] = *reinterpret_cast<const unsigned*>(&h);
+          for (int q2 = 0; q2 < 4; ++q2) {
+            float p[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const int c = kc8 * 8 + 2 * q2 + i;
+              asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p[i]) : "f"(fmaf(sv[c], kScale, -sub)));
+              p[i] = (see >> c) & 1u ? p[i] : 0.f;                     // keys the row does not see drop out
+            }
+            add += p[0] + p[1];
+            const __half2 hp = __floats2half2_rn(p[0], p[1]);
+            pk[q2] = *reinterpret_cast<const unsigned*>(&hp);
+          }
+          *reinterpret_cast<uint4*>(pd + ((size_t)(4 * h + kc8) * 128 + m) * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
-        *reinterpret_cast<uint4*>(pd + ((size_t)(4 * hf + kc8) * 128 + m) * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
+      umma::fence_before_sync();
+      __syncwarp();
+      if (l == 0) umma::mbar_arrive_relaxed(&sEmpty[s]);
       lsum += add;
       umma::fence_async_smem();
       umma::fence_before_sync();
       __syncwarp();
       if (l == 0) fl_mbar_arrive(&pFull[s]);
     }
-    // ---------------------------------------------------------------- epilogue: each warp of a pair writes half of the channels
-    float* half_sum = &half_max[n & 1][0][0];                           // the buffer the last step did not use
-    if (hf == 1) half_sum[m] = lsum;
-    pair_sync();
-    if (hf == 0) { lsum += half_sum[m]; half_sum[128 + m] = lsum; }
-    pair_sync();
-    lsum = half_sum[128 + m];
+    // ---------------------------------------------------------------- epilogue: each warpgroup writes half of the channels
+    auto both_sync = [] { asm volatile("bar.sync 9, 256;\n" ::: "memory"); };
+    both_sync();
+    float* sum_s = reinterpret_cast<float*>(&seen_s[0][0][0]);           // 128 floats: no step reads its words any more
+    const float last_ref = n > 0 ? ref_s[(n - 1) & 1][m] : -INFINITY;
+    if (m_ref != last_ref) lsum *= exp2f(m_ref - last_ref);
+    m_ref = last_ref;
+    if (hf == 1) sum_s[m] = lsum;
+    both_sync();
+    if (hf == 0) { sum_s[m] += lsum; ref_s[(n & 1)][m] = m_ref; }
     if (n > 0) warp_wait(&pvDone[(n - 1) % kFlStages], ((n - 1) / kFlStages) & 1);
     umma::fence_after_sync();
-    if (P.partials) {                                                   // the tile is split: leave (m, l, acc) of this share
-      float* rec = P.partials + (((size_t)blockIdx.z * a.R + row0 + r) * P.Hq + g * gqa + hq) * CR_QSA_PART;
-      if (rowok && hf == 0) *reinterpret_cast<float2*>(rec) = make_float2(m_ref * 0.6931471805599453f, lsum);
+    // O to shared memory (every tile and probability has been read), padded so that neither side has bank conflicts
 #pragma unroll 1
-      for (int c8 = 4 * hf; c8 < 4 * hf + 4; ++c8) {
-        float o[32];
-        umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
-        if (!rowok) continue;
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) *reinterpret_cast<float2*>(rec + 2 + 32 * c8 + c) = n > 0 ? make_float2(o[c], o[c + 1]) : make_float2(0.f, 0.f);
-      }
-    }
-    const bool ok = !P.partials && rowok && lsum > 0.f && !dead;
-    const float inv = ok ? 1.f / lsum : 0.f;
-    const int gr = row0 + r, h = g * gqa + hq;
-    const size_t W = (size_t)P.Hq * 256;
-    const float* gate = a.q + ((size_t)gr * P.Hq + h) * 512 + 256;
-#pragma unroll 1
-    for (int c8 = 4 * hf; c8 < 4 * hf + 4 && !P.partials; ++c8) {
+    for (int c8 = 4 * hf; c8 < 4 * hf + 4; ++c8) {
       float o[32];
-      umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);     // warp-collective: every lane takes part
-      if (!ok) continue;
+      umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+      float* dst = reinterpret_cast<float*>(sm) + m * kFlOutLd + 32 * c8;
 #pragma unroll
-      for (int c = 0; c < 32; ++c) o[c] *= inv;
-      if (a.context) {
-        float4* cx = reinterpret_cast<float4*>(a.context + ((size_t)gr * P.Hq + h) * 256 + 32 * c8);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) cx[c] = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-      }
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float4 gv = *reinterpret_cast<const float4*>(gate + 32 * c8 + 4 * c);
-        o[4 * c] *= sigmoidf_(gv.x); o[4 * c + 1] *= sigmoidf_(gv.y); o[4 * c + 2] *= sigmoidf_(gv.z); o[4 * c + 3] *= sigmoidf_(gv.w);
-      }
-      const size_t at = (size_t)gr * W + h * 256 + 32 * c8;
-      if (P.gated) {
-        float4* dst = reinterpret_cast<float4*>(P.gated + at);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) dst[c] = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-      } else if (P.fmt == CR_OUT_RAW_F32) {
-        float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + at);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) dst[c] = make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-      } else {
-        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.out) + at);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          unsigned pk[4];
-#pragma unroll
-          for (int q2 = 0; q2 < 4; ++q2) {
-            const __nv_bfloat162 b2 = __floats2bfloat162_rn(o[8 * c + 2 * q2], o[8 * c + 2 * q2 + 1]);
-            pk[q2] = *reinterpret_cast<const unsigned*>(&b2);
-          }
-          dst[c] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        }
-      }
+      for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
     }
   }
   umma::fence_before_sync();
   __syncthreads();
   if (w == kFlIssuer) umma::tmem_dealloc(tm, 512);
-}
-
-// The reference's out-projection input from gated fp32 rows: fp16(WHT128(RoundH(RoundH(o) * suh)) / sqrt(128))
-// (engine/layers/qsa_long.h:476-489).  grid (Hq, R), 64 threads: a warp per 128-channel group.
-__global__ void __launch_bounds__(64) qsa_out_transform_kernel(cr_qsa_args a, const float* gated, int Hq, const int* tile_count, int RT, int flash_max) {
-  const int h = blockIdx.x, r = blockIdx.y, half = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (tile_count[r / RT] > flash_max) return;             // a row of the row-wise kernels, which transform their own output
-  const int W = Hq * 256, c0 = h * 256 + half * 128 + lane * 4;
-  const float4 o = *reinterpret_cast<const float4*>(gated + (size_t)r * W + c0);
-  const __half* suh = reinterpret_cast<const __half*>(a.suh_o) + c0;
-  float v[4] = {round_h(round_h(o.x) * __half2float(suh[0])), round_h(round_h(o.y) * __half2float(suh[1])),
-                round_h(round_h(o.z) * __half2float(suh[2])), round_h(round_h(o.w) * __half2float(suh[3]))};
-  wht128(v);
-  __half* dst = reinterpret_cast<__half*>(a.out);
+  if (dead) return;
+  // Output rows, a warp per (row, head): lane l holds the channels 4 l .. + 3 and 128 + 4 l .. + 3.
+  const float* sums = reinterpret_cast<const float*>(&seen_s[0][0][0]);
+  constexpr int kWarps = kFlThreads / 32, kBatch = 4;      // gates of four rows are in flight before the first is used
+  const int live = min(P.RT, a.R - row0) * gqa;
+#pragma unroll 1
+  for (int m0 = w; m0 < live; m0 += kBatch * kWarps) {
+    float4 gate[kBatch][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) dst[out_index(r, c0 + i, W, a.pack_rows, a.pack_off)] = __float2half(v[i] * kHadNorm);
+    for (int k = 0; k < kBatch; ++k) {
+      const int m = m0 + k * kWarps;
+      if (m >= live || P.partials) break;
+      const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)(row0 + m / gqa) * P.Hq + g * gqa + m % gqa) * 512 + 256) + l;
+      gate[k][0] = src[0]; gate[k][1] = src[32];
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int m = m0 + k * kWarps, gr = row0 + m / gqa, h = g * gqa + m % gqa;
+      if (m >= live) break;
+      const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(sm) + m * kFlOutLd) + l;
+      float4 o[2] = {src[0], src[32]};
+      const float lsum = sums[m];
+      if (P.partials) {                                    // the tile is split: (m, l, acc) of this share
+        float* rec = P.partials + (((size_t)blockIdx.z * a.R + gr) * P.Hq + h) * CR_QSA_PART;
+        if (l == 0) *reinterpret_cast<float2*>(rec) = make_float2(ref_s[n & 1][m] * 0.6931471805599453f, lsum);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (n == 0) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          *reinterpret_cast<float2*>(rec + 2 + 128 * i + 4 * l) = make_float2(o[i].x, o[i].y);
+          *reinterpret_cast<float2*>(rec + 4 + 128 * i + 4 * l) = make_float2(o[i].z, o[i].w);
+        }
+        continue;
+      }
+      const float inv = 1.f / lsum;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        emit_group(a, P.Hq, gr, h, 128 * i + 4 * l, make_float4(o[i].x * inv, o[i].y * inv, o[i].z * inv, o[i].w * inv), gate[k][i], P.fmt);
+    }
+  }
 }
 
 cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int2* list, int* count, cudaStream_t stream) {
@@ -513,30 +542,27 @@ cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int
   return CR_OK;
 }
 
-// Attention of the rows of `a` over the union lists; `gated` (rows x Hq x 256 floats) is needed for CR_OUT_EXL3_WHT.
+// Attention of the rows of `a` over the union lists; splits > 1 leaves records in `partials` for qsa_merge_launch.
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* gated, float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream) {
+                           float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream) {
   static PerDeviceOnce configured;
   if (cr_status st = once_per_device(configured, [] {
-        CR_CUDA(cudaFuncSetAttribute(qsa_flash_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem));
+        CR_CUDA(cudaFuncSetAttribute(qsa_flash_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem));
+        CR_CUDA(cudaFuncSetAttribute(qsa_flash_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem));
         return CR_OK;
       })) return st;
   FlashParams P;
   P.a = a; P.q_hi = q_hi; P.list = list; P.count = count;
   P.RT = qsa_union_rows(g); P.cap = qsa_union_cap(P.RT);
   P.Hq = g->q_heads; P.Hkv = g->kv_heads; P.fmt = (int)fmt;
-  P.gated = fmt == CR_OUT_EXL3_WHT && splits == 1 ? gated : nullptr;
   P.partials = splits > 1 ? partials : nullptr;
   P.flash_max = flash_max;
-  CR_REQUIRE(fmt != CR_OUT_EXL3_WHT || gated, "qsa flash: the EXL3 output needs the gated fp32 scratch");
   const int tiles = (a.R + P.RT - 1) / P.RT;
   use_stream(stream);
-  qsa_flash_tc_kernel<<<dim3(tiles, g->kv_heads, splits), kFlThreads, kFlashSmem, stream>>>(P);
+  const dim3 grid(g->kv_heads, tiles, splits);
+  if (g->kv_heads == 2) qsa_flash_tc_kernel<2><<<grid, kFlThreads, kFlashSmem, stream>>>(P);
+  else qsa_flash_tc_kernel<0><<<grid, kFlThreads, kFlashSmem, stream>>>(P);
   CR_LAUNCH_CHECK("qsa_flash_tc_kernel");
-  if (P.gated) {
-    qsa_out_transform_kernel<<<dim3(g->q_heads, a.R), 64, 0, stream>>>(a, gated, g->q_heads, count, P.RT, flash_max);
-    CR_LAUNCH_CHECK("qsa_out_transform_kernel");
-  }
   return CR_OK;
 }
 

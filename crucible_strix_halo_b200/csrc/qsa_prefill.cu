@@ -13,10 +13,9 @@ int qsa_union_rows(const cr_geometry* g);
 int qsa_union_cap(int RT);
 cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int2* list, int* count, cudaStream_t stream);
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* gated, float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream);
+                           float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream);
 
-// Scratch of a part: [partial records of split tiles][gated fp32 rows for the EXL3 transform of the tiled kernel][union
-// lists, 2 ints per entry][union counts].  The list area is sized for tiles of 8 rows, the smallest tile.
+// Scratch of a part: [partial records of split tiles][union lists, 2 ints per entry][union counts].  The list area is sized for tiles of 8 rows, the smallest tile.
 //
 // A short part has fewer (tile, KV head) pairs than the GPU has SMs, and each walks its whole union list: its tiles are
 // then split along the list, as many ways as fill the SMs once, and a merge kernel combines the records.  117 rows at
@@ -32,12 +31,16 @@ static size_t partial_bytes(const cr_geometry* g, int rows) {
   const int all = rows * kMaxTileSplits;
   return (size_t)(all < kPartialRows ? all : kPartialRows) * g->q_heads * CR_QSA_PART * sizeof(float);
 }
-static size_t gated_bytes(const cr_geometry* g, int rows) { return (size_t)rows * g->q_heads * 256 * sizeof(float); }
 static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_cap(8) * 2; }
-// A tile goes to the tiled tensor-core kernel when its rows share enough blocks: at most this many union entries per
-// row of the tile (of 513 possible).  Measured on B200 at 262,144 context: a step of 16 entries costs the tiled kernel
-// about 3 us per (tile, KV head) when its gathers miss L2, the row-wise kernels about 69 SM-us per (row, KV head).
-constexpr int kFlashEntriesPerRow = 320;
+// A tile goes to the tiled tensor-core kernel when its rows share enough blocks: at most this many union entries per row
+// of the tile (of 513 possible).  Both kernels' times are linear in their work: 2,048 rows cost the tiled one 2.45 us per
+// entry and row (1,231 us at 502 unrelated entries), the row-wise one 855 us with 16 heads and 1,700 us with 24, where
+// its streams take two warps; the lines cross at 349 entries and above 513.
+constexpr int kFlashEntriesPerRow = 340;
+static int entries_per_row(const cr_geometry* g) { return g->q_heads / g->kv_heads <= 8 ? kFlashEntriesPerRow : 513; }
+// A part of so few rows is quicker row-wise whatever its rows share (20 rows at 20,000 positions: 24 us against 32 us of
+// lists, split tiles and merge).
+constexpr int kRowWiseRows = 24;
 
 static cr_status check_part(const cr_geometry* g, const cr_qsa_prefill_args* args, int skip, cr_out_format fmt, const char* who) {
   CR_REQUIRE(args, "%s: null args", who);
@@ -68,19 +71,18 @@ static cr_qsa_args output_rows(const cr_geometry* g, cr_qsa_args q, int skip, cr
 static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, const cr_qsa_args& q, int skip, cr_out_format fmt,
                         cudaStream_t stream) {
   char* scratch = (char*)args->scratch;
-  if (options().qsa_union_rows >= 0 && args->q_hi) {
-    float* gated = reinterpret_cast<float*>(scratch + partial_bytes(g, q.R));
-    int2* list = reinterpret_cast<int2*>(scratch + partial_bytes(g, q.R) + gated_bytes(g, q.R));
+  if (args->q_hi && (options().qsa_union_rows > 0 || (options().qsa_union_rows == 0 && q.R > kRowWiseRows))) {
+    int2* list = reinterpret_cast<int2*>(scratch + partial_bytes(g, q.R));
     int* count = reinterpret_cast<int*>(list + list_ints(q.R) / 2);
     const int RT = qsa_union_rows(g);
     const int splits = tile_splits(g, q.R);
-    const QsaTileSplit tiles = {count, RT, options().qsa_union_rows > 0 ? INT_MAX : kFlashEntriesPerRow * RT};   // an explicit tile size forces the tiled kernel
+    const QsaTileSplit tiles = {count, RT, options().qsa_union_rows > 0 ? 513 : entries_per_row(g)};   // an explicit tile size forces the tiled kernel
     if (cr_status s = qsa_union_build_launch(g, q, list, count, stream)) return s;
     if (cr_status s = qsa_flash_launch(g, q, reinterpret_cast<const __half*>(args->q_hi) + (size_t)skip * g->q_heads * 256, list, count,
-                                       gated, reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, stream)) return s;
+                                       reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, stream)) return s;
     if (splits > 1)
       if (cr_status s = qsa_merge_launch(g, q, splits, reinterpret_cast<const float*>(scratch), fmt, stream, &tiles)) return s;
-    if (tiles.max == INT_MAX) return CR_OK;
+    if (tiles.max >= 513) return CR_OK;                // no list is longer
     // the tiles with little sharing: row-wise split-KV attention (its CTAs of tiled rows exit at once)
     return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream, &tiles);
   }
@@ -90,7 +92,7 @@ static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, c
 
 extern "C" size_t cr_qsa_prefill_scratch_bytes(const cr_geometry* g, int rows) {
   if (!g || rows < 1) return 0;
-  return cr::partial_bytes(g, rows) + cr::gated_bytes(g, rows) + cr::list_ints(rows) * sizeof(int) + (size_t)((rows + 7) / 8) * sizeof(int);
+  return cr::partial_bytes(g, rows) + cr::list_ints(rows) * sizeof(int) + (size_t)((rows + 7) / 8) * sizeof(int);
 }
 
 extern "C" size_t cr_qsa_union_list_ints(const cr_geometry* g, int rows) {

@@ -40,16 +40,18 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
-// One poll: true once the phase with the given parity has completed (the hardware may suspend the thread for
-// a short, system-dependent time while the phase is pending).
+// One poll: true once the phase with the given parity has completed.  While the phase is pending the hardware may suspend
+// the thread for up to the hinted time and wakes it when the phase completes: waiting threads then take no issue slots
+// and no shared-memory bandwidth from the warps they wait for.
+constexpr uint32_t kSuspendNs = 20000;
 __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}\n"
       : "=r"(done)
-      : "r"(addr), "r"(parity)
+      : "r"(addr), "r"(parity), "r"(kSuspendNs)
       : "memory");
   return done != 0;
 }
@@ -61,10 +63,10 @@ __device__ __forceinline__ bool mbar_try_relaxed(uint32_t addr, uint32_t parity)
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.relaxed.cta.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.relaxed.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}\n"
       : "=r"(done)
-      : "r"(addr), "r"(parity)
+      : "r"(addr), "r"(parity), "r"(kSuspendNs)
       : "memory");
   return done != 0;
 }
@@ -79,17 +81,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 // Waits with a bound in time: gives up after max_ns nanoseconds (or as soon as *abort is set by another
-// thread that gave up) and returns false.  The clock is read only when the first poll fails.
+// thread that gave up) and returns false.  The clock is not read before a few polls have failed.
 template <bool RELAXED = false>
 __device__ __forceinline__ bool mbar_wait_timed(uint64_t* bar, uint32_t parity, const volatile int* abort, uint64_t max_ns = 2000000000ull) {
   const uint32_t addr = smem_u32(bar);
   auto poll = [&]() { return RELAXED ? mbar_try_relaxed(addr, parity) : mbar_try(addr, parity); };
-  if (poll()) return true;
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i)
+    if (poll()) return true;
   uint64_t t0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   for (;;) {
 #pragma unroll 1
-    for (int i = 0; i < 64; ++i)   // the clock and the abort flag are slow to read: look at them rarely
+    for (int i = 0; i < 8; ++i)   // the clock and the abort flag are slow to read: look at them rarely
       if (poll()) return true;
     uint64_t t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
