@@ -41,18 +41,18 @@ __device__ __forceinline__ void st_half4(uint16_t* p, const float4 v) {
   else { p[0] = (uint16_t)u0; p[1] = (uint16_t)(u0 >> 16); p[2] = (uint16_t)u1; p[3] = (uint16_t)(u1 >> 16); }
 }
 
-// A head of 128 (N4 = 1) or 256 (N4 = 2) values spread over a warp: lane l holds elements 4 l .. 4 l + 3 (and 128 + 4 l ..).
+// A head of 256 values spread over a warp: lane l holds elements 4 l .. 4 l + 3 and 128 + 4 l .. + 3.
 // CN-RMSNorm, then split-half RoPE of the first 64: lanes 0-7 hold the first half of the pairs, lanes 8-15 the second.
 // c4 / s4: cosines and sines of the frequencies 4 (l % 8) .. + 3.
-template <bool VEC, int N4>
-__device__ __forceinline__ void norm_rope(float4 (&x)[N4], const float* w1, const float4 c4, const float4 s4) {
+template <bool VEC>
+__device__ __forceinline__ void norm_rope(float4 (&x)[2], const float* w1, const float4 c4, const float4 s4) {
   const int l = threadIdx.x & 31;
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < N4; ++i) ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
-  const float rs = rsqrtf(warp_sum(ss) / (128.f * N4) + kEps);
+  for (int i = 0; i < 2; ++i) ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+  const float rs = rsqrtf(warp_sum(ss) / 256.f + kEps);
 #pragma unroll
-  for (int i = 0; i < N4; ++i) {
+  for (int i = 0; i < 2; ++i) {
     const float4 w = ld4<VEC>(w1 + 128 * i + 4 * l);
     x[i] = make_float4(x[i].x * rs * w.x, x[i].y * rs * w.y, x[i].z * rs * w.z, x[i].w * rs * w.w);
   }
@@ -64,6 +64,22 @@ __device__ __forceinline__ void norm_rope(float4 (&x)[N4], const float* w1, cons
     x[0] = make_float4(x[0].x * c4.x + sg * o.x * s4.x, x[0].y * c4.y + sg * o.y * s4.y, x[0].z * c4.z + sg * o.z * s4.z,
                        x[0].w * c4.w + sg * o.w * s4.w);
   }
+}
+
+// A head of the indexer (128 values), strided over a warp: lane l holds the elements l, 32 + l, 64 + l, 96 + l.  The sum of
+// squares is the left-to-right sum of the four 32-element butterflies: selections hang on the last bit of these rows, so
+// the order of the additions stays what it is.  cj / sj: cosine and sine of frequency l.
+__device__ __forceinline__ void norm_rope_idx(float (&x)[4], const float* w1, float cj, float sj) {
+  const int l = threadIdx.x & 31;
+  float t[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) t[i] = warp_sum(x[i] * x[i]);
+  const float rs = rsqrtf((((t[0] + t[1]) + t[2]) + t[3]) / 128.f + kEps);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = x[i] * rs * w1[32 * i + l];
+  const float a = x[0], b = x[1];
+  x[0] = a * cj - b * sj;
+  x[1] = b * cj + a * sj;
 }
 
 // Rows at which a call keeps only the newest raw keys of a ring (a longer call writes the ring once, at its end).
@@ -83,24 +99,21 @@ __device__ __forceinline__ bool raw_after_pool(const cr_qsa_args& a, int r) {
 template <bool VEC>
 __device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
   const int l = threadIdx.x & 31;
-  float4 k4[4];
+  float k[4][4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const int pos = b * 4 + t;
-    k4[t] = ld4<VEC>(pos >= a.pos0 ? a.idx + (size_t)(pos - a.pos0) * 640 + 512 + 4 * l : a.c.ik_raw + raw_offset(a.c.raw_slots, pos, 4 * l));
+    const float* src = pos >= a.pos0 ? a.idx + (size_t)(pos - a.pos0) * 640 + 512 + l : a.c.ik_raw + raw_offset(a.c.raw_slots, pos, l);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) k[t][i] = src[32 * i];
   }
-  float cj, sj;
+  float cj, sj, x[4];
   rope_terms(a, l, b * 4, cj, sj);
-  float4 c4, s4;
-  const int f0 = 4 * (l & 7);
-  c4.x = __shfl_sync(0xffffffffu, cj, f0); c4.y = __shfl_sync(0xffffffffu, cj, f0 + 1); c4.z = __shfl_sync(0xffffffffu, cj, f0 + 2); c4.w = __shfl_sync(0xffffffffu, cj, f0 + 3);
-  s4.x = __shfl_sync(0xffffffffu, sj, f0); s4.y = __shfl_sync(0xffffffffu, sj, f0 + 1); s4.z = __shfl_sync(0xffffffffu, sj, f0 + 2); s4.w = __shfl_sync(0xffffffffu, sj, f0 + 3);
-  float4 x[1];
-  x[0] = make_float4(round_h((((0.f + k4[0].x) + k4[1].x) + k4[2].x + k4[3].x) * 0.25f), round_h((((0.f + k4[0].y) + k4[1].y) + k4[2].y + k4[3].y) * 0.25f),
-                     round_h((((0.f + k4[0].z) + k4[1].z) + k4[2].z + k4[3].z) * 0.25f), round_h((((0.f + k4[0].w) + k4[1].w) + k4[2].w + k4[3].w) * 0.25f));
-  norm_rope<VEC>(x, a.ik_norm1, c4, s4);
-  float* dst = a.c.ik_pool + pool_offset(b, 4 * l);
-  dst[0] = x[0].x; dst[32] = x[0].y; dst[64] = x[0].z; dst[96] = x[0].w;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = round_h((((k[0][i] + k[1][i]) + k[2][i]) + k[3][i]) * 0.25f);
+  norm_rope_idx(x, a.ik_norm1, cj, sj);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a.c.ik_pool[pool_offset(b, 32 * i + l)] = x[i];
   if (b == a.pos0 / 4 && a.c.raw_slots != 0) {            // the ring rows that had to wait for the reads above
     __syncwarp();
     for (int r = max(0, a.R - a.c.raw_slots); r < a.R; ++r)
@@ -142,8 +155,8 @@ __global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ Q
     else if (u < Hq + 2 * Hkv + 5) { src = u < Hq + 2 * Hkv + 4 || !queries_only ? a.idx + (size_t)r * 640 + (u - Hq - 2 * Hkv) * 128 : nullptr; wide = false; }
     x[i][0] = x[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (src) {
-      x[i][0] = ld4<VEC>(src + 4 * l);
-      if (wide) x[i][1] = ld4<VEC>(src + 128 + 4 * l);
+      if (wide) { x[i][0] = ld4<VEC>(src + 4 * l); x[i][1] = ld4<VEC>(src + 128 + 4 * l); }
+      else x[i][0] = make_float4(src[l], src[32 + l], src[64 + l], src[96 + l]);
     }
   }
   if (w == 0) {
@@ -174,14 +187,17 @@ __global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ Q
       st_half4<VEC>(h, x[i][0]);
       st_half4<VEC>(h + 128, x[i][1]);
     } else if (u < Hq + 2 * Hkv + 4) {
-      float4 y[1] = {x[i][0]};
-      norm_rope<VEC>(y, a.iq_norm1, c4, s4);
-      st4<VEC>(a.idx + (size_t)r * 640 + (u - Hq - 2 * Hkv) * 128 + 4 * l, y[0]);
+      float y[4] = {x[i][0].x, x[i][0].y, x[i][0].z, x[i][0].w};
+      norm_rope_idx(y, a.iq_norm1, cs[l], sn[l]);
+      float* dst = a.idx + (size_t)r * 640 + (u - Hq - 2 * Hkv) * 128 + l;
+      dst[0] = y[0]; dst[32] = y[1]; dst[64] = y[2]; dst[96] = y[3];
     } else if (queries_only) {
       continue;
     } else if (u == Hq + 2 * Hkv + 4) {
-      if (raw_kept(a, r) && !raw_after_pool(a, r))
-        st4<VEC>(a.c.ik_raw + raw_offset(a.c.raw_slots, p, 4 * l), x[i][0]);
+      if (raw_kept(a, r) && !raw_after_pool(a, r)) {
+        float* dst = a.c.ik_raw + raw_offset(a.c.raw_slots, p, l);
+        dst[0] = x[i][0].x; dst[32] = x[i][0].y; dst[64] = x[i][0].z; dst[96] = x[i][0].w;
+      }
     } else if (u == Hq + 2 * Hkv + 5) {
       if (p % 4 == 3) pool_block<VEC>(a, p / 4);
     }
