@@ -18,9 +18,10 @@
 // Bound: the gather.  Random 512-byte rows of a 512 MB cache arrive at 8.5 TB/s (16 MB: 20 TB/s).  The form before this
 // one (a CTA per (row, KV head, split), heads as M rows, Q re-read from shared memory for every tile, partials merged by
 // a second kernel) was held by shared-memory reads and barriers: 2,048 rows at 262,144 positions took 1,875 us plus
-// 180 us of merge, 849 us now (10.1 TB/s of gathers: the rows walk
-// their ascending positions side by side, so the rows in flight share a region of the cache that L2 holds); 72 verify
-// rows at 131,072 105 + 12 us, 53 us now; four decode rows at 262,144 17 + 9 us, 14 us now.
+// 180 us of merge, 744 us now (11.6 TB/s of gathers: the rows walk their ascending positions side by side, so the rows in
+// flight share a region of the cache that L2 holds; from L2 alone 666 us, where every byte's way into and out of shared
+// memory takes three quarters of its bandwidth); 72 verify rows at 131,072 105 + 12 us, 53 us now; four decode rows at
+// 262,144 17 + 9 us, 13 us now.
 #include <climits>
 #include <cooperative_groups.h>
 #include "qsa.cuh"
@@ -46,7 +47,10 @@ struct AttnShape {
   int cluster;                                 // CTAs per unit (spu = all streams then)
 };
 
-__device__ __forceinline__ void attn_cp16(unsigned dst, const void* src, bool valid) {
+__device__ __forceinline__ void attn_cp16(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+}
+__device__ __forceinline__ void attn_cp16_or_zero(unsigned dst, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
 }
@@ -79,11 +83,12 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// grid (cluster x ceil(Rmax * Hkv / units per CTA), 1, spans).
-template <int NG>
+// grid (cluster x ceil(Rmax * Hkv / units per CTA), 1, spans).  HKV: the cache's KV heads where they are two (row pitches
+// become constants), else 0.
+template <int NG, int HKV>
 __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __grid_constant__ QsaParams P, const AttnShape shape, float* partials,
                                                                        int p0, int p1, int fmt) {
-  extern __shared__ __align__(128) unsigned char ring_raw[];
+  extern __shared__ __align__(1024) unsigned char ring_raw[];
   __shared__ float ml_s[kMaxWarps][8][2];              // (m, l) of every stream's heads
   __shared__ float cta_ml[16][2];                      // of the CTA's merged unit, read by the cluster
   pdl_release();
@@ -136,25 +141,37 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
       return e < e_hi ? (ns < 0 || e >= full ? (e >= full ? nb : e) : sel[e]) : -1;
     };
     int ids = load_ids(0), ids_next = load_ids(1);
-    const size_t row_bytes = (size_t)P.Hkv * 512;
+    const size_t row_bytes = HKV ? (size_t)HKV * 512 : (size_t)P.Hkv * 512;
     const char* kc = reinterpret_cast<const char*>(a.c.k) + (size_t)g * 512 + l * 16;
     const char* vc = reinterpret_cast<const char*>(a.c.v) + (size_t)g * 512 + l * 16;
-    const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
+    const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring), ring_l = ring_s + l * 16;
     const int lo_pos = max(p0, 0), hi_pos = min(p, p1 - 1);          // visible positions
+    // Tiles before this one (of the stream's) hold complete selected blocks inside the window: nothing to mask.
+    const int whole_tiles = p0 <= 0 && p1 > p ? (full - e0) >> 2 : 0;
     int blk[4];                                          // blocks of the tile whose K half was issued last
-    auto issue = [&](const char* base, int half) {       // the 16 rows of the tile in blk, into slot half % kSlots
-      const unsigned slot = ring_s + (half % kSlots) * kHalfBytes;
+    auto issue = [&](const char* base, int half, bool whole) {       // the 16 rows of the tile in blk, into slot half % kSlots
+      const unsigned slot = ring_l + (half % kSlots) * kHalfBytes;    // slots are 512-byte aligned: the swizzle is one XOR
 #pragma unroll
-      for (int i = 0; i < kTok / NG; ++i) {
-        const int k = hg * (kTok / NG) + i;
-        const int b = NG == 1 ? blk[i >> 2] : (hg == 0 ? blk[i >> 2] : blk[2 + (i >> 2)]);
-        const int pos = 4 * b + (k & 3);
-        const bool ok = b >= 0 && pos >= lo_pos && pos <= hi_pos;
-        attn_cp16(slot + k * 512 + ((l ^ (k & 7)) << 4), base + (ok ? (size_t)pos * row_bytes : 0), ok);
+      for (int i4 = 0; i4 < kTok / 4 / NG; ++i4) {
+        const int b = NG == 1 ? blk[i4] : (hg == 0 ? blk[i4] : blk[2 + i4]);
+        const char* src = base + (size_t)(unsigned)b * (4 * row_bytes);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int kk = 4 * i4 + i;                     // row of this warp's share: 8 hg + kk where two warps share a stream
+          const unsigned dst = (slot ^ ((kk & 7) << 4)) + (NG == 1 ? kk : 8 * hg + kk) * 512;
+          if (whole) {
+            attn_cp16(dst, src + i * row_bytes);
+          } else {
+            const int pos = 4 * b + i;
+            const bool ok = b >= 0 && pos >= lo_pos && pos <= hi_pos;
+            attn_cp16_or_zero(dst, ok ? src + i * row_bytes : base, ok);
+          }
+        }
       }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
-    auto visible = [&]() {                               // bit k: position k of the tile in blk is attended
+    auto visible = [&](bool whole) {                     // bit k: position k of the tile in blk is attended
+      if (whole) return 0xFFFFu;
       const int b = l < kTok ? (l < 8 ? (l < 4 ? blk[0] : blk[1]) : (l < 12 ? blk[2] : blk[3])) : -1;
       const int pos = 4 * b + (l & 3);
       return __ballot_sync(0xffffffffu, b >= 0 && pos >= lo_pos && pos <= hi_pos);
@@ -169,11 +186,11 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
       else asm volatile("bar.sync %0, 64;\n" ::"r"(1 + stream) : "memory");
     };
     unsigned see = 0, see_next = 0;
-    if (tiles > 0) { take_blocks(0); see = visible(); issue(kc, 0); }
+    if (tiles > 0) { take_blocks(0); see = visible(0 < whole_tiles); issue(kc, 0, 0 < whole_tiles); }
     commit();
-    if (tiles > 0) issue(vc, 1);
+    if (tiles > 0) issue(vc, 1, 0 < whole_tiles);
     commit();
-    if (tiles > 1) { take_blocks(1); see_next = visible(); issue(kc, 2); }
+    if (tiles > 1) { take_blocks(1); see_next = visible(1 < whole_tiles); issue(kc, 2, 1 < whole_tiles); }
     commit();
     // Query heads of the group as column fragments, fp16 head and remainder, while the first halves are in flight.
     unsigned qh[16][2], ql[16][2];
@@ -192,7 +209,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     constexpr float kScale = 0.0625f * 1.4426950408889634f;           // logits / 16, in powers of two
     // this lane's ldmatrix rows: K: matrices (positions 0-7 | 8-15) x (first | second 8 channels); V: the transpose of that
     const int mi = l >> 3, k_row = (l & 7) + (mi & 1) * 8, v_row = (l & 7) + (mi >> 1) * 8;
-    const unsigned k_addr = k_row * 512, v_addr = v_row * 512;
+    const unsigned k_addr = k_row * 512 + (((mi >> 1) ^ (l & 7)) << 4), v_addr = v_row * 512 + (((mi & 1) ^ (l & 7)) << 4);   // ^ 32 per 16 channels
     for (int i = 0; i < tiles; ++i) {
       asm volatile("cp.async.wait_group 2;\n" ::: "memory");
       pair_sync();
@@ -201,12 +218,12 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
 #pragma unroll
       for (int ks = 0; ks < 16; ++ks) {
         unsigned ka[4];
-        ldsm_x4(ka, ks_base + (((2 * ks + (mi >> 1)) ^ (l & 7)) << 4));
+        ldsm_x4(ka, ks_base ^ (ks << 5));
         mma_f16(s, ka, qh[ks][0], qh[ks][1]);
         mma_f16(s2, ka, ql[ks][0], ql[ks][1]);
       }
       pair_sync();                                       // the K half is free
-      if (i + 1 < tiles) issue(vc, 2 * i + 3);           // blk still holds tile i + 1
+      if (i + 1 < tiles) issue(vc, 2 * i + 3, i + 1 < whole_tiles);   // blk still holds tile i + 1
       commit();
       const bool v0 = (see >> g8) & 1u, v1 = (see >> (g8 + 8)) & 1u;
 #pragma unroll
@@ -217,7 +234,9 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
         mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], o));
         mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], o));
       }
-      if (__any_sync(0xffffffffu, mx[0] > m_run[0] || mx[1] > m_run[1])) {
+      // The reference maximum moves only when a logit exceeds it by more than 2^8: O is rescaled once or twice per stream, and
+      // probabilities up to 256 lose nothing in their fp16 head and remainder.
+      if (__any_sync(0xffffffffu, mx[0] > m_run[0] + 8.f || mx[1] > m_run[1] + 8.f)) {
         float corr[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -245,13 +264,13 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
 #pragma unroll
       for (int mt = 0; mt < 16; ++mt) {
         unsigned va[4];
-        ldsm_x4_trans(va, vs_base + (((2 * mt + (mi & 1)) ^ (l & 7)) << 4));
+        ldsm_x4_trans(va, vs_base ^ (mt << 5));
         mma_f16(O[mt], va, ph[0], ph[1]);
         mma_f16(O[mt], va, pl[0], pl[1]);
       }
       pair_sync();                                       // the V half is free
       see = see_next;
-      if (i + 2 < tiles) { take_blocks(i + 2); see_next = visible(); issue(kc, 2 * i + 4); }
+      if (i + 2 < tiles) { take_blocks(i + 2); see_next = visible(i + 2 < whole_tiles); issue(kc, 2 * i + 4, i + 2 < whole_tiles); }
       commit();
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -407,12 +426,12 @@ static AttnShape attn_shape(int streams, long long units, int tiles, int sms) {
   return best;
 }
 
-template <int NG>
+template <int NG, int HKV>
 static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long units, int tiles, float* partials, int p0, int p1, int fmt, cudaStream_t stream) {
   static PerDeviceOnce configured;
   constexpr size_t smem = kAttnSmem<NG> + 12 * 256 * sizeof(float);   // + the merged unit of a cluster's CTA
   if (cr_status st = once_per_device(configured, [] {
-        CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG, HKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         return CR_OK;
       })) return st;
   const AttnShape shape = attn_shape(kStreams<NG>, units, tiles, sm_count());
@@ -430,7 +449,7 @@ static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long un
     attr[na].val.clusterDim.x = shape.cluster; attr[na].val.clusterDim.y = 1; attr[na++].val.clusterDim.z = 1;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
-  CR_CUDA(cudaLaunchKernelEx(&cfg, qsa_attn_kernel<NG>, P, shape, partials, p0, p1, fmt));
+  CR_CUDA(cudaLaunchKernelEx(&cfg, qsa_attn_kernel<NG, HKV>, P, shape, partials, p0, p1, fmt));
   CR_LAUNCH_CHECK("qsa_attn_kernel");
   return CR_OK;
 }
@@ -452,8 +471,9 @@ cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
       last = max(last, spans[s0 + s].pos0 + spans[s0 + s].R - 1);
     }
     const int most = (min(last / 4 + 1, CR_SEL_BLOCKS + 1) + 3) / 4, Rmax = qsa_max_rows(spans + s0, n);
-    const cr_status st = g->q_heads / g->kv_heads <= 8 ? attn_launch_t<1>(P, Rmax, n, units, most, partials, p0, p1, (int)fmt, stream)
-                                                       : attn_launch_t<2>(P, Rmax, n, units, most, partials, p0, p1, (int)fmt, stream);
+    const bool one = g->q_heads / g->kv_heads <= 8, two_kv = g->kv_heads == 2;
+    auto launch = one ? (two_kv ? attn_launch_t<1, 2> : attn_launch_t<1, 0>) : (two_kv ? attn_launch_t<2, 2> : attn_launch_t<2, 0>);
+    const cr_status st = launch(P, Rmax, n, units, most, partials, p0, p1, (int)fmt, stream);
     if (st) return st;
     for (int s = 0; s < n; ++s) row_base += spans[s0 + s].R;
   }

@@ -33,14 +33,15 @@ static size_t partial_bytes(const cr_geometry* g, int rows) {
 }
 static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_cap(8) * 2; }
 // A tile goes to the tiled tensor-core kernel when its rows share enough blocks: at most this many union entries per row
-// of the tile (of 513 possible).  Both kernels' times are linear in their work: 2,048 rows cost the tiled one 2.45 us per
-// entry and row (1,231 us at 502 unrelated entries), the row-wise one 855 us with 16 heads and 1,700 us with 24, where
-// its streams take two warps; the lines cross at 349 entries and above 513.
-constexpr int kFlashEntriesPerRow = 340;
-static int entries_per_row(const cr_geometry* g) { return g->q_heads / g->kv_heads <= 8 ? kFlashEntriesPerRow : 513; }
-// A part of so few rows is quicker row-wise whatever its rows share (20 rows at 20,000 positions: 24 us against 32 us of
-// lists, split tiles and merge).
-constexpr int kRowWiseRows = 24;
+// of the tile (of 513 possible).  Both kernels' times are linear in their work: 2,048 rows cost the tiled one 2.5 us per
+// entry and row (1,250 us at 502 unrelated entries), the row-wise one 744 us with 16 heads and 1,500 us with 24, where its
+// streams take two warps; the lines cross at 298 entries and above 513.
+constexpr int kFlashEntriesPerRow = 298;
+static bool one_warp_streams(const cr_geometry* g) { return g->q_heads / g->kv_heads <= 8; }
+static int entries_per_row(const cr_geometry* g) { return one_warp_streams(g) ? kFlashEntriesPerRow : 513; }
+// A part of so few rows is quicker row-wise whatever its rows share: 40 rows of 16 heads at 20,000 positions take 29 us
+// against 32 us of lists, split tiles and merge, 20 rows of 24 heads 34 us against 30 us.
+static int row_wise_rows(const cr_geometry* g) { return one_warp_streams(g) ? 40 : 16; }
 
 static cr_status check_part(const cr_geometry* g, const cr_qsa_prefill_args* args, int skip, cr_out_format fmt, const char* who) {
   CR_REQUIRE(args, "%s: null args", who);
@@ -71,7 +72,7 @@ static cr_qsa_args output_rows(const cr_geometry* g, cr_qsa_args q, int skip, cr
 static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, const cr_qsa_args& q, int skip, cr_out_format fmt,
                         cudaStream_t stream) {
   char* scratch = (char*)args->scratch;
-  if (args->q_hi && (options().qsa_union_rows > 0 || (options().qsa_union_rows == 0 && q.R > kRowWiseRows))) {
+  if (args->q_hi && (options().qsa_union_rows > 0 || (options().qsa_union_rows == 0 && q.R > row_wise_rows(g)))) {
     int2* list = reinterpret_cast<int2*>(scratch + partial_bytes(g, q.R));
     int* count = reinterpret_cast<int*>(list + list_ints(q.R) / 2);
     const int RT = qsa_union_rows(g);
