@@ -1,268 +1,344 @@
 // Gated DeltaNet decode / speculative-verify step for sm_100a.
 //
-// One thread-block CLUSTER of 4 CTAs per (value head, span): CTA c of the cluster owns value columns
-// [32c, 32c+32) of the head's 128x128 fp32 state (16 KB, 16 registers per thread), because the delta rule
-// never mixes value columns.  The only cross-column quantity, the RMS of the 128-wide readout, is
-// exchanged through distributed shared memory once per call.  The state slice is streamed with 128-bit loads
-// (each warp load covers 4 key rows x 128 B) while the row prologue (conv + SiLU, L2 norms, a/b GEMV) runs.
+// One CTA of 8 warps per (value head, span).  A warp owns 16 value columns of the head's 128 x 128 fp32 state, because the
+// delta rule never mixes value columns; a lane holds 4 columns x 16 keys of it in registers (as pairs of keys, for the
+// two-lane fp32 instructions), so a row of the pass costs a warp eight 128-bit reads of shared memory, eleven shuffles and no
+// barrier, and the rows (replayed ones first) run back to back.  Everything the pass reads is asked for at the start: raw
+// rows with their halo and the pending rows into shared memory, the state into L2 and, behind the a / b dot products, into
+// registers, the gate rows during the recurrence.
 //
 // Semantics follow GdnKernel (engine/layers/ops.h:252-401): replay of pending rows, per-row update with the
 // readout from the updated state, state stored after row commit-1, rows >= commit recorded as
 // (khat, v, decay, beta), gated RMSNorm readout, raw-row ring update.
-#include <cooperative_groups.h>
+//
+// Bound: latency of a few dependent memory round trips; with many rows the update chain.  Reads of k and q from shared memory
+// set the pace of every form with less state per lane: 8 sessions x (9 rows + 4 replayed) took 94 us with a quarter of the
+// columns per CTA and two barriers a row, 52 us with 8 columns per warp and none, 32 us now; 4 sessions x 1 row took 12.3 us,
+// 10.5 us now (one session 6.8, now 9: 32 CTAs pull 64 KB of state each).
 #include "common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace cr {
 
 constexpr int kStepRows = CR_MAX_STEP_ROWS;
+constexpr int kStepThreads = 256, kStepWarps = kStepThreads / 32;
+constexpr int kReplayChunk = 16;                       // pending rows staged at a time
+constexpr int kRawCols = 384;                          // channels of a head: 128 q, 128 k, 128 v
 
 struct GdnStepParams {
   cr_gdn_args span[kMaxSpans];
   int Hv, Hk, hidden, pend_rows, fmt;
+  int rows, replay;                                    // most of any span: the shared-memory layout
 };
 
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256)
-gdn_step_kernel(const __grid_constant__ GdnStepParams P) {
-  const cr_gdn_args& a = P.span[blockIdx.y];
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int h = blockIdx.x >> 2;
-  const int t = threadIdx.x, w = t >> 5, l = t & 31;
-  const int rep = P.Hv / P.Hk, kh = h / rep;
-  const int KW = P.Hk * 128, VW = P.Hv * 128, C = 2 * KW + VW;
-  const int colbase = rank * 32, c4 = (l & 7) * 4;
-  const int R = a.R;
+// Floats of dynamic shared memory: raw rows with halo, q, k and v rows (the readout replaces v), staged pending rows.
+__host__ __device__ inline int step_smem_floats(int rows, int replay) {
+  const int rep = replay < kReplayChunk ? replay : kReplayChunk;
+  return (rows + 3) * kRawCols + rows * kRawCols + rep * 258;
+}
 
-  __shared__ __align__(16) float qs[kStepRows][128];
-  __shared__ __align__(16) float ks[kStepRows][128];
-  __shared__ __align__(16) float vs[kStepRows][32];
-  __shared__ __align__(16) float ys[kStepRows][32];
-  __shared__ __align__(16) float kbuf[128];
-  __shared__ __align__(16) float part[8][32];
-  __shared__ __align__(16) float party[8][32];
-  __shared__ float red_qk[kStepRows][8], red_a[kStepRows][8], red_b[kStepRows][8];
+// Two fp32 lanes in one 64-bit register: half the instructions of the row updates.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float x, float y) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y)); return r; }
+__device__ __forceinline__ float2 unpack2(f2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ void load_f2x2(const float* p, f2& a, f2& b) {      // four floats, 16-byte aligned
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  a = v.x; b = v.y;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void step_cp(float* dst, const float* src, bool valid) {
+  const int bytes = valid ? BYTES : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(BYTES), "r"(bytes));
+}
+
+__global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_constant__ GdnStepParams P) {
+  extern __shared__ __align__(16) float step_sm[];
+  __shared__ float ab_warp[kStepWarps][kStepRows][2];          // a / b dot products by warp
   __shared__ float dec[kStepRows], bet[kStepRows];
-  __shared__ float ssq[kStepRows];                       // read by the other CTAs of the cluster
-  __shared__ __align__(16) float ob[kStepRows][128];     // rank 0's copy is written by the whole cluster
+  const cr_gdn_args& a = P.span[blockIdx.y];
+  const int h = blockIdx.x, t = threadIdx.x, w = t >> 5, l = t & 31;
+  const int kg = l & 7, col4 = 16 * w + 4 * (l >> 3);          // keys 32 i + 4 kg + j of the columns col4 .. col4 + 3
+  const int own = (l & 1) * 2 + ((l >> 1) & 1);                // the column (of the four) whose sums end up in this lane
+  const int rep = P.Hv / P.Hk, kh = h / rep, KW = P.Hk * 128, VW = P.Hv * 128, C = 2 * KW + VW;
+  const int R = a.R;
+  float* raw = step_sm;                                        // [R + 3][384]: rows -3 .. R - 1
+  float* qs = raw + (P.rows + 3) * kRawCols;                   // [R][128]
+  float* ks = qs + P.rows * 128;
+  float* vs = ks + P.rows * 128;                               // a column's y replaces its v once that has been read
+  float* pk = vs + P.rows * 128;                               // staged pending rows: keys | values, then (decay, beta)
+  float* pg = pk + min(P.replay, kReplayChunk) * 256;
+  pdl_release();
+  pdl_wait();
 
-  // ---- state slice -> registers: lane holds key rows 16w + 4i + l/8 (i < 4), columns colbase + c4 .. +3
-  float S[4][4];
-  int krow[4];
-  float* st = a.state + (size_t)h * 16384 + colbase + c4;
+  // ---- everything the pass reads is asked for: state (L2), raw rows and pending rows (shared memory)
+  float* st = a.state + (size_t)h * 16384;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    krow[i] = 16 * w + 4 * i + (l >> 3);
-    const float4 v = *reinterpret_cast<const float4*>(st + (size_t)krow[i] * 128);
-    S[i][0] = v.x; S[i][1] = v.y; S[i][2] = v.z; S[i][3] = v.w;
-  }
-
-  // One delta-rule update of the register slice.  kv: the 128 normalised key values; qv: the query values or
-  // nullptr (replay has no readout).  Two block barriers per call.
-  auto update = [&](const float* kv, const float* qv, float decay, float beta, const float vcol[4], float* yrow) {
-    float kk[4], m[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      kk[i] = kv[krow[i]];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        S[i][c] *= decay;
-        m[c] = fmaf(S[i][c], kk[i], m[c]);
+  for (int i = 0; i < 2; ++i) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(st + (size_t)(t + 256 * i) * 32));
+  const float* qkv = reinterpret_cast<const float*>(a.qkv);
+  {
+    // a warp takes every eighth row, a lane the same channels of each: 96 pieces of 4 channels, or 384 single ones
+    const bool vec = (((uintptr_t)qkv | (uintptr_t)a.hist) & 15) == 0;
+    const int per = vec ? kRawCols / 4 : kRawCols;
+    for (int rr = w; rr < R + 3; rr += kStepWarps) {
+      const int p = a.pos0 + rr - 3;
+      const float* row = rr >= 3 ? qkv + (size_t)(rr - 3) * C : a.hist + (size_t)(p & 15) * C;
+      for (int i = l; i < per; i += 32) {
+        const int c = vec ? 4 * i : i;
+        const float* src = row + (c < 128 ? kh * 128 + c : (c < 256 ? KW + kh * 128 + c - 128 : 2 * KW + h * 128 + c - 256));
+        if (vec) step_cp<16>(raw + rr * kRawCols + c, src, p >= 0);
+        else step_cp<4>(raw + rr * kRawCols + c, src, p >= 0);
       }
     }
+  }
+  auto stage_pending = [&](int i0, int n) {
+    for (int i = w; i < n; i += kStepWarps) {
+      const float* pe = a.pend + ((size_t)h * P.pend_rows + i0 + i) * CR_PEND_FLOATS;
+      for (int c = l; c < 258; c += 32) step_cp<4>(c < 256 ? pk + i * 256 + c : pg + 2 * i + c - 256, pe + c, true);
+    }
+  };
+  if (a.replay > 0) stage_pending(0, min(a.replay, kReplayChunk));
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+
+  // ---- a / b dot products: all threads on one row, or four groups of 64 threads on every fourth row
+  const int groups = R == 1 ? 1 : 4, lanes = kStepThreads / groups, grp = t / lanes;
+  {
+    constexpr int kMost = (kStepRows + 3) / 4;                 // rows of a group
+    f2 pa[kMost], pb[kMost];
+#pragma unroll
+    for (int k = 0; k < kMost; ++k) pa[k] = pb[k] = 0ull;
+    const __half* wa = reinterpret_cast<const __half*>(a.ab) + (size_t)h * P.hidden;
+    const __half* wb = reinterpret_cast<const __half*>(a.ab) + (size_t)(P.Hv + h) * P.hidden;
+#pragma unroll 2
+    for (int u = t & (lanes - 1); u < P.hidden / 8; u += lanes) {
+      const uint4 ua = *reinterpret_cast<const uint4*>(wa + u * 8), ub = *reinterpret_cast<const uint4*>(wb + u * 8);
+      const __half2* ha = reinterpret_cast<const __half2*>(&ua);
+      const __half2* hb = reinterpret_cast<const __half2*>(&ub);
+      f2 fa[4], fb[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 x = __half22float2(ha[j]), y = __half22float2(hb[j]);
+        fa[j] = pack2(x.x, x.y); fb[j] = pack2(y.x, y.y);
+      }
+#pragma unroll
+      for (int k = 0; k < kMost; ++k) {
+        const int r = grp + 4 * k;
+        if (r >= R) break;
+        f2 x[4];
+        load_f2x2(a.x + (size_t)r * P.hidden + u * 8, x[0], x[1]);
+        load_f2x2(a.x + (size_t)r * P.hidden + u * 8 + 4, x[2], x[3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { pa[k] = fma2(fa[j], x[j], pa[k]); pb[k] = fma2(fb[j], x[j], pb[k]); }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kMost; ++k) {
+      const int r = grp + 4 * k;
+      if (r >= R) break;
+      const float2 xa = unpack2(pa[k]), xb = unpack2(pb[k]);
+      const float sa = warp_sum(xa.x + xa.y), sb = warp_sum(xb.x + xb.y);
+      if (l == 0) { ab_warp[w][r][0] = sa; ab_warp[w][r][1] = sb; }
+    }
+  }
+  // The state, from L2 by now: its registers are not needed while the dot products hold theirs.
+  f2 S[4][8];                                                  // [column][pair of keys 32 (m / 2) + 4 kg + 2 (m % 2)]
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float* s2 = st + (size_t)(32 * i + 4 * kg + 2 * j) * 128 + col4;
+      const float4 x = *reinterpret_cast<const float4*>(s2), y = *reinterpret_cast<const float4*>(s2 + 128);
+      S[0][2 * i + j] = pack2(x.x, y.x); S[1][2 * i + j] = pack2(x.y, y.y);
+      S[2][2 * i + j] = pack2(x.z, y.z); S[3][2 * i + j] = pack2(x.w, y.w);
+    }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+
+  // The sums over the eight key groups of four values per lane: every lane ends up with that of its own column.
+  auto reduce4 = [&](const float (&x)[4]) {
+    const bool hi = l & 1, odd = l & 2;
+    float a0 = hi ? x[2] : x[0], a1 = hi ? x[3] : x[1];
+    a0 += __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 1);
+    a1 += __shfl_xor_sync(0xffffffffu, hi ? x[1] : x[3], 1);
+    float s = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 2);
+    return s + __shfl_xor_sync(0xffffffffu, s, 4);
+  };
+  // One delta-rule update with the 128 key values kv and the head's value row v; the readout of the updated state goes over
+  // v where qv is given.
+  auto update = [&](const float* kv, const float* qv, float decay, float beta, float* v) {
+    f2 k2[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) load_f2x2(kv + 32 * i + 4 * kg, k2[2 * i], k2[2 * i + 1]);
+    float m[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      m[c] += __shfl_xor_sync(0xffffffffu, m[c], 8);
-      m[c] += __shfl_xor_sync(0xffffffffu, m[c], 16);
+      f2 x = mul2(S[c][0], k2[0]), y = mul2(S[c][1], k2[1]);
+#pragma unroll
+      for (int i = 2; i < 8; i += 2) { x = fma2(S[c][i], k2[i], x); y = fma2(S[c][i + 1], k2[i + 1], y); }
+      const float2 z = unpack2(add2(x, y));
+      m[c] = z.x + z.y;
     }
-    if (l < 8) *reinterpret_cast<float4*>(&part[w][c4]) = make_float4(m[0], m[1], m[2], m[3]);
-    __syncthreads();
-    float mem[4] = {0.f, 0.f, 0.f, 0.f};
+    const float mine = beta * (v[col4 + own] - decay * reduce4(m));
+    const float pair = __shfl_xor_sync(0xffffffffu, mine, 2);   // the deltas of the four columns back to every lane
+    const float d0 = (l & 2) ? pair : mine, d1 = (l & 2) ? mine : pair;
+    const float e0 = __shfl_xor_sync(0xffffffffu, d0, 1), e1 = __shfl_xor_sync(0xffffffffu, d1, 1);
+    const float delta[4] = {(l & 1) ? e0 : d0, (l & 1) ? e1 : d1, (l & 1) ? d0 : e0, (l & 1) ? d1 : e1};
+    const f2 g2 = pack2(decay, decay);
 #pragma unroll
-    for (int ww = 0; ww < 8; ++ww) {
-      const float4 p = *reinterpret_cast<const float4*>(&part[ww][c4]);
-      mem[0] += p.x; mem[1] += p.y; mem[2] += p.z; mem[3] += p.w;
-    }
-    float delta[4], y[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = 0; c < 4; ++c) {
+      const f2 d2 = pack2(delta[c], delta[c]);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) delta[c] = beta * (vcol[c] - mem[c]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float qq = qv ? qv[krow[i]] : 0.f;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        S[i][c] = fmaf(kk[i], delta[c], S[i][c]);
-        y[c] = fmaf(S[i][c], qq, y[c]);
-      }
+      for (int i = 0; i < 8; ++i) S[c][i] = fma2(k2[i], d2, mul2(g2, S[c][i]));
     }
     if (qv) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        y[c] += __shfl_xor_sync(0xffffffffu, y[c], 8);
-        y[c] += __shfl_xor_sync(0xffffffffu, y[c], 16);
-      }
-      if (l < 8) *reinterpret_cast<float4*>(&party[w][c4]) = make_float4(y[0], y[1], y[2], y[3]);
-    }
-    __syncthreads();
-    if (qv && t < 32) {
-      float s = 0.f;
+      for (int i = 0; i < 4; ++i) load_f2x2(qv + 32 * i + 4 * kg, k2[2 * i], k2[2 * i + 1]);
+      float o[4];
 #pragma unroll
-      for (int ww = 0; ww < 8; ++ww) s += party[ww][t];
-      yrow[t] = s;
+      for (int c = 0; c < 4; ++c) {
+        f2 x = mul2(S[c][0], k2[0]), y = mul2(S[c][1], k2[1]);
+#pragma unroll
+        for (int i = 2; i < 8; i += 2) { x = fma2(S[c][i], k2[i], x); y = fma2(S[c][i + 1], k2[i + 1], y); }
+        const float2 z = unpack2(add2(x, y));
+        o[c] = z.x + z.y;
+      }
+      const float y = reduce4(o);
+      if (kg < 4) v[col4 + own] = y;                            // the warp has read its v before the shuffles
     }
   };
 
   // ---- lazy commit: fold the accepted rows of the previous pass into the state (no readout)
-  for (int i = 0; i < a.replay; ++i) {
-    const float* pe = a.pend + ((size_t)h * P.pend_rows + i) * CR_PEND_FLOATS;
-    __syncthreads();
-    if (t < 128) kbuf[t] = pe[t];
-    __syncthreads();
-    float vcol[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) vcol[c] = pe[128 + colbase + c4 + c];
-    update(kbuf, nullptr, pe[256], pe[257], vcol, nullptr);
-  }
-  // Every CTA of the cluster has read the old pending rows before any of them records new ones.
-  if (a.replay > 0 && R > a.commit) cluster.sync();
-
-  // ---- row prologue for all rows: conv + SiLU, squared norms, a/b dot products
-  const float A = -__expf(a.A_log[h]), dtb = a.dt_bias[h];
-  const float* qkv = reinterpret_cast<const float*>(a.qkv);
-  const float* zrow = reinterpret_cast<const float*>(a.z);
-  for (int r = 0; r < R; ++r) {
-    const int p = a.pos0 + r;
-    auto tap = [&](int ch, int back) -> float {
-      const int rr = r - back;
-      if (rr >= 0) return qkv[(size_t)rr * C + ch];
-      if (p - back < 0) return 0.f;
-      return a.hist[(size_t)((p - back) & 15) * C + ch];
-    };
-    auto conv = [&](int ch) -> float {
-      const float4 wv = *reinterpret_cast<const float4*>(a.conv + (size_t)ch * 4);
-      float c = wv.x * tap(ch, 3);
-      c = fmaf(wv.y, tap(ch, 2), c);
-      c = fmaf(wv.z, tap(ch, 1), c);
-      c = fmaf(wv.w, tap(ch, 0), c);
-      return siluf_(c);
-    };
-    const float cqk = conv(t < 128 ? kh * 128 + t : KW + kh * 128 + (t - 128));
-    if (t < 128) qs[r][t] = cqk; else ks[r][t - 128] = cqk;
-    if (t < 32) vs[r][t] = conv(2 * KW + h * 128 + colbase + t);
-    float pa = 0.f, pb = 0.f;
-    const float* xr = a.x + (size_t)r * P.hidden;
-    const __half* wa = reinterpret_cast<const __half*>(a.ab) + (size_t)h * P.hidden;
-    const __half* wb = reinterpret_cast<const __half*>(a.ab) + (size_t)(P.Hv + h) * P.hidden;
-    for (int i8 = t; i8 < P.hidden / 8; i8 += 256) {
-      const float4 x0 = *reinterpret_cast<const float4*>(xr + i8 * 8);
-      const float4 x1 = *reinterpret_cast<const float4*>(xr + i8 * 8 + 4);
-      const uint4 ua = *reinterpret_cast<const uint4*>(wa + i8 * 8);
-      const uint4 ub = *reinterpret_cast<const uint4*>(wb + i8 * 8);
-      const __half2* ha = reinterpret_cast<const __half2*>(&ua);
-      const __half2* hb = reinterpret_cast<const __half2*>(&ub);
-      const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 fa = __half22float2(ha[j]), fb = __half22float2(hb[j]);
-        pa = fmaf(fa.x, xs[2 * j], pa); pa = fmaf(fa.y, xs[2 * j + 1], pa);
-        pb = fmaf(fb.x, xs[2 * j], pb); pb = fmaf(fb.y, xs[2 * j + 1], pb);
-      }
+  for (int i0 = 0; i0 < a.replay; i0 += kReplayChunk) {
+    const int n = min(a.replay - i0, kReplayChunk);
+    if (i0 > 0) {
+      __syncthreads();                                         // the chunk before has been used
+      stage_pending(i0, n);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();
     }
-    const float s2 = warp_sum(cqk * cqk);
-    pa = warp_sum(pa);
-    pb = warp_sum(pb);
-    if (l == 0) { red_qk[r][w] = s2; red_a[r][w] = pa; red_b[r][w] = pb; }
+    for (int i = 0; i < n; ++i) update(pk + i * 256, nullptr, pg[2 * i], pg[2 * i + 1], pk + i * 256 + 128);
+  }
+
+  // ---- conv + SiLU: a thread takes q or k channel t of all rows and a v channel of every other row
+  {
+    const float4 wqk = *reinterpret_cast<const float4*>(a.conv + (size_t)((t < 128 ? 0 : KW - 128) + kh * 128 + t) * 4);
+    const float4 wv = *reinterpret_cast<const float4*>(a.conv + (size_t)(2 * KW + h * 128 + (t & 127)) * 4);
+    auto conv = [&](const float4& c, float x0, float x1, float x2, float x3) {
+      float s = c.x * x0;
+      s = fmaf(c.y, x1, s);
+      s = fmaf(c.z, x2, s);
+      s = fmaf(c.w, x3, s);
+      return siluf_(s);
+    };
+    float* dst = t < 128 ? qs + t : ks + t - 128;
+    float x0 = raw[t], x1 = raw[kRawCols + t], x2 = raw[2 * kRawCols + t];
+#pragma unroll 4
+    for (int r = 0; r < R; ++r) {
+      const float x3 = raw[(r + 3) * kRawCols + t];
+      dst[r * 128] = conv(wqk, x0, x1, x2, x3);
+      x0 = x1; x1 = x2; x2 = x3;
+    }
+    for (int r = t >> 7; r < R; r += 2) {
+      const float* x = raw + r * kRawCols + 256 + (t & 127);
+      vs[r * 128 + (t & 127)] = conv(wv, x[0], x[kRawCols], x[2 * kRawCols], x[3 * kRawCols]);
+    }
   }
   __syncthreads();
-  for (int r = 0; r < R; ++r) {
-    if (t < 128) {
-      const float sq = red_qk[r][0] + red_qk[r][1] + red_qk[r][2] + red_qk[r][3];
-      qs[r][t] *= rsqrtf(sq + kEps) * kInvSqrt128;
-    } else {
-      const float sk = red_qk[r][4] + red_qk[r][5] + red_qk[r][6] + red_qk[r][7];
-      ks[r][t - 128] *= rsqrtf(sk + kEps);
-    }
+  for (int i = w; i < 2 * R; i += kStepWarps) {                // a warp normalises a row of q or k
+    float4* row = reinterpret_cast<float4*>((i < R ? qs + i * 128 : ks + (i - R) * 128) + 4 * l);
+    const float4 x = *row;
+    const float sc = rsqrtf(warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w) + kEps) * (i < R ? kInvSqrt128 : 1.f);
+    *row = make_float4(x.x * sc, x.y * sc, x.z * sc, x.w * sc);
   }
   if (t < R) {
     float pa = 0.f, pb = 0.f;
-#pragma unroll
-    for (int ww = 0; ww < 8; ++ww) { pa += red_a[t][ww]; pb += red_b[t][ww]; }
-    const float sp = pa + dtb;
+    const int per = kStepWarps / groups, w0 = R == 1 ? 0 : (t & 3) * per;
+    for (int k = w0; k < w0 + per; ++k) { pa += ab_warp[k][t][0]; pb += ab_warp[k][t][1]; }
+    const float sp = pa + a.dt_bias[h];
     const float softplus = sp > 20.f ? sp : log1pf(expf(sp));
-    dec[t] = expf(A * softplus);
+    dec[t] = expf(-__expf(a.A_log[h]) * softplus);
     bet[t] = sigmoidf_(pb);
   }
+  float z[2][4];                                               // gate rows w and w + 8: in flight during the recurrence
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[k][i] = w + 8 * k < R ? reinterpret_cast<const float*>(a.z)[(size_t)(w + 8 * k) * VW + h * 128 + 4 * l + i] : 0.f;
   __syncthreads();
 
-  // ---- speculative rows: record (khat, v, decay, beta) for the next pass's replay
-  for (int r = a.commit; r < R; ++r) {
-    float* pe = a.pend + ((size_t)h * P.pend_rows + (r - a.commit)) * CR_PEND_FLOATS;
-    if (rank == 0) {
-      if (t < 128) pe[t] = ks[r][t];
-      if (t == 128) pe[256] = dec[r];
-      if (t == 129) pe[257] = bet[r];
+  // ---- raw-row ring (slots of this call never alias the three slots any CTA reads: R + 3 <= 16) and speculative rows:
+  // (khat, v, decay, beta) for the next pass's replay, whose old rows every warp of this head has used
+  for (int r = w; r < R; r += kStepWarps) {
+    float* hs = a.hist + (size_t)((a.pos0 + r) & 15) * C;
+    const float* x = raw + (r + 3) * kRawCols;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = l + 32 * i;
+      hs[2 * KW + h * 128 + c] = x[256 + c];
+      if (h % rep == 0) { hs[kh * 128 + c] = x[c]; hs[KW + kh * 128 + c] = x[128 + c]; }
     }
-    if (t < 32) pe[128 + colbase + t] = vs[r][t];
+    if (r >= a.commit) {
+      float* pe = a.pend + ((size_t)h * P.pend_rows + (r - a.commit)) * CR_PEND_FLOATS;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { pe[l + 32 * i] = ks[r * 128 + l + 32 * i]; pe[128 + l + 32 * i] = vs[r * 128 + l + 32 * i]; }
+      if (l < 2) pe[256 + l] = l == 0 ? dec[r] : bet[r];
+    }
   }
+  if (R > a.commit) __syncthreads();                           // the readout overwrites v
 
   // ---- the recurrence
   for (int r = 0; r < R; ++r) {
-    float vcol[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) vcol[c] = vs[r][c4 + c];
-    update(ks[r], qs[r], dec[r], bet[r], vcol, ys[r]);
+    update(ks + r * 128, qs + r * 128, dec[r], bet[r], vs + r * 128);
     if (r == a.commit - 1) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float4*>(st + (size_t)krow[i] * 128) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float2 x[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) x[c] = unpack2(S[c][2 * i + j]);
+          float* s2 = st + (size_t)(32 * i + 4 * kg + 2 * j) * 128 + col4;
+          *reinterpret_cast<float4*>(s2) = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
+          *reinterpret_cast<float4*>(s2 + 128) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+        }
     }
   }
   __syncthreads();
 
-  // ---- gated RMSNorm over the head's 128 columns: partial sums of squares exchanged through DSMEM
-  for (int r = w; r < R; r += 8) {
-    const float v = ys[r][l];
-    const float s = warp_sum(v * v);
-    if (l == 0) ssq[r] = s;
-  }
-  cluster.sync();
-  float* ob0 = cluster.map_shared_rank(&ob[0][0], 0);
-  for (int r = w; r < R; r += 8) {
-    float tot = 0.f;
+  // ---- gated RMSNorm over the head's 128 columns, a warp per row, lane l the columns 4 l .. 4 l + 3
 #pragma unroll
-    for (int k = 0; k < 4; ++k) tot += cluster.map_shared_rank(ssq, k)[r];
-    const int col = h * 128 + colbase + l;
-    const float o = ys[r][l] * rsqrtf(tot * (1.f / 128.f) + kEps) * a.gamma[colbase + l] *
-                    sigmoidf_(zrow[(size_t)r * VW + col]);
-    if (P.fmt == CR_OUT_RAW_F32) reinterpret_cast<float*>(a.out)[(size_t)r * VW + col] = o;
-    else if (P.fmt == CR_OUT_RAW_BF16) reinterpret_cast<__nv_bfloat16*>(a.out)[(size_t)r * VW + col] = __float2bfloat16(o);
-    else ob0[r * 128 + colbase + l] = round_h(round_h(o) * __half2float(reinterpret_cast<const __half*>(a.suh_out)[col]));
-  }
-  cluster.sync();   // remote reads of ssq and remote writes of ob are complete
-  if (P.fmt == CR_OUT_EXL3_WHT && rank == 0) {
-    for (int r = w; r < R; r += 8) {
-      float v[4];
+  for (int k = 0; k < 2; ++k) {
+    const int r = w + 8 * k;
+    if (r >= R) break;
+    const float4 y = *reinterpret_cast<const float4*>(vs + r * 128 + 4 * l);
+    const float rs = rsqrtf(warp_sum(y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w) * (1.f / 128.f) + kEps);
+    const float yv[4] = {y.x, y.y, y.z, y.w};
+    float o[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = ob[r][l * 4 + i];
-      wht128(v);
-      __half* dst = reinterpret_cast<__half*>(a.out);
+    for (int i = 0; i < 4; ++i) o[i] = yv[i] * rs * a.gamma[4 * l + i] * sigmoidf_(z[k][i]);
+    const size_t at = (size_t)r * VW + h * 128 + 4 * l;
+    if (P.fmt == CR_OUT_RAW_F32) {
+      float* dst = reinterpret_cast<float*>(a.out) + at;
+      if (((uintptr_t)dst & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+      else { dst[0] = o[0]; dst[1] = o[1]; dst[2] = o[2]; dst[3] = o[3]; }
+    } else if (P.fmt == CR_OUT_RAW_BF16) {
+      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + at;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        dst[out_index(r, h * 128 + l * 4 + i, VW, a.pack_rows, a.pack_off)] = __float2half(v[i] * kHadNorm);
-    }
-  }
-
-  // ---- raw-row ring: slots of this call never alias the three slots any CTA reads (R + 3 <= 16)
-  for (int r = 0; r < R; ++r) {
-    float* hs = a.hist + (size_t)((a.pos0 + r) & 15) * C;
-    const float* q = qkv + (size_t)r * C;
-    if (t < 32) {
-      const int ch = 2 * KW + h * 128 + colbase + t;
-      hs[ch] = q[ch];
-    } else if (t < 96 && h % rep == 0) {
-      const int ch = (t < 64 ? 0 : KW) + kh * 128 + colbase + ((t - 32) & 31);
-      hs[ch] = q[ch];
+      for (int i = 0; i < 4; i += 2) {
+        const __nv_bfloat162 b = __floats2bfloat162_rn(o[i], o[i + 1]);
+        if (((uintptr_t)dst & 3) == 0) *reinterpret_cast<__nv_bfloat162*>(dst + i) = b;
+        else { dst[i] = b.x; dst[i + 1] = b.y; }
+      }
+    } else {
+      float su[4];
+      load_half4(a.suh_out + h * 128 + 4 * l, su);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = round_h(round_h(o[i]) * su[i]);
+      wht128(o);
+      store_half4(reinterpret_cast<uint16_t*>(a.out) + out_index(r, h * 128 + 4 * l, VW, a.pack_rows, a.pack_off), o, kHadNorm);
     }
   }
 }
@@ -295,7 +371,18 @@ extern "C" cr_status cr_gdn_step(const cr_geometry* g, const cr_gdn_args* spans,
     const int n = n_spans - s0 < kMaxSpans ? n_spans - s0 : kMaxSpans;
     for (int s = 0; s < n; ++s) P.span[s] = spans[s0 + s];
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.hidden = g->hidden; P.pend_rows = pend_rows; P.fmt = (int)fmt;
-    gdn_step_kernel<<<dim3(4 * g->gdn_vheads, n), 256, 0, (cudaStream_t)stream>>>(P);
+    static PerDeviceOnce configured;
+    if (cr_status st = once_per_device(configured, [] {
+          CR_CUDA(cudaFuncSetAttribute(gdn_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(step_smem_floats(kStepRows, kReplayChunk) * sizeof(float))));
+          return CR_OK;
+        })) return st;
+    P.rows = P.replay = 0;
+    for (int s = 0; s < n; ++s) {
+      P.rows = P.rows > P.span[s].R ? P.rows : P.span[s].R;
+      P.replay = P.replay > P.span[s].replay ? P.replay : P.span[s].replay;
+    }
+    CR_CUDA(launch_pdl(gdn_step_kernel, dim3(g->gdn_vheads, n), dim3(kStepThreads), step_smem_floats(P.rows, P.replay) * sizeof(float),
+                       (cudaStream_t)stream, P));
     CR_LAUNCH_CHECK("gdn_step_kernel");
   }
   return CR_OK;
