@@ -1,4 +1,4 @@
-"""Builds libcrucible_attn.so (sm_100a) in-tree with nvcc.
+"""Builds libcrucible_attn.so (sm_100a) in-tree with nvcc, and _binding.so (the host path of layers.py) with g++.
 
     python -m crucible_strix_halo_b200.build [--force]
 """
@@ -13,6 +13,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libcrucible_attn.so")
+BINDING = os.path.join(PKG, "_binding.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-O3"]
 
@@ -52,6 +53,27 @@ def build_library(force=False, verbose=False):
     return LIB
 
 
+def build_binding(force=False):
+    """Needs the library and torch's headers; links against both (the library is found beside the binding)."""
+    src = os.path.join(PKG, "native", "binding.cpp")
+    if not force and _newer(BINDING, [src, os.path.join(ROOT, "include", "crucible_attn.h")]):
+        return BINDING
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    libs = cpp_extension.library_paths(device_type="cuda")
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+          *["-I" + d for d in cpp_extension.include_paths(device_type="cuda") + [sysconfig.get_paths()["include"]]], src, "-o", BINDING,
+          "-L" + PKG, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN", *["-L" + d for d in libs], "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    return BINDING
+
+
+def build_all(force=False, verbose=False):
+    build_library(force, verbose)
+    build_binding(force)
+    return LIB
+
+
 if __name__ == "__main__":
     force = "--force" in sys.argv
-    print(build_library(force, verbose="-v" in sys.argv))
+    print(build_all(force, verbose="-v" in sys.argv))

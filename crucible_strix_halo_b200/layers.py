@@ -1,16 +1,16 @@
 """Torch-tensor wrappers over the C ABI: they own device buffers the way the engine's SequenceState does
-(engine/runtime/sequence_state.h:84-112) and fill the argument structs of include/crucible_attn.h.
-Plumbing only: every computation happens in libcrucible_attn.so."""
+(engine/runtime/sequence_state.h:84-112); _binding (native/binding.cpp) fills the argument structs of
+include/crucible_attn.h from them.  Plumbing only: every computation happens in libcrucible_attn.so."""
 import ctypes as C
 
 import torch
 
-from . import capi
-from .capi import (GdnArgs, GdnPrefillArgs, QsaArgs, QsaCache, QsaPrefillArgs, Geometry, check, dptr, lib)
+from . import _binding, capi
+from .capi import QsaArgs, QsaCache, Geometry, check, dptr, lib
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(_binding.current_stream())
 
 
 def _out_dtype(fmt):
@@ -44,26 +44,10 @@ class GdnSession:
         return self.state[:self.g.gdn_vheads * 16384].view(self.g.gdn_vheads, 128, 128)
 
 
-def _gdn_args(w: GdnWeights, s: GdnSession, qkv, z, x, out, pos0, R, replay, commit, pack_rows=0, pack_off=0):
-    return GdnArgs(dptr(qkv), dptr(z), dptr(x), dptr(w.ab), dptr(w.conv), dptr(w.A_log), dptr(w.dt_bias),
-                   dptr(w.gamma), dptr(s.hist), dptr(s.state), dptr(w.suh), dptr(out), dptr(s.pend),
-                   pos0, R, replay, commit, pack_rows, pack_off)
-
-
 def gdn_step(w: GdnWeights, spans, fmt=capi.OUT_RAW_F32, outs=None):
     """spans: list of dicts(session, qkv [R,C] f32, z [R,Hv*128] f32, x [R,hidden] f32, pos0, replay, commit).
     One launch for all spans (LaunchGdnCore / packed verify).  Returns the list of outputs [R, Hv*128]."""
-    g = w.g
-    given, outs, arr = outs, [], (GdnArgs * len(spans))()
-    pend_rows = spans[0]["session"].pend_rows
-    for i, sp in enumerate(spans):
-        R = sp["qkv"].shape[0]
-        out = given[i] if given is not None else torch.empty(R, g.gdn_vheads * 128, device=sp["qkv"].device, dtype=_out_dtype(fmt))
-        outs.append(out)
-        arr[i] = _gdn_args(w, sp["session"], sp["qkv"], sp["z"], sp["x"], out, sp["pos0"], R,
-                           sp.get("replay", 0), sp.get("commit", R))
-    check(lib.cr_gdn_step(C.byref(g), arr, len(spans), pend_rows, fmt, _stream()))
-    return outs
+    return _binding.gdn_step(w, spans, fmt, outs)
 
 
 class GdnPrefillPlan:
@@ -79,10 +63,7 @@ class GdnPrefillPlan:
     def run(self, s: GdnSession, qkv, z, ab_logits, pos0, algo=capi.GDN_SERIAL_F32):
         R = qkv.shape[0]
         assert R == self.rows
-        a = GdnPrefillArgs(_gdn_args(self.w, s, qkv, z, None, self.out, pos0, R, 0, R), dptr(ab_logits), self.in_dtype,
-                           dptr(self.workspace), self.workspace.numel(), dptr(self.raw_y))
-        check(lib.cr_gdn_prefill(C.byref(self.w.g), C.byref(a), algo, self.fmt, _stream()))
-        return self.out
+        return _binding.gdn_prefill(self, s, qkv, z, ab_logits, pos0, algo)
 
 
 class QsaWeights:
@@ -140,18 +121,7 @@ class QsaStepPlan:
 
     def run(self, spans, want_context=False, outs=None):
         """spans: list of dicts(session, q [R,Hq,512] f32 (modified in place), k, v [R,Hkv*256], idx [R,640], pos0)."""
-        g = self.w.g
-        arr = (QsaArgs * len(spans))()
-        given, outs, ctxs = outs, [], []
-        for i, sp in enumerate(spans):
-            R = sp["q"].shape[0]
-            out = given[i] if given is not None else torch.empty(R, g.q_heads * 256, device=sp["q"].device, dtype=_out_dtype(self.fmt))
-            ctx = torch.empty(R, g.q_heads, 256, device=sp["q"].device, dtype=torch.float32) if want_context else None
-            outs.append(out)
-            ctxs.append(ctx)
-            arr[i] = qsa_args(self.w, sp["session"], sp["q"], sp["k"], sp["v"], sp["idx"], out, sp["pos0"], ctx)
-        check(lib.cr_qsa_step(C.byref(g), arr, len(spans), dptr(self.scratch), self.scratch.numel(), self.fmt, _stream()))
-        return (outs, ctxs) if want_context else outs
+        return _binding.qsa_step(self, spans, want_context, outs)
 
 
 class QsaPrefillPlan:
@@ -167,10 +137,7 @@ class QsaPrefillPlan:
     def run(self, s: QsaSession, q, k, v, idx, pos0, skip=0, context=None):
         R = q.shape[0]
         assert R <= self.rows and s.scores.shape[0] >= R
-        a = QsaPrefillArgs(qsa_args(self.w, s, q, k, v, idx, self.out, pos0, context), dptr(self.q_hi),
-                           dptr(self.scratch), self.scratch.numel())
-        check(lib.cr_qsa_prefill(C.byref(self.w.g), C.byref(a), skip, self.fmt, _stream()))
-        return self.out[:R]
+        return _binding.qsa_prefill(self, s, q, k, v, idx, pos0, skip, context)
 
 
 def checkpoint_spans(gdn_sessions, qsa_sessions, position):
@@ -207,13 +174,4 @@ class SlotCheckpoint:
 def proj_gemm(x, w, outs):
     """x [R, K] bf16, w [N, K] bf16 (out x in); outs: list of (tensor [R, cols] bf16 or fp32, contiguous rows) whose
     widths add up to N.  One cr_proj_gemm launch (the input or output GEMM group of a prefill layer)."""
-    R, K = x.shape
-    N = w.shape[0]
-    arr = (capi.ProjOut * len(outs))()
-    col = 0
-    for i, o in enumerate(outs):
-        cols = o.shape[-1] if o.dim() == 2 else o[0].numel()
-        arr[i] = capi.ProjOut(o.data_ptr(), col, cols, cols, 1 if o.dtype == torch.float32 else 0)
-        col += cols
-    check(lib.cr_proj_gemm(dptr(x), dptr(w), R, K, N, arr, len(outs), _stream()))
-    return outs
+    return _binding.proj_gemm(x, w, outs)
