@@ -63,10 +63,10 @@ __device__ __forceinline__ bool mbar_try_relaxed(uint32_t addr, uint32_t parity)
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.relaxed.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.relaxed.cta.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}\n"
       : "=r"(done)
-      : "r"(addr), "r"(parity), "r"(kSuspendNs)
+      : "r"(addr), "r"(parity)
       : "memory");
   return done != 0;
 }
@@ -87,13 +87,13 @@ __device__ __forceinline__ bool mbar_wait_timed(uint64_t* bar, uint32_t parity, 
   const uint32_t addr = smem_u32(bar);
   auto poll = [&]() { return RELAXED ? mbar_try_relaxed(addr, parity) : mbar_try(addr, parity); };
 #pragma unroll 1
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < (RELAXED ? 1 : 4); ++i)
     if (poll()) return true;
   uint64_t t0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
   for (;;) {
 #pragma unroll 1
-    for (int i = 0; i < 8; ++i)   // the clock and the abort flag are slow to read: look at them rarely
+    for (int i = 0; i < (RELAXED ? 64 : 8); ++i)   // the clock and the abort flag are slow to read: look at them rarely
       if (poll()) return true;
     uint64_t t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
