@@ -368,7 +368,7 @@ size_t cr_spans_bytes(const cr_span* spans, int n);
 
 /* Copies the spans, in order and back to back, into `buffer` (save) or out of it (restore): the copy loops of
  * SlotCheckpointIO::Save / Restore (engine/runtime/slot_checkpoint_io.h:49-73) and CopySnapshotSpans
- * (engine/runtime/snapshot_bytes.h:692-704) as one kernel per 96 spans on `stream`, in order with the forwards
+ * (engine/runtime/snapshot_bytes.h:692-704) as one kernel per 1,200 spans on `stream`, in order with the forwards
  * around it.  `buffer` is device memory, or pinned host memory the device can address (a conversation snapshot).
  * The ledger (RetainedPrefix) and the token history that belong to a checkpoint are host data and stay with the
  * caller.  CR_ERR_INVALID if the buffer is smaller than the spans, or a span is not 16-byte aligned and sized. */
