@@ -1,18 +1,23 @@
 // Exact top-512 of a row of indexer scores for sm_100a (the job of LaunchQsaTop, engine/layers/qsa_long.h:111-380):
 // the 512 best blocks in the total order (score descending, block id ascending), emitted in ascending block id.
 //
-// Method: group maxima, pivot, filter, bisect, mark, compact.  One CTA of 1024 threads per row.
+// Method: group maxima, pivot, filter, histogram, mark, compact.  One CTA of 1024 threads per row.
 //   1. Scores are >= +0, so their fp32 bit patterns order like unsigned integers (key = pattern + 1; 0 = no element).
 //      Thread t reads the elements t, t + 1024, ... (its group) and keeps their maximum.
-//   2. The pivot is the 512th largest of the 1024 group maxima, found by bisection over the key bits: 31 block-wide
-//      counts, no sorting and no atomics.  At least 512 elements are >= the pivot (those maxima themselves), so every
-//      element that can be among the best 512, ties included, is >= the pivot; with unrelated scores about 700 are.
+//   2. The pivot is a lower bound of the 512th largest of the 1024 group maxima: they are counted in 2,048 bins of the key
+//      range below the largest, and a suffix scan finds the bin that holds the 512th.  At least 512 elements are >= the
+//      bin's lower edge (those maxima themselves), so every element that can be among the best 512, ties included, is; with
+//      unrelated scores about 700 are.
 //   3. A second pass gathers the elements >= the pivot into a shared-memory list (warp-aggregated appends).
-//   4. The 512th largest key of the list is found by the same bisection; keys above it are taken, and of the keys
-//      equal to it the lowest indices (counted among the ties).
+//   4. The same histogram over the list, between its known bounds, finds the bin of the 512th key: everything above is
+//      taken, and the few elements inside the bin are ranked against each other (key, then index).  A crowded bin is
+//      divided again, down to single keys; of equal keys the lowest indices are taken.
 //   5. The taken elements set their bit in a bitmap over the row, which is compacted in index order: a prefix sum over
 //      word popcounts gives every thread its output offset.
 //   Rows of at most 4096 elements skip 1-3: every element goes into the list.
+//   Bound: block barriers of a latency chain (the row itself is read at L2 speed).  As 31-step bisections with a
+//   block-wide count per bit, a row of 2,300 blocks took 16 us, 7 now; 2,048 rows of 65,536 blocks 268 -> 203 us (long
+//   rows are read four elements at a time), of 8,192 blocks 125 -> 68 us.
 //   When more than 4096 elements pass the pivot (long runs of equal scores), the row takes the slow exact path: the
 //   same bisection over the whole row, counting with plain reductions, then the values above the 512th best pattern
 //   plus its first ties in index order from a second bitmap.
@@ -37,6 +42,9 @@ struct RowSource {                         // scores[i], block id = id_base + i
   int id_base;
   __device__ __forceinline__ bool get(int i, unsigned& bits) const { bits = __float_as_uint(scores[i]); return true; }
   __device__ __forceinline__ int id(int i) const { return id_base + i; }
+  // Four consecutive elements, where the row starts at a 16-byte boundary and its buffer goes on to the next one.
+  bool quads;
+  __device__ __forceinline__ uint4 get4(int q) const { return reinterpret_cast<const uint4*>(scores)[q]; }
 };
 struct GatheredSource {                    // candidates of several ranks: element i = rank i / 512, slot i % 512
   const float* scores;
@@ -50,7 +58,13 @@ struct GatheredSource {                    // candidates of several ranks: eleme
     return true;
   }
   __device__ __forceinline__ int id(int i) const { return ids[at(i)]; }
+  static constexpr bool quads = false;
+  __device__ __forceinline__ uint4 get4(int) const { return make_uint4(0u, 0u, 0u, 0u); }
 };
+__device__ __forceinline__ RowSource row_source(const cr_qsa_args& a, int r, int b0) {
+  const float* s = a.scores + (size_t)r * a.sstride + b0;
+  return RowSource{s, b0, ((uintptr_t)s & 15) == 0 && a.sstride % 4 == 0 && b0 % 4 == 0};
+}
 
 // ---- block-wide helpers ------------------------------------------------------------------------------------
 __device__ __forceinline__ unsigned block_sum_u32(unsigned v, unsigned* red) {   // red: 33 words
@@ -68,8 +82,15 @@ __device__ __forceinline__ unsigned block_sum_u32(unsigned v, unsigned* red) {  
   __syncthreads();
   return red[32];
 }
-// Exclusive prefix sum of one value per thread over the block (1024 threads); *total receives the sum.
-__device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* red, unsigned* total) {
+// Largest of one value per thread; one barrier (red: 32 words, free again after the caller's next barrier).
+__device__ __forceinline__ unsigned block_max_u32(unsigned v, unsigned* red) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  return __reduce_max_sync(0xffffffffu, red[threadIdx.x & 31]);
+}
+// Exclusive prefix sum of one value per thread over the block (1024 threads); one barrier before red is written, one after.
+__device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* red) {
   const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned inc = v;
 #pragma unroll
@@ -80,20 +101,7 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* r
   __syncthreads();
   if (l == 31) red[w] = inc;
   __syncthreads();
-  if (w == 0) {
-    const unsigned mine = red[l];
-    unsigned winc = mine;
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-      const unsigned o = __shfl_up_sync(0xffffffffu, winc, s);
-      if (l >= s) winc += o;
-    }
-    red[l] = winc - mine;                    // exclusive over warps
-    if (l == 31) red[32] = winc;
-  }
-  __syncthreads();
-  *total = red[32];
-  return red[w] + inc - v;
+  return __reduce_add_sync(0xffffffffu, l < w ? red[l] : 0u) + inc - v;
 }
 // Shared memory of one CTA: candidate list (32 KB), bitmap over the row's elements (count bits), small arrays.
 struct SelectSmem {
@@ -101,6 +109,9 @@ struct SelectSmem {
   unsigned* bitmap;            // ceil(count / 32) words
   unsigned* red;               // 33 words
   unsigned* counter;           // 1 word
+  int* hist;                   // kBins counters, zero between uses
+  int* found;                  // 3 words
+  uint2* ties;                 // kRankCap entries
 };
 
 constexpr int kBatch = 8;      // loads a thread issues before it uses any of them
@@ -127,57 +138,139 @@ __device__ __forceinline__ void for_each_key(const Src& src, int count, F&& f) {
   }
 }
 
-// The largest T with at least `want` keys >= T, over keys spread one per thread (mine; 0 = none).
-__device__ __forceinline__ unsigned bisect_one_per_thread(unsigned mine, int want) {
-  unsigned T = 0u;
-  for (int bit = 30; bit >= 0; --bit) {
-    const unsigned trial = T | (1u << bit);
-    if (__syncthreads_count(mine >= trial) >= want) T = trial;
-  }
-  return T;
-}
-// The same over the candidate list: thread t holds the list entries t, t + 1024, ... (at most 4).  Every key lies in
-// [lo, hi]: the bits above the first bit in which lo and hi differ are settled, and the search starts below them.
-__device__ __forceinline__ unsigned bisect_list(const uint2* cand, int m, int want, unsigned lo, unsigned hi) {
-  unsigned k[4];
+// The same four elements at a time (src.quads): f(i, keys) for the elements i .. i + 3, keys past the end 0.  All lanes of a
+// warp make the same number of calls.
+template <typename Src, typename F>
+__device__ __forceinline__ void for_each_quad(const Src& src, int count, F&& f) {
+  const int lane = threadIdx.x & 31, quads = (count + 3) >> 2;
+  constexpr int kDeep = 2;
+  for (int q0 = threadIdx.x; q0 - lane < quads; q0 += kSelThreads * kDeep) {
+    uint4 v[kDeep];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) { const int i = threadIdx.x + q * kSelThreads; k[q] = i < m ? cand[i].x : 0u; }
-  if (lo >= hi) return lo;
-  const int top = 31 - __clz(lo ^ hi);                             // the first differing bit
-  unsigned T = lo & ~((2u << top) - 1u);
-  for (int bit = top; bit >= 0; --bit) {
-    const unsigned trial = T | (1u << bit);
-    const int c = (k[0] >= trial) + (k[1] >= trial) + (k[2] >= trial) + (k[3] >= trial);
-    int total;
-    if (m <= kSelThreads) total = __syncthreads_count(c);
-    else total = __syncthreads_count(c & 1) + 2 * __syncthreads_count(c & 2) + 4 * __syncthreads_count(c & 4);
-    if (total >= want) T = trial;
+    for (int k = 0; k < kDeep; ++k) {
+      const int q = q0 + k * kSelThreads;
+      v[k] = q < quads ? src.get4(q) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int k = 0; k < kDeep; ++k) {
+      const int q = q0 + k * kSelThreads, i = 4 * q;
+      if (q - lane >= quads) break;                                 // warp uniform
+      f(i, make_uint4(i < count ? v[k].x + 1u : 0u, i + 1 < count ? v[k].y + 1u : 0u, i + 2 < count ? v[k].z + 1u : 0u, i + 3 < count ? v[k].w + 1u : 0u));
+    }
   }
-  return T;
 }
 
-// The list sm.cand[0, m) holds (key, index) pairs that include the `want` best elements of the row (want <= m <= kSortCap):
-// marks those in sm.bitmap.  The want-th largest key by bisection; keys above it are taken, and of the keys equal to it
-// the lowest indices (counted among the ties).
-__device__ __forceinline__ void select_from_list(int m, int want, const SelectSmem& sm, unsigned lo = 0u, unsigned hi = 0x7FFFFFFFu) {
-  const int t = threadIdx.x;
-  const unsigned T = bisect_list(sm.cand, m, want, lo, hi);
-  int gt = 0, eq = 0;
-  for (int i = t; i < m; i += kSelThreads) { const unsigned k = sm.cand[i].x; gt += k > T; eq += k == T; }
-  const int n_gt = (int)block_sum_u32((unsigned)gt, sm.red), n_eq = (int)block_sum_u32((unsigned)eq, sm.red);
-  const int need = want - n_gt;                                    // ties to take: 1 <= need <= n_eq
-  for (int i = t; i < m; i += kSelThreads) {
-    const uint2 c = sm.cand[i];
-    bool take = c.x > T;
-    if (c.x == T) {
-      if (need >= n_eq) take = true;
-      else {                                                       // rank among the ties by index
-        int before = 0;
-        for (int j = 0; j < m; ++j) { const uint2 o = sm.cand[j]; before += (o.x == T && o.y < c.y); }
-        take = before < need;
-      }
+// ---- threshold by histogram ----------------------------------------------------------------------------------
+constexpr int kBins = 2048;
+constexpr int kRankCap = 512;              // elements of the threshold bin that are ranked against each other
+
+struct Threshold { int bin, above, in_bin; };   // the bin that holds the want-th largest; elements in higher bins; in it
+// sm.hist filled and visible.  The bin of the want-th largest counted element; bin = -1 when fewer were counted.  Two
+// barriers; the histogram is zero again afterwards (visible after the caller's next barrier).
+__device__ __forceinline__ Threshold find_threshold(const SelectSmem& sm, int want) {
+  constexpr int PER = kBins / kSelThreads;
+  const int t = threadIdx.x, l = t & 31, w = t >> 5, first = kBins - 1 - t * PER;   // this thread's bins, descending
+  int c[PER], sum = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) { c[i] = sm.hist[first - i]; sm.hist[first - i] = 0; sum += c[i]; }
+  int inc = sum;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, inc, s);
+    if (l >= s) inc += o;
+  }
+  if (l == 31) sm.red[w] = (unsigned)inc;
+  if (t == 0) sm.found[0] = -1;
+  __syncthreads();
+  int before = (int)__reduce_add_sync(0xffffffffu, l < w ? sm.red[l] : 0u) + inc - sum;   // elements in higher bins
+  if (before < want && before + sum >= want) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      if (before < want && before + c[i] >= want) { sm.found[0] = first - i; sm.found[1] = before; sm.found[2] = c[i]; }
+      before += c[i];
     }
-    if (take) atomicOr(&sm.bitmap[c.y >> 5], 1u << (c.y & 31));
+  }
+  __syncthreads();
+  return Threshold{sm.found[0], sm.found[1], sm.found[2]};
+}
+// Bits by which keys in [lo, hi] are shifted to fall into kBins bins.
+__device__ __forceinline__ int bin_shift(unsigned lo, unsigned hi) {
+  const unsigned span = hi > lo ? hi - lo : 0u;
+  return span < (unsigned)kBins ? 0 : 21 - __clz(span);
+}
+
+// A lower bound of the want-th largest of one key per thread (0: none), such that at least `want` keys are >= it; 1 when
+// there are fewer.  largest: the largest of all keys.  sm.hist zero on entry.
+__device__ __forceinline__ unsigned pivot_of(unsigned mine, unsigned largest, int want, const SelectSmem& sm) {
+  unsigned shift = 14;                                             // the four octaves below the largest key
+#pragma unroll 1
+  for (int round = 0; round < 2; ++round, shift = 20) {            // then everything
+    const unsigned width = (unsigned)kBins << shift, lo = largest >= width ? largest - width + 1u : 1u;
+    if (mine >= lo) atomicAdd(&sm.hist[(mine - lo) >> shift], 1);
+    __syncthreads();
+    const Threshold th = find_threshold(sm, want);
+    __syncthreads();
+    if (th.bin >= 0) return lo + ((unsigned)th.bin << shift);
+  }
+  return 1u;
+}
+
+// The list sm.cand[0, m) holds (key, index) pairs that include the `want` best elements of the row (want <= m <= kSortCap),
+// keys in [lo, hi]: marks those in sm.bitmap.  sm.hist zero and the list visible on entry; ends with a barrier.
+__device__ __forceinline__ void select_from_list(int m, int want, const SelectSmem& sm, unsigned lo, unsigned hi) {
+  const int t = threadIdx.x;
+  constexpr int PER = kSortCap / kSelThreads;
+  uint2 c[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) { const int i = t + q * kSelThreads; c[q] = i < m ? sm.cand[i] : make_uint2(0u, 0u); }
+  // The first division covers the four octaves below the largest key (or less, if the list does); should they hold too few,
+  // the whole range.
+  const int full = bin_shift(lo, hi);
+  int need = want, shift = full < 14 ? full : 14;
+  unsigned first = full <= 14 ? lo : hi - ((unsigned)kBins << 14) + 1u, last;   // keys of the threshold bin
+  Threshold th;
+  for (;;) {
+    const unsigned width = (unsigned)kBins << shift;
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const unsigned d = c[q].x - first;
+      if (c[q].x >= first && c[q].x != 0u && d < width) atomicAdd(&sm.hist[d >> shift], 1);
+    }
+    __syncthreads();
+    th = find_threshold(sm, need);
+    if (th.bin < 0) {
+      shift = full; first = lo;
+      __syncthreads();
+      continue;
+    }
+    need -= th.above;
+    first += (unsigned)th.bin << shift;
+    last = first + ((1u << shift) - 1u);
+    if (need == th.in_bin || th.in_bin <= kRankCap || shift == 0) break;
+    shift = shift > 11 ? shift - 11 : 0;
+    __syncthreads();                                               // the histogram is zero again for everybody
+  }
+  const bool all = need == th.in_bin, ranked = !all && th.in_bin <= kRankCap;
+  if (ranked) {
+    if (t == 0) *sm.counter = 0u;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PER; ++q)
+      if (c[q].x >= first && c[q].x <= last && c[q].x != 0u) sm.ties[atomicAdd(sm.counter, 1u)] = c[q];
+    __syncthreads();
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    if (c[q].x < first || c[q].x == 0u) continue;
+    bool take = c[q].x > last || all;
+    if (!take) {                                                   // inside the bin: better keys, then lower indices first
+      const uint2* list = ranked ? sm.ties : sm.cand;              // a bin too crowded to rank holds one key only
+      const int n = ranked ? th.in_bin : m;
+      int before = 0;
+      for (int j = 0; j < n; ++j) { const uint2 o = list[j]; before += (o.x > c[q].x && o.x <= last) || (o.x == c[q].x && o.y < c[q].y); }
+      take = before < need;
+    }
+    if (take) atomicOr(&sm.bitmap[c[q].y >> 5], 1u << (c[q].y & 31));
   }
   __syncthreads();
 }
@@ -191,17 +284,19 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
   const int t = threadIdx.x, l = t & 31;
   const int words = (count + 31) >> 5;
   for (int i = t; i < words; i += kSelThreads) sm.bitmap[i] = 0u;
+  for (int i = t; i < kBins; i += kSelThreads) sm.hist[i] = 0;
   if (t == 0) *sm.counter = 0u;
-  unsigned pivot = 1u;                                             // every element passes
+  unsigned pivot = 1u, mine = 0u, largest = 0u;                    // pivot 1: every element passes
   if (count > kSortCap) {
-    unsigned mine = 0u;
-    for_each_key<false>(src, count, [&](int, unsigned key) { mine = key > mine ? key : mine; });
-    pivot = bisect_one_per_thread(mine, want);                     // 0 when fewer than `want` groups hold an element
-    if (pivot == 0u) pivot = 1u;
+    if (src.quads) for_each_quad(src, count, [&](int, const uint4& k) { mine = max(max(max(mine, k.x), max(k.y, k.z)), k.w); });
+    else for_each_key<false>(src, count, [&](int, unsigned key) { mine = key > mine ? key : mine; });
+    largest = block_max_u32(mine, sm.red);
+    pivot = pivot_of(mine, largest, want, sm);
+  } else {
+    __syncthreads();
   }
-  __syncthreads();
   // ---- the elements >= pivot, as (key, index) pairs
-  for_each_key<true>(src, count, [&](int i, unsigned key) {
+  auto append = [&](int i, unsigned key) {
     const bool pass = key >= pivot;
     const unsigned m = __ballot_sync(0xffffffffu, pass);
     if (m) {
@@ -211,10 +306,24 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
       const unsigned at = base + __popc(m & ((1u << l) - 1u));
       if (pass && at < (unsigned)kSortCap) sm.cand[at] = make_uint2(key, (unsigned)i);
     }
-  });
-  __syncthreads();
+  };
+  if (src.quads) {
+    for_each_quad(src, count, [&](int i, const uint4& k) {
+      const unsigned best = max(max(k.x, k.y), max(k.z, k.w));
+      mine = max(mine, best);
+      if (!__any_sync(0xffffffffu, best >= pivot)) return;         // most quads of a long row
+      append(i, k.x); append(i + 1, k.y); append(i + 2, k.z); append(i + 3, k.w);
+    });
+  } else {
+    for_each_key<true>(src, count, [&](int i, unsigned key) {
+      mine = max(mine, key);
+      append(i, key);
+    });
+  }
+  if (count > kSortCap) __syncthreads();
+  else largest = block_max_u32(mine, sm.red);
   const int m = (int)*sm.counter;
-  if (m >= want && m <= kSortCap) { select_from_list(m, want, sm, pivot); return; }
+  if (m >= want && m <= kSortCap) { select_from_list(m, want, sm, pivot, largest); return; }
   select_slow(src, count, want, sm);
 }
 
@@ -243,8 +352,7 @@ __device__ __forceinline__ void select_slow(const Src& src, int count, int want,
   const int per = (words + kSelThreads - 1) / kSelThreads, w0 = t * per, w1 = min(w0 + per, words);
   unsigned mine = 0u;
   for (int w = w0; w < w1; ++w) mine += __popc(ties[w]);
-  unsigned total = 0u;
-  unsigned before = block_exclusive_scan(mine, sm.red, &total);
+  unsigned before = block_exclusive_scan(mine, sm.red);
   for (int w = w0; w < w1 && before < need; ++w) {
     unsigned e = ties[w];
     const unsigned c = __popc(e);
@@ -267,8 +375,7 @@ __device__ __forceinline__ void select_emit(const Src& src, int count, const Sel
   const int per = (words + kSelThreads - 1) / kSelThreads, w0 = t * per, w1 = min(w0 + per, words);
   unsigned mine = 0u;
   for (int w = w0; w < w1; ++w) mine += __popc(sm.bitmap[w]);
-  unsigned total = 0u;
-  unsigned at = block_exclusive_scan(mine, sm.red, &total);
+  unsigned at = block_exclusive_scan(mine, sm.red);
   for (int w = w0; w < w1; ++w) {
     unsigned m = sm.bitmap[w];
     while (m) {
@@ -287,12 +394,15 @@ __device__ __forceinline__ SelectSmem carve(unsigned char* raw, int max_count) {
   sm.bitmap = reinterpret_cast<unsigned*>(raw + (size_t)kSortCap * 8);
   sm.red = sm.bitmap + ((max_count + 31) >> 5);
   sm.counter = sm.red + 33;
+  sm.found = reinterpret_cast<int*>(sm.counter + 1);
+  sm.hist = sm.found + 3;
+  sm.ties = reinterpret_cast<uint2*>(raw + (size_t)kSortCap * 8 + (((size_t)((max_count + 31) / 32) + 33 + 1 + 3 + kBins) * 4 + 7) / 8 * 8);
   return sm;
 }
-static size_t select_smem_bytes(int max_count) { return (size_t)kSortCap * 8 + (size_t)((max_count + 31) / 32) * 4 + 34 * 4 + 16; }
+static size_t select_smem_bytes(int max_count) { return (size_t)kSortCap * 8 + ((size_t)((max_count + 31) / 32) + 37 + kBins) * 4 + 8 + (size_t)kRankCap * 8; }
 
 // grid (rows, spans): the selection of one row.
-__global__ void __launch_bounds__(kSelThreads) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
+__global__ void __launch_bounds__(kSelThreads, 2) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
   extern __shared__ __align__(16) unsigned char raw[];
   pdl_release();
   pdl_wait();
@@ -302,7 +412,7 @@ __global__ void __launch_bounds__(kSelThreads) qsa_topk_kernel(const __grid_cons
   const int nb = (a.pos0 + r + 1) / 4;
   if (nb <= CR_SEL_BLOCKS) { if (threadIdx.x == 0) a.nsel[r] = -1; return; }
   const SelectSmem sm = carve(raw, max_count);
-  const RowSource src{a.scores + (size_t)r * a.sstride, 0};
+  const RowSource src = row_source(a, r, 0);
   select_mark(src, nb, CR_SEL_BLOCKS, sm);
   select_emit(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
   if (threadIdx.x == 0) a.nsel[r] = CR_SEL_BLOCKS;
@@ -372,7 +482,10 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
     mine = u[k] > mine ? u[k] : mine;
   }
   const int words = (nb + 31) >> 5;
-  if (rank == 0) for (int i = t; i < words; i += kSelThreads) sm.bitmap[i] = 0u;
+  if (rank == 0) {
+    for (int i = t; i < words; i += kSelThreads) sm.bitmap[i] = 0u;
+    for (int i = t; i < kBins; i += kSelThreads) sm.hist[i] = 0;
+  }
   if (t == 0) *sm.counter = 0u;
   const unsigned sorted = warp_sort_desc(mine);
   if (l < 4) top4[(t >> 5) * 4 + l] = sorted;
@@ -422,7 +535,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
       }
     }
     __syncthreads();
-    const RowSource src{sc, 0};
+    const RowSource src = row_source(a, r, 0);
     if (total >= CR_SEL_BLOCKS && total <= kSortCap) select_from_list(total, CR_SEL_BLOCKS, sm, pivot, largest);
     else select_slow(src, nb, CR_SEL_BLOCKS, sm);
     select_emit(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
@@ -432,7 +545,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
 }
 
 // A rank's candidates among blocks [b0, b1): its best 512 (score, id), ascending id, unused slots -1.
-__global__ void __launch_bounds__(kSelThreads) qsa_candidates_kernel(const __grid_constant__ QsaParams P, int b0, int b1, float* cand_scores,
+__global__ void __launch_bounds__(kSelThreads, 2) qsa_candidates_kernel(const __grid_constant__ QsaParams P, int b0, int b1, float* cand_scores,
                                                                      int* cand_ids, int max_count) {
   extern __shared__ __align__(16) unsigned char raw[];
   const cr_qsa_args& a = P.span[0];
@@ -450,7 +563,7 @@ __global__ void __launch_bounds__(kSelThreads) qsa_candidates_kernel(const __gri
     return;
   }
   const SelectSmem sm = carve(raw, max_count);
-  const RowSource src{a.scores + (size_t)r * a.sstride + b0, b0};
+  const RowSource src = row_source(a, r, b0);
   select_mark(src, count, CR_SEL_BLOCKS, sm);
   select_emit(src, count, sm, ci, cs);
 }

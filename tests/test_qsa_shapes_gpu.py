@@ -99,3 +99,31 @@ def test_union_lists_past_one_bitmap_window(pos0, R):
             for b in blocks:
                 want[int(b)] = want.get(int(b), 0) | 1 << (r - t * RT)
         np.testing.assert_array_equal(got[t, :int(cnt[t])], np.array(sorted(want.items()), np.int32))
+
+
+# histogram levels of the selection: everything in one bin, crowded bins that are divided, many equal keys around the
+# threshold, an outlier that leaves the window below the largest key empty; rows read four elements at a time and singly
+@pytest.mark.parametrize("nb", [600, 4096, 4097, 9001, 20000])
+@pytest.mark.parametrize("pattern", ["close", "steps", "outlier", "zeros", "ramp"])
+def test_selection_threshold_patterns(nb, pattern):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(nb)
+    u = torch.rand(3, nb, device="cuda", generator=gen)
+    sc = {"close": 1.0 + u * 1e-5, "steps": (u * 7).floor() / 7, "outlier": u * 1e-6, "zeros": torch.where(u < 0.95, torch.zeros_like(u), u),
+          "ramp": torch.arange(nb, device="cuda").expand(3, nb) * 1e-3}[pattern]
+    if pattern == "outlier":
+        sc[:, 5] = 3e4
+    for pad in (0, 1, 4):                                            # sstride a multiple of four or not
+        s = layers.QsaSession(g, 4 * nb + 8, max_rows=3)
+        s.sstride = nb + pad
+        s.scores = torch.zeros(3, s.sstride, device="cuda")
+        s.scores[:, :nb] = sc
+        z = torch.zeros(3, 16, 512, device="cuda")
+        args = layers.qsa_args(w, s, z, z, z, z, z, 4 * nb - 1)
+        cs, ci = torch.empty(3, 512, device="cuda"), torch.empty(3, 512, device="cuda", dtype=torch.int32)
+        capi.check(capi.lib.cr_qsa_shard_candidates(C.byref(g), C.byref(args), 0, nb, capi.dptr(cs), capi.dptr(ci), None))
+        for r in range(3):
+            v = sc[r].double().cpu().numpy()
+            want = np.sort(np.lexsort((np.arange(nb), -v))[:512])
+            np.testing.assert_array_equal(ci[r].cpu().numpy(), want)
+            np.testing.assert_array_equal(cs[r].cpu().numpy(), sc[r].cpu().numpy()[want])
