@@ -45,14 +45,18 @@ inline cr_status once_per_device(PerDeviceOnce& f, F&& fn) {
 const cr_options& options();
 inline bool pdl_enabled() { return options().pdl != 0; }
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_chained(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_chained(pdl_enabled(), kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 
@@ -101,10 +105,29 @@ int proj_gemm_status_read();  void proj_gemm_status_clear();
 
 // ---- device math ---------------------------------------------------------------------------------
 __device__ __forceinline__ float round_h(float v) { return __half2float(__float2half_rn(v)); }
-// __fdividef: reciprocal + multiply (2 ulp), instead of the IEEE division sequence; the denominators lie in [1, inf].
-__device__ __forceinline__ float sigmoidf_(float v) { return __fdividef(1.f, 1.f + __expf(-v)); }
-__device__ __forceinline__ float siluf_(float v) { return __fdividef(v, 1.f + __expf(-v)); }
+// Base-2 exponential, reciprocal and inverse square root as one instruction each: the special-function unit's own results
+// (2 ulp, 1 ulp, 2 ulp), without the range fix-ups that __expf, __fdividef and rsqrtf put around it for denormals.  Where
+// these are used a denormal argument or result stands beside a 1 or an epsilon.
+__device__ __forceinline__ float ex2_ftz(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float rcp_ftz(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float rsqrt_ftz(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+constexpr float kLog2e = 1.4426950408889634f;
+// The denominators lie in [1, inf].
+__device__ __forceinline__ float sigmoidf_(float v) { return rcp_ftz(1.f + ex2_ftz(v * -kLog2e)); }
+__device__ __forceinline__ float siluf_(float v) { return v * sigmoidf_(v); }
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t u) { return __uint_as_float((uint32_t)u << 16); }
+
+// Two fp32 lanes in one 64-bit register: half the instructions of a row update.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float x, float y) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y)); return r; }
+__device__ __forceinline__ float2 unpack2(f2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ void load_f2x2(const float* p, f2& a, f2& b) {      // four floats, 16-byte aligned
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  a = v.x; b = v.y;
+}
 
 // Round to tf32 (10-bit mantissa, nearest, ties away): the tensor-core unit ignores the low 13 bits of an
 // fp32 operand, so operands are rounded when they are written.  Integer add + mask gives the same bits as
@@ -112,6 +135,9 @@ __device__ __forceinline__ float bf16_bits_to_float(uint16_t u) { return __uint_
 // rate of the special-function unit (about one warp instruction per 7 cycles per scheduler, measured), which
 // made it the longest part of every epilogue that used it.
 __device__ __forceinline__ float tf32r(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
+
+// The same rounding of a value that only a tensor core reads: the low 13 bits, which it ignores, stay as they are.
+__device__ __forceinline__ float tf32_operand(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

@@ -10,15 +10,19 @@
 //      in block-row order), then W = T (beta e^G K) and Ut = T (beta V) on tensor cores with tf32 operands; the
 //      v columns run conv + SiLU from the staged raw rows.
 // Outputs go straight into the layouts the scan consumes (K-major tiles for the tcgen05 scan).
-// Two CTAs fit per SM (110 KB of shared memory, 128 registers x 256 threads each), so one CTA's barriers and loads
-// hide behind the other's math.
+// Two CTAs of 16 warps fit per SM (113 KB of shared memory, 64 registers x 512 threads each).  With 8 warps each a phase
+// lasted about as long alone on an SM as beside another CTA: latency of shuffles, shared-memory loads and barriers, not
+// issue slots, set the pace.  With 16 warps, pairs of fp32 in one instruction, the norms taken from registers and products
+// of the inverse reading both factors 16 bytes at a time the kernel issues 60 % of the time.  7,104 rows, 16 / 32 heads:
+// 256 -> 232 us; 333 rows 36 -> 26 us; 64 rows 32 -> 16 us; 1,999 fp32 rows, 16 / 48 heads: 131 -> 120 us.
 #include "gdn_chunk.cuh"
 
 namespace cr {
 
 constexpr int kRawRows = 67;                               // 64 rows + 3 halo rows
 constexpr int kStageBytes = kRawRows * 128 * 2;            // one 128-channel bf16 tile (or 64 fp32 channels)
-constexpr size_t kLocalSmem = (size_t)(64 * kLdK + 64 * kLdX + 64 * kLdM + 15 * 64 + 3 * 256) * sizeof(float) + kStageBytes + 256;
+constexpr int kLocalThreads = 512;
+constexpr size_t kLocalSmem = (size_t)(64 * kLdK + 64 * kLdX + 64 * kLdM + 15 * 64 + 8 * 256) * sizeof(float) + kStageBytes + 256;
 
 // Starts the copy of rows row0-3 .. row0+63 of channels [ch0, ch0+CH) into dst[67][CH] (element type of the input)
 // as one cp.async group; rows past the end of the call are zero-filled.  Rows before the call come from the input
@@ -27,155 +31,192 @@ template <bool BF16, int CH>
 __device__ __forceinline__ void stage_issue(const GdnPrefillParams& P, int C, int row0, int ch0, void* dst) {
   constexpr int EPV = BF16 ? 8 : 4;                        // elements per 16-byte piece
   constexpr int PPR = CH / EPV;                            // pieces per row
+  constexpr int RPP = kLocalThreads / PPR;                 // rows per pass
   const cr_gdn_args& a = P.a;
-  for (int i = threadIdx.x; i < kRawRows * PPR; i += 256) {
-    const int rr = i / PPR, pc = i % PPR, r = row0 - 3 + rr, ch = ch0 + pc * EPV;
-    uint4* d = reinterpret_cast<uint4*>(dst) + i;
+  const int pc = threadIdx.x % PPR, rr0 = threadIdx.x / PPR;
+  uint4* d = reinterpret_cast<uint4*>(dst) + threadIdx.x;
+  const char* src = reinterpret_cast<const char*>(a.qkv) + ((long long)(row0 - 3 + rr0) * C + ch0 + pc * EPV) * (BF16 ? 2 : 4);
+  const long long step = (long long)RPP * C * (BF16 ? 2 : 4);
+#pragma unroll
+  for (int k = 0; k * RPP < kRawRows; ++k, src += step) {
+    const int rr = rr0 + k * RPP, r = row0 - 3 + rr;
+    if ((k + 1) * RPP > kRawRows && rr >= kRawRows) break;
     if (r >= 0 || P.halo_in) {
-      const bool valid = r < a.R;
-      cp_async16(d, reinterpret_cast<const char*>(a.qkv) + (valid ? ((long long)r * C + ch) * (BF16 ? 2 : 4) : 0ll), valid);
+      cp_async16(d + k * kLocalThreads, r < a.R ? src : reinterpret_cast<const char*>(a.qkv), r < a.R);
     } else {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (a.pos0 + r >= 0) {
-        const float* hs = a.hist + (size_t)((a.pos0 + r) & 15) * C + ch;
+        const float* hs = a.hist + (size_t)((a.pos0 + r) & 15) * C + ch0 + pc * EPV;
         if constexpr (BF16) {
           __nv_bfloat162 b[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) b[k] = __floats2bfloat162_rn(hs[2 * k], hs[2 * k + 1]);
+          for (int i = 0; i < 4; ++i) b[i] = __floats2bfloat162_rn(hs[2 * i], hs[2 * i + 1]);
           v = *reinterpret_cast<const uint4*>(b);
         } else {
           v = *reinterpret_cast<const uint4*>(hs);
         }
       }
-      *d = v;
+      d[k * kLocalThreads] = v;
     }
   }
   cp_async_commit();
 }
-template <bool BF16, int CH>
-__device__ __forceinline__ void stage_raw(const GdnPrefillParams& P, int C, int row0, int ch0, void* dst) {
-  stage_issue<BF16, CH>(P, C, row0, ch0, dst);
-  cp_async_wait_all();
-}
 template <bool BF16>
-__device__ __forceinline__ float2 staged_pair(const void* buf, int CH, int rr, int ch) {
-  if constexpr (BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const __nv_bfloat16*>(buf) + rr * CH + ch));
-  else return *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(buf) + rr * CH + ch);
-}
-template <bool BF16>
-__device__ __forceinline__ float staged_one(const void* buf, int CH, int rr, int ch) {
-  if constexpr (BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(buf)[rr * CH + ch]);
-  else return reinterpret_cast<const float*>(buf)[rr * CH + ch];
+__device__ __forceinline__ f2 staged_pair(const void* buf, int CH, int rr, int ch) {
+  if constexpr (BF16) {
+    const unsigned v = *reinterpret_cast<const unsigned*>(reinterpret_cast<const __nv_bfloat16*>(buf) + rr * CH + ch);
+    return pack2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u));
+  } else {
+    return *reinterpret_cast<const f2*>(reinterpret_cast<const float*>(buf) + rr * CH + ch);
+  }
 }
 
-// T = (I + L)^-1 for the 64x64 unit lower-triangular I + L held in LT, exact fp32, in place, by 16x16 blocks:
-// diagonal blocks by forward substitution (one thread per column, column in registers), then block row by block
-// row, T_ab = -T_aa (sum_{c=b}^{a-1} L_ac T_cb): every phase is a product of 16-long unrolled dot products with
-// all 256 threads busy (thread = element (t/16, t%16) of each block of the row).
-__device__ __forceinline__ void invert_unit_lower_64(float* LT, float* Ms) {
-  const int t = threadIdx.x, i = t >> 4, j = t & 15;
+// conv(4) + SiLU of two channels (conv row ch, staged column col) over N rows from the staged rows of a tile.
+template <bool BF16, int N>
+__device__ __forceinline__ void conv_rows(const float* conv, int ch, const void* src, int CH, int row, int col, f2 (&out)[N]) {
+  const float4 w0 = *reinterpret_cast<const float4*>(conv + (size_t)ch * 4), w1 = *reinterpret_cast<const float4*>(conv + (size_t)(ch + 1) * 4);
+  const f2 t0 = pack2(w0.x, w1.x), t1 = pack2(w0.y, w1.y), t2 = pack2(w0.z, w1.z), t3 = pack2(w0.w, w1.w);
+  f2 x0 = staged_pair<BF16>(src, CH, row, col), x1 = staged_pair<BF16>(src, CH, row + 1, col), x2 = staged_pair<BF16>(src, CH, row + 2, col);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const f2 x3 = staged_pair<BF16>(src, CH, row + 3 + i, col);       // staged row index = chunk row + 3
+    const f2 c = fma2(t3, x3, fma2(t2, x2, fma2(t1, x1, mul2(t0, x0))));
+    const float2 e = unpack2(mul2(c, pack2(-kLog2e, -kLog2e)));
+    const float2 d = unpack2(add2(pack2(ex2_ftz(e.x), ex2_ftz(e.y)), pack2(1.f, 1.f)));
+    out[i] = mul2(c, pack2(rcp_ftz(d.x), rcp_ftz(d.y)));
+    x0 = x1; x1 = x2; x2 = x3;
+  }
+}
+// Sums of eight values over the warp; lane l returns the sum of value l >> 2.
+__device__ __forceinline__ float warp_sum8(float (&s)[8]) {
+  const int l = threadIdx.x & 31;
+#pragma unroll
+  for (int k = 4; k >= 1; k >>= 1) {      // a lane keeps the half of the values that its bit of l >> 2 names
+    const bool up = (l >> 2) & k;
+#pragma unroll
+    for (int i = 0; i < k; ++i) {
+      const float keep = up ? s[i + k] : s[i], give = up ? s[i] : s[i + k];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * k);
+    }
+  }
+  float v = s[0];
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// T = (I + L)^-1 for the 64x64 unit lower-triangular I + L held in LT, in place, exact fp32, rounded to tf32 at the very
+// end.  The diagonal 16 x 16 blocks come first (invert_diagonal: one thread per column by forward substitution, the two
+// warps that do it need no barrier).  Then blocks (1,0) and (3,2), then the 32 x 32 block below the diagonal, each as
+// T_ab = -T_aa (L_ab T_bb): a product per phase, all 512 threads busy.  What a product reads down a column is kept
+// transposed as well, so that both factors come four to a load.
+//
+// Transposed 16 x 16 blocks: row j (a column of T), 16-byte unit u at u ^ (j / 2), free of bank conflicts for 16 rows.
+__device__ __forceinline__ float* tr16(float* block, int j, int u) { return block + j * 16 + ((u ^ (j >> 1)) & 3) * 4; }
+__device__ __forceinline__ void invert_diagonal(float* LT, float* Tt) {   // t < 64; Tt: T_00, T_11, T_22 and then T_10, transposed
+  const int b = threadIdx.x >> 4, j = threadIdx.x & 15;
+  float* B = LT + 16 * b * kLdM + 16 * b;
   float D[16];
-  if (t < 64) {
-    const int b = t >> 4;
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      float acc = (r == j) ? 1.f : 0.f;
+  for (int r = 0; r < 16; ++r) {
+    float acc = (r == j) ? 1.f : 0.f;
 #pragma unroll
-      for (int m = 0; m < r; ++m) acc = fmaf(-LT[(16 * b + r) * kLdM + 16 * b + m], D[m], acc);
-      D[r] = acc;
-    }
+    for (int m = 0; m < r; ++m) acc = fmaf(-B[r * kLdM + m], D[m], acc);
+    D[r] = acc;
   }
-  __syncthreads();
-  if (t < 64) {
-    const int b = t >> 4;
+  __syncwarp();                          // both blocks of the warp have been read
 #pragma unroll
-    for (int r = 0; r < 16; ++r) LT[(16 * b + r) * kLdM + 16 * b + j] = D[r];
+  for (int r = 0; r < 16; ++r) B[r * kLdM + j] = D[r];
+  if (b < 3)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) *reinterpret_cast<float4*>(tr16(Tt + b * 256, j, u)) = make_float4(D[4 * u], D[4 * u + 1], D[4 * u + 2], D[4 * u + 3]);
+}
+// acc += sum over m < 16 of a[m] times row j of a transposed block, even and odd m apart
+__device__ __forceinline__ f2 dot16(f2 acc, const float* a, float* block, int j) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    f2 a0, a1, b0, b1;
+    load_f2x2(a + 4 * u, a0, a1);
+    load_f2x2(tr16(block, j, u), b0, b1);
+    acc = fma2(a1, b1, fma2(a0, b0, acc));
   }
-  __syncthreads();
-  for (int a = 1; a < 4; ++a) {          // block row a: its L blocks are still untouched
-    float macc[3] = {0.f, 0.f, 0.f};     // M_ab = sum_{c=b}^{a-1} L_ac T_cb for b = 0 .. a-1; L_ac[i][m] is read once
-#pragma unroll
-    for (int cb = 0; cb < 3; ++cb) {
-      if (cb < a) {
-        const float* Lr = LT + (16 * a + i) * kLdM + 16 * cb;
-#pragma unroll
-        for (int m4 = 0; m4 < 16; m4 += 4) {
-          const float4 lv = *reinterpret_cast<const float4*>(Lr + m4);
-          const float lm[4] = {lv.x, lv.y, lv.z, lv.w};
-#pragma unroll
-          for (int mm = 0; mm < 4; ++mm) {
-            const float* Tc = LT + (16 * cb + m4 + mm) * kLdM + j;
-#pragma unroll
-            for (int b = 0; b < 3; ++b)
-              if (b <= cb) macc[b] = fmaf(lm[mm], Tc[16 * b], macc[b]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      if (b < a) Ms[b * 256 + t] = macc[b];
+  return acc;
+}
+__device__ __forceinline__ float sum2(f2 v) { const float2 x = unpack2(v); return x.x + x.y; }
+__device__ __forceinline__ void round_quadrant(float* Q) {   // 32 x 32 at Q, two elements per thread
+  float2* p = reinterpret_cast<float2*>(Q + (threadIdx.x >> 4) * kLdM + 2 * (threadIdx.x & 15));
+  const float2 v = *p;
+  *p = make_float2(tf32_operand(v.x), tf32_operand(v.y));
+}
+__device__ __forceinline__ void invert_unit_lower_64(float* LT, float* Tt, float* Ms) {   // after a barrier behind invert_diagonal
+  const int t = threadIdx.x, half = t >> 8, i = (t >> 4) & 15, j = t & 15;
+  auto put = [&](float* block, float v) { tr16(block, j, i >> 2)[i & 3] = v; };   // element (i, j)
+  {
+    const float* row = LT + (32 * half + 16 + i) * kLdM + 32 * half;
+    put(Ms + half * 256, sum2(dot16(0ull, row, Tt + half * 512, j)));
     __syncthreads();
-    {                                    // T_ab = -T_aa M_ab  (T_aa lower triangular: m <= i); the T_aa row is read once
-      const float* Tr = LT + (16 * a + i) * kLdM + 16 * a;
-      float tr[16];
-#pragma unroll
-      for (int m4 = 0; m4 < 16; m4 += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(Tr + m4);
-        tr[m4] = m4 <= i ? v.x : 0.f; tr[m4 + 1] = m4 + 1 <= i ? v.y : 0.f;
-        tr[m4 + 2] = m4 + 2 <= i ? v.z : 0.f; tr[m4 + 3] = m4 + 3 <= i ? v.w : 0.f;
-      }
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        if (b < a) {
-          const float* Mc = Ms + b * 256 + j;
-          float m0 = 0.f, m1 = 0.f;
-#pragma unroll
-          for (int m = 0; m < 16; m += 2) {
-            m0 = fmaf(tr[m], Mc[m * 16], m0);
-            m1 = fmaf(tr[m + 1], Mc[(m + 1) * 16], m1);
-          }
-          LT[(16 * a + i) * kLdM + 16 * b + j] = -(m0 + m1);
-        }
-      }
-    }
+    const float v = -sum2(dot16(0ull, row + 16, Ms + half * 256, j));
+    LT[(32 * half + 16 + i) * kLdM + 32 * half + j] = v;
+    if (half == 0) put(Tt + 768, v);
+    __syncthreads();
+  }
+  {   // a thread has rows 32 + i and 48 + i of one column; columns 16-31 meet a zero block of T in the first product
+    const float *hi = LT + (32 + i) * kLdM, *lo = LT + (48 + i) * kLdM;
+    f2 m0 = 0ull, m1 = 0ull;
+    if (half == 0) { m0 = dot16(m0, hi, Tt, j); m1 = dot16(m1, lo, Tt, j); }
+    float* below = Tt + (half == 0 ? 768 : 256);
+    put(Ms + half * 512, sum2(dot16(m0, hi + 16, below, j)));
+    put(Ms + half * 512 + 256, sum2(dot16(m1, lo + 16, below, j)));
+    __syncthreads();
+    const float t0 = -sum2(dot16(0ull, hi + 32, Ms + half * 512, j));
+    const float t1 = -sum2(dot16(dot16(0ull, lo + 32, Ms + half * 512, j), lo + 48, Ms + half * 512 + 256, j));
+    LT[(32 + i) * kLdM + 16 * half + j] = tf32_operand(t0);
+    LT[(48 + i) * kLdM + 16 * half + j] = tf32_operand(t1);
+    round_quadrant(LT);
+    __syncthreads();
+    round_quadrant(LT + 32 * kLdM + 32);
     __syncthreads();
   }
 }
 
 // Operands for the tcgen05 scan are written as K-major tiles float[K/4][rows][4] (plus Qt = e^G Q and K'^T).
 template <bool BF16>
-__global__ void __launch_bounds__(256, 2) gdn_chunk_local_kernel(GdnPrefillParams P, ChunkWs ws) {
+__global__ void __launch_bounds__(kLocalThreads, 2) gdn_chunk_local_kernel(GdnPrefillParams P, ChunkWs ws) {
   extern __shared__ __align__(16) float sm[];
   float* Ks = sm;                       // [64][132] khat (tf32)
   float* Qs = Ks + 64 * kLdK;           // [64][132] qhat (tf32), later [64][136] X = beta e^G K / beta V
   char* RB = reinterpret_cast<char*>(Qs + 64 * kLdX);      // raw staging tile
-  float* LT = reinterpret_cast<float*>(RB + kStageBytes);  // [64][68] L
+  float* LT = reinterpret_cast<float*>(RB + kStageBytes);  // [64][68] L, then T
   float* Gs = LT + 64 * kLdM;           // [3][64] cumulative log decay per value head
   float* bs = Gs + 3 * 64;              // [3][64] beta
   float* es = bs + 3 * 64;              // [3][64] beta * exp(G)
   float* egs = es + 3 * 64;             // [3][64] exp(G)
   float* scs = egs + 3 * 64;            // [3][64] exp(G_end - G)
-  float* Ms = scs + 3 * 64;             // [3][256] scratch of the blocked inverse
+  float* Ms = scs + 3 * 64;             // [4][16][16] scratch of the blocked inverse; first the partial sums of the L2 norms
+  float* Tt = Ms + 4 * 256;             // [4][16][16] blocks of T, transposed
   const cr_gdn_args& a = P.a;
   const int c = blockIdx.x, kh = blockIdx.y;
   const int t = threadIdx.x, w = t >> 5, l = t & 31, g = l >> 2, tq = l & 3;
   const int R = a.R, r0 = c * kChunk, valid = min(kChunk, R - r0);
   const int rep = P.Hv / P.Hk, KW = P.Hk * 128, VW = P.Hv * 128, C = 2 * KW + VW;
-  constexpr int CH = BF16 ? 128 : 64;   // channels per staging round
-  constexpr int PAIRS = CH / 2, RSEG = 256 / PAIRS, RPT = 64 / RSEG;
+  const int v_first = rep * (int)blockIdx.z / (int)gridDim.z, v_last = rep * ((int)blockIdx.z + 1) / (int)gridDim.z;   // value heads of this CTA
+  constexpr int VCH = BF16 ? 128 : 64;  // channels of v per staging round
 
-  // ---- 1. q and k of the key head.  With bf16 inputs a whole 128-channel tile is one staging round: q goes to the
-  // staging tile and k to the (still unused) L tile, both in flight at once; the first v tile follows as soon as
-  // the staging tile is free, so its latency hides behind the Gram products.
+  pdl_release();
+  pdl_wait();
+  // ---- 1. q and k of the key head, raw rows of both in flight at once: bf16 rows of q in the staging tile and of k in
+  // the (still unused) L tile; fp32 rows of q as two 64-channel halves in those two and of k in the place of qhat.
   char* RB2 = reinterpret_cast<char*>(LT);
   if constexpr (BF16) {
     stage_issue<true, 128>(P, C, r0, kh * 128, RB);
     stage_issue<true, 128>(P, C, r0, KW + kh * 128, RB2);
+  } else {
+    stage_issue<false, 64>(P, C, r0, kh * 128, RB);
+    stage_issue<false, 64>(P, C, r0, kh * 128 + 64, RB2);
+    stage_issue<false, 128>(P, C, r0, KW + kh * 128, Qs);
   }
   // Gates while the first tiles are in flight: g = -exp(A_log) softplus(a + dt_bias), beta = sigmoid(b), prefix sum of
   // g inside the chunk; one warp per value head.  The tables are read after later barriers.
-  if (w < rep) {
+  if (w >= v_first && w < v_last) {
     const int h = kh * rep + w;
     const float A = -expf(a.A_log[h]), dtb = a.dt_bias[h];
     float gv[2], bv[2];
@@ -205,182 +246,160 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_local_kernel(GdnPrefillParam
     float* Gg = ws.G + ((size_t)h * ws.chunks + c) * 64;
     Gg[2 * l] = G0; Gg[2 * l + 1] = G1;
   }
+  // A thread has two channels of eight rows, of q and of k: conv, SiLU and its share of the row sums stay in registers
+  // until the two warps that share a row have exchanged their sums.
+  const int pair = t & 63, rb = (t >> 6) * 8, ch2 = 2 * pair;
+  f2 val[2][8];
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    if (part == 0) cp_async_wait_but_one(); else cp_async_wait_all();   // k is the last group
+    __syncthreads();
+    if constexpr (BF16) conv_rows<true>(a.conv, (part ? KW : 0) + kh * 128 + ch2, part ? RB2 : RB, 128, rb, ch2, val[part]);
+    else if (part) conv_rows<false>(a.conv, KW + kh * 128 + ch2, Qs, 128, rb, ch2, val[1]);
+    else conv_rows<false>(a.conv, kh * 128 + ch2, pair < 32 ? RB : RB2, 64, rb, ch2 & 63, val[0]);
+    float s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = sum2(mul2(val[part][i], val[part][i]));
+    const float sum = warp_sum8(s);     // of row rb + (l >> 2)
+    if ((l & 3) == 0) Ms[part * 128 + (rb + (l >> 2)) * 2 + (w & 1)] = sum;
+  }
+  __syncthreads();
+  // The raw rows have been read: v of the first value head may come in.
+  stage_issue<BF16, VCH>(P, C, r0, 2 * KW + (kh * rep + v_first) * 128, RB);
+  // L2 norms, scale, round to tf32; rows past the end are zero.  Lane 8 part + i has the factor of row rb + i.
+  const float2 sums = *reinterpret_cast<const float2*>(Ms + (l >> 3 & 1) * 128 + (rb + (l & 7)) * 2);
+  const float norm = rb + (l & 7) < valid ? rsqrt_ftz(sums.x + sums.y + kEps) * (l & 8 ? 1.f : kInvSqrt128) : 0.f;
+#pragma unroll
   for (int part = 0; part < 2; ++part) {
     float* dst = part ? Ks : Qs;
-    for (int round = 0; round < 128 / CH; ++round) {
-      const char* src = RB;
-      if constexpr (BF16) {
-        if (part == 0) cp_async_wait_but_one(); else cp_async_wait_all();
-        __syncthreads();
-        src = part ? RB2 : RB;
-      } else {
-        __syncthreads();                // staging tile free
-        stage_raw<BF16, CH>(P, C, r0, (part ? KW : 0) + kh * 128 + round * CH, RB);
-        __syncthreads();
-      }
-      const int cp = t % PAIRS, seg = t / PAIRS, chl = 2 * cp, chg = (part ? KW : 0) + kh * 128 + round * CH + chl;
-      const float4 w0 = *reinterpret_cast<const float4*>(a.conv + (size_t)chg * 4);
-      const float4 w1 = *reinterpret_cast<const float4*>(a.conv + (size_t)(chg + 1) * 4);
-      const int rb = seg * RPT;         // first chunk row of this thread; staged row index = chunk row + 3
-      float2 x0 = staged_pair<BF16>(src, CH, rb, chl), x1 = staged_pair<BF16>(src, CH, rb + 1, chl), x2 = staged_pair<BF16>(src, CH, rb + 2, chl);
 #pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        const float2 x3 = staged_pair<BF16>(src, CH, rb + 3 + i, chl);
-        float c0 = w0.x * x0.x, c1 = w1.x * x0.y;
-        c0 = fmaf(w0.y, x1.x, c0); c1 = fmaf(w1.y, x1.y, c1);
-        c0 = fmaf(w0.z, x2.x, c0); c1 = fmaf(w1.z, x2.y, c1);
-        c0 = fmaf(w0.w, x3.x, c0); c1 = fmaf(w1.w, x3.y, c1);
-        const bool live = rb + i < valid;
-        *reinterpret_cast<float2*>(dst + (rb + i) * kLdK + round * CH + chl) = make_float2(live ? siluf_(c0) : 0.f, live ? siluf_(c1) : 0.f);
-        x0 = x1; x1 = x2; x2 = x3;
-      }
+    for (int i = 0; i < 8; ++i) {
+      const float sc = __shfl_sync(0xffffffffu, norm, 8 * part + i);
+      const float2 o = unpack2(mul2(val[part][i], pack2(sc, sc)));
+      *reinterpret_cast<float2*>(dst + (rb + i) * kLdK + ch2) = make_float2(tf32r(o.x), tf32r(o.y));
     }
   }
   __syncthreads();
-  if constexpr (BF16) stage_issue<true, 128>(P, C, r0, 2 * KW + kh * rep * 128, RB);   // v of the first value head
-  for (int i = t; i < 64 * 32; i += 256) {   // L2 norms (a warp holds one row), scale, round to tf32
-    const int row = i >> 5, c4 = (i & 31) * 4;
-    float4 q = *reinterpret_cast<float4*>(Qs + row * kLdK + c4), k = *reinterpret_cast<float4*>(Ks + row * kLdK + c4);
-    float sq = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w, sk = k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w;
+  // per value head: K'^T = (e^{G_end - G} K)^T, K-major over tokens (unit (token / 4, key) holds 4 tokens of one
+  // key; the decay towards the chunk end is folded into K so that the scan multiplies U itself), and
+  // Qt = e^G Q, K-major over keys
+  for (int vi = v_first; vi < v_last; ++vi) {
+    float* kt = ws.Kt + ((size_t)(kh * rep + vi) * ws.chunks + c) * 8192;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      sk += __shfl_xor_sync(0xffffffffu, sk, o);
+    for (int k = 0; k < 4; ++k) {
+      const int key = t & 127, tc = (t >> 7) + 4 * k;
+      const float4 sc = *reinterpret_cast<const float4*>(scs + vi * 64 + 4 * tc);
+      const float* K = Ks + 4 * tc * kLdK + key;
+      *reinterpret_cast<float4*>(kt + (size_t)(tc * 128 + key) * 4) =
+          make_float4(tf32_operand(sc.x * K[0]), tf32_operand(sc.y * K[kLdK]), tf32_operand(sc.z * K[2 * kLdK]), tf32_operand(sc.w * K[3 * kLdK]));
     }
-    sq = rsqrtf(sq + kEps) * kInvSqrt128;
-    sk = rsqrtf(sk + kEps);
-    q = make_float4(tf32r(q.x * sq), tf32r(q.y * sq), tf32r(q.z * sq), tf32r(q.w * sq));
-    k = make_float4(tf32r(k.x * sk), tf32r(k.y * sk), tf32r(k.z * sk), tf32r(k.w * sk));
-    *reinterpret_cast<float4*>(Qs + row * kLdK + c4) = q;
-    *reinterpret_cast<float4*>(Ks + row * kLdK + c4) = k;
-  }
-  __syncthreads();
-  {
-    // per value head: K'^T = (e^{G_end - G} K)^T, K-major over tokens (unit (token / 4, key) holds 4 tokens of one
-    // key; the decay towards the chunk end is folded into K so that the scan multiplies U itself), and
-    // Qt = e^G Q, K-major over keys
-    for (int vi = 0; vi < rep; ++vi) {
-      float* kt = ws.Kt + ((size_t)(kh * rep + vi) * ws.chunks + c) * 8192;
-      for (int i = t; i < 16 * 128; i += 256) {
-        const int key = i & 127, tc = i >> 7;
-        const float4 sc = *reinterpret_cast<const float4*>(scs + vi * 64 + 4 * tc);
-        *reinterpret_cast<float4*>(kt + (size_t)i * 4) =
-            make_float4(tf32r(sc.x * Ks[(4 * tc) * kLdK + key]), tf32r(sc.y * Ks[(4 * tc + 1) * kLdK + key]),
-                        tf32r(sc.z * Ks[(4 * tc + 2) * kLdK + key]), tf32r(sc.w * Ks[(4 * tc + 3) * kLdK + key]));
-      }
-      float* qt = ws.WQ + ((size_t)(kh * rep + vi) * ws.chunks + c) * 16384;
-      for (int i = t; i < 32 * 64; i += 256) {
-        const int row = i & 63, kc = i >> 6;
-        const float4 q = *reinterpret_cast<const float4*>(Qs + row * kLdK + kc * 4);
-        const float e = egs[vi * 64 + row];
-        *reinterpret_cast<float4*>(qt + (size_t)(kc * 128 + 64 + row) * 4) = make_float4(tf32r(e * q.x), tf32r(e * q.y), tf32r(e * q.z), tf32r(e * q.w));
-      }
+    float* qt = ws.WQ + ((size_t)(kh * rep + vi) * ws.chunks + c) * 16384;
+    const int row = t & 63;
+    const float e = egs[vi * 64 + row];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int kc = (t >> 6) + 8 * k;
+      const float4 q = *reinterpret_cast<const float4*>(Qs + row * kLdK + kc * 4);
+      *reinterpret_cast<float4*>(qt + (size_t)(kc * 128 + 64 + row) * 4) = make_float4(tf32_operand(e * q.x), tf32_operand(e * q.y), tf32_operand(e * q.z), tf32_operand(e * q.w));
     }
   }
-  // ---- 2. Gram matrices stay in registers: warps 0-3 hold K K^T, warps 4-7 hold Q K^T, 16 rows each
-  const int mt = w & 3;
-  float gram[8][4];
+  // ---- 2. Gram matrices stay in registers: K K^T in warps 0-3 and 8-11, Q K^T in the others, 16 rows and 32 columns each;
+  // the row blocks are dealt so that every scheduler gets one of each.
+  const int mt = (w + (w >> 2)) & 3, n_first = (w >> 3) * 4;
+  const bool is_kk = (w & 4) == 0;
+  float gram[4][4];
 #pragma unroll
-  for (int n = 0; n < 8; ++n) gram[n][0] = gram[n][1] = gram[n][2] = gram[n][3] = 0.f;
-  const int n_used = 2 * mt + 2;        // column tiles at or below the diagonal of row block mt; the rest is masked
-  warp_gemm_nk_ldm<8, 16>(gram, (w < 4 ? Ks : Qs) + mt * 16 * kLdK, kLdK, Ks, kLdK, n_used);
+  for (int n = 0; n < 4; ++n) gram[n][0] = gram[n][1] = gram[n][2] = gram[n][3] = 0.f;
+  const int n_used = 2 * mt + 2 - n_first;   // column tiles at or below the diagonal of row block mt; the rest is masked
+  if (n_used > 0) warp_gemm_nk_ldm<4, 16>(gram, (is_kk ? Ks : Qs) + mt * 16 * kLdK, kLdK, Ks + n_first * 8 * kLdK, kLdK, n_used);
 
   // ---- 3. per value head
-  for (int vi = 0; vi < rep; ++vi) {
+  for (int vi = v_first; vi < v_last; ++vi) {
     const int h = kh * rep + vi;
     const size_t unit = (size_t)h * ws.chunks + c;
     const float* Gv = Gs + vi * 64; const float* bv = bs + vi * 64; const float* ev = es + vi * 64;
-    __syncthreads();                    // previous head done with LT and the staging tile; qhat no longer needed
-    {   // L (warps 0-3) and QKd (warps 4-7) straight from the Gram fragments
+    __syncthreads();                    // previous head done with LT and X; qhat no longer needed
+    {   // L and QKd straight from the Gram fragments
       float* qkd = ws.QKp + unit * 4096;
 #pragma unroll
-      for (int n = 0; n < 8; ++n)
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int hrow = 0; hrow < 2; ++hrow) {
-          const int row = mt * 16 + g + 8 * hrow, col = n * 8 + 2 * tq;
+          const int row = mt * 16 + g + 8 * hrow, col = (n_first + n) * 8 + 2 * tq;
           if (n >= n_used) {            // above the diagonal: nothing reads L there, QKd is zero
-            if (w >= 4) *reinterpret_cast<float2*>(qkd + ((col >> 2) * 64 + row) * 4 + (col & 3)) = make_float2(0.f, 0.f);
+            if (!is_kk) *reinterpret_cast<float2*>(qkd + ((col >> 2) * 64 + row) * 4 + (col & 3)) = make_float2(0.f, 0.f);
             continue;
           }
           const float Gr = Gv[row];
-          const float p0 = __expf(fminf(Gr - Gv[col], 0.f)), p1 = __expf(fminf(Gr - Gv[col + 1], 0.f));
+          const float p0 = ex2_ftz(fminf(Gr - Gv[col], 0.f) * kLog2e), p1 = ex2_ftz(fminf(Gr - Gv[col + 1], 0.f) * kLog2e);
           const float v0 = gram[n][2 * hrow], v1 = gram[n][2 * hrow + 1];
-          if (w < 4) {
+          if (is_kk) {
             const float b = bv[row];
             *reinterpret_cast<float2*>(LT + row * kLdM + col) = make_float2(col < row ? b * v0 * p0 : 0.f, col + 1 < row ? b * v1 * p1 : 0.f);
           } else {
             const int at = ((col >> 2) * 64 + row) * 4 + (col & 3);
-            *reinterpret_cast<float2*>(qkd + at) = make_float2(col <= row ? tf32r(v0 * p0) : 0.f, col + 1 <= row ? tf32r(v1 * p1) : 0.f);
+            *reinterpret_cast<float2*>(qkd + at) = make_float2(col <= row ? tf32_operand(v0 * p0) : 0.f, col + 1 <= row ? tf32_operand(v1 * p1) : 0.f);
           }
         }
     }
-    for (int i = t; i < 64 * 32; i += 256) {   // X = beta e^G K
-      const int row = i >> 5, c4 = (i & 31) * 4;
-      const float4 kv = *reinterpret_cast<const float4*>(Ks + row * kLdK + c4);
-      const float e = ev[row];
-      *reinterpret_cast<float4*>(Qs + row * kLdX + c4) = make_float4(tf32r(e * kv.x), tf32r(e * kv.y), tf32r(e * kv.z), tf32r(e * kv.w));
-    }
-    // raw v rows of value head h, 128 channels per round with bf16 inputs (already in flight), 64 with fp32 inputs
-    constexpr int VCH = BF16 ? 128 : 64;
-    if constexpr (BF16) cp_async_wait_all();
-    else stage_raw<BF16, VCH>(P, C, r0, 2 * KW + h * 128, RB);
     __syncthreads();
-    invert_unit_lower_64(LT, Ms);       // ends with a barrier; T stays fp32 and is rounded as the products load it
-    // T is lower triangular: row block m needs k < 16 (m + 1).  A warp takes 32 columns of two row blocks, (3, 0) or
-    // (2, 1), ten k steps either way.
-    const int qn = w & 3, m_hi = w < 4 ? 3 : 2, m_lo = w < 4 ? 0 : 1;
+    if (w < 2) invert_diagonal(LT, Tt);
+    else {
+      for (int row = w - 2; row < 64; row += 14) {   // X = beta e^G K
+        const int c4 = 4 * l;
+        const float4 kv = *reinterpret_cast<const float4*>(Ks + row * kLdK + c4);
+        const float e = ev[row];
+        *reinterpret_cast<float4*>(Qs + row * kLdX + c4) = make_float4(tf32_operand(e * kv.x), tf32_operand(e * kv.y), tf32_operand(e * kv.z), tf32_operand(e * kv.w));
+      }
+    }
+    __syncthreads();
+    invert_unit_lower_64(LT, Tt, Ms);       // ends with a barrier
+    // T is lower triangular: row block m needs k < 16 (m + 1).  A warp takes 16 (or 8) columns of two row blocks, (3, 0)
+    // or (2, 1), ten k steps either way.
+    const int qn = w & 7, m_hi = w < 8 ? 3 : 2, m_lo = w < 8 ? 0 : 1;
     {   // W = T X
-      float acc[2][4][4];
+      float acc[2][2][4];
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) acc[k][n][0] = acc[k][n][1] = acc[k][n][2] = acc[k][n][3] = 0.f;
-      warp_gemm_tril_pair<4, true>(acc[0], acc[1], LT, kLdM, m_hi, m_lo, Qs + qn * 32, kLdX);
+        for (int n = 0; n < 2; ++n) acc[k][n][0] = acc[k][n][1] = acc[k][n][2] = acc[k][n][3] = 0.f;
+      warp_gemm_tril_pair<2>(acc[0], acc[1], LT, kLdM, m_hi, m_lo, Qs + qn * 16, kLdX);
       float* dst = ws.WQ + unit * 16384;
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const int col = qn * 32 + n * 8 + 2 * tq, r_lo = (k ? m_lo : m_hi) * 16 + g;
-          *reinterpret_cast<float2*>(dst + ((col >> 2) * 128 + r_lo) * 4 + (col & 3)) = make_float2(tf32r(acc[k][n][0]), tf32r(acc[k][n][1]));
-          *reinterpret_cast<float2*>(dst + ((col >> 2) * 128 + r_lo + 8) * 4 + (col & 3)) = make_float2(tf32r(acc[k][n][2]), tf32r(acc[k][n][3]));
+        for (int n = 0; n < 2; ++n) {
+          const int col = qn * 16 + n * 8 + 2 * tq, r_lo = (k ? m_lo : m_hi) * 16 + g;
+          *reinterpret_cast<float2*>(dst + ((col >> 2) * 128 + r_lo) * 4 + (col & 3)) = make_float2(tf32_operand(acc[k][n][0]), tf32_operand(acc[k][n][1]));
+          *reinterpret_cast<float2*>(dst + ((col >> 2) * 128 + r_lo + 8) * 4 + (col & 3)) = make_float2(tf32_operand(acc[k][n][2]), tf32_operand(acc[k][n][3]));
         }
     }
-    __syncthreads();                    // X = beta e^G K consumed
-    for (int round = 0; round < 128 / VCH; ++round) {   // X = beta SiLU(conv(v)) from the staged raw rows
-      if (round) {
-        __syncthreads();
-        stage_raw<BF16, VCH>(P, C, r0, 2 * KW + h * 128 + round * VCH, RB);
-        __syncthreads();
-      }
-      constexpr int VP = VCH / 2, VSEG = 256 / VP, VR = 64 / VSEG;
-      const int cp = t % VP, seg = t / VP, chl = 2 * cp, chg = 2 * KW + h * 128 + round * VCH + chl, rb = seg * VR;
-      const float4 w0 = *reinterpret_cast<const float4*>(a.conv + (size_t)chg * 4);
-      const float4 w1 = *reinterpret_cast<const float4*>(a.conv + (size_t)(chg + 1) * 4);
-      float2 x0 = staged_pair<BF16>(RB, VCH, rb, chl), x1 = staged_pair<BF16>(RB, VCH, rb + 1, chl), x2 = staged_pair<BF16>(RB, VCH, rb + 2, chl);
+#pragma unroll 1
+    for (int round = 0; round < 128 / VCH; ++round) {   // X = beta SiLU(conv(v)) from the staged raw rows, then Ut = T X
+      cp_async_wait_all();
+      __syncthreads();                  // the raw rows are there; X = beta e^G K consumed
+      constexpr int VP = VCH / 2, VR = 64 / (kLocalThreads / VP);
+      const int vch = 2 * (t % VP), vr = (t / VP) * VR;
+      f2 v[VR];
+      conv_rows<BF16>(a.conv, 2 * KW + h * 128 + round * VCH + vch, RB, VCH, vr, vch, v);
 #pragma unroll
       for (int i = 0; i < VR; ++i) {
-        const float2 x3 = staged_pair<BF16>(RB, VCH, rb + 3 + i, chl);
-        float c0 = w0.x * x0.x, c1 = w1.x * x0.y;
-        c0 = fmaf(w0.y, x1.x, c0); c1 = fmaf(w1.y, x1.y, c1);
-        c0 = fmaf(w0.z, x2.x, c0); c1 = fmaf(w1.z, x2.y, c1);
-        c0 = fmaf(w0.w, x3.x, c0); c1 = fmaf(w1.w, x3.y, c1);
-        const float b = rb + i < valid ? bv[rb + i] : 0.f;
-        *reinterpret_cast<float2*>(Qs + (rb + i) * kLdX + round * VCH + chl) = make_float2(tf32r(b * siluf_(c0)), tf32r(b * siluf_(c1)));
-        x0 = x1; x1 = x2; x2 = x3;
+        const float b = vr + i < valid ? bv[vr + i] : 0.f;
+        const float2 x = unpack2(mul2(v[i], pack2(b, b)));
+        *reinterpret_cast<float2*>(Qs + (vr + i) * kLdX + round * VCH + vch) = make_float2(tf32_operand(x.x), tf32_operand(x.y));
       }
-    }
-    __syncthreads();
-    if constexpr (BF16) {   // staging tile consumed: start the next value head's rows
-      if (vi + 1 < rep) stage_issue<true, 128>(P, C, r0, 2 * KW + (h + 1) * 128, RB);
-    }
-    {   // Ut = T X  (stored fp32: it is added, not multiplied, in the scan)
-      float acc[2][4][4];
+      __syncthreads();
+      // staging tile consumed: start the next rows
+      if (round + 1 < 128 / VCH) stage_issue<BF16, VCH>(P, C, r0, 2 * KW + h * 128 + (round + 1) * VCH, RB);
+      else if (vi + 1 < v_last) stage_issue<BF16, VCH>(P, C, r0, 2 * KW + (h + 1) * 128, RB);
+      // Ut = T X  (stored fp32: it is added, not multiplied, in the scan)
+      constexpr int NT = VCH / 64;
+      float acc[2][NT][4];
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int n = 0; n < 4; ++n) acc[k][n][0] = acc[k][n][1] = acc[k][n][2] = acc[k][n][3] = 0.f;
-      warp_gemm_tril_pair<4, true>(acc[0], acc[1], LT, kLdM, m_hi, m_lo, Qs + qn * 32, kLdX);
+        for (int n = 0; n < NT; ++n) acc[k][n][0] = acc[k][n][1] = acc[k][n][2] = acc[k][n][3] = 0.f;
+      warp_gemm_tril_pair<NT>(acc[0], acc[1], LT, kLdM, m_hi, m_lo, Qs + round * VCH + qn * NT * 8, kLdX);
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int mt2 = k ? m_lo : m_hi;
@@ -388,8 +407,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_local_kernel(GdnPrefillParam
         // 128-bit load, a warp 512 contiguous bytes
         float* dst = ws.Ut + unit * 8192 + (size_t)mt2 * 2048;
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const int col = qn * 32 + n * 8 + 2 * tq;
+        for (int n = 0; n < NT; ++n) {
+          const int col = round * VCH + (qn * NT + n) * 8 + 2 * tq;
           float* d = dst + (g >> 2) * 512 + col * 4 + (g & 3);
           d[0] = acc[k][n][0]; d[4] = acc[k][n][1]; d[1024] = acc[k][n][2]; d[1028] = acc[k][n][3];
         }
@@ -405,9 +424,11 @@ cr_status gdn_chunk_local_launch(const cr_geometry* g, const GdnPrefillParams& P
         CR_CUDA(cudaFuncSetAttribute(gdn_chunk_local_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLocalSmem));
         return CR_OK;
       })) return st;
-  const dim3 grid(ws.chunks, g->gdn_kheads);
-  if (bf16_in) gdn_chunk_local_kernel<true><<<grid, 256, kLocalSmem, stream>>>(P, ws);
-  else gdn_chunk_local_kernel<false><<<grid, 256, kLocalSmem, stream>>>(P, ws);
+  // A short call has a CTA per value head instead of one per key head (q and k prepared once per value head) while all of
+  // them are resident at once.
+  const int rep = g->gdn_vheads / g->gdn_kheads;
+  const dim3 grid(ws.chunks, g->gdn_kheads, ws.chunks * g->gdn_vheads <= 2 * sm_count() ? rep : 1);
+  CR_CUDA(launch_chained(P.chained, bf16_in ? gdn_chunk_local_kernel<true> : gdn_chunk_local_kernel<false>, grid, dim3(kLocalThreads), kLocalSmem, stream, P, ws));
   CR_LAUNCH_CHECK("gdn_chunk_local_kernel");
   return CR_OK;
 }

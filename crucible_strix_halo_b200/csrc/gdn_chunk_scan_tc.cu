@@ -71,6 +71,8 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
+  pdl_release();
+  pdl_wait();
   const uint32_t tm = tmem_slot;
   bool gave_up = false;                                    // a thread that gave up once does not wait again
   auto wait = [&](uint64_t* bar, uint32_t parity) {
@@ -245,7 +247,7 @@ cr_status gdn_chunk_scan_tc_launch(const cr_geometry* g, const GdnPrefillParams&
         CR_CUDA(cudaFuncSetAttribute(gdn_chunk_scan_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScanSmem));
         return CR_OK;
       })) return st;
-  gdn_chunk_scan_tc_kernel<<<g->gdn_vheads, kScanThreads, kScanSmem, stream>>>(P, ws);
+  CR_CUDA(launch_chained(P.chained, gdn_chunk_scan_tc_kernel, dim3(g->gdn_vheads), dim3(kScanThreads), kScanSmem, stream, P, ws));
   CR_LAUNCH_CHECK("gdn_chunk_scan_tc_kernel");
   return CR_OK;
 }

@@ -6,7 +6,7 @@
 //              beta = sigmoid(b)                                   -> workspace (qn, kn, vn, glog, beta)
 //   scan       delta rule over the rows from the carried state     -> raw readout y, new state
 //   gdn_gate   y * rsqrt(mean y^2 + eps) * gamma * sigmoid(z), output transform
-//   gdn_ring   last 16 raw rows -> hist ring (GdnPrefillHistoryKernel, prefill_gdn.h:274-282)
+//              and, in blocks of its own, the last 16 raw rows -> hist ring (GdnPrefillHistoryKernel, prefill_gdn.h:274-282)
 #include "common.cuh"
 #include <algorithm>
 #include <mutex>
@@ -156,7 +156,8 @@ __global__ void __launch_bounds__(256) gdn_scan_serial_kernel(GdnPrefillParams P
 // ---- gated readout -----------------------------------------------------------------------------------
 // One warp per four consecutive (row, head) units; lane l holds columns 4l..4l+3 of each (the WHT layout).  All
 // loads of the four units are issued before anything is consumed: the kernel is a stream, and bytes in flight per
-// thread are what its bandwidth depends on.
+// thread are what its bandwidth depends on.  Blocks past the units copy the last rows of the call to the raw-row ring
+// (P.ring_rows of them, in the last part of a call): everything that read the ring has ended by then.
 constexpr int kGateUnits = 4;
 template <bool BF16>
 __global__ void __launch_bounds__(256) gdn_gate_kernel(GdnPrefillParams P) {
@@ -164,6 +165,17 @@ __global__ void __launch_bounds__(256) gdn_gate_kernel(GdnPrefillParams P) {
   const int VW = P.Hv * 128, l = threadIdx.x & 31;
   const long long total = (long long)a.R * P.Hv;
   const long long unit0 = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * kGateUnits;
+  pdl_release();
+  pdl_wait();
+  if (blockIdx.x >= P.gate_blocks) {
+    const int C = 2 * P.Hk * 128 + VW, i = ((int)(blockIdx.x - P.gate_blocks) * 256 + threadIdx.x) * 4;
+    if (i >= P.ring_rows * C) return;
+    const int r = a.R - P.ring_rows + i / C, ch = i % C;             // a short last part reaches back into the one before it
+    const long long at = (long long)r * C + ch;
+    *reinterpret_cast<float4*>(a.hist + (size_t)((a.pos0 + r) & 15) * C + ch) =
+        make_float4(load_in<BF16>(a.qkv, at), load_in<BF16>(a.qkv, at + 1), load_in<BF16>(a.qkv, at + 2), load_in<BF16>(a.qkv, at + 3));
+    return;
+  }
   if (unit0 >= total) return;
   float4 y4[kGateUnits], z4[kGateUnits];
 #pragma unroll
@@ -204,28 +216,14 @@ __global__ void __launch_bounds__(256) gdn_gate_kernel(GdnPrefillParams P) {
       pk.x = *reinterpret_cast<const unsigned*>(&lo); pk.y = *reinterpret_cast<const unsigned*>(&hi);
       *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(a.out) + base) = pk;
     } else {
-      const __half* suh = reinterpret_cast<const __half*>(a.suh_out) + h * 128 + l * 4;
+      float su[4];
+      load_half4(reinterpret_cast<const uint16_t*>(a.suh_out) + h * 128 + l * 4, su);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) o[i] = round_h(round_h(o[i]) * __half2float(suh[i]));
+      for (int i = 0; i < 4; ++i) o[i] = round_h(round_h(o[i]) * su[i]);
       wht128(o);
-      __half* dst = reinterpret_cast<__half*>(a.out);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        dst[out_index(r, h * 128 + l * 4 + i, VW, a.pack_rows, a.pack_off)] = __float2half(o[i] * kHadNorm);
+      store_half4(reinterpret_cast<uint16_t*>(a.out) + out_index(r, h * 128 + l * 4, VW, a.pack_rows, a.pack_off), o, kHadNorm);
     }
   }
-}
-
-// ---- raw-row ring --------------------------------------------------------------------------------------
-template <bool BF16>
-__global__ void __launch_bounds__(256) gdn_ring_kernel(GdnPrefillParams P) {
-  const cr_gdn_args& a = P.a;
-  const int C = 2 * P.Hk * 128 + P.Hv * 128;
-  const int keep = min(a.R, 16);
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= (long long)keep * C) return;
-  const int r = a.R - keep + (int)(i / C), ch = (int)(i % C);
-  a.hist[(size_t)((a.pos0 + r) & 15) * C + ch] = load_in<BF16>(a.qkv, (size_t)r * C + ch);
 }
 
 // ---- materialize -----------------------------------------------------------------------------------------
@@ -373,6 +371,7 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
   const size_t in_elt = bf ? 2 : 4, out_elt = fmt == CR_OUT_RAW_F32 ? 4 : 2;
   const size_t Cw = 2 * (size_t)g->gdn_kheads * 128 + (size_t)g->gdn_vheads * 128, VWs = (size_t)g->gdn_vheads * 128;
   GdnPrefillParams P;
+  const bool pipelined = algo == CR_GDN_CHUNK_TC && a.R > gdn_part_rows() && !profiling();
   // The call runs in parts of gdn_part_rows() rows; the state carries from part to part.
   auto part_params = [&](int p0, int buf, int rows = 0) {
     P.a = a;
@@ -385,19 +384,20 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
     P.ab_logits = (const char*)args->ab_logits + (size_t)p0 * 2 * g->gdn_vheads * in_elt;
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.fmt = (int)fmt;
     P.tf32 = 0;
+    P.chained = pdl_enabled() && !pipelined;
     P.halo_in = p0 > 0;
-
-
+    P.gate_blocks = (unsigned)(((long long)P.a.R * g->gdn_vheads + 8 * kGateUnits - 1) / (8 * kGateUnits));
+    P.ring_rows = p0 + P.a.R == a.R ? std::min(a.R, 16) : 0;
     gdn_workspace_layout(g, part_rows, &P, (char*)args->workspace + (size_t)buf * part_bytes);
     if (args->raw_y) P.yraw = args->raw_y + (size_t)p0 * VWs;
   };
   auto gate = [&](cudaStream_t st) -> cr_status {
-    const unsigned gg = (unsigned)(((long long)P.a.R * g->gdn_vheads + 8 * kGateUnits - 1) / (8 * kGateUnits));
-    if (bf) gdn_gate_kernel<true><<<gg, 256, 0, st>>>(P); else gdn_gate_kernel<false><<<gg, 256, 0, st>>>(P);
+    const unsigned blocks = P.gate_blocks + (unsigned)((P.ring_rows * (long long)Cw + 1023) / 1024);
+    CR_CUDA(launch_chained(P.chained, bf ? gdn_gate_kernel<true> : gdn_gate_kernel<false>, dim3(blocks), dim3(256), 0, st, P));
     CR_LAUNCH_CHECK("gdn_gate_kernel");
     return CR_OK;
   };
-  if (algo == CR_GDN_CHUNK_TC && a.R > gdn_part_rows() && !profiling()) {
+  if (pipelined) {
     // Pipeline over parts on two internal streams that fork from the caller's stream and join it again.  The
     // scan of part p is enqueued before the local kernel of part p + 1 and on the stream of higher priority, so
     // that its CTAs (one whole SM each) are placed while the SMs are empty; the local kernel then fills the rest.
@@ -464,11 +464,6 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
       if (cr_status s = gate(stream)) return s;
     }
   }
-  P.a = a;
-  const int C = 2 * g->gdn_kheads * 128 + g->gdn_vheads * 128;
-  const unsigned rg = (unsigned)(((long long)(a.R < 16 ? a.R : 16) * C + 255) / 256);
-  if (bf) gdn_ring_kernel<true><<<rg, 256, 0, stream>>>(P); else gdn_ring_kernel<false><<<rg, 256, 0, stream>>>(P);
-  CR_LAUNCH_CHECK("gdn_ring_kernel");
   return CR_OK;
 }
 

@@ -21,6 +21,9 @@ struct GdnPrefillParams {
   char* chunk_ws;          // workspace of the chunked scan
   int Hv, Hk, fmt;
   int halo_in;             // 1: rows before this part's first row are read from the input (a later part of one call)
+  unsigned gate_blocks;    // blocks of the gate kernel that gate; those behind them fill the ring
+  int ring_rows;           // rows of the raw-row ring this part writes
+  bool chained;            // launch with programmatic dependence on the kernel ahead (not across the streams of the part pipeline)
   int tf32;                // 1: prep rounds q/k to tf32 (operands of the tensor-core scan)
 };
 

@@ -36,18 +36,6 @@ __host__ __device__ inline int step_smem_floats(int rows, int replay) {
   return (rows + 3) * kRawCols + rows * kRawCols + rep * 258;
 }
 
-// Two fp32 lanes in one 64-bit register: half the instructions of the row updates.
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pack2(float x, float y) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y)); return r; }
-__device__ __forceinline__ float2 unpack2(f2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ void load_f2x2(const float* p, f2& a, f2& b) {      // four floats, 16-byte aligned
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-  a = v.x; b = v.y;
-}
-
 template <int BYTES>
 __device__ __forceinline__ void step_cp(float* dst, const float* src, bool valid) {
   const int bytes = valid ? BYTES : 0;

@@ -37,3 +37,35 @@ def test_projection_cuts(R, K, N):
     assert capi.lib.cr_device_check() == 0
     ref = x.float() @ w.float().t()
     assert (torch.cat(outs, 1) - ref).abs().max().item() < 2e-4          # order of the fp32 additions only
+
+
+# chunked scan against the serial one: a single ragged chunk, rows fewer than the ring holds, both sides of the size where a
+# CTA takes one value head (296 / value heads chunks), one to three value heads per key head
+@pytest.mark.parametrize("geometry", [(16, 32), (16, 48), (4, 4)])
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("R", [1, 17, 63, 64, 385, 576, 577])
+def test_gdn_chunk_prefill_splits(geometry, bf16, R):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, geometry[1], geometry[0])
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    C, Hv, pos0 = g.gdn_channels, g.gdn_vheads, 100
+    dt = torch.bfloat16 if bf16 else torch.float32
+    w = layers.GdnWeights(g, rn(C, 4, std=0.5), rn(Hv) - 1, rn(Hv, std=0.5), 1 + rn(128, std=0.1))
+    qkv, z, ab = rn(R, C).to(dt), rn(R, Hv * 128).to(dt), rn(R, 2 * Hv).to(dt)
+    hist = rn(16, C).bfloat16().float()
+    state = rn(Hv * 16384 + 64, std=0.1)
+    got = []
+    for algo in (capi.GDN_SERIAL_F32, capi.GDN_CHUNK_TC):
+        s = layers.GdnSession(g)
+        s.hist.copy_(hist)
+        s.state.copy_(state)
+        plan = layers.GdnPrefillPlan(w, R, in_dtype=capi.IN_BF16 if bf16 else capi.IN_F32)
+        got.append((plan.run(s, qkv, z, ab, pos0, algo).clone(), s.state_view().clone(), s.hist.clone()))
+    assert capi.lib.cr_device_check() == 0
+    (o0, s0, h0), (o1, s1, h1) = got
+    ring = hist.clone()
+    for r in range(max(0, R - 16), R):
+        ring[(pos0 + r) % 16] = qkv[r].float()
+    assert torch.equal(h0, ring) and torch.equal(h1, ring)
+    assert (o1 - o0).abs().max() < 4e-3 * o0.abs().max() and (s1 - s0).abs().max() < 4e-3 * s0.abs().max()
