@@ -46,13 +46,13 @@ NCU_TRAFFIC = {
     "gdn_prefill_32k": {"gdn_chunk_scan_tc_kernel": ("token", (526.36e6 + 102.34e6) / 7104),
                         "gdn_chunk_local_kernel": ("token", (121.44e6 + 464.28e6) / 7104),
                         "gdn_gate_kernel": ("token", (174.63e6 + 37.16e6) / 7104)},
-    "decode_262k": {"qsa_score_kernel": ("step", 134.25e6 + 3.57e6), "qsa_attn_split_kernel": ("step", 16.87e6),
-                    "qsa_topk_cluster_kernel": ("step", 1.11e6), "qsa_merge_kernel": ("step", 2.21e6), "qsa_prep_kernel": ("step", 0.13e6),
+    "decode_262k": {"qsa_score_kernel": ("step", 134.25e6 + 3.57e6), "qsa_attn_kernel": ("step", 16.87e6),
+                    "qsa_topk_cluster_kernel": ("step", 1.11e6), "qsa_prep_kernel": ("step", 0.13e6),
                     "gdn_step_kernel": ("step", 9.47e6)},
-    "qsa_prefill_262k": {"qsa_attn_split_kernel": ("step", 6737.66e6 + 135.26e6), "qsa_score_tc_kernel": ("step", 475.9e6),
+    "qsa_prefill_262k": {"qsa_attn_kernel": ("step", 6737.66e6 + 135.26e6), "qsa_score_tc_kernel": ("step", 475.9e6),
                          "qsa_topk_kernel": ("step", 537.4e6 + 7.0e6)},
     "qsa_attend_262k_drift": {"qsa_flash_tc_kernel": ("step", 704.4e6 + 13.6e6)},
-    "verify_131k": {"qsa_attn_split_kernel": ("step", 281.55e6 + 29.26e6), "gdn_step_kernel": ("step", 23.2e6)},
+    "verify_131k": {"qsa_attn_kernel": ("step", 281.55e6 + 29.26e6), "gdn_step_kernel": ("step", 23.2e6)},
 }
 DECODE_BYTES_PER_SESSION = 65536 * 512 + 2051 * 2048 + 2 * 2097152   # pool scan + K/V gather + GDN state in/out
 
@@ -262,7 +262,7 @@ class Decode262k:
         self.h2d = self.h_in.numel() * 4
         self.d2h = self.h_out.numel() * 4
         # per-kernel algorithmic bytes: pool scan; K/V gather; GDN state in + out; scores read by the select
-        self.kernel_bytes = {"qsa_score_kernel": 65536 * 512 * S, "qsa_attn_split_kernel": 2051 * 2048 * S,
+        self.kernel_bytes = {"qsa_score_kernel": 65536 * 512 * S, "qsa_attn_kernel": 2051 * 2048 * S,
                              "gdn_step_kernel": 2 * 2097152 * S, "qsa_topk_cluster_kernel": 65536 * 4 * S}
         self.side = torch.cuda.Stream()
         self.graph = None
@@ -373,7 +373,7 @@ class QsaPrefill262k:
         self.units_per_step = R
         # gathered K/V rows of every query row + one pass over the pooled keys + the rows in and out
         self.alg_bytes = R * 2051 * 2048 + 65536 * 512 + self.h2d + self.d2h
-        self.kernel_bytes = {"qsa_attn_split_kernel": R * 2051 * 2048, "qsa_flash_tc_kernel": R * 2051 * 2048}
+        self.kernel_bytes = {"qsa_attn_kernel": R * 2051 * 2048, "qsa_flash_tc_kernel": R * 2051 * 2048}
         # useful flops: attention 4 * Hq * D * n per row + scoring 2 * 4 * 128 * nb per row
         self.alg_flops = R * (4 * 16 * 256 * 2051) + sum(1024 * ((self.POS0 + r + 1) // 4) for r in range(R))
 

@@ -112,7 +112,7 @@ extern "C" cr_status cr_device_check(void) {
   if (st == 0) return CR_OK;
   cr::set_error("a bounded device-side wait gave up (status word 0x%x:%s%s%s%s%s); the outputs of that launch are undefined",
                 st, st & 1 ? " gdn_chunk_scan_tc_kernel" : "", st & 2 ? " qsa_score_tc_kernel" : "", st & 4 ? " qsa_flash_tc_kernel" : "",
-                st & 8 ? " debug_wait_kernel" : "", st & 16 ? " proj_gemm_kernel" : "");
+                st & 8 ? " debug_wait_kernel" : "", st & 16 ? " proj_gemm kernels" : "");
   return CR_ERR_TIMEOUT;
 }
 

@@ -214,20 +214,18 @@ cr_status cr_qsa_select(const cr_geometry* g, const cr_qsa_args* spans, int n_sp
                         size_t scratch_bytes, void* stream);
 
 /* Replaces LaunchQsaAttn / QsaAttnTailKernel (engine/layers/qsa_long.h:399-534): split-KV attention over the
- * attended positions, log-sum-exp merge, sigmoid gate, output transform.  `scratch` holds
- * cr_qsa_scratch_bytes(g, total rows) bytes of split-KV partials; it needs no initialisation (every record the
- * merge reads is written by the same call first).  Two launches: the split kernel, then a merge kernel; no
- * block waits on another block and there are no counters (the reference's `sync` words have no counterpart). */
+ * attended positions, log-sum-exp merge, sigmoid gate, output transform, in one launch: the parts of a row are merged on
+ * chip, over a thread-block cluster where a row spans several blocks, and there are no counters (the reference's `sync`
+ * words have no counterpart).  `scratch` of cr_qsa_scratch_bytes(g, total rows) bytes is part of the contract, as the
+ * reference's launcher takes it; it needs no initialisation. */
 cr_status cr_qsa_attn(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void* scratch,
                       size_t scratch_bytes, cr_out_format fmt, void* stream);
 
 /* No counterpart in the reference (its engine always owns scratch).  Same work and output as cr_qsa_attn, for
  * callers that cannot allocate device memory or pass scratch: a serving process whose HBM is fully committed to
  * caches, a plugin without access to its host's allocator, or a caller that must not allocate while a stream
- * capture is open.  The split-KV partials live in an array inside the library (8.45 MB per GPU, held until the
- * process exits).  Limit: total rows x q_heads <= CR_STATIC_ATTN_MAX_ROW_HEADS, else CR_ERR_INVALID.  All calls on
- * a device share the array: calls whose kernels may overlap on the GPU race.  The first call on a device resolves
- * the array's address; make it before any stream capture starts. */
+ * capture is open.  Nothing is held between calls, and calls may overlap.  Limit: total rows x q_heads <=
+ * CR_STATIC_ATTN_MAX_ROW_HEADS, else CR_ERR_INVALID. */
 enum { CR_STATIC_ATTN_MAX_ROW_HEADS = 256 };
 cr_status cr_qsa_attn_static(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cr_out_format fmt,
                              void* stream);
