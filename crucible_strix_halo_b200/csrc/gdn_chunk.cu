@@ -12,10 +12,11 @@ size_t gdn_chunk_layout(const cr_geometry* g, int rows, ChunkWs* ws, char* base)
   auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
   const size_t oU = take(Hv * chunks * 64 * 128 * 4), oG = take(Hv * chunks * 64 * 4);
   const size_t oWQ = take(Hv * chunks * 16384 * 4), oQKp = take(Hv * chunks * 4096 * 4);
-  const size_t oKt = take(Hv * chunks * 8192 * 4);
+  const size_t oKt = take(Hv * chunks * 8192 * 4), oR = take(Hv * chunks * 4);
   if (ws) {
     ws->Ut = (float*)(base + oU); ws->G = (float*)(base + oG);
     ws->WQ = (float*)(base + oWQ); ws->QKp = (float*)(base + oQKp); ws->Kt = (float*)(base + oKt);
+    ws->ready = (unsigned*)(base + oR);
     ws->chunks = (int)chunks;
   }
   return off;

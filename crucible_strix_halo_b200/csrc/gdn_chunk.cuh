@@ -25,6 +25,7 @@ struct ChunkWs {
   float* WQ;   // [Hv][chunks][32][128][4] rows 0-63 W, rows 64-127 e^G Q, one K-major tf32 tile
   float* QKp;  // [Hv][chunks][16][64][4]  QKd as a K-major tf32 tile
   float* Kt;   // [Hv][chunks][16][128][4] (e^{G_end - G} K)^T as a K-major tf32 tile
+  unsigned* ready;   // [chunks][Hv]       1 once the operands of (chunk, head) are written
   int chunks;
 };
 

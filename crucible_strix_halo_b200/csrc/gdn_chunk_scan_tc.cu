@@ -17,8 +17,9 @@
 // recurrent passes through shared memory.  Four compute warpgroups split the columns of every accumulator
 // (warp w reaches lanes 32 (w % 4) .. +31, so each warpgroup covers all lanes); the fp32 master state is spread
 // the same way (thread = column v, 32 keys).  One issuer warp feeds the tensor core, one loader warp keeps two
-// chunks of operand tiles in flight (224 KB of shared memory, two stages).  Warps synchronise only through
-// mbarriers.  Every wait is bounded: a wait that gives up raises a status word, after which no thread waits
+// chunks of operand tiles in flight (224 KB of shared memory, two stages).  It may run beside the kernel that writes the
+// operands: the loader looks at the marks of finished chunks (ChunkWs::ready) and tells the compute warps.  Warps synchronise
+// only through mbarriers.  Every wait is bounded: a wait that gives up raises a status word, after which no thread waits
 // again; the kernel runs to its end, frees its tensor memory and returns.
 #include "gdn_chunk.cuh"
 #include "umma.cuh"
@@ -37,11 +38,40 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_u32(bar)) : "memory");
 }
 
+__device__ __forceinline__ unsigned load_acquire_gpu(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int load_acquire_cta(const int* p) {
+  int v;
+  asm volatile("ld.acquire.cta.shared.s32 %0, [%1];\n" : "=r"(v) : "r"(umma::smem_u32(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_release_cta(int* p, int v) { asm volatile("st.release.cta.shared.s32 [%0], %1;\n" ::"r"(umma::smem_u32(p)), "r"(v) : "memory"); }
+// Until reached(), or two seconds have passed or *abort is set: then false.
+template <class F>
+__device__ __forceinline__ bool wait_until(F&& reached, const volatile int* abort) {
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i)
+    if (reached()) return true;
+  uint64_t t0, t1;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i)
+      if (reached()) return true;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+    if (t1 - t0 > 2000000000ull || *abort) return false;
+  }
+}
+
 __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnPrefillParams P, ChunkWs ws) {
   extern __shared__ __align__(128) float sm[];
   __shared__ __align__(8) uint64_t bars[12];
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int dead;
+  __shared__ int avail;                                    // chunks whose operands are known to be written
   uint64_t* full = &bars[0];                               // one per stage: all three tiles of a chunk
   uint64_t *d1 = &bars[4], *d2 = &bars[5], *d3 = &bars[6];
   uint64_t *uReady = &bars[8], *sReady = &bars[9];
@@ -66,13 +96,13 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
     umma::mbar_init(&yDone[1], 4 * kWG);
     umma::mbar_fence_init();
     dead = 0;
+    avail = 0;
   }
   if (w == kIssuer) umma::tmem_alloc(&tmem_slot, 512);
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   pdl_release();
-  pdl_wait();
   const uint32_t tm = tmem_slot;
   bool gave_up = false;                                    // a thread that gave up once does not wait again
   auto wait = [&](uint64_t* bar, uint32_t parity) {
@@ -95,40 +125,66 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
 
   if (w == kLoader) {
     // ------------------------------------------------------------------ loader: two chunks of tiles in flight
-    if (l == 0) {
-      auto load = [&](int c) {
-        const int s = c & 1;
-        float* A1s = sm + s * kStageFloats;
-        const float* a = ws.WQ + ((size_t)h * nch + c) * 16384;
-        umma::mbar_expect_tx(&full[s], kStageFloats * 4);
-        umma::bulk_load(A1s, a, 32768, &full[s]);
-        umma::bulk_load(A1s + 8192, a + 8192, 32768, &full[s]);
-        umma::bulk_load(A1s + 16384, ws.Kt + ((size_t)h * nch + c) * 8192, 32768, &full[s]);
-        umma::bulk_load(A1s + 24576, ws.QKp + ((size_t)h * nch + c) * 4096, 16384, &full[s]);
-      };
-      // The tiles of a chunk are asked into L2 kLead chunks before their copy to shared memory is issued, and the
-      // rows of Ut that the compute threads read themselves one chunk before they are read.
-      constexpr int kLead = 2;
-      auto prefetch = [&](int c) {
-        if (c >= nch) return;
-        const size_t unit = (size_t)h * nch + c;
-        umma::bulk_prefetch_l2(ws.WQ + unit * 16384, 65536);
-        umma::bulk_prefetch_l2(ws.Kt + unit * 8192, 32768);
-        umma::bulk_prefetch_l2(ws.QKp + unit * 4096, 16384);
-        umma::bulk_prefetch_l2(ws.Ut + unit * 8192, 32768);
-      };
-      for (int c = 0; c < 2 + kLead; ++c) prefetch(c);
-      load(0);
-      if (nch > 1) load(1);
-      // The stage of chunk c is free once every MMA of chunk c has completed.  Each stage has its own barrier, which
-      // completes once per use of the stage and cannot complete again before this warp has refilled the stage: a
-      // loader that falls behind never sees a phase it was not waiting for.
-      for (int c = 0; c + 2 < nch; ++c) {
-        wait(&empty[c & 1], (c >> 1) & 1);
-        if (gave_up || dead) break;                        // no more copies once any wait has run out
-        load(c + 2);
-        prefetch(c + 2 + kLead);
+    // The warp looks at the marks of the next 32 chunks at once, early enough that neither the look nor the fence behind it
+    // stands between a stage that becomes free and the copy into it.
+    int known = 0;                                         // chunks whose operands are written
+    auto ready = [&](int c) {
+      if (known > c || gave_up) return;
+      uint64_t t0 = 0;
+      for (unsigned poll = 0;; ++poll) {
+        const unsigned mask = __ballot_sync(0xffffffffu, known + l < nch && load_acquire_gpu(ws.ready + (size_t)(known + l) * P.Hv + h) != 0);
+        known += mask == 0xffffffffu ? 32 : __ffs(~mask) - 1;
+        if (known > c) break;
+        if (poll % 64 == 0) {
+          uint64_t t1;
+          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+          if (poll == 0) t0 = t1;
+          if (__any_sync(0xffffffffu, t1 - t0 > 2000000000ull || dead)) { gave_up = true; dead = 1; g_gdn_scan_status = 1; return; }
+        }
       }
+      if (l == 0) {
+        asm volatile("fence.proxy.async;\n" ::: "memory"); // written by ordinary stores, read by the copy engine
+        store_release_cta(&avail, known);
+      }
+    };
+    auto load = [&](int c) {
+      if (l != 0 || gave_up) return;
+      const int s = c & 1;
+      float* A1s = sm + s * kStageFloats;
+      const float* a = ws.WQ + ((size_t)h * nch + c) * 16384;
+      umma::mbar_expect_tx(&full[s], kStageFloats * 4);
+      umma::bulk_load(A1s, a, 32768, &full[s]);
+      umma::bulk_load(A1s + 8192, a + 8192, 32768, &full[s]);
+      umma::bulk_load(A1s + 16384, ws.Kt + ((size_t)h * nch + c) * 8192, 32768, &full[s]);
+      umma::bulk_load(A1s + 24576, ws.QKp + ((size_t)h * nch + c) * 4096, 16384, &full[s]);
+    };
+    // The tiles of a chunk are asked into L2 kLead chunks before their copy to shared memory is issued, and the
+    // rows of Ut that the compute threads read themselves one chunk before they are read.  What was written beside this
+    // kernel is in L2 already.
+    constexpr int kLead = 2;
+    auto prefetch = [&](int c) {
+      if (l != 0 || c >= nch || c >= known) return;
+      const size_t unit = (size_t)h * nch + c;
+      umma::bulk_prefetch_l2(ws.WQ + unit * 16384, 65536);
+      umma::bulk_prefetch_l2(ws.Kt + unit * 8192, 32768);
+      umma::bulk_prefetch_l2(ws.QKp + unit * 4096, 16384);
+      umma::bulk_prefetch_l2(ws.Ut + unit * 8192, 32768);
+    };
+    ready(0);
+    load(0);
+    if (nch > 1) ready(1);
+    if (nch > 1) load(1);
+    if (nch > 2) ready(2);
+    for (int c = 2; c < 2 + kLead; ++c) prefetch(c);
+    // The stage of chunk c is free once every MMA of chunk c has completed.  Each stage has its own barrier, which
+    // completes once per use of the stage and cannot complete again before this warp has refilled the stage: a
+    // loader that falls behind never sees a phase it was not waiting for.
+    for (int c = 0; c + 2 < nch; ++c) {
+      if (l == 0) wait(&empty[c & 1], (c >> 1) & 1);
+      if (__any_sync(0xffffffffu, gave_up || dead)) break; // no more copies once any wait has run out
+      load(c + 2);
+      if (c + 3 < nch) ready(c + 3);
+      prefetch(c + 2 + kLead);
     }
   } else if (w == kIssuer) {
     // ------------------------------------------------------------------ issuer: tensor-core work
@@ -182,13 +238,19 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
 
     float ut[16];                                          // Ut of column v, tokens 16 wg .. +15
     float Gend = 0.f;
+    int seen = 0;                                          // chunks this warp knows to be written
     auto fetch_rows = [&](int c) {
+      // The acquiring look waits for the thread's stores of Y, on the chain: only when the last one does not cover c.
+      if (seen <= c) {
+        if (l == 0 && !gave_up && !wait_until([&] { return (seen = load_acquire_cta(&avail)) > c; }, &dead)) { gave_up = true; dead = 1; g_gdn_scan_status = 1; }
+        seen = __shfl_sync(0xffffffffu, seen, 0);
+      }
       const size_t unit = (size_t)h * nch + c;
-      Gend = ws.G[unit * 64 + 63];
+      Gend = __ldcg(ws.G + unit * 64 + 63);
       const float* up = ws.Ut + unit * 8192 + (size_t)wg * 2048 + v * 4;   // [token / 16][(token % 16) / 4][v][token % 4]
 #pragma unroll
       for (int j = 0; j < 16; j += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(up + j * 128);
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(up + j * 128));
         ut[j] = x.x; ut[j + 1] = x.y; ut[j + 2] = x.z; ut[j + 3] = x.w;
       }
     };
@@ -238,6 +300,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
   }
   umma::fence_before_sync();
   __syncthreads();
+  pdl_wait();                                              // whoever waits for this kernel waits for the one ahead of it too
   if (w == kIssuer) umma::tmem_dealloc(tm, 512);
 }
 
