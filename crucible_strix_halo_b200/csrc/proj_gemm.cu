@@ -62,12 +62,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 }
 
 // ---- CTA pairs: the cta_group::2 forms --------------------------------------------------------------------------
-// Shared-cluster address of a barrier (or anything) of CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(umma::smem_u32(p)), "r"(rank));
-  return r;
-}
 // A box into this CTA's shared memory whose bytes complete on a barrier of either CTA of the pair.
 __device__ __forceinline__ void pair_load_box_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
@@ -75,24 +69,6 @@ __device__ __forceinline__ void pair_load_box_2d(void* dst, const CUtensorMap* m
                "l"(map), "r"(c0), "r"(c1), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ void pair_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// One arrival on the barrier at this offset in both CTAs when every MMA issued so far has completed.
-__device__ __forceinline__ void pair_commit(uint64_t* bar) {
-  const uint16_t both = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(umma::smem_u32(bar)), "h"(both)
-               : "memory");
-}
-__device__ __forceinline__ void pair_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory"); }
 
 // Columns col .. col + 31 of one row to the output that owns them.
@@ -163,8 +139,7 @@ proj_gemm_pair_kernel(const __grid_constant__ ProjParams P, const __grid_constan
     prefetch_map(&wmap);
   }
   if (w == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(umma::smem_u32(&tmem_slot)), "r"(512) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    umma::pair_tmem_alloc(&tmem_slot, 512);
   }
   umma::fence_before_sync();
   cluster.sync();                                                       // both CTAs' barriers are ready
@@ -191,7 +166,7 @@ proj_gemm_pair_kernel(const __grid_constant__ ProjParams P, const __grid_constan
           if (gave_up) break;
           unsigned char* st = sm + s * kPStageBytes;
           if (rank == 0) umma::mbar_expect_tx(&full[s], 2 * kPStageBytes);
-          const uint32_t bar = cluster_addr(&full[s], 0);
+          const uint32_t bar = umma::cluster_addr(&full[s], 0);
           pair_load_box_2d(st, &xmap, kb * kGK, m0 + 128 * (int)rank, bar);
           pair_load_box_2d(st + kTileBytes, &wmap, kb * kGK, n0 + 128 * (int)rank, bar);
         }
@@ -214,11 +189,11 @@ proj_gemm_pair_kernel(const __grid_constant__ ProjParams P, const __grid_constan
           const unsigned char* st = sm + s * kPStageBytes;
 #pragma unroll
           for (int ks = 0; ks < kGK / 16; ++ks)
-            pair_mma(tm + acc * 256, tma::desc_sw128(st + ks * 32, 16, 1024), tma::desc_sw128(st + kTileBytes + ks * 32, 16, 1024), idesc,
+            umma::pair_mma(tm + acc * 256, tma::desc_sw128(st + ks * 32, 16, 1024), tma::desc_sw128(st + kTileBytes + ks * 32, 16, 1024), idesc,
                      (kb > 0 || ks > 0) ? 1u : 0u);
-          pair_commit(&empty[s]);                                           // the stage is free in both CTAs once these MMAs have read it
+          umma::pair_commit(&empty[s]);                                           // the stage is free in both CTAs once these MMAs have read it
         }
-        if (!gave_up) pair_commit(&accFull[acc]);
+        if (!gave_up) umma::pair_commit(&accFull[acc]);
       }
     }
   } else {
@@ -243,13 +218,13 @@ proj_gemm_pair_kernel(const __grid_constant__ ProjParams P, const __grid_constan
       }
       umma::fence_before_sync();
       __syncwarp();
-      if (l == 0) pair_arrive(cluster_addr(&accEmpty[acc], 0));
+      if (l == 0) umma::pair_arrive(umma::cluster_addr(&accEmpty[acc], 0));
     }
   }
   umma::fence_before_sync();
   __syncwarp();
   cluster.sync();                                                          // neither CTA leaves while the other may still use its memory
-  if (w == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tm), "r"(512) : "memory");
+  if (w == 1) umma::pair_tmem_dealloc(tm, 512);
 }
 
 // ---- few rows: 128 x TN tiles, K split over a cluster ----------------------------------------------------------------

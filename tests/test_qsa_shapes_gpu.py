@@ -127,3 +127,25 @@ def test_selection_threshold_patterns(nb, pattern):
             want = np.sort(np.lexsort((np.arange(nb), -v))[:512])
             np.testing.assert_array_equal(ci[r].cpu().numpy(), want)
             np.testing.assert_array_equal(cs[r].cpu().numpy(), sc[r].cpu().numpy()[want])
+
+
+# scores of prefill parts: dense rows in front of scored ones, ragged row tiles, fewer visits than CTA pairs, runs of a pair
+# that cross into the next row tile
+@pytest.mark.parametrize("start,R", [(2040, 70), (2100, 17), (9003, 117), (33000, 65), (6001, 257), (20000, 700)])
+def test_prefill_part_scores(start, R):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.GEOM_BENCH
+    gen = torch.Generator(device="cuda").manual_seed(start)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    w = layers.QsaWeights(g, 1 + 0.1 * rn(256), 1 + 0.1 * rn(256), 1 + 0.1 * rn(128), 1 + 0.1 * rn(128))
+    s = layers.QsaSession(g, start + R, max_rows=R)
+    s.ik_pool.copy_(rn(s.ik_pool.numel()))
+    q, k, v, idx = rn(R, g.q_heads, 512), rn(R, 512), rn(R, 512), rn(R, 640)
+    layers.QsaPrefillPlan(w, R).run(s, q, k, v, idx, start)
+    assert capi.lib.cr_device_check() == 0
+    pool = s.pool_rows((start + R) // 4).double()
+    want = torch.relu(torch.einsum("rhd,bd->rhb", idx[:, :512].view(R, 4, 128).double(), pool)).sum(1) / 128 ** 0.5
+    for r in range(R):
+        nb = (start + r + 1) // 4
+        if nb > capi.SEL_BLOCKS:
+            assert (s.scores[r, :nb].double() - want[r, :nb]).abs().max().item() < 2e-4, r
