@@ -32,14 +32,14 @@ cr_status qsa_validate(const cr_geometry* g, const cr_qsa_args* spans, int n_spa
 int qsa_max_rows(const cr_qsa_args* spans, int n);
 void qsa_fill_params(QsaParams& P, const cr_geometry* g, const cr_qsa_args* spans, int n);
 cr_status qsa_prep_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, int u0, __half* q_hi, int q_skip,
-                          cudaStream_t stream, bool queries_only = false);
+                          cudaStream_t stream, bool queries_only = false, bool mark_dense = false);
 cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, int b_lo = 0, int b_hi = INT_MAX);
 // Prefill parts (many rows): the scores as four GEMMs on tcgen05 tensor cores.
 cr_status qsa_score_tc_launch(const QsaParams& P, int n, cudaStream_t stream);
 // Spans of 3..16 rows (verify passes): the scores as an HBM stream through mma.sync, every block of every row.
 cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream);
-cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream);
-cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream);
+cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
+cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
 struct QsaTileSplit { const int* count; int rows, max; };   // see QsaParams::tile_count
 // Attention of the spans' rows over the attended positions inside [p0, p1): outputs, or with `partials` one (m, l, acc[256])
 // record per (row, head).

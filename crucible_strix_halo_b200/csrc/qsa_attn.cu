@@ -532,8 +532,8 @@ extern "C" cr_status cr_qsa_step(const cr_geometry* g, const cr_qsa_args* spans,
   const size_t need = cr_qsa_scratch_bytes(g, (int)total_rows(spans, n_spans));
   CR_REQUIRE(scratch && scratch_bytes >= need, "cr_qsa_step: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
   cudaStream_t st = (cudaStream_t)stream;
-  if (cr_status s = qsa_prep_launch(g, spans, n_spans, 0, nullptr, 0, st)) return s;
-  if (cr_status s = qsa_select_launch(g, spans, n_spans, st)) return s;
+  if (cr_status s = qsa_prep_launch(g, spans, n_spans, 0, nullptr, 0, st, false, true)) return s;
+  if (cr_status s = qsa_select_launch(g, spans, n_spans, st, true)) return s;
   return qsa_attn_launch(g, spans, n_spans, nullptr, 0, INT_MAX, fmt, st);
 }
 

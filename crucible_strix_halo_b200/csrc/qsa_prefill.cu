@@ -125,8 +125,8 @@ extern "C" cr_status cr_qsa_prefill(const cr_geometry* g, const cr_qsa_prefill_a
   if (cr_status s = check_part(g, args, skip, fmt, "cr_qsa_prefill")) return s;
   cudaStream_t stream = (cudaStream_t)stream_;
   // cache rows + query prep for the whole part (rows below skip get cache work only)
-  if (cr_status s = qsa_prep_launch(g, &args->input, 1, 0, reinterpret_cast<__half*>(args->q_hi), skip, stream)) return s;
+  if (cr_status s = qsa_prep_launch(g, &args->input, 1, 0, reinterpret_cast<__half*>(args->q_hi), skip, stream, false, skip == 0)) return s;
   const cr_qsa_args q = output_rows(g, args->input, skip, fmt);
-  if (cr_status s = qsa_select_launch(g, &q, 1, stream)) return s;
+  if (cr_status s = qsa_select_launch(g, &q, 1, stream, skip == 0)) return s;
   return attend(g, args, q, skip, fmt, stream);
 }

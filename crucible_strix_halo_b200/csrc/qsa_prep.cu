@@ -126,7 +126,8 @@ __device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
 // Units: [0, Hq) query heads, [.., + Hkv) key heads, [.., + Hkv) value heads, 4 indexer-query heads, the raw indexer key, and
 // the pooled key of the block that the row completes.  u0 skips leading units (u0 = Hq runs the cache units only).
 // q_hi (optional): fp16 copy of the prepared queries [R][Hq][256] for the prefill attention kernels; rows < q_skip are
-// not written to q_hi.  queries_only: only the query and indexer-query units do anything (a rank of a split-KV group that
+// not written to q_hi.  mark_dense: rows that attend every block say so here (nsel = -1), which saves a call of such rows
+// alone the launch of the selection.  queries_only: only the query and indexer-query units do anything (a rank of a split-KV group that
 // does not own the rows' positions still normalises the queries).
 //
 // Bound: HBM for a part (query rows in and out, fp16 copies, cache rows), latency for a step.  A head lives in one warp
@@ -135,7 +136,7 @@ __device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
 // takes a row per CTA with all loads of a warp issued first (UPW = 5).  2,048 rows at 262,144 positions: 98.8 us as one
 // CTA per (row, unit), 28 us now (4.9 TB/s).
 template <int UPW, bool VEC>
-__global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ QsaParams P, int u0, __half* q_hi, int q_skip, int queries_only) {
+__global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ QsaParams P, int u0, __half* q_hi, int q_skip, int queries_only, int mark_dense) {
   pdl_release();
   pdl_wait();
   const cr_qsa_args& a = P.span[blockIdx.z];
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ Q
     } else if (queries_only) {
       continue;
     } else if (u == Hq + 2 * Hkv + 4) {
+      if (mark_dense && l == 0 && (p + 1) / 4 <= CR_SEL_BLOCKS) a.nsel[r] = -1;
       if (raw_kept(a, r) && !raw_after_pool(a, r)) {
         float* dst = a.c.ik_raw + raw_offset(a.c.raw_slots, p, l);
         dst[0] = x[i][0].x; dst[32] = x[i][0].y; dst[64] = x[i][0].z; dst[96] = x[i][0].w;
@@ -237,7 +239,7 @@ void qsa_fill_params(QsaParams& P, const cr_geometry* g, const cr_qsa_args* span
 }
 
 cr_status qsa_prep_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, int u0, __half* q_hi, int q_skip,
-                          cudaStream_t stream, bool queries_only) {
+                          cudaStream_t stream, bool queries_only, bool mark_dense) {
   use_stream(stream);
   for (int s0 = 0; s0 < n_spans; s0 += kMaxSpans) {
     const int n = n_spans - s0 < kMaxSpans ? n_spans - s0 : kMaxSpans;
@@ -256,7 +258,7 @@ cr_status qsa_prep_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     const bool bulk = (long long)Rmax * n > 128;    // below that a CTA per row would leave SMs idle
     auto kernel = bulk ? (vec ? qsa_prep_kernel<kBulk, true> : qsa_prep_kernel<kBulk, false>) : (vec ? qsa_prep_kernel<1, true> : qsa_prep_kernel<1, false>);
     const int per_cta = 8 * (bulk ? kBulk : 1);
-    CR_CUDA(launch_pdl(kernel, dim3((units + per_cta - 1) / per_cta, Rmax, n), dim3(256), 0, stream, P, u0, q_hi, q_skip, queries_only ? 1 : 0));
+    CR_CUDA(launch_pdl(kernel, dim3((units + per_cta - 1) / per_cta, Rmax, n), dim3(256), 0, stream, P, u0, q_hi, q_skip, queries_only ? 1 : 0, mark_dense ? 1 : 0));
     CR_LAUNCH_CHECK("qsa_prep_kernel");
   }
   return CR_OK;

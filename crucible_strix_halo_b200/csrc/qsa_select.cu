@@ -204,9 +204,9 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
   return CR_OK;
 }
 
-cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream) {
+cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked) {
   if (cr_status s = qsa_score_launch(g, spans, n_spans, stream)) return s;
-  return qsa_topk_launch(g, spans, n_spans, stream);
+  return qsa_topk_launch(g, spans, n_spans, stream, dense_marked);
 }
 
 }  // namespace cr

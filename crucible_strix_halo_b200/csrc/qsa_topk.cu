@@ -597,7 +597,7 @@ static cr_status select_configure() {
   });
 }
 
-cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream) {
+cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked) {
   use_stream(stream);
   if (cr_status st = select_configure()) return st;
   for (int s0 = 0; s0 < n_spans; s0 += kMaxSpans) {
@@ -608,6 +608,7 @@ cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     int nb_max = 0;
     for (int s = 0; s < n; ++s) nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
     CR_REQUIRE(nb_max <= kMaxSelectCount, "qsa select: %d blocks exceed the selectable range of %d", nb_max, kMaxSelectCount);
+    if (dense_marked && nb_max <= CR_SEL_BLOCKS) continue;          // no row of these spans selects
     if ((long long)Rmax * n <= 64 && nb_max >= 16384) {             // few long rows: 8 SMs per row
       if (nb_max <= 65536) CR_CUDA(launch_pdl(qsa_topk_cluster_kernel<8>, dim3(8 * Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
       else CR_CUDA(launch_pdl(qsa_topk_cluster_kernel<32>, dim3(8 * Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));

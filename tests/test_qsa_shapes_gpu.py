@@ -149,3 +149,22 @@ def test_prefill_part_scores(start, R):
         nb = (start + r + 1) // 4
         if nb > capi.SEL_BLOCKS:
             assert (s.scores[r, :nb].double() - want[r, :nb]).abs().max().item() < 2e-4, r
+
+
+# rows on both sides of the first selection: spans without any selecting row (no selection launch), with one, and both in a step
+@pytest.mark.parametrize("starts,R", [([1500], 1), ([2046], 1), ([2050], 1), ([2045, 700], 5), ([10, 2051], 3)])
+def test_step_marks_dense_rows(starts, R):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.GEOM_BENCH
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    w = layers.QsaWeights(g, 1 + 0.1 * rn(256), 1 + 0.1 * rn(256), 1 + 0.1 * rn(128), 1 + 0.1 * rn(128))
+    spans = []
+    for p in starts:
+        s = layers.QsaSession(g, p + R, R)
+        s.nsel.fill_(77)
+        spans.append(dict(session=s, q=rn(R, g.q_heads, 512), k=rn(R, 512), v=rn(R, 512), idx=rn(R, 640), pos0=p))
+    layers.QsaStepPlan(w, len(starts) * R).run(spans)
+    for x in spans:
+        want = [-1 if (x["pos0"] + r + 1) // 4 <= capi.SEL_BLOCKS else capi.SEL_BLOCKS for r in range(R)]
+        assert x["session"].nsel.tolist() == want
