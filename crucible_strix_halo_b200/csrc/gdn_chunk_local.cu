@@ -446,8 +446,10 @@ __global__ void __launch_bounds__(HALVES * kLocalThreads, 3 - HALVES) gdn_chunk_
     const LocalUnit x = unit_at(u, split, P.Hv, P.Hk);
     if (t < x.n) ws.ready[(size_t)x.c * P.Hv + x.h0 + t] = 0;
   }
-  __threadfence();                      // before the scan, which is let in below, can look
-  local_sync();
+  // The scan, which is let in below, must not see a mark of the call before.  One thread's release counts for the whole CTA,
+  // so the marks of both halves have to be zero before any thread gets there.
+  __threadfence();
+  __syncthreads();
   pdl_release();
 #pragma unroll 1
   for (int u = first; u < units; u += step) {

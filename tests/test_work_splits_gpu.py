@@ -69,3 +69,42 @@ def test_gdn_chunk_prefill_splits(geometry, bf16, R):
         ring[(pos0 + r) % 16] = qkv[r].float()
     assert torch.equal(h0, ring) and torch.equal(h1, ring)
     assert (o1 - o0).abs().max() < 4e-3 * o0.abs().max() and (s1 - s0).abs().max() < 4e-3 * s0.abs().max()
+
+
+# Calls in a row on one plan, with nothing between them: every call writes its operands where the one before had its own, and its
+# scan must not take those for new.  The workspace of the first call holds marks that say everything is written.  Rows: a CTA
+# with a unit for one half, units for both, several per half.
+@pytest.mark.parametrize("geometry", [(16, 32), (16, 48)])
+@pytest.mark.parametrize("R", [64, 577, 1999])
+def test_gdn_prefill_calls_share_a_workspace(geometry, R):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, geometry[1], geometry[0])
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    C, Hv = g.gdn_channels, g.gdn_vheads
+    w = layers.GdnWeights(g, rn(C, 4, std=0.5), rn(Hv) - 1, rn(Hv, std=0.5), 1 + rn(128, std=0.1))
+    inputs = [(rn(R, C), rn(R, Hv * 128), rn(R, 2 * Hv)) for _ in range(2)]
+    state = [rn(Hv * 16384 + 64, std=0.1) for _ in range(2)]
+
+    def session(i):
+        s = layers.GdnSession(g)
+        s.state.copy_(state[i])
+        return s
+
+    serial = layers.GdnPrefillPlan(w, R)
+    want = []
+    for i in range(2):
+        s = session(i)
+        want.append((serial.run(s, *inputs[i], 0, capi.GDN_SERIAL_F32).clone(), s.state_view()))
+    plan = layers.GdnPrefillPlan(w, R)
+    plan.workspace.fill_(0xFF)                                   # marks set, operands NaN
+    got = [session(k & 1) for k in range(12)]
+    torch.cuda.synchronize()
+    for k, s in enumerate(got):
+        out = plan.run(s, *inputs[k & 1], 0, capi.GDN_CHUNK_TC)
+    assert capi.lib.cr_device_check() == 0
+    out1, _ = want[1]
+    assert (out - out1).abs().max() < 4e-3 * out1.abs().max()    # the last call had the second inputs
+    for k, s in enumerate(got):
+        ref = want[k & 1][1]
+        assert (s.state_view() - ref).abs().max() < 4e-3 * ref.abs().max(), k
