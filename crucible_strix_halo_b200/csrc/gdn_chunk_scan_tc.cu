@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
           if (__any_sync(0xffffffffu, t1 - t0 > 2000000000ull || dead)) { gave_up = true; dead = 1; g_gdn_scan_status = 1; return; }
         }
       }
+      __syncwarp();                                        // every lane's looks come before lane 0's release: a vote orders no memory
       if (l == 0) {
         asm volatile("fence.proxy.async;\n" ::: "memory"); // written by ordinary stores, read by the copy engine
         store_release_cta(&avail, known);
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_chunk_scan_tc_kernel(GdnP
       // The acquiring look waits for the thread's stores of Y, on the chain: only when the last one does not cover c.
       if (seen <= c) {
         if (l == 0 && !gave_up && !wait_until([&] { return (seen = load_acquire_cta(&avail)) > c; }, &dead)) { gave_up = true; dead = 1; g_gdn_scan_status = 1; }
+        __syncwarp();                                      // lane 0's look comes before the other lanes' loads: a shuffle orders no memory
         seen = __shfl_sync(0xffffffffu, seen, 0);
       }
       const size_t unit = (size_t)h * nch + c;

@@ -73,9 +73,9 @@ def test_gdn_chunk_prefill_splits(geometry, bf16, R):
 
 # Calls in a row on one plan, with nothing between them: every call writes its operands where the one before had its own, and its
 # scan must not take those for new.  The workspace of the first call holds marks that say everything is written.  Rows: a CTA
-# with a unit for one half, units for both, several per half.
+# with a unit for one half, units for both, several per half; more chunks than the scan's loader looks at in one go (32).
 @pytest.mark.parametrize("geometry", [(16, 32), (16, 48)])
-@pytest.mark.parametrize("R", [64, 577, 1999])
+@pytest.mark.parametrize("R", [64, 577, 1999, 2113])
 def test_gdn_prefill_calls_share_a_workspace(geometry, R):
     from crucible_strix_halo_b200 import capi, layers
     g = capi.Geometry(256, 16, 2, geometry[1], geometry[0])
