@@ -34,6 +34,7 @@ __device__ __forceinline__ int local_tid() {
 }
 __device__ __forceinline__ void local_sync() { asm volatile("bar.sync %0, 512;\n" ::"r"(1 + (int)(threadIdx.x >> 9)) : "memory"); }
 
+constexpr int kCleared = 3;                                // barrier: the marks of the CTA are cleared
 constexpr int kRawRows = 67;                               // 64 rows + 3 halo rows
 constexpr int kStageBytes = kRawRows * 128 * 2;            // one 128-channel bf16 tile (or 64 fp32 channels)
 constexpr int kLocalThreads = 512;
@@ -442,25 +443,30 @@ __global__ void __launch_bounds__(HALVES * kLocalThreads, 3 - HALVES) gdn_chunk_
   const int units = split * P.Hv + (ws.chunks - split) * P.Hk;
   const int step = HALVES * gridDim.x, half = threadIdx.x >> 9, first = blockIdx.x + half * gridDim.x, t = local_tid();
   pdl_wait();
-  for (int u = first; u < units; u += step) {
-    const LocalUnit x = unit_at(u, split, P.Hv, P.Hk);
-    if (t < x.n) ws.ready[(size_t)x.c * P.Hv + x.h0 + t] = 0;
+  // The scan, which is let in below, must not see a mark of the call before.  One thread's release counts for the whole CTA, so
+  // the first half clears the marks of both and releases alone; the other half meets it (kCleared) before its first mark.
+  if (half == 0) {
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      const LocalUnit x = unit_at(u, split, P.Hv, P.Hk);
+      if (t < x.n) ws.ready[(size_t)x.c * P.Hv + x.h0 + t] = 0;
+    }
+    __threadfence();
+    local_sync();
+    pdl_release();
+    if (HALVES == 2) asm volatile("bar.arrive %0, 1024;\n" ::"n"(kCleared) : "memory");
   }
-  // The scan, which is let in below, must not see a mark of the call before.  One thread's release counts for the whole CTA,
-  // so the marks of both halves have to be zero before any thread gets there.
-  __threadfence();
-  __syncthreads();
-  pdl_release();
 #pragma unroll 1
   for (int u = first; u < units; u += step) {
     const LocalUnit x = unit_at(u, split, P.Hv, P.Hk);
     const int rep = P.Hv / P.Hk;
     local_unit<BF16>(P, ws, sm + half * (kLocalSmem / sizeof(float)), x.c, x.h0 / rep, x.h0 % rep, x.h0 % rep + x.n);
     asm volatile("fence.proxy.async;\n" ::: "memory");                      // the scan reads the tiles with bulk copies
+    if (HALVES == 2 && half == 1 && u == first) asm volatile("bar.sync %0, 1024;\n" ::"n"(kCleared) : "memory");
     local_sync();
     const LocalUnit y = unit_at(u, split, P.Hv, P.Hk);
     if (t < y.n) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(ws.ready + (size_t)y.c * P.Hv + y.h0 + t), "r"(1u) : "memory");
   }
+  if (HALVES == 2 && half == 1 && first >= units) asm volatile("bar.sync %0, 1024;\n" ::"n"(kCleared) : "memory");
 }
 
 cr_status gdn_chunk_local_launch(const cr_geometry* g, const GdnPrefillParams& P, const ChunkWs& ws, bool bf16_in, cudaStream_t stream) {
