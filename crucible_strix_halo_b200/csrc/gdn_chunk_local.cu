@@ -69,7 +69,7 @@ __device__ __forceinline__ void stage_issue(const GdnPrefillParams& P, int C, in
           for (int i = 0; i < 4; ++i) b[i] = __floats2bfloat162_rn(hs[2 * i], hs[2 * i + 1]);
           v = *reinterpret_cast<const uint4*>(b);
         } else {
-          v = *reinterpret_cast<const uint4*>(hs);
+          v = make_uint4(__float_as_uint(hs[0]), __float_as_uint(hs[1]), __float_as_uint(hs[2]), __float_as_uint(hs[3]));
         }
       }
       d[k * kLocalThreads] = v;

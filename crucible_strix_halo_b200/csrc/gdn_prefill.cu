@@ -172,8 +172,10 @@ __global__ void __launch_bounds__(256) gdn_gate_kernel(GdnPrefillParams P) {
     if (i >= P.ring_rows * C) return;
     const int r = a.R - P.ring_rows + i / C, ch = i % C;             // a short last part reaches back into the one before it
     const long long at = (long long)r * C + ch;
-    *reinterpret_cast<float4*>(a.hist + (size_t)((a.pos0 + r) & 15) * C + ch) =
-        make_float4(load_in<BF16>(a.qkv, at), load_in<BF16>(a.qkv, at + 1), load_in<BF16>(a.qkv, at + 2), load_in<BF16>(a.qkv, at + 3));
+    const float4 x = make_float4(load_in<BF16>(a.qkv, at), load_in<BF16>(a.qkv, at + 1), load_in<BF16>(a.qkv, at + 2), load_in<BF16>(a.qkv, at + 3));
+    float* dst = a.hist + (size_t)((a.pos0 + r) & 15) * C + ch;
+    if (((uintptr_t)dst & 15) == 0) *reinterpret_cast<float4*>(dst) = x;
+    else { dst[0] = x.x; dst[1] = x.y; dst[2] = x.z; dst[3] = x.w; }       // the ring lies at any float address
     return;
   }
   if (unit0 >= total) return;

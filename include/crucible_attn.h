@@ -77,7 +77,7 @@ typedef struct {
   const float* A_log;      /* [Hv] */
   const float* dt_bias;    /* [Hv] */
   const float* gamma;      /* [128] direct gamma */
-  float* hist;             /* [16][channels] ring of raw qkv rows, slot = pos & 15 */
+  float* hist;             /* [16][channels] ring of raw qkv rows, slot = pos & 15; any float address */
   float* state;            /* [Hv][128 key][128 value] fp32, followed by 64 scale floats */
   const uint16_t* suh_out; /* fp16 [Hv*128], CR_OUT_EXL3_WHT only */
   void* out;               /* [R][Hv*128] in the chosen cr_out_format (xh_out in the reference) */

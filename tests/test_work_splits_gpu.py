@@ -108,3 +108,29 @@ def test_gdn_prefill_calls_share_a_workspace(geometry, R):
     for k, s in enumerate(got):
         ref = want[k & 1][1]
         assert (s.state_view() - ref).abs().max() < 4e-3 * ref.abs().max(), k
+
+
+# The raw-row ring at an address that is a multiple of 4 bytes only: what a call reads of it (the three rows before the call) and
+# what it writes are the same as with an aligned ring, bit for bit.
+@pytest.mark.parametrize("algo", ["serial", "chunk"])
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_gdn_prefill_ring_at_any_float_address(algo, bf16, offset):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, 4, 2)
+    gen = torch.Generator(device="cuda").manual_seed(offset)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    C, Hv, R, pos0 = g.gdn_channels, 4, 21, 5
+    dt = torch.bfloat16 if bf16 else torch.float32
+    w = layers.GdnWeights(g, rn(C, 4, std=0.5), rn(Hv) - 1, rn(Hv, std=0.5), 1 + rn(128, std=0.1))
+    qkv, z, ab, hist = rn(R, C).to(dt), rn(R, Hv * 128).to(dt), rn(R, 2 * Hv).to(dt), rn(16, C).bfloat16().float()
+    plan = layers.GdnPrefillPlan(w, R, in_dtype=capi.IN_BF16 if bf16 else capi.IN_F32)
+    got = []
+    for shift in (0, offset):
+        s = layers.GdnSession(g)
+        room = torch.zeros(16 * C + 4, device="cuda")
+        s.hist = room[shift:shift + 16 * C].view(16, C)
+        s.hist.copy_(hist)
+        out = plan.run(s, qkv, z, ab, pos0, capi.GDN_SERIAL_F32 if algo == "serial" else capi.GDN_CHUNK_TC)
+        got.append((out.clone(), s.state.clone(), s.hist.clone(), room[:shift].sum() + room[shift + 16 * C:].sum()))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and got[1][3] == 0
