@@ -74,6 +74,16 @@ cr_geometry geometry(PyObject* w) {                  // w.g, a ctypes structure
   if (!out.kv_heads) { PyErr_SetString(PyExc_TypeError, "weights need a Geometry"); throw Error(); }
   return out;
 }
+// A call into the library, without the interpreter lock: other host threads go on meanwhile, on streams or GPUs of their own.
+// The argument structs are filled and nothing of Python is touched until the lock is back, also when `f` throws.
+template <typename F>
+cr_status unlocked(F&& f) {
+  struct Lock {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Lock() { PyEval_RestoreThread(state); }
+  } released;
+  return f();
+}
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 at::ScalarType out_type(long fmt) {
   return fmt == CR_OUT_RAW_F32 ? at::kFloat : fmt == CR_OUT_RAW_BF16 ? at::kBFloat16 : at::kHalf;
@@ -160,7 +170,8 @@ PyObject* gdn_step(PyObject*, PyObject* args) {      // (weights, spans, fmt, ou
       a[i].commit = (int)item_or(sp, s_commit, R);
       a[i].out = output(outs, given, i, {R, W}, out_type(fmt), qkv);
     }
-    check(cr_gdn_step(&g, a.data(), (int)n, (int)pend_rows, (cr_out_format)fmt, stream()));
+    void* const st = stream();
+    check(unlocked([&] { return cr_gdn_step(&g, a.data(), (int)n, (int)pend_rows, (cr_out_format)fmt, st); }));
     Py_INCREF(outs.p);
     return outs.p;
   });
@@ -196,7 +207,9 @@ PyObject* qsa_step(PyObject*, PyObject* args) {      // (plan, spans, want_conte
     }
     Ref scratch(PyObject_GetAttr(plan, s_scratch));
     const at::Tensor& sc = tensor(scratch);
-    check(cr_qsa_step(&g, a.data(), (int)n, sc.data_ptr(), (size_t)sc.numel(), (cr_out_format)fmt, stream()));
+    void *const st = stream(), *const at = sc.data_ptr();
+    const size_t bytes = (size_t)sc.numel();
+    check(unlocked([&] { return cr_qsa_step(&g, a.data(), (int)n, at, bytes, (cr_out_format)fmt, st); }));
     if (want) return PyTuple_Pack(2, outs.p, contexts.p);
     Py_INCREF(outs.p);
     return outs.p;
@@ -225,7 +238,9 @@ PyObject* gdn_prefill(PyObject*, PyObject* args) {   // (plan, session, qkv, z, 
     a.workspace = wst.data_ptr();
     a.workspace_bytes = (size_t)wst.numel();
     attr(a.raw_y, plan, s_raw_y);
-    check(cr_gdn_prefill(&g, &a, (cr_gdn_algo)algo, (cr_out_format)long_attr(plan, s_fmt), stream()));
+    const cr_out_format fmt = (cr_out_format)long_attr(plan, s_fmt);
+    void* const st = stream();
+    check(unlocked([&] { return cr_gdn_prefill(&g, &a, (cr_gdn_algo)algo, fmt, st); }));
     return PyObject_GetAttr(plan, s_out);
   });
 }
@@ -253,7 +268,9 @@ PyObject* qsa_prefill(PyObject*, PyObject* args) {   // (plan, session, q, k, v,
     const at::Tensor& sc = tensor(scratch);
     a.scratch = sc.data_ptr();
     a.scratch_bytes = (size_t)sc.numel();
-    check(cr_qsa_prefill(&g, &a, skip, (cr_out_format)long_attr(plan, s_fmt), stream()));
+    const cr_out_format fmt = (cr_out_format)long_attr(plan, s_fmt);
+    void* const st = stream();
+    check(unlocked([&] { return cr_qsa_prefill(&g, &a, skip, fmt, st); }));
     return wrap(tensor(out).narrow(0, 0, qt.size(0)));
   });
 }
@@ -273,7 +290,10 @@ PyObject* proj_gemm(PyObject*, PyObject* args) {     // (x, w, outs)
       o[i] = cr_proj_out{t.data_ptr(), col, cols, cols, t.scalar_type() == at::kFloat ? 1 : 0};
       col += cols;
     }
-    check(cr_proj_gemm(xt.data_ptr(), wt.data_ptr(), (int)xt.size(0), (int)xt.size(1), (int)wt.size(0), o.data(), (int)n, stream()));
+    const void *const xp = xt.data_ptr(), *const wp = wt.data_ptr();
+    const int R = (int)xt.size(0), K = (int)xt.size(1), N = (int)wt.size(0);
+    void* const st = stream();
+    check(unlocked([&] { return cr_proj_gemm(xp, wp, R, K, N, o.data(), (int)n, st); }));
     Py_INCREF(outs);
     return outs;
   });
