@@ -2,6 +2,7 @@
 // attributes; through ctypes that, the stream look-up and the outputs took 15 us per GDN call and 24 us per QSA call, three
 // times their launches.  Here the same objects (weights, sessions, plans, span dicts) are read with the CPython API and the
 // argument structs of include/crucible_attn.h are filled on the stack.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAStream.h>
@@ -84,7 +85,7 @@ cr_status unlocked(F&& f) {
   } released;
   return f();
 }
-void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }   // throws without a usable GPU
 at::ScalarType out_type(long fmt) {
   return fmt == CR_OUT_RAW_F32 ? at::kFloat : fmt == CR_OUT_RAW_BF16 ? at::kBFloat16 : at::kHalf;
 }
@@ -115,8 +116,8 @@ PyObject* guarded(F&& f) {
     return f();
   } catch (const Error&) {
     return nullptr;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {                                    // the exception that torch's own functions give for it
+    torch::translate_exception_to_python(std::current_exception());
     return nullptr;
   }
 }
@@ -299,7 +300,9 @@ PyObject* proj_gemm(PyObject*, PyObject* args) {     // (x, w, outs)
   });
 }
 
-PyObject* current_stream(PyObject*, PyObject*) { return PyLong_FromVoidPtr(stream()); }
+PyObject* current_stream(PyObject*, PyObject*) {
+  return guarded([] { return PyLong_FromVoidPtr(stream()); });
+}
 
 PyMethodDef methods[] = {{"current_stream", current_stream, METH_NOARGS, nullptr},
                          {"gdn_step", gdn_step, METH_VARARGS, nullptr},       {"qsa_step", qsa_step, METH_VARARGS, nullptr},

@@ -46,3 +46,17 @@ def test_calls_release_the_interpreter_lock(tmp_path):
         (tmp_path / "_binding.so").write_bytes(f.read())
     r = subprocess.run([sys.executable, "-c", UNLOCKED, str(tmp_path)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def _without_gpu(code):
+    """Runs `code` in a process of its own that sees no GPU; it prints what it has to say."""
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="", PYTHONPATH=os.path.dirname(PKG))
+    r = subprocess.run([sys.executable, "-c", "import torch\nfrom crucible_strix_halo_b200 import _binding, layers\n" + code], capture_output=True,
+                       text=True, timeout=300, env=env)
+    assert r.returncode == 0, "status %d\n%s" % (r.returncode, r.stderr[-2000:])
+    return r.stdout.split()
+
+
+@pytest.mark.parametrize("call", ["_binding.current_stream()", "layers.proj_gemm(torch.zeros(1, 64).bfloat16(), torch.zeros(32, 64).bfloat16(), [torch.zeros(1, 32)])"])
+def test_no_gpu_is_an_exception(call):
+    assert _without_gpu("try:\n    %s\nexcept RuntimeError:\n    print('refused')" % call) == ["refused"]
