@@ -281,12 +281,14 @@ PyObject* proj_gemm(PyObject*, PyObject* args) {     // (x, w, outs)
     PyObject *x, *w, *outs;
     if (!PyArg_ParseTuple(args, "OOO", &x, &w, &outs)) throw Error();
     const at::Tensor &xt = tensor(x), &wt = tensor(w);
+    if (xt.dim() != 2) { PyErr_SetString(PyExc_ValueError, "x must be a matrix [rows, inner]"); throw Error(); }
     Ref list(PySequence_Fast(outs, "outs must be a sequence"));
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(list.p);
     std::vector<cr_proj_out> o(n);
     int col = 0;
     for (Py_ssize_t i = 0; i < n; ++i) {
       const at::Tensor& t = tensor(PySequence_Fast_GET_ITEM(list.p, i));
+      if (t.dim() != 2 && t.size(0) == 0) { PyErr_SetString(PyExc_IndexError, "an output that is not a matrix needs a first row"); throw Error(); }
       const int cols = (int)(t.dim() == 2 ? t.size(1) : t.numel() / t.size(0));
       o[i] = cr_proj_out{t.data_ptr(), col, cols, cols, t.scalar_type() == at::kFloat ? 1 : 0};
       col += cols;

@@ -60,3 +60,11 @@ def _without_gpu(code):
 @pytest.mark.parametrize("call", ["_binding.current_stream()", "layers.proj_gemm(torch.zeros(1, 64).bfloat16(), torch.zeros(32, 64).bfloat16(), [torch.zeros(1, 32)])"])
 def test_no_gpu_is_an_exception(call):
     assert _without_gpu("try:\n    %s\nexcept RuntimeError:\n    print('refused')" % call) == ["refused"]
+
+
+@pytest.mark.parametrize("x,out,error", [((1, 64), (0,), "IndexError"), ((1, 64), (0, 4, 8), "IndexError"), ((1, 64), (), "IndexError"),
+                                         ((1, 8, 8), (1, 32), "ValueError"), ((64,), (1, 32), "ValueError"), ((), (1, 32), "ValueError")])
+def test_projection_shapes_that_are_refused(x, out, error):
+    """Outputs without rows that are not matrices (the width is looked up in the first row), and inputs that are not matrices."""
+    code = "try:\n    layers.proj_gemm(torch.zeros(%s).bfloat16(), torch.zeros(32, 64).bfloat16(), [torch.zeros(%s)])\nexcept %s:\n    print('refused')"
+    assert _without_gpu(code % (x, out, error)) == ["refused"]
