@@ -1,21 +1,26 @@
 // Gated DeltaNet decode / speculative-verify step for sm_100a.
 //
-// One CTA of 8 warps per (value head, span).  A warp owns 16 value columns of the head's 128 x 128 fp32 state, because the
-// delta rule never mixes value columns; a lane holds 4 columns x 16 keys of it in registers (as pairs of keys, for the
-// two-lane fp32 instructions), so a row of the pass costs a warp eight 128-bit reads of shared memory, eleven shuffles and no
-// barrier, and the rows (replayed ones first) run back to back.  Everything the pass reads is asked for at the start: raw
-// rows with their halo and the pending rows into shared memory, the state into L2 and, behind the a / b dot products, into
-// registers, the gate rows during the recurrence.
+// A cluster of 1, 2 or 4 CTAs of 8 warps per (value head, span).  The delta rule never mixes value columns, so a CTA has its
+// share of the columns of the head's 128 x 128 fp32 state and a warp 16 of them (8 in clusters); a lane holds 4 (2) columns x 16
+// keys in registers (as pairs of keys, for the two-lane fp32 instructions), so a row of the pass costs a warp eight 128-bit
+// reads of shared memory, eleven (nine) shuffles and no barrier, and the rows (replayed ones first) run back to back.
+// Everything the pass reads is asked for at the start: raw rows with their halo and the pending rows into shared memory, the
+// state into L2 and, behind the a / b dot products, into registers, the gate rows during the recurrence.  The CTAs of a cluster
+// prepare the same rows; what they exchange is the readout, once, for the norm over the head's columns.
 //
 // Semantics follow GdnKernel (engine/layers/ops.h:252-401): replay of pending rows, per-row update with the
 // readout from the updated state, state stored after row commit-1, rows >= commit recorded as
 // (khat, v, decay, beta), gated RMSNorm readout, raw-row ring update.
 //
 // Bound: latency of a few dependent memory round trips; with many rows the update chain.  Reads of k and q from shared memory
-// set the pace of every form with less state per lane: 8 sessions x (9 rows + 4 replayed) took 94 us with a quarter of the
-// columns per CTA and two barriers a row, 52 us with 8 columns per warp and none, 32 us now; 4 sessions x 1 row took 12.3 us,
-// 10.5 us now (one session 6.8, now 9: 32 CTAs pull 64 KB of state each).
+// set the pace of every form with less state per lane: 8 sessions x (9 rows + 4 replayed), 32 heads, took 95 us with a quarter
+// of the columns per CTA and two barriers a row, 52 us with 8 columns per warp and none, 32 us now.  One session x 1 row, 32
+// heads, state in L2 / in HBM: 6.8 / 9.2 us in that first form, 8.6 / 9.1 on a CTA per head, which pulls 64 KB of state, 6.6 / 7.1
+// as clusters of four.  4 sessions x 1 row: 9.8 / 12.9, now 8.8 / 10.1.  (Plain launches; chained ones take 0.5 to 0.8 less.)
+#include <cooperative_groups.h>
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cr {
 
@@ -31,7 +36,7 @@ struct GdnStepParams {
 };
 
 // Floats of dynamic shared memory: raw rows with halo, q, k and v rows (the readout replaces v), staged pending rows.
-__host__ __device__ inline int step_smem_floats(int rows, int replay) {
+__host__ __device__ constexpr int step_smem_floats(int rows, int replay) {
   const int rep = replay < kReplayChunk ? replay : kReplayChunk;
   return (rows + 3) * kRawCols + rows * kRawCols + rep * 258;
 }
@@ -42,14 +47,18 @@ __device__ __forceinline__ void step_cp(float* dst, const float* src, bool valid
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(BYTES), "r"(bytes));
 }
 
+// A head is a cluster of CL CTAs (grid x: CL per head); CTA k has 128 / CL of its value columns, NC of them per lane.
+template <int CL>
 __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_constant__ GdnStepParams P) {
+  constexpr int NC = CL == 1 ? 4 : 2, kWarpCols = 4 * NC, kOwners = 128 / CL / kWarpCols;   // columns of a lane, of a warp; warps that own columns
   extern __shared__ __align__(16) float step_sm[];
   __shared__ float ab_warp[kStepWarps][kStepRows][2];          // a / b dot products by warp
   __shared__ float dec[kStepRows], bet[kStepRows];
   const cr_gdn_args& a = P.span[blockIdx.y];
-  const int h = blockIdx.x, t = threadIdx.x, w = t >> 5, l = t & 31;
-  const int kg = l & 7, col4 = 16 * w + 4 * (l >> 3);          // keys 32 i + 4 kg + j of the columns col4 .. col4 + 3
-  const int own = (l & 1) * 2 + ((l >> 1) & 1);                // the column (of the four) whose sums end up in this lane
+  const int h = blockIdx.x / CL, rank = blockIdx.x % CL, t = threadIdx.x, w = t >> 5, l = t & 31;
+  const int kg = l & 7, col = rank * (128 / CL) + kWarpCols * w + NC * (l >> 3);   // keys 32 i + 4 kg + j of the columns col .. col + NC - 1
+  const int own = NC == 4 ? (l & 1) * 2 + ((l >> 1) & 1) : l & 1;                  // the column (of the NC) whose sums end up in this lane
+  const bool owner = kOwners == kStepWarps || w < kOwners;
   const int rep = P.Hv / P.Hk, kh = h / rep, KW = P.Hk * 128, VW = P.Hv * 128, C = 2 * KW + VW;
   const int R = a.R;
   float* raw = step_sm;                                        // [R + 3][384]: rows -3 .. R - 1
@@ -64,7 +73,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
   // ---- everything the pass reads is asked for: state (L2), raw rows and pending rows (shared memory)
   float* st = a.state + (size_t)h * 16384;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(st + (size_t)(t + 256 * i) * 32));
+  for (int i = 0; i < 2 / CL + (CL > 2); ++i)                  // 128 / CL columns of the 128 rows, 128 bytes at a time
+    if (CL < 4 || t < 128) {
+      const int line = t + 256 * i;
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(st + (size_t)(line / (4 / CL)) * 128 + rank * (128 / CL) + line % (4 / CL) * 32));
+    }
   const float* qkv = reinterpret_cast<const float*>(a.qkv);
   {
     // a warp takes every eighth row, a lane the same channels of each: 96 pieces of 4 channels, or 384 single ones
@@ -131,51 +144,73 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
     }
   }
   // The state, from L2 by now: its registers are not needed while the dot products hold theirs.
-  f2 S[4][8];                                                  // [column][pair of keys 32 (m / 2) + 4 kg + 2 (m % 2)]
+  f2 S[NC][8];                                                 // [column][pair of keys 32 (m / 2) + 4 kg + 2 (m % 2)]
+  if (owner) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const float* s2 = st + (size_t)(32 * i + 4 * kg + 2 * j) * 128 + col4;
-      const float4 x = *reinterpret_cast<const float4*>(s2), y = *reinterpret_cast<const float4*>(s2 + 128);
-      S[0][2 * i + j] = pack2(x.x, y.x); S[1][2 * i + j] = pack2(x.y, y.y);
-      S[2][2 * i + j] = pack2(x.z, y.z); S[3][2 * i + j] = pack2(x.w, y.w);
+    for (int i = 0; i < 8; ++i) {
+      const float* s2 = st + (size_t)(32 * (i >> 1) + 4 * kg + 2 * (i & 1)) * 128 + col;
+      if constexpr (NC == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(s2), y = *reinterpret_cast<const float4*>(s2 + 128);
+        S[0][i] = pack2(x.x, y.x); S[1][i] = pack2(x.y, y.y); S[2][i] = pack2(x.z, y.z); S[3][i] = pack2(x.w, y.w);
+      } else {
+        const float2 x = *reinterpret_cast<const float2*>(s2), y = *reinterpret_cast<const float2*>(s2 + 128);
+        S[0][i] = pack2(x.x, y.x); S[1][i] = pack2(x.y, y.y);
+      }
     }
+  }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
 
-  // The sums over the eight key groups of four values per lane: every lane ends up with that of its own column.
-  auto reduce4 = [&](const float (&x)[4]) {
-    const bool hi = l & 1, odd = l & 2;
-    float a0 = hi ? x[2] : x[0], a1 = hi ? x[3] : x[1];
-    a0 += __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 1);
-    a1 += __shfl_xor_sync(0xffffffffu, hi ? x[1] : x[3], 1);
-    float s = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 2);
+  // The sums over the eight key groups of NC values per lane: every lane ends up with that of its own column.  A column's sum
+  // has the same order for every NC, so a pass gives the same bits whatever else shares its launch.
+  auto reduce = [&](const float (&x)[NC]) {
+    const bool hi = l & 1;
+    float s;
+    if constexpr (NC == 4) {
+      const bool odd = l & 2;
+      float a0 = hi ? x[2] : x[0], a1 = hi ? x[3] : x[1];
+      a0 += __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 1);
+      a1 += __shfl_xor_sync(0xffffffffu, hi ? x[1] : x[3], 1);
+      s = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 2);
+    } else {
+      s = (hi ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[1], 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+    }
     return s + __shfl_xor_sync(0xffffffffu, s, 4);
   };
   // One delta-rule update with the 128 key values kv and the head's value row v; the readout of the updated state goes over
   // v where qv is given.
   auto update = [&](const float* kv, const float* qv, float decay, float beta, float* v) {
+    if (!owner) return;
     f2 k2[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) load_f2x2(kv + 32 * i + 4 * kg, k2[2 * i], k2[2 * i + 1]);
-    float m[4];
+    auto columns = [&](float (&m)[NC]) {                        // this lane's share of k2 . S
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      f2 x = mul2(S[c][0], k2[0]), y = mul2(S[c][1], k2[1]);
+      for (int c = 0; c < NC; ++c) {
+        f2 x = mul2(S[c][0], k2[0]), y = mul2(S[c][1], k2[1]);
 #pragma unroll
-      for (int i = 2; i < 8; i += 2) { x = fma2(S[c][i], k2[i], x); y = fma2(S[c][i + 1], k2[i + 1], y); }
-      const float2 z = unpack2(add2(x, y));
-      m[c] = z.x + z.y;
+        for (int i = 2; i < 8; i += 2) { x = fma2(S[c][i], k2[i], x); y = fma2(S[c][i + 1], k2[i + 1], y); }
+        const float2 z = unpack2(add2(x, y));
+        m[c] = z.x + z.y;
+      }
+    };
+    float m[NC];
+    columns(m);
+    const float mine = beta * (v[col + own] - decay * reduce(m));
+    float delta[NC];                                            // back to every lane
+    if constexpr (NC == 4) {
+      const float pair = __shfl_xor_sync(0xffffffffu, mine, 2);
+      const float d0 = (l & 2) ? pair : mine, d1 = (l & 2) ? mine : pair;
+      const float e0 = __shfl_xor_sync(0xffffffffu, d0, 1), e1 = __shfl_xor_sync(0xffffffffu, d1, 1);
+      delta[0] = (l & 1) ? e0 : d0; delta[1] = (l & 1) ? e1 : d1; delta[2] = (l & 1) ? d0 : e0; delta[3] = (l & 1) ? d1 : e1;
+    } else {
+      const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
+      delta[0] = (l & 1) ? other : mine; delta[1] = (l & 1) ? mine : other;
     }
-    const float mine = beta * (v[col4 + own] - decay * reduce4(m));
-    const float pair = __shfl_xor_sync(0xffffffffu, mine, 2);   // the deltas of the four columns back to every lane
-    const float d0 = (l & 2) ? pair : mine, d1 = (l & 2) ? mine : pair;
-    const float e0 = __shfl_xor_sync(0xffffffffu, d0, 1), e1 = __shfl_xor_sync(0xffffffffu, d1, 1);
-    const float delta[4] = {(l & 1) ? e0 : d0, (l & 1) ? e1 : d1, (l & 1) ? d0 : e0, (l & 1) ? d1 : e1};
     const f2 g2 = pack2(decay, decay);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < NC; ++c) {
       const f2 d2 = pack2(delta[c], delta[c]);
 #pragma unroll
       for (int i = 0; i < 8; ++i) S[c][i] = fma2(k2[i], d2, mul2(g2, S[c][i]));
@@ -183,17 +218,9 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
     if (qv) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) load_f2x2(qv + 32 * i + 4 * kg, k2[2 * i], k2[2 * i + 1]);
-      float o[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        f2 x = mul2(S[c][0], k2[0]), y = mul2(S[c][1], k2[1]);
-#pragma unroll
-        for (int i = 2; i < 8; i += 2) { x = fma2(S[c][i], k2[i], x); y = fma2(S[c][i + 1], k2[i + 1], y); }
-        const float2 z = unpack2(add2(x, y));
-        o[c] = z.x + z.y;
-      }
-      const float y = reduce4(o);
-      if (kg < 4) v[col4 + own] = y;                            // the warp has read its v before the shuffles
+      columns(m);
+      const float y = reduce(m);
+      if (kg < NC) v[col + own] = y;                            // the warp has read its v before the shuffles
     }
   };
 
@@ -209,6 +236,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
     }
     for (int i = 0; i < n; ++i) update(pk + i * 256, nullptr, pg[2 * i], pg[2 * i + 1], pk + i * 256 + 128);
   }
+  if (CL > 1 && a.replay > 0 && R > a.commit) cg::this_cluster().sync();   // every CTA has its pending rows before new ones are recorded
 
   // ---- conv + SiLU: a thread takes q or k channel t of all rows and a v channel of every other row
   {
@@ -250,16 +278,19 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
     dec[t] = expf(-__expf(a.A_log[h]) * softplus);
     bet[t] = sigmoidf_(pb);
   }
-  float z[2][4];                                               // gate rows w and w + 8: in flight during the recurrence
+  constexpr int kGateRows = (kStepRows + CL * kStepWarps - 1) / (CL * kStepWarps);
+  float z[kGateRows][4];                                       // this warp's gate rows: in flight during the recurrence
 #pragma unroll
-  for (int k = 0; k < 2; ++k)
+  for (int k = 0; k < kGateRows; ++k) {
+    const int r = rank + CL * (w + kStepWarps * k);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) z[k][i] = w + 8 * k < R ? reinterpret_cast<const float*>(a.z)[(size_t)(w + 8 * k) * VW + h * 128 + 4 * l + i] : 0.f;
+    for (int i = 0; i < 4; ++i) z[k][i] = r < R ? reinterpret_cast<const float*>(a.z)[(size_t)r * VW + h * 128 + 4 * l + i] : 0.f;
+  }
   __syncthreads();
 
   // ---- raw-row ring (slots of this call never alias the three slots any CTA reads: R + 3 <= 16) and speculative rows:
   // (khat, v, decay, beta) for the next pass's replay, whose old rows every warp of this head has used
-  for (int r = w; r < R; r += kStepWarps) {
+  for (int r = rank + CL * w; r < R; r += CL * kStepWarps) {
     float* hs = a.hist + (size_t)((a.pos0 + r) & 15) * C;
     const float* x = raw + (r + 3) * kRawCols;
 #pragma unroll
@@ -280,28 +311,33 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
   // ---- the recurrence
   for (int r = 0; r < R; ++r) {
     update(ks + r * 128, qs + r * 128, dec[r], bet[r], vs + r * 128);
-    if (r == a.commit - 1) {
+    if (owner && r == a.commit - 1) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i) {
+        float2 x[NC];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          float2 x[4];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) x[c] = unpack2(S[c][2 * i + j]);
-          float* s2 = st + (size_t)(32 * i + 4 * kg + 2 * j) * 128 + col4;
+        for (int c = 0; c < NC; ++c) x[c] = unpack2(S[c][i]);
+        float* s2 = st + (size_t)(32 * (i >> 1) + 4 * kg + 2 * (i & 1)) * 128 + col;
+        if constexpr (NC == 4) {
           *reinterpret_cast<float4*>(s2) = make_float4(x[0].x, x[1].x, x[2].x, x[3].x);
           *reinterpret_cast<float4*>(s2 + 128) = make_float4(x[0].y, x[1].y, x[2].y, x[3].y);
+        } else {
+          *reinterpret_cast<float2*>(s2) = make_float2(x[0].x, x[1].x);
+          *reinterpret_cast<float2*>(s2 + 128) = make_float2(x[0].y, x[1].y);
         }
+      }
     }
   }
-  __syncthreads();
+  if constexpr (CL == 1) __syncthreads();
+  else cg::this_cluster().sync();                              // the readout of all columns is there
 
-  // ---- gated RMSNorm over the head's 128 columns, a warp per row, lane l the columns 4 l .. 4 l + 3
+  // ---- gated RMSNorm over the head's 128 columns, a warp per row (the rows dealt over the cluster), lane l the columns 4 l .. 4 l + 3
+  const float* yv_s = CL == 1 ? vs : cg::this_cluster().map_shared_rank(vs, l * CL / 32);
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int r = w + 8 * k;
+  for (int k = 0; k < kGateRows; ++k) {
+    const int r = rank + CL * (w + kStepWarps * k);
     if (r >= R) break;
-    const float4 y = *reinterpret_cast<const float4*>(vs + r * 128 + 4 * l);
+    const float4 y = *reinterpret_cast<const float4*>(yv_s + r * 128 + 4 * l);
     const float rs = rsqrtf(warp_sum(y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w) * (1.f / 128.f) + kEps);
     const float yv[4] = {y.x, y.y, y.z, y.w};
     float o[4];
@@ -329,6 +365,36 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
       store_half4(reinterpret_cast<uint16_t*>(a.out) + out_index(r, h * 128 + 4 * l, VW, a.pack_rows, a.pack_off), o, kHadNorm);
     }
   }
+  if constexpr (CL > 1) cg::this_cluster().sync();             // the rows stay until every CTA has read them
+}
+
+// With more than half of an SM's shared memory a CTA has an SM of its own.  Calls that fit the SMs once ask for that: let in while
+// the kernel ahead still holds most SMs, the CTAs would pair up on the free ones and stay there, and a pair takes half as long
+// again (steps of 3 sessions x 1 row, 32 heads, one behind the other: 12.7 us paired, 9.0 us).
+constexpr size_t kAloneSmem = 116 * 1024;
+static_assert(step_smem_floats(kStepRows, kReplayChunk) * sizeof(float) <= kAloneSmem, "the longest pass fits");
+
+template <int CL>
+static cr_status step_launch(const GdnStepParams& P, int n, cudaStream_t stream) {
+  static PerDeviceOnce configured;
+  if (cr_status st = once_per_device(configured, [] {
+        CR_CUDA(cudaFuncSetAttribute(gdn_step_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAloneSmem));
+        return CR_OK;
+      })) return st;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(P.Hv * CL, n); cfg.blockDim = dim3(kStepThreads); cfg.stream = stream;
+  cfg.dynamicSmemBytes = P.Hv * CL * n <= sm_count() ? kAloneSmem : step_smem_floats(P.rows, P.replay) * sizeof(float);
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (pdl_enabled()) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na++].val.programmaticStreamSerializationAllowed = 1; }
+  if (CL > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = CL; attr[na].val.clusterDim.y = 1; attr[na++].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr; cfg.numAttrs = na;
+  CR_CUDA(cudaLaunchKernelEx(&cfg, gdn_step_kernel<CL>, P));
+  CR_LAUNCH_CHECK("gdn_step_kernel");
+  return CR_OK;
 }
 
 }  // namespace cr
@@ -359,19 +425,17 @@ extern "C" cr_status cr_gdn_step(const cr_geometry* g, const cr_gdn_args* spans,
     const int n = n_spans - s0 < kMaxSpans ? n_spans - s0 : kMaxSpans;
     for (int s = 0; s < n; ++s) P.span[s] = spans[s0 + s];
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.hidden = g->hidden; P.pend_rows = pend_rows; P.fmt = (int)fmt;
-    static PerDeviceOnce configured;
-    if (cr_status st = once_per_device(configured, [] {
-          CR_CUDA(cudaFuncSetAttribute(gdn_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(step_smem_floats(kStepRows, kReplayChunk) * sizeof(float))));
-          return CR_OK;
-        })) return st;
     P.rows = P.replay = 0;
     for (int s = 0; s < n; ++s) {
       P.rows = P.rows > P.span[s].R ? P.rows : P.span[s].R;
       P.replay = P.replay > P.span[s].replay ? P.replay : P.span[s].replay;
     }
-    CR_CUDA(launch_pdl(gdn_step_kernel, dim3(g->gdn_vheads, n), dim3(kStepThreads), step_smem_floats(P.rows, P.replay) * sizeof(float),
-                       (cudaStream_t)stream, P));
-    CR_LAUNCH_CHECK("gdn_step_kernel");
+    // Few heads leave SMs idle: a head is spread over as many CTAs as there are SMs for.  States in HBM, 1 / 9 rows: 32 heads
+    // 9.1 / 21.2 us on one CTA each, 8.0 / 18.3 on two, 7.1 / 17.3 on four; 64 heads 9.3 / 21.7, 8.4 / 18.9, 8.6 / 19.8; 96 heads
+    // 9.7 / 22.1, 10.8 / 22.5: once two CTAs share an SM the work that a head's CTAs repeat (rows, dot products) costs more.
+    const int heads = n * P.Hv, cl = 4 * heads <= sm_count() ? 4 : (2 * heads <= sm_count() ? 2 : 1);
+    const auto launch = cl == 4 ? step_launch<4> : cl == 2 ? step_launch<2> : step_launch<1>;
+    if (cr_status st = launch(P, n, (cudaStream_t)stream)) return st;
   }
   return CR_OK;
 }

@@ -134,3 +134,38 @@ def test_gdn_prefill_ring_at_any_float_address(algo, bf16, offset):
         out = plan.run(s, qkv, z, ab, pos0, capi.GDN_SERIAL_F32 if algo == "serial" else capi.GDN_CHUNK_TC)
         got.append((out.clone(), s.state.clone(), s.hist.clone(), room[:shift].sum() + room[shift + 16 * C:].sum()))
     assert all(torch.equal(a, b) for a, b in zip(*got)) and got[1][3] == 0
+
+
+# A GDN step alone and beside 1 to 5 other sessions: its heads run as clusters of four, of two (2 sessions x 32 heads; 48 heads),
+# as single CTAs with an SM each and two to an SM, and give the same bits.  Rows and replayed rows from the fewest to the most,
+# more replayed rows than are staged at once, rows that are recorded where replayed ones lay.
+@pytest.mark.parametrize("heads", [32, 48])
+@pytest.mark.parametrize("R,replay,commit", [(1, 0, 1), (4, 2, 1), (9, 8, 1), (13, 17, 5), (13, 0, 13)])
+@pytest.mark.parametrize("fmt", [0, 1, 2])
+def test_gdn_step_clusters(heads, R, replay, commit, fmt):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(512, 16, 2, heads, 16)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    C, W = g.gdn_channels, heads * 128
+    w = layers.GdnWeights(g, rn(C, 4, std=0.5), rn(heads) - 1, rn(heads, std=0.5), 1 + rn(128, std=0.1), ab=rn(2 * heads, 512, std=0.05), suh=1 + rn(W, std=0.1))
+    rows = [(rn(R, C), rn(R, W), rn(R, 512)) for _ in range(6)]
+    begin = [(rn(heads * 16384 + 64, std=0.1), rn(16, C), torch.cat([rn(heads, 20, 256, std=0.2), torch.rand(heads, 20, 2, device="cuda", generator=gen)], 2)) for _ in range(6)]
+
+    def span(i):
+        s = layers.GdnSession(g, pend_rows=20)
+        for to, x in zip((s.state, s.hist, s.pend), begin[i]):
+            to.copy_(x)
+        qkv, z, x = rows[i]
+        return dict(session=s, qkv=qkv, z=z, x=x, pos0=7, replay=replay, commit=commit)
+
+    def results(spans, outs):
+        s = spans[0]["session"]
+        return outs[0], s.state, s.hist, s.pend
+
+    alone = [span(0)]
+    want = results(alone, layers.gdn_step(w, alone, fmt))
+    assert torch.isfinite(want[0].float()).all() and torch.isfinite(want[1]).all()
+    for n in (2, 3, 4, 6):
+        spans = [span(i) for i in range(n)]
+        assert all(torch.equal(a, b) for a, b in zip(want, results(spans, layers.gdn_step(w, spans, fmt)))), n
