@@ -774,7 +774,6 @@ class SplitKvPrefill262k:
         self.sel_mine = torch.zeros(Rr, 512, device="cuda", dtype=torch.int32); self.nsel_mine = torch.zeros(Rr, device="cuda", dtype=torch.int32)
         self.part = torch.empty(R, 16, 258, device="cuda"); self.my_part = torch.empty(world, Rr, 16, 258, device="cuda")
         self.out_mine = torch.empty(Rr, 4096, device="cuda", dtype=torch.bfloat16)
-        self.scratch = torch.empty(R * 16 * 4 * 258 * 4, dtype=torch.uint8, device="cuda")
         # the argument block of this rank's rows: same buffers, row pointers moved to row r0, selections and outputs of its own
         mine = capi.QsaArgs.from_buffer_copy(self.args)
         mine.q += r0 * 16 * 512 * 4; mine.idx += r0 * 640 * 4; mine.k += r0 * 512 * 4; mine.v += r0 * 512 * 4
@@ -820,7 +819,7 @@ class SplitKvPrefill262k:
             self.sel.copy_(self.sel_mine); self.nsel.copy_(self.nsel_mine)
         if timed: self.ev[3].record()
         capi.check(capi.lib.cr_qsa_shard_attn(C.byref(g), arr, self.p0, self.p1 if self.rank < self.world - 1 else 2 ** 31 - 1,
-                                              self.part.data_ptr(), self.scratch.data_ptr(), self.scratch.numel(), st))
+                                              self.part.data_ptr(), None, 0, st))
         if timed: self.ev[4].record()
         if self.world > 1:
             dist.all_to_all_single(self.my_part.view(-1, 16, 258), self.part)

@@ -501,54 +501,35 @@ static cr_status check_out(const cr_qsa_args* spans, int n, cr_out_format fmt, c
   return CR_OK;
 }
 
-static size_t total_rows(const cr_qsa_args* spans, int n) {
-  size_t r = 0;
-  for (int s = 0; s < n; ++s) r += (size_t)spans[s].R;
-  return r;
-}
-
 }  // namespace cr
 
+// What the reference's callers size by; the entry points below ignore their scratch, the parts of a row being merged on chip.
 extern "C" size_t cr_qsa_scratch_bytes(const cr_geometry* g, int rows) {
   if (!g || rows < 1) return 0;
   return (size_t)rows * g->q_heads * CR_QSA_SPLITS * CR_QSA_PART * sizeof(float);
 }
 
-extern "C" cr_status cr_qsa_attn(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void* scratch, size_t scratch_bytes,
-                                 cr_out_format fmt, void* stream) {
+extern "C" cr_status cr_qsa_attn(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void*, size_t, cr_out_format fmt, void* stream) {
   using namespace cr;
   if (cr_status s = qsa_validate(g, spans, n_spans, CR_MAX_STEP_ROWS, "cr_qsa_attn")) return s;
   if (cr_status s = check_out(spans, n_spans, fmt, "cr_qsa_attn")) return s;
-  const size_t need = cr_qsa_scratch_bytes(g, (int)total_rows(spans, n_spans));
-  CR_REQUIRE(scratch && scratch_bytes >= need, "cr_qsa_attn: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
   return qsa_attn_launch(g, spans, n_spans, nullptr, 0, INT_MAX, fmt, (cudaStream_t)stream);
 }
 
-extern "C" cr_status cr_qsa_step(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void* scratch, size_t scratch_bytes,
-                                 cr_out_format fmt, void* stream) {
+extern "C" cr_status cr_qsa_step(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void*, size_t, cr_out_format fmt, void* stream) {
   using namespace cr;
   if (cr_status s = qsa_validate(g, spans, n_spans, CR_MAX_STEP_ROWS, "cr_qsa_step")) return s;
   if (cr_status s = check_out(spans, n_spans, fmt, "cr_qsa_step")) return s;
-  const size_t need = cr_qsa_scratch_bytes(g, (int)total_rows(spans, n_spans));
-  CR_REQUIRE(scratch && scratch_bytes >= need, "cr_qsa_step: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   if (cr_status s = qsa_prep_launch(g, spans, n_spans, 0, nullptr, 0, st, false, true)) return s;
   if (cr_status s = qsa_select_launch(g, spans, n_spans, st, true)) return s;
   return qsa_attn_launch(g, spans, n_spans, nullptr, 0, INT_MAX, fmt, st);
 }
 
-extern "C" cr_status cr_qsa_shard_attn(const cr_geometry* g, const cr_qsa_args* a, int p0, int p1, float* partials, void* scratch,
-                                       size_t scratch_bytes, void* stream) {
+extern "C" cr_status cr_qsa_shard_attn(const cr_geometry* g, const cr_qsa_args* a, int p0, int p1, float* partials, void*, size_t, void* stream) {
   using namespace cr;
   if (cr_status s = qsa_validate(g, a, 1, CR_MAX_PREFILL_ROWS, "cr_qsa_shard_attn", 0)) return s;
   CR_REQUIRE(partials && p0 >= 0 && p1 >= p0, "cr_qsa_shard_attn: bad position window or null output");
-  // A part's rows take up to 4 splits each; a window that holds a fraction of the cache holds about that fraction of a
-  // row's 2,051 attended positions, so it takes fewer (a split whose list is longer than expected walks it in chunks).
-  const long long cache = (long long)a->pos0 + a->R, window = (p1 < cache ? p1 : cache) - p0;
-  const int part_splits = window <= 0 ? 1 : (int)((4 * window + cache - 1) / cache);
-  const int splits = a->R <= CR_MAX_STEP_ROWS ? CR_QSA_SPLITS : (part_splits < 1 ? 1 : part_splits > 4 ? 4 : part_splits);
-  const size_t need = (size_t)a->R * g->q_heads * splits * CR_QSA_PART * sizeof(float);
-  CR_REQUIRE(scratch && scratch_bytes >= need, "cr_qsa_shard_attn: scratch of %zu bytes needed, %zu given", need, scratch_bytes);
   return qsa_attn_launch(g, a, 1, partials, p0, p1, CR_OUT_RAW_F32, (cudaStream_t)stream);
 }
 

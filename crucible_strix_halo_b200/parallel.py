@@ -153,7 +153,6 @@ class CudaQsaBackend:
         self.capi, self.torch, self.g, self.rows, self.fmt, self.out = capi, torch, geometry, rows, fmt, out
         self.args = args
         self.arr = (capi.QsaArgs * 1)(args)
-        self.scratch = torch.empty(rows * geometry.q_heads * 32 * 258 * 4, dtype=torch.uint8, device="cuda")
         self.sel = torch.zeros(rows, 512, device="cuda", dtype=torch.int32)        # the part's selection, wherever it was merged
         self.nsel = torch.zeros(rows, device="cuda", dtype=torch.int32)
 
@@ -199,7 +198,7 @@ class CudaQsaBackend:
     def shard_attn(self, p0, p1):
         parts = self.torch.empty(self.rows, self.g.q_heads, 258, device="cuda")
         self.capi.check(self.capi.lib.cr_qsa_shard_attn(C.byref(self.g), self.arr, p0, min(p1, 2 ** 31 - 1), parts.data_ptr(),
-                                                          self.scratch.data_ptr(), self.scratch.numel(), self._stream()))
+                                                          None, 0, self._stream()))
         return parts
 
     def merge_partials(self, parts, r0, r1):

@@ -184,8 +184,8 @@ typedef struct {
 
 /* Scratch sizing (engine/layers/qsa_long.h:226, :396; engine/layers/ops.h:420;
  * engine/layers/cache_storage.h:40-46). */
-size_t cr_qsa_scratch_bytes(const cr_geometry* g, int rows);         /* split-KV partials: rows x Hq x 32 x 258 floats
-                                                                        (a pass of many rows uses fewer splits of it) */
+size_t cr_qsa_scratch_bytes(const cr_geometry* g, int rows);         /* rows x Hq x 32 x 258 floats, what QsaScratchFloats
+                                                                        call sites allocate; nothing here needs it */
 size_t cr_qsa_select_scratch_bytes(const cr_geometry* g, int rows);  /* 0: the select kernels keep their candidate
                                                                         lists on chip; kept so that
                                                                         QsaSelectScratchFloats call sites compile */
@@ -217,8 +217,7 @@ cr_status cr_qsa_select(const cr_geometry* g, const cr_qsa_args* spans, int n_sp
 /* Replaces LaunchQsaAttn / QsaAttnTailKernel (engine/layers/qsa_long.h:399-534): split-KV attention over the
  * attended positions, log-sum-exp merge, sigmoid gate, output transform, in one launch: the parts of a row are merged on
  * chip, over a thread-block cluster where a row spans several blocks, and there are no counters (the reference's `sync`
- * words have no counterpart).  `scratch` of cr_qsa_scratch_bytes(g, total rows) bytes is part of the contract, as the
- * reference's launcher takes it; it needs no initialisation. */
+ * words have no counterpart).  `scratch` stands where the reference's launcher takes it and is ignored: NULL and 0 will do. */
 cr_status cr_qsa_attn(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void* scratch,
                       size_t scratch_bytes, cr_out_format fmt, void* stream);
 
@@ -232,7 +231,7 @@ cr_status cr_qsa_attn_static(const cr_geometry* g, const cr_qsa_args* spans, int
                              void* stream);
 
 /* prep + select + attn, the whole AttentionCore of a QSA layer for decode / verify
- * (engine/runtime/batch_forward.h:300-333). */
+ * (engine/runtime/batch_forward.h:300-333).  `scratch` as in cr_qsa_attn. */
 cr_status cr_qsa_step(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, void* scratch,
                       size_t scratch_bytes, cr_out_format fmt, void* stream);
 
@@ -294,7 +293,7 @@ cr_status cr_qsa_shard_select(const cr_geometry* g, const cr_qsa_args* a, int b0
 cr_status cr_qsa_merge_candidates(const cr_geometry* g, const cr_qsa_args* a, int ranks,
                                   const float* cand_scores, const int* cand_ids, void* stream);
 /* Attention over the attended positions inside [p0, p1) only; writes one partial (m, l, acc[256]) per
- * (row, head): partials [rows][Hq][258]. */
+ * (row, head): partials [rows][Hq][258].  `scratch` as in cr_qsa_attn. */
 cr_status cr_qsa_shard_attn(const cr_geometry* g, const cr_qsa_args* a, int p0, int p1, float* partials,
                             void* scratch, size_t scratch_bytes, void* stream);
 /* LSE merge of gathered partials [ranks][rows][Hq][258] + gate + output transform. */

@@ -60,3 +60,27 @@ def test_static_scratch_rejects_oversized_calls():
     arr, keep = _spans(capi, layers, w, g, rng, ctxs=[600, 600], rows=[9, 8])     # 17 rows x 16 heads = 272 > 256
     assert capi.lib.cr_qsa_attn_static(C.byref(g), arr, 2, capi.OUT_RAW_F32, None) == capi.ERR_INVALID
     assert b"exceed the built-in scratch" in capi.lib.cr_last_error()
+
+
+def test_attention_without_scratch_equals_static():
+    """cr_qsa_attn and cr_qsa_shard_attn take no scratch: NULL and 0."""
+    from crucible_strix_halo_b200 import capi, layers
+    torch.manual_seed(2)
+    g = capi.GEOM_BENCH
+    rng = np.random.default_rng(2)
+    w = layers.QsaWeights(g, *[1 + 0.1 * rng.normal(size=n) for n in (256, 256, 128, 128)])
+    arr, keep = _spans(capi, layers, w, g, rng, ctxs=[2500], rows=[3])
+    out = keep[0][2]
+    capi.check(capi.lib.cr_qsa_prep(C.byref(g), arr, 1, None))
+    capi.check(capi.lib.cr_qsa_select(C.byref(g), arr, 1, None, 0, None))
+    capi.check(capi.lib.cr_qsa_attn_static(C.byref(g), arr, 1, capi.OUT_RAW_F32, None))
+    want = out.clone()
+    out.zero_()
+    capi.check(capi.lib.cr_qsa_attn(C.byref(g), arr, 1, None, 0, capi.OUT_RAW_F32, None))
+    assert torch.equal(out, want) and want.abs().max() > 0
+    parts = torch.empty(2, 3, 16, 258, device="cuda")
+    for i, (p0, p1) in enumerate([(0, 1200), (1200, 1 << 30)]):
+        capi.check(capi.lib.cr_qsa_shard_attn(C.byref(g), arr, p0, p1, parts[i].data_ptr(), None, 0, None))
+    out.zero_()
+    capi.check(capi.lib.cr_qsa_merge_partials(C.byref(g), arr, 2, parts.data_ptr(), capi.OUT_RAW_F32, None))
+    assert torch.allclose(out, want, rtol=0, atol=2e-4)          # two partial sums of fp32-level products
