@@ -150,19 +150,6 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Sum over a block of NT threads; red holds NT/32 floats; every thread gets the same fixed-order result.
-template <int NT>
-__device__ __forceinline__ float block_sum(float v, float* red) {
-  v = warp_sum(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = 0.f;
-#pragma unroll
-  for (int i = 0; i < NT / 32; ++i) t += red[i];
-  return t;
-}
-
 // In-warp natural-order Sylvester-Hadamard of 128 values, lane l holding elements 4l..4l+3; unnormalised.
 __device__ __forceinline__ void wht128(float v[4]) {
   const int lane = threadIdx.x & 31;

@@ -37,37 +37,6 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], flo
         "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
 
-// acc[16 x 8NT] += A[16 x 8KT] B.  A row-major in shared memory (lda % 32 == 4), or A_T: stored [k][m]
-// (lda % 32 == 8).  B stored [k][n] (ldb % 32 == 8), or B_NK: stored [n][k] (ldb % 32 == 4).
-// Operands hold tf32-rounded values.  Bank-conflict free for the stated strides.
-template <int NT, int KT, bool A_T, bool B_NK>
-__device__ __forceinline__ void warp_gemm(float (&acc)[NT][4], const float* A, int lda, const float* B, int ldb) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int kk = 0; kk < KT; ++kk) {
-    float a[4];
-    if constexpr (!A_T) {
-      a[0] = A[g * lda + kk * 8 + t];       a[1] = A[(g + 8) * lda + kk * 8 + t];
-      a[2] = A[g * lda + kk * 8 + t + 4];   a[3] = A[(g + 8) * lda + kk * 8 + t + 4];
-    } else {
-      a[0] = A[(kk * 8 + t) * lda + g];     a[1] = A[(kk * 8 + t) * lda + g + 8];
-      a[2] = A[(kk * 8 + t + 4) * lda + g]; a[3] = A[(kk * 8 + t + 4) * lda + g + 8];
-    }
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      float b0, b1;
-      if constexpr (B_NK) {
-        b0 = B[(n * 8 + g) * ldb + kk * 8 + t];
-        b1 = B[(n * 8 + g) * ldb + kk * 8 + t + 4];
-      } else {
-        b0 = B[(kk * 8 + t) * ldb + n * 8 + g];
-        b1 = B[(kk * 8 + t + 4) * ldb + n * 8 + g];
-      }
-      mma_tf32(acc[n], a, b0, b1);
-    }
-  }
-}
-
 // Four 8 x 4 pieces of tf32 values (8 rows of 16 bytes each) in one instruction: lane L passes the address of row
 // L % 8 of piece L / 8 and receives element (L / 4, L % 4) of every piece, which is the layout of the m16n8k8
 // fragments.  Rows must be 16-byte aligned.

@@ -34,10 +34,6 @@ constexpr int kStageFloats = 16384 + 8192 + 4096;         // [W ; e^G Q] 64 KB, 
 constexpr size_t kScanSmem = (size_t)2 * kStageFloats * sizeof(float) + 128;
 constexpr uint32_t kColS = 0, kColD2 = 128, kColD1 = 256;   // D1 of chunk c at kColD1 + 128 (c & 1)
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_u32(bar)) : "memory");
-}
-
 __device__ __forceinline__ unsigned load_acquire_gpu(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");

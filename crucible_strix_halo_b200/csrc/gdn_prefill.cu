@@ -76,9 +76,7 @@ __global__ void __launch_bounds__(256) gdn_prep_kernel(GdnPrefillParams P) {
       if (i >= rows) break;
       const float ss = red[i][part * 4] + red[i][part * 4 + 1] + red[i][part * 4 + 2] + red[i][part * 4 + 3];
       const float sc = rsqrtf(ss + kEps) * (part ? 1.f : kInvSqrt128);
-      float o = val[i] * sc;
-      if (P.tf32) o = tf32r(o);
-      dst[((size_t)(r0 + i) * P.Hk + u) * 128 + j] = o;
+      dst[((size_t)(r0 + i) * P.Hk + u) * 128 + j] = val[i] * sc;
     }
   } else {
 #pragma unroll
@@ -385,7 +383,6 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
     P.a.commit = P.a.R;
     P.ab_logits = (const char*)args->ab_logits + (size_t)p0 * 2 * g->gdn_vheads * in_elt;
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.fmt = (int)fmt;
-    P.tf32 = 0;
     P.chained = pdl_enabled() && !pipelined;
     P.halo_in = p0 > 0;
     P.gate_blocks = (unsigned)(((long long)P.a.R * g->gdn_vheads + 8 * kGateUnits - 1) / (8 * kGateUnits));

@@ -9,7 +9,7 @@ namespace cr {
 // two workspaces used in turn.  The scan pays a fixed cost per launch (state load and store, pipeline fill, 15 to
 // 40 us measured), which argues for long parts; the first local kernel and the last scan have nothing to run
 // beside, which argues for short ones.  A part's intermediates take about 72 KB per row.
-int gdn_part_rows();   // 64 x cr_options.gdn_part_chunks (kGdnPartRowsDefault unless a host changed it)
+int gdn_part_rows();   // 64 x cr_options.gdn_part_chunks (kGdnPartChunksDefault unless a host changed it)
 
 struct GdnPrefillParams {
   cr_gdn_args a;
@@ -24,7 +24,6 @@ struct GdnPrefillParams {
   unsigned gate_blocks;    // blocks of the gate kernel that gate; those behind them fill the ring
   int ring_rows;           // rows of the raw-row ring this part writes
   bool chained;            // launch with programmatic dependence on the kernel ahead (not across the streams of the part pipeline)
-  int tf32;                // 1: prep rounds q/k to tf32 (operands of the tensor-core scan)
 };
 
 bool gdn_chunk_available();

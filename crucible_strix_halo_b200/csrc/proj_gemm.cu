@@ -53,9 +53,6 @@ __device__ __forceinline__ void load_box_2d(void* dst, const CUtensorMap* map, i
                "l"(map), "r"(c0), "r"(c1), "r"(umma::smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void gemm_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_u32(bar)) : "memory");
-}
 // Instruction descriptor for kind::f16 with bf16 operands (format 1), fp32 accumulation, both operands K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);

@@ -11,9 +11,6 @@
 // algorithm allows.
 #pragma once
 #include <cstdint>
-#ifndef CR_MBAR_BACKOFF
-#define CR_MBAR_BACKOFF 0
-#endif
 #include <cuda_runtime.h>
 
 namespace cr {
@@ -203,10 +200,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 // Asks the copy engine to bring [src, src + bytes) into L2 (16-byte aligned, multiple of 16); nothing is signalled.
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
-}
-// K-major operand with padded planes: float[K/4][plane_units][4], rows < plane_units.
-__device__ __forceinline__ uint64_t desc_kmajor_padded(const float* base, int plane_units, int k0) {
-  return smem_desc(base + (size_t)(k0 / 4) * plane_units * 4, (uint32_t)plane_units * 16u, 128u);
 }
 }  // namespace umma
 }  // namespace cr
