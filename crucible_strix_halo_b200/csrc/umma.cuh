@@ -70,13 +70,6 @@ __device__ __forceinline__ bool mbar_try_relaxed(uint32_t addr, uint32_t parity)
 __device__ __forceinline__ void mbar_arrive_relaxed(uint64_t* bar) {
   asm volatile("mbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
-// Waits for the phase with the given parity; gives up after `limit` polls and returns false.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = 1u << 22) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t i = 0; i < limit; ++i)
-    if (mbar_try(addr, parity)) return true;
-  return false;
-}
 // Waits with a bound in time: gives up after max_ns nanoseconds (or as soon as *abort is set by another
 // thread that gave up) and returns false.  The clock is not read before a few polls have failed.
 template <bool RELAXED = false>

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(128) umma_test_kernel(const float* A, const fl
     for (int k0 = 0; k0 < K; k0 += 8) umma::mma_tf32_ss(tmem, umma::desc_kmajor(As, 128, k0), umma::desc_kmajor(Bs, N, k0), idesc, k0 > 0);
     umma::commit(&bar);
   }
-  const bool ok = umma::mbar_wait(&bar, 0);
+  const bool ok = umma::mbar_wait_timed(&bar, 0, nullptr);
   umma::fence_after_sync();
   for (int c0 = 0; c0 < N; c0 += 32) {
     float v[32];
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(128) umma_f16_test_kernel(const __half* A, con
     }
     umma::commit(&bar);
   }
-  const bool ok = umma::mbar_wait(&bar, 0);
+  const bool ok = umma::mbar_wait_timed(&bar, 0, nullptr);
   umma::fence_after_sync();
   for (int c0 = 0; c0 < N; c0 += 32) {
     float v[32];
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(128) umma_kv_step_test_kernel(const __grid_con
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
-  bool ok = umma::mbar_wait(&bars[0], 0);
+  bool ok = umma::mbar_wait_timed(&bars[0], 0, nullptr);
   if (t == 0 && ok) {
     constexpr uint32_t idS = umma::idesc_f16(128, 64, false, false), idO = umma::idesc_f16(128, 256, false, true);
     for (int ks = 0; ks < 16; ++ks)
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(128) umma_kv_step_test_kernel(const __grid_con
       umma::mma_f16_ss(tmem, umma::smem_desc(Ps + (size_t)kk * 2 * 128 * 16, 128 * 16, 128), tma::desc_sw128(Vt + kk * 2048, tma::kGroupBytes, 1024), idO, kk > 0);
     umma::commit(&bars[1]);
   }
-  ok = ok && umma::mbar_wait(&bars[1], 0);
+  ok = ok && umma::mbar_wait_timed(&bars[1], 0, nullptr);
   umma::fence_after_sync();
   for (int c0 = 0; c0 < 320; c0 += 32) {
     float v[32];
