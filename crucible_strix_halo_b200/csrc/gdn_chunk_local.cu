@@ -487,13 +487,14 @@ cr_status gdn_chunk_local_launch(const cr_geometry* g, const GdnPrefillParams& P
     const int split = nch * Hv <= 2 * room ? nch : std::min(nch, room / Hv), units = split * Hv + (nch - split) * g->gdn_kheads;
     CR_CUDA(launch_pdl(bf16_in ? gdn_chunk_local_kernel<true, 2> : gdn_chunk_local_kernel<false, 2>, dim3(std::min(units, room)), dim3(2 * kLocalThreads),
                        2 * kLocalSmem, stream, P, ws, split));
+    CR_LAUNCH_CHECK("gdn_chunk_local_kernel<2>");        // under a name of its own in stage timing
   } else {
     // A CTA per unit, to run wherever there is room.
     const int split = nch * Hv <= 2 * sm_count() ? nch : 0;
     CR_CUDA(launch_chained(P.chained, bf16_in ? gdn_chunk_local_kernel<true, 1> : gdn_chunk_local_kernel<false, 1>, dim3(split * Hv + (nch - split) * g->gdn_kheads),
                            dim3(kLocalThreads), kLocalSmem, stream, P, ws, split));
+    CR_LAUNCH_CHECK("gdn_chunk_local_kernel");
   }
-  CR_LAUNCH_CHECK("gdn_chunk_local_kernel");
   return CR_OK;
 }
 

@@ -371,7 +371,7 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
   const size_t in_elt = bf ? 2 : 4, out_elt = fmt == CR_OUT_RAW_F32 ? 4 : 2;
   const size_t Cw = 2 * (size_t)g->gdn_kheads * 128 + (size_t)g->gdn_vheads * 128, VWs = (size_t)g->gdn_vheads * 128;
   GdnPrefillParams P;
-  const bool pipelined = algo == CR_GDN_CHUNK_TC && a.R > gdn_part_rows() && !profiling();
+  const bool in_parts = algo == CR_GDN_CHUNK_TC && a.R > gdn_part_rows(), pipelined = in_parts && !profiling();
   // The call runs in parts of gdn_part_rows() rows; the state carries from part to part.
   auto part_params = [&](int p0, int buf, int rows = 0) {
     P.a = a;
@@ -383,7 +383,7 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
     P.a.commit = P.a.R;
     P.ab_logits = (const char*)args->ab_logits + (size_t)p0 * 2 * g->gdn_vheads * in_elt;
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.fmt = (int)fmt;
-    P.chained = pdl_enabled() && !pipelined;
+    P.chained = pdl_enabled() && !in_parts;              // with stage timing too: it times the kernels that a live call runs
     P.halo_in = p0 > 0;
     P.gate_blocks = (unsigned)(((long long)P.a.R * g->gdn_vheads + 8 * kGateUnits - 1) / (8 * kGateUnits));
     P.ring_rows = p0 + P.a.R == a.R ? std::min(a.R, 16) : 0;

@@ -169,3 +169,27 @@ def test_gdn_step_clusters(heads, R, replay, commit, fmt):
     for n in (2, 3, 4, 6):
         spans = [span(i) for i in range(n)]
         assert all(torch.equal(a, b) for a, b in zip(want, results(spans, layers.gdn_step(w, spans, fmt)))), n
+
+
+# Stage timing keeps a call on one stream but times the form of the chunk-local kernel that the call runs without it: units on CTAs
+# of their own in a call of several parts, two units to a CTA in a call of one.
+@pytest.mark.parametrize("R,form", [(2500, "gdn_chunk_local_kernel"), (1500, "gdn_chunk_local_kernel<2>")])
+def test_gdn_stage_timing_times_the_live_form(R, form):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, 32, 16)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    w = layers.GdnWeights(g, rn(g.gdn_channels, 4, std=0.5), rn(32) - 1, rn(32, std=0.5), 1 + rn(128, std=0.1))
+    inputs = rn(R, g.gdn_channels), rn(R, 4096), rn(R, 64)
+    old = capi.set_options(gdn_part_chunks=32)
+    try:
+        outs = []
+        for timing in (0, 1):
+            capi.check(capi.lib.cr_profile_enable(timing))
+            plan = layers.GdnPrefillPlan(w, R)
+            outs.append(plan.run(layers.GdnSession(g), *inputs, 0, capi.GDN_CHUNK_TC))
+        names = capi.profile_collect()
+    finally:
+        capi.check(capi.lib.cr_profile_enable(0))
+        capi.set_options(gdn_part_chunks=old.gdn_part_chunks)
+    assert [n for n in names if "local" in n] == [form] and torch.equal(*outs)
