@@ -375,23 +375,39 @@ constexpr size_t kAloneSmem = 116 * 1024;
 static_assert(step_smem_floats(kStepRows, kReplayChunk) * sizeof(float) <= kAloneSmem, "the longest pass fits");
 
 template <int CL>
-static cr_status step_launch(const GdnStepParams& P, int n, cudaStream_t stream) {
-  static PerDeviceOnce configured;
-  if (cr_status st = once_per_device(configured, [] {
+static cudaLaunchConfig_t step_config(dim3 grid, size_t smem, cudaStream_t stream, cudaLaunchAttribute (&attr)[2]) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(kStepThreads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = attr;
+  if (CL > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = CL; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  return cfg;
+}
+// Heads whose clusters of CL CTAs, an SM to each, the device holds at once (looked up once per device).
+template <int CL>
+static cr_status step_heads(int& heads) {
+  static PerDeviceOnce looked_up;
+  static int table[64];
+  int dev = 0;
+  CR_CUDA(cudaGetDevice(&dev));
+  if (cr_status st = once_per_device(looked_up, [dev] {
         CR_CUDA(cudaFuncSetAttribute(gdn_step_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAloneSmem));
+        cudaLaunchAttribute attr[2];
+        cudaLaunchConfig_t cfg = step_config<CL>(dim3(CL), kAloneSmem, nullptr, attr);
+        if (CL > 1) CR_CUDA(cudaOccupancyMaxActiveClusters(&table[dev & 63], gdn_step_kernel<CL>, &cfg));
+        else table[dev & 63] = sm_count();
         return CR_OK;
       })) return st;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(P.Hv * CL, n); cfg.blockDim = dim3(kStepThreads); cfg.stream = stream;
-  cfg.dynamicSmemBytes = P.Hv * CL * n <= sm_count() ? kAloneSmem : step_smem_floats(P.rows, P.replay) * sizeof(float);
+  heads = table[dev & 63];
+  return CR_OK;
+}
+template <int CL>
+static cr_status step_launch(const GdnStepParams& P, int n, bool alone, cudaStream_t stream) {
   cudaLaunchAttribute attr[2];
-  int na = 0;
-  if (pdl_enabled()) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na++].val.programmaticStreamSerializationAllowed = 1; }
-  if (CL > 1) {
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = CL; attr[na].val.clusterDim.y = 1; attr[na++].val.clusterDim.z = 1;
-  }
-  cfg.attrs = attr; cfg.numAttrs = na;
+  cudaLaunchConfig_t cfg = step_config<CL>(dim3(P.Hv * CL, n), alone ? kAloneSmem : step_smem_floats(P.rows, P.replay) * sizeof(float), stream, attr);
+  if (pdl_enabled()) { attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1; }
   CR_CUDA(cudaLaunchKernelEx(&cfg, gdn_step_kernel<CL>, P));
   CR_LAUNCH_CHECK("gdn_step_kernel");
   return CR_OK;
@@ -430,12 +446,16 @@ extern "C" cr_status cr_gdn_step(const cr_geometry* g, const cr_gdn_args* spans,
       P.rows = P.rows > P.span[s].R ? P.rows : P.span[s].R;
       P.replay = P.replay > P.span[s].replay ? P.replay : P.span[s].replay;
     }
-    // Few heads leave SMs idle: a head is spread over as many CTAs as there are SMs for.  States in HBM, 1 / 9 rows: 32 heads
-    // 9.1 / 21.2 us on one CTA each, 8.0 / 18.3 on two, 7.1 / 17.3 on four; 64 heads 9.3 / 21.7, 8.4 / 18.9, 8.6 / 19.8; 96 heads
-    // 9.7 / 22.1, 10.8 / 22.5: once two CTAs share an SM the work that a head's CTAs repeat (rows, dot products) costs more.
-    const int heads = n * P.Hv, cl = 4 * heads <= sm_count() ? 4 : (2 * heads <= sm_count() ? 2 : 1);
-    const auto launch = cl == 4 ? step_launch<4> : cl == 2 ? step_launch<2> : step_launch<1>;
-    if (cr_status st = launch(P, n, (cudaStream_t)stream)) return st;
+    // Few heads leave SMs idle: a head is spread over as many CTAs as there are SMs for, all clusters at once.  States in HBM, 1 / 9
+    // rows: 32 heads 9.1 / 21.2 us on one CTA each, 8.0 / 18.3 on two, 7.1 / 17.3 on four; 64 heads 9.3 / 21.7, 8.4 / 18.9, 8.6 / 19.8;
+    // 96 heads 9.7 / 22.1, 10.8 / 22.5: once two CTAs share an SM the work that a head's CTAs repeat (rows, dot products) costs more.
+    int fit4, fit2, fit1;
+    if (cr_status st = step_heads<4>(fit4)) return st;
+    if (cr_status st = step_heads<2>(fit2)) return st;
+    if (cr_status st = step_heads<1>(fit1)) return st;
+    const int heads = n * P.Hv;
+    const auto launch = heads <= fit4 ? step_launch<4> : (heads <= fit2 ? step_launch<2> : step_launch<1>);
+    if (cr_status st = launch(P, n, heads <= fit1, (cudaStream_t)stream)) return st;
   }
   return CR_OK;
 }
