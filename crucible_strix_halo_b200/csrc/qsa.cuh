@@ -11,19 +11,27 @@ struct QsaParams {
   int base[kMaxSpans];
   int Hq, Hkv, n;
   int b_lo, b_hi;          // scoring only: the blocks [b_lo, b_hi) are scored (a rank's own blocks; 0, INT_MAX = all)
-  // Prefill parts that mix the tiled and the row-wise attention: tile_count[r / tile_rows] is the size of the union
-  // list of row r's tile; the row-wise kernel serves the rows whose tile has more than tile_max entries for each of its
-  // rows (null: all).
-  const int* tile_count;
-  int tile_rows, tile_max;
+  // Prefill parts whose rows go to the tiled or to the row-wise attention by their union lists (null: all row-wise).
+  const int* tile_count;   // entries of every tile's list
+  int tile_rows, tile_max; // rows of a tile; entries per row up to which the tiled kernel is the quicker one
+  bool tile_whole;         // one decision for the whole part
 };
-// rows: rows of the part, of which the last tile may hold fewer than tile_rows
-__host__ __device__ __forceinline__ bool qsa_tile_shares(int entries, int tile, int tile_rows, int rows, int per_row) {
-  const int in_tile = rows - tile * tile_rows;
-  return entries <= per_row * (in_tile < tile_rows ? in_tile : tile_rows);
+// Which kernel serves the rows of `tile`: true, the tiled one.  Called by whole warps.  rows: rows of the part, of which the last tile
+// may hold fewer than tile_rows; it follows the tile before it, because a launch for those rows alone takes longer than they
+// save: a tile of 4 rows has few entries and many per row.
+__device__ __forceinline__ bool qsa_tile_shares(const int* count, int tile, int tile_rows, int rows, int per_row, bool whole) {
+  if (per_row >= CR_SEL_BLOCKS + 1) return true;         // no list is longer
+  if (whole) {
+    int sum = 0;
+    for (int i = threadIdx.x & 31; i * tile_rows < rows; i += 32) sum += count[i];
+    return __reduce_add_sync(0xffffffffu, sum) <= per_row * rows;
+  }
+  const int most = per_row * tile_rows;
+  if ((tile + 1) * tile_rows > rows && tile > 0) return count[tile] <= most && count[tile - 1] <= most;
+  return count[tile] <= most;
 }
 __device__ __forceinline__ bool qsa_row_is_tiled(const QsaParams& P, int r) {
-  return P.tile_count && qsa_tile_shares(P.tile_count[r / P.tile_rows], r / P.tile_rows, P.tile_rows, P.span[0].R, P.tile_max);
+  return P.tile_count && qsa_tile_shares(P.tile_count, r / P.tile_rows, P.tile_rows, P.span[0].R, P.tile_max, P.tile_whole);
 }
 
 // score_blocks >= 0: the score stride must cover that many blocks (a rank's own range, or 0 for entries that never touch
@@ -40,7 +48,7 @@ cr_status qsa_score_tc_launch(const QsaParams& P, int n, cudaStream_t stream);
 cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream);
 cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
 cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
-struct QsaTileSplit { const int* count; int rows, max; };   // see QsaParams::tile_count
+struct QsaTileSplit { const int* count; int rows, max; bool whole; };   // see QsaParams::tile_count
 // Attention of the spans' rows over the attended positions inside [p0, p1): outputs, or with `partials` one (m, l, acc[256])
 // record per (row, head).
 cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int p0, int p1, cr_out_format fmt,

@@ -13,7 +13,7 @@ int qsa_union_rows(const cr_geometry* g);
 int qsa_union_cap(int RT);
 cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int2* list, int* count, cudaStream_t stream);
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* partials, int splits, cr_out_format fmt, int flash_max, cudaStream_t stream);
+                           float* partials, int splits, cr_out_format fmt, int flash_max, bool flash_whole, cudaStream_t stream);
 
 // Scratch of a part: [partial records of split tiles][union lists, 2 ints per entry][union counts].  The list area is sized for tiles of 8 rows, the smallest tile.
 //
@@ -32,16 +32,31 @@ static size_t partial_bytes(const cr_geometry* g, int rows) {
   return (size_t)(all < kPartialRows ? all : kPartialRows) * g->q_heads * CR_QSA_PART * sizeof(float);
 }
 static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_cap(8) * 2; }
-// A tile goes to the tiled tensor-core kernel when its rows share enough blocks: at most this many union entries per row
-// of the tile (of 513 possible).  Both kernels' times are linear in their work: 2,048 rows cost the tiled one 2.5 us per
-// entry and row (1,250 us at 502 unrelated entries), the row-wise one 744 us with 16 heads and 1,500 us with 24, where its
-// streams take two warps; the lines cross at 298 entries and above 513.
-constexpr int kFlashEntriesPerRow = 298;
+// Which of the two kernels serves a part, or a tile of it.  Measured on parts of 2 to 2,048 rows at 8 K to 262 K positions, where the
+// position hardly matters (sparse rows, us of the attention stage):
+//   row-wise, up to 8 heads per KV head   5 + 24 for each wave of one (row, KV head) per SM: 29 to 74 rows, 50 to 148, 190 at 512,
+//                                         664 at 2,048;
+//   row-wise, 9 to 12 heads (two warps)   23 to 16 rows, 34 to 37, then 4 + 52.5 per wave: 57 to 74 rows, 110 to 148, 1,470 at 2,048;
+//   tiled                                 24 + 1.3 to 1.5 for each entry of a row and wave of CTAs, divided by the splits of a list: 128
+//                                         rows of 16 heads 33 at 42 entries and 70 at 264, 1,024 rows 78 and 340, 2,048 rows 150 and 700.
+// Two warps: the tiled kernel from 17 rows on, whatever the rows share (at 513 entries, the most there are, the lines cross between
+// 80 and 512 rows).
+// One warp: a part of one wave row-wise (64 rows at 42 entries, nearly the fewest: 27 to 29 tiled).  Above that the lists decide.
+// While every tile has an SM of its own, a tile left out makes the tiled kernel no quicker and the row-wise launch beside it costs
+// its whole waves (192 rows about the line, tile by tile: 108 us, either kernel alone 81 to 86), so the part goes one way; lists
+// built in vain cost 12 us.  The lines cross at 241 entries per row for 128 rows, 250 for 512, 206 for 768 (one CTA per tile).
+// Longer parts decide tile by tile: 165 entries for 1,204 rows, 243 for 2,048, two waves of CTAs either way.
 static bool one_warp_streams(const cr_geometry* g) { return g->q_heads / g->kv_heads <= 8; }
-static int entries_per_row(const cr_geometry* g) { return one_warp_streams(g) ? kFlashEntriesPerRow : 513; }
-// A part of so few rows is quicker row-wise whatever its rows share: 40 rows of 16 heads at 20,000 positions take 29 us
-// against 32 us of lists, split tiles and merge, 20 rows of 24 heads 34 us against 30 us.
-static int row_wise_rows(const cr_geometry* g) { return one_warp_streams(g) ? 40 : 16; }
+static bool rows_go_row_wise(const cr_geometry* g, int rows) { return one_warp_streams(g) ? rows * g->kv_heads <= sm_count() : rows <= 16; }
+static QsaTileSplit tile_rule(const cr_geometry* g, int rows, const int* count, int RT) {
+  if (!one_warp_streams(g)) return {count, RT, CR_SEL_BLOCKS + 1, false};
+  auto waves = [](int n) { return (n + sm_count() - 1) / sm_count(); };
+  const int ctas = (rows + RT - 1) / RT * g->kv_heads;
+  const bool whole = ctas <= sm_count();
+  const double per_entry = 1.4 * RT / 16 * waves(ctas) / tile_splits(g, rows);
+  const double line = (5 + 24.0 * waves(rows * g->kv_heads) - (whole ? 12 : 26)) / per_entry;
+  return {count, RT, line < CR_SEL_BLOCKS + 1 ? (int)line : CR_SEL_BLOCKS + 1, whole};
+}
 
 static cr_status check_part(const cr_geometry* g, const cr_qsa_prefill_args* args, int skip, cr_out_format fmt, const char* who) {
   CR_REQUIRE(args, "%s: null args", who);
@@ -72,18 +87,19 @@ static cr_qsa_args output_rows(const cr_geometry* g, cr_qsa_args q, int skip, cr
 static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, const cr_qsa_args& q, int skip, cr_out_format fmt,
                         cudaStream_t stream) {
   char* scratch = (char*)args->scratch;
-  if (args->q_hi && (options().qsa_union_rows > 0 || (options().qsa_union_rows == 0 && q.R > row_wise_rows(g)))) {
+  if (args->q_hi && (options().qsa_union_rows > 0 || (options().qsa_union_rows == 0 && !rows_go_row_wise(g, q.R)))) {
     int2* list = reinterpret_cast<int2*>(scratch + partial_bytes(g, q.R));
     int* count = reinterpret_cast<int*>(list + list_ints(q.R) / 2);
     const int RT = qsa_union_rows(g);
     const int splits = tile_splits(g, q.R);
-    const QsaTileSplit tiles = {count, RT, options().qsa_union_rows > 0 ? 513 : entries_per_row(g)};   // an explicit tile size forces the tiled kernel
+    QsaTileSplit tiles = tile_rule(g, q.R, count, RT);
+    if (options().qsa_union_rows > 0) tiles.max = CR_SEL_BLOCKS + 1;   // an explicit tile size forces the tiled kernel
     if (cr_status s = qsa_union_build_launch(g, q, list, count, stream)) return s;
     if (cr_status s = qsa_flash_launch(g, q, reinterpret_cast<const __half*>(args->q_hi) + (size_t)skip * g->q_heads * 256, list, count,
-                                       reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, stream)) return s;
+                                       reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, tiles.whole, stream)) return s;
     if (splits > 1)
       if (cr_status s = qsa_merge_launch(g, q, splits, reinterpret_cast<const float*>(scratch), fmt, stream, &tiles)) return s;
-    if (tiles.max >= 513) return CR_OK;                // no list is longer
+    if (tiles.max > CR_SEL_BLOCKS) return CR_OK;       // no list is longer
     // the tiles with little sharing: row-wise split-KV attention (its CTAs of tiled rows exit at once)
     return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream, &tiles);
   }

@@ -168,3 +168,42 @@ def test_step_marks_dense_rows(starts, R):
     for x in spans:
         want = [-1 if (x["pos0"] + r + 1) // 4 <= capi.SEL_BLOCKS else capi.SEL_BLOCKS for r in range(R)]
         assert x["session"].nsel.tolist() == want
+
+
+# Which kernel serves a part: one wave row-wise; then all tiles one way by their lists together (75 rows, a ragged part, as many tiles as
+# have an SM each); then tile by tile, a ragged last tile with the one before it.  Tiles that share their blocks, tiles that do not, and
+# both in turn, against the row-wise kernel (tolerance of the fp16 queries and probabilities of the tiled one).
+@pytest.mark.parametrize("Hq", [16, 24])
+@pytest.mark.parametrize("R", [16, 17, 74, 75, 148, 1184, 1185, 1204])
+@pytest.mark.parametrize("pattern", ["shared", "scattered", "mixed", "mixed last shared"])
+def test_prefill_kernel_choice(Hq, R, pattern):
+    capi, layers, g, w = _weights(Hq)
+    start = 20480
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    s = layers.QsaSession(g, start + R, max_rows=R)
+    s.k.copy_(rn(start + R, 2, 256)); s.v.copy_(rn(start + R, 2, 256))
+    RT = 128 // (Hq // 2)
+    tile = torch.arange(R, device="cuda") // RT
+    last = int(tile[-1])
+    share = {"shared": tile >= 0, "scattered": tile < 0, "mixed": (tile - last) % 2 == 1, "mixed last shared": (tile - last) % 2 == 0}[pattern]
+    score = rn(R, start // 4) * torch.where(share, 0.05, 1.0)[:, None] + rn(last + 1, start // 4)[tile] * share[:, None]
+    s.sel.copy_(score.topk(512, dim=1).indices.sort(dim=1).values.int())
+    s.nsel.fill_(512)
+    q = rn(R, Hq, 512)
+    zero = torch.zeros(R, 640, device="cuda")
+    got = {}
+    for mode in (0, -1):
+        old = capi.set_options(qsa_union_rows=mode)
+        try:
+            plan = layers.QsaPrefillPlan(w, R)
+            plan.q_hi.copy_(q[:, :, :256])
+            plan.out.fill_(float("nan"))
+            a = capi.QsaPrefillArgs(layers.qsa_args(w, s, q, zero, zero, zero, plan.out, start), capi.dptr(plan.q_hi), capi.dptr(plan.scratch), plan.scratch.numel())
+            capi.check(capi.lib.cr_qsa_prefill_attend(C.byref(g), C.byref(a), 0, capi.OUT_RAW_F32, None))
+            torch.cuda.synchronize()
+            got[mode] = plan.out
+        finally:
+            capi.check(capi.lib.cr_set_options(C.byref(old)))
+    assert capi.lib.cr_device_check() == 0
+    assert (got[0] - got[-1]).abs().max().item() < 4e-3
