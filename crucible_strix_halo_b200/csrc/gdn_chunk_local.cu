@@ -18,7 +18,7 @@
 //
 // The scan reads a chunk as soon as it is written: units are walked in chunk order and mark what they finish, and in a call of one
 // part the scan's CTAs run beside this kernel, on SMs that it leaves to them.  The call then takes what the longer of the two
-// takes, not their sum: 1,999 rows, 16 / 32 heads, 193 -> 156 us, 16 / 48 heads from fp32 rows 247 -> 217 us, 7,104 rows 570 ->
+// takes, not their sum: 1,999 rows, 16 / 32 heads, 193 -> 156 us, 16 / 48 heads from fp32 rows 247 -> 225 us, 7,104 rows 570 ->
 // 410 us.  The scan waits for this kernel and never the other way, and is let in when every CTA here is resident.
 #include <algorithm>
 #include "gdn_chunk.cuh"

@@ -18,7 +18,7 @@
 // Bound: the gather.  Random 512-byte rows of a 512 MB cache arrive at 8.5 TB/s (16 MB: 20 TB/s).  The form before this
 // one (a CTA per (row, KV head, split), heads as M rows, Q re-read from shared memory for every tile, partials merged by
 // a second kernel) was held by shared-memory reads and barriers: 2,048 rows at 262,144 positions took 1,875 us plus
-// 180 us of merge, 744 us now (11.6 TB/s of gathers: the rows walk their ascending positions side by side, so the rows in
+// 180 us of merge, 700 us now (12 TB/s of gathers: the rows walk their ascending positions side by side, so the rows in
 // flight share a region of the cache that L2 holds; from L2 alone 666 us, where every byte's way into and out of shared
 // memory takes three quarters of its bandwidth); 72 verify rows at 131,072 105 + 12 us, 53 us now; four decode rows at
 // 262,144 17 + 9 us, 13 us now.

@@ -37,7 +37,7 @@ static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_
 //   row-wise, up to 8 heads per KV head   5 + 24 for each wave of one (row, KV head) per SM: 29 to 74 rows, 50 to 148, 190 at 512,
 //                                         664 at 2,048;
 //   row-wise, 9 to 12 heads (two warps)   23 to 16 rows, 34 to 37, then 4 + 52.5 per wave: 57 to 74 rows, 110 to 148, 1,470 at 2,048;
-//   tiled                                 24 + 1.3 to 1.5 for each entry of a row and wave of CTAs, divided by the splits of a list: 128
+//   tiled                                 24 + 1.3 for each entry of a row and wave of CTAs, divided by the splits of a list: 128
 //                                         rows of 16 heads 33 at 42 entries and 70 at 264, 1,024 rows 78 and 340, 2,048 rows 150 and 700.
 // Two warps: the tiled kernel from 17 rows on, whatever the rows share (at 513 entries, the most there are, the lines cross between
 // 80 and 512 rows).
@@ -53,7 +53,7 @@ static QsaTileSplit tile_rule(const cr_geometry* g, int rows, const int* count, 
   auto waves = [](int n) { return (n + sm_count() - 1) / sm_count(); };
   const int ctas = (rows + RT - 1) / RT * g->kv_heads;
   const bool whole = ctas <= sm_count();
-  const double per_entry = 1.4 * RT / 16 * waves(ctas) / tile_splits(g, rows);
+  const double per_entry = 1.3 * RT / 16 * waves(ctas) / tile_splits(g, rows);
   const double line = (5 + 24.0 * waves(rows * g->kv_heads) - (whole ? 12 : 26)) / per_entry;
   return {count, RT, line < CR_SEL_BLOCKS + 1 ? (int)line : CR_SEL_BLOCKS + 1, whole};
 }
@@ -100,7 +100,7 @@ static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, c
     if (splits > 1)
       if (cr_status s = qsa_merge_launch(g, q, splits, reinterpret_cast<const float*>(scratch), fmt, stream, &tiles)) return s;
     if (tiles.max > CR_SEL_BLOCKS) return CR_OK;       // no list is longer
-    // the tiles with little sharing: row-wise split-KV attention (its CTAs of tiled rows exit at once)
+    // the tiles with little sharing: row-wise attention (its CTAs of tiled rows exit at once)
     return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream, &tiles);
   }
   return qsa_attn_launch(g, &q, 1, nullptr, 0, INT_MAX, fmt, stream);

@@ -5,7 +5,7 @@
 // engine/runtime/snapshot_bytes.h:692-704).  The copy is a grid-stride walk over 16 KB pieces of all spans together, so
 // 133 spans of a 48-layer model between 2 KB and 2 MiB fill every SM evenly; each thread issues its four 128-bit
 // loads before the first store.  HBM-bound: bytes read + bytes written = 2 x the spans' bytes.  The 132 spans (104 MB) of a
-// 48-layer stream out and back: 86 us as two launches of at most 96 spans each way, 75 us as one (0.85 of the copy bandwidth).
+// 48-layer stream out and back: 86 us as two launches of at most 96 spans each way, 72 us as one (0.88 of the copy bandwidth).
 #include "common.cuh"
 
 namespace cr {
