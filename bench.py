@@ -40,18 +40,19 @@ sys.path.insert(0, ROOT)
 
 GDN_BYTES_PER_TOKEN = (8192 + 4096) * 2 + 4096 * 2 + 2 * 32 * 4      # bf16 qkv + z in, bf16 out, fp32 a/b logits
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one launch from the ncu captures summarised under
-# profiles/, per unit of work (GDN: per token of a 7,104-token part; decode: per step of 4 sessions), scaled to
+# profiles/, per unit of work (GDN: per token of a 7,104-token part, the chunk-local kernel of a 4,544-token one; decode: per step of 4
+# sessions), scaled to
 # the launch by the units it processes (traffic grows in proportion to them).
 NCU_TRAFFIC = {
     "gdn_prefill_32k": {"gdn_chunk_scan_tc_kernel": ("token", (526.38e6 + 99.4e6) / 7104),
-                        "gdn_chunk_local_kernel": ("token", (120.62e6 + 476.6e6) / 7104),
+                        "gdn_chunk_local_kernel": ("token", (75.55e6 + 282.96e6) / 4544),
                         "gdn_gate_kernel": ("token", (174.89e6 + 34.3e6) / 7104)},
     "decode_262k": {"qsa_score_kernel": ("step", 134.24e6 + 0.13e6), "qsa_attn_kernel": ("step", 16.98e6),
                     "qsa_topk_cluster_kernel": ("step", 1.11e6), "qsa_prep_kernel": ("step", 0.13e6),
                     "gdn_step_kernel": ("step", 9.47e6)},
     "qsa_prefill_262k": {"qsa_attn_kernel": ("step", 3500e6 + 14.7e6), "qsa_score_tc_kernel": ("step", 141.3e6 + 483.3e6),
                          "qsa_topk_kernel": ("step", 537.0e6 + 3.7e6)},
-    "qsa_attend_262k_drift": {"qsa_flash_tc_kernel": ("step", 704.4e6 + 13.6e6)},
+    "qsa_attend_262k_drift": {"qsa_flash_tc_kernel": ("step", 1005.3e6 + 11.4e6)},
     "verify_131k": {"qsa_attn_kernel": ("step", 288.1e6 + 0.1e6), "gdn_step_kernel": ("step", 23.3e6)},
 }
 DECODE_BYTES_PER_SESSION = 65536 * 512 + 2051 * 2048 + 2 * 2097152   # pool scan + K/V gather + GDN state in/out
