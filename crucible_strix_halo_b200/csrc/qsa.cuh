@@ -14,24 +14,33 @@ struct QsaParams {
   // Prefill parts whose rows go to the tiled or to the row-wise attention by their union lists (null: all row-wise).
   const int* tile_count;   // entries of every tile's list
   int tile_rows, tile_max; // rows of a tile; entries per row up to which the tiled kernel is the quicker one
-  bool tile_whole;         // one decision for the whole part
+  int tile_mixed;          // >= 0: one decision for the whole part, with this line where some tile has to go row-wise all the same
 };
+// Tiles of more entries per row than this go row-wise whatever their part does: they would gain little, and the row-wise kernel
+// splits queries and probabilities into two fp16 numbers where the tiled one rounds them to one.
+constexpr int kTileMost = 298;
 // Which kernel serves the rows of `tile`: true, the tiled one.  Called by whole warps.  rows: rows of the part, of which the last tile
-// may hold fewer than tile_rows; it follows the tile before it, because a launch for those rows alone takes longer than they
-// save: a tile of 4 rows has few entries and many per row.
-__device__ __forceinline__ bool qsa_tile_shares(const int* count, int tile, int tile_rows, int rows, int per_row, bool whole) {
+// may hold fewer than tile_rows.
+__device__ __forceinline__ bool qsa_tile_shares(const int* count, int tile, int tile_rows, int rows, int per_row, int mixed) {
   if (per_row >= CR_SEL_BLOCKS + 1) return true;         // no list is longer
-  if (whole) {
+  const int here = min(tile_rows, rows - tile * tile_rows);
+  if (count[tile] > kTileMost * here) return false;
+  if (mixed >= 0) {
     int sum = 0;
-    for (int i = threadIdx.x & 31; i * tile_rows < rows; i += 32) sum += count[i];
-    return __reduce_add_sync(0xffffffffu, sum) <= per_row * rows;
+    bool over = false;
+    for (int i = threadIdx.x & 31; i * tile_rows < rows; i += 32) {
+      const int n = count[i];
+      sum += n;
+      over |= n > kTileMost * min(tile_rows, rows - i * tile_rows);
+    }
+    const int line = __any_sync(0xffffffffu, over) ? mixed : per_row;
+    return (int)__reduce_add_sync(0xffffffffu, sum) <= line * rows;
   }
-  const int most = per_row * tile_rows;
-  if ((tile + 1) * tile_rows > rows && tile > 0) return count[tile] <= most && count[tile - 1] <= most;
-  return count[tile] <= most;
+  // A last tile of few rows has few entries and many per row: it follows the tile before it.
+  return count[here < tile_rows && tile > 0 ? tile - 1 : tile] <= per_row * (tile > 0 ? tile_rows : here);
 }
 __device__ __forceinline__ bool qsa_row_is_tiled(const QsaParams& P, int r) {
-  return P.tile_count && qsa_tile_shares(P.tile_count, r / P.tile_rows, P.tile_rows, P.span[0].R, P.tile_max, P.tile_whole);
+  return P.tile_count && qsa_tile_shares(P.tile_count, r / P.tile_rows, P.tile_rows, P.span[0].R, P.tile_max, P.tile_mixed);
 }
 
 // score_blocks >= 0: the score stride must cover that many blocks (a rank's own range, or 0 for entries that never touch
@@ -48,7 +57,7 @@ cr_status qsa_score_tc_launch(const QsaParams& P, int n, cudaStream_t stream);
 cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream);
 cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
 cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
-struct QsaTileSplit { const int* count; int rows, max; bool whole; };   // see QsaParams::tile_count
+struct QsaTileSplit { const int* count; int rows, max, mixed; };   // see QsaParams::tile_count
 // Attention of the spans' rows over the attended positions inside [p0, p1): outputs, or with `partials` one (m, l, acc[256])
 // record per (row, head).
 cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, float* partials, int p0, int p1, cr_out_format fmt,

@@ -462,7 +462,7 @@ cr_status qsa_attn_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     const int n = n_spans - s0 < kMaxSpans ? n_spans - s0 : kMaxSpans;
     QsaParams P;
     qsa_fill_params(P, g, spans + s0, n);
-    if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; P.tile_whole = tiles->whole; }
+    if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; P.tile_mixed = tiles->mixed; }
     long long units = 0;
     int last = 0;                                        // newest position of any row
     for (int s = 0; s < n; ++s) {
@@ -484,7 +484,7 @@ cr_status qsa_merge_launch(const cr_geometry* g, const cr_qsa_args& a, int npart
                            const QsaTileSplit* tiles) {
   QsaParams P;
   qsa_fill_params(P, g, &a, 1);
-  if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; P.tile_whole = tiles->whole; }
+  if (tiles) { P.tile_count = tiles->count; P.tile_rows = tiles->rows; P.tile_max = tiles->max; P.tile_mixed = tiles->mixed; }
   use_stream(stream);
   CR_CUDA(launch_pdl(qsa_merge_kernel, dim3(g->q_heads, a.R), dim3(64), 0, stream, P, partials, nparts, (int)fmt));
   CR_LAUNCH_CHECK("qsa_merge_kernel");

@@ -65,7 +65,7 @@ struct FlashParams {
   float* partials;        // splits > 1: records (m, l, acc[256]) [split][R][Hq][258] for the merge kernel, else null
   int cap, RT, Hq, Hkv, fmt;
   int flash_max;          // entries per row of a tile: longer lists are left to the row-wise kernel,
-  bool flash_whole;       // all lists of the part together
+  int flash_mixed;        // as QsaParams::tile_mixed
 };
 
 int qsa_union_rows(const cr_geometry* g) {
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
   const int gqa = P.Hq / P.Hkv;
   const int cnt = P.count[tile];
   const int n_all = (cnt + kFlBlocks - 1) / kFlBlocks;   // steps of the tile; this CTA's share is [step0, step0 + n)
-  if (n_all == 0 || !qsa_tile_shares(P.count, tile, P.RT, a.R, P.flash_max, P.flash_whole)) return;           // a tile without rows, or one the row-wise kernels serve
+  if (n_all == 0 || !qsa_tile_shares(P.count, tile, P.RT, a.R, P.flash_max, P.flash_mixed)) return;           // a tile without rows, or one the row-wise kernels serve
   const int step0 = (int)((long long)n_all * blockIdx.z / gridDim.z), n = (int)((long long)n_all * (blockIdx.z + 1) / gridDim.z) - step0;
   if ((umma::smem_u32(sm) & 1023u) != 0) {               // the swizzled tiles need their atoms on 1 KB boundaries
     if (t == 0) g_qsa_flash_status = 1;
@@ -545,7 +545,7 @@ cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int
 
 // Attention of the rows of `a` over the union lists; splits > 1 leaves records in `partials` for qsa_merge_launch.
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* partials, int splits, cr_out_format fmt, int flash_max, bool flash_whole, cudaStream_t stream) {
+                           float* partials, int splits, cr_out_format fmt, int flash_max, int flash_mixed, cudaStream_t stream) {
   static PerDeviceOnce configured;
   if (cr_status st = once_per_device(configured, [] {
         CR_CUDA(cudaFuncSetAttribute(qsa_flash_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlashSmem));
@@ -557,7 +557,7 @@ cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __h
   P.RT = qsa_union_rows(g); P.cap = qsa_union_cap(P.RT);
   P.Hq = g->q_heads; P.Hkv = g->kv_heads; P.fmt = (int)fmt;
   P.partials = splits > 1 ? partials : nullptr;
-  P.flash_max = flash_max; P.flash_whole = flash_whole;
+  P.flash_max = flash_max; P.flash_mixed = flash_mixed;
   const int tiles = (a.R + P.RT - 1) / P.RT;
   use_stream(stream);
   const dim3 grid(g->kv_heads, tiles, splits);

@@ -5,6 +5,7 @@
 // row-wise kernel of the decode path (qsa_attn.cu) serves the tiles whose rows share little, and every row with
 // cr_options.qsa_union_rows = -1.  Rows of a part are independent once the cache and the pool hold the
 // part, so causality inside the part falls out of pos0 + r.
+#include <algorithm>
 #include <climits>
 #include "qsa.cuh"
 
@@ -13,7 +14,7 @@ int qsa_union_rows(const cr_geometry* g);
 int qsa_union_cap(int RT);
 cr_status qsa_union_build_launch(const cr_geometry* g, const cr_qsa_args& a, int2* list, int* count, cudaStream_t stream);
 cr_status qsa_flash_launch(const cr_geometry* g, const cr_qsa_args& a, const __half* q_hi, const int2* list, const int* count,
-                           float* partials, int splits, cr_out_format fmt, int flash_max, bool flash_whole, cudaStream_t stream);
+                           float* partials, int splits, cr_out_format fmt, int flash_max, int flash_mixed, cudaStream_t stream);
 
 // Scratch of a part: [partial records of split tiles][union lists, 2 ints per entry][union counts].  The list area is sized for tiles of 8 rows, the smallest tile.
 //
@@ -44,18 +45,19 @@ static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_
 // One warp: a part of one wave row-wise (64 rows at 42 entries, nearly the fewest: 27 to 29 tiled).  Above that the lists decide.
 // While every tile has an SM of its own, a tile left out makes the tiled kernel no quicker and the row-wise launch beside it costs
 // its whole waves (192 rows about the line, tile by tile: 108 us, either kernel alone 81 to 86), so the part goes one way; lists
-// built in vain cost 12 us.  The lines cross at 241 entries per row for 128 rows, 250 for 512, 206 for 768 (one CTA per tile).
-// Longer parts decide tile by tile: 165 entries for 1,204 rows, 243 for 2,048, two waves of CTAs either way.
+// built in vain cost 15 us at 128 rows and 27 at 512, and a wave of row-wise CTAs for a tile past kTileMost 30.  With the lists paid for
+// the lines cross at 263 entries per row for 128 and 512 rows, 213 for 768 (one CTA per tile).  Longer parts decide tile by tile:
+// 165 entries for 1,204 rows, 243 for 2,048, two waves of CTAs either way.
 static bool one_warp_streams(const cr_geometry* g) { return g->q_heads / g->kv_heads <= 8; }
 static bool rows_go_row_wise(const cr_geometry* g, int rows) { return one_warp_streams(g) ? rows * g->kv_heads <= sm_count() : rows <= 16; }
 static QsaTileSplit tile_rule(const cr_geometry* g, int rows, const int* count, int RT) {
-  if (!one_warp_streams(g)) return {count, RT, CR_SEL_BLOCKS + 1, false};
+  if (!one_warp_streams(g)) return {count, RT, CR_SEL_BLOCKS + 1, -1};
   auto waves = [](int n) { return (n + sm_count() - 1) / sm_count(); };
-  const int ctas = (rows + RT - 1) / RT * g->kv_heads;
-  const bool whole = ctas <= sm_count();
-  const double per_entry = 1.3 * RT / 16 * waves(ctas) / tile_splits(g, rows);
-  const double line = (5 + 24.0 * waves(rows * g->kv_heads) - (whole ? 12 : 26)) / per_entry;
-  return {count, RT, line < CR_SEL_BLOCKS + 1 ? (int)line : CR_SEL_BLOCKS + 1, whole};
+  const bool whole = (rows + RT - 1) / RT * g->kv_heads <= sm_count();
+  const double per_entry = 1.3 * RT / 16 * waves(std::max(rows / RT, 1) * g->kv_heads) / tile_splits(g, rows);   // a ragged last tile is short
+  const double row_wise = 5 + 24.0 * waves(rows * g->kv_heads), vain = 12 + 0.03 * rows;
+  auto line = [&](double more) { return std::max(std::min((int)((row_wise - 24 + more) / per_entry), kTileMost), 0); };
+  return {count, RT, line(whole ? vain : -2), whole ? line(vain - 30) : -1};
 }
 
 static cr_status check_part(const cr_geometry* g, const cr_qsa_prefill_args* args, int skip, cr_out_format fmt, const char* who) {
@@ -96,7 +98,7 @@ static cr_status attend(const cr_geometry* g, const cr_qsa_prefill_args* args, c
     if (options().qsa_union_rows > 0) tiles.max = CR_SEL_BLOCKS + 1;   // an explicit tile size forces the tiled kernel
     if (cr_status s = qsa_union_build_launch(g, q, list, count, stream)) return s;
     if (cr_status s = qsa_flash_launch(g, q, reinterpret_cast<const __half*>(args->q_hi) + (size_t)skip * g->q_heads * 256, list, count,
-                                       reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, tiles.whole, stream)) return s;
+                                       reinterpret_cast<float*>(scratch), splits, fmt, tiles.max, tiles.mixed, stream)) return s;
     if (splits > 1)
       if (cr_status s = qsa_merge_launch(g, q, splits, reinterpret_cast<const float*>(scratch), fmt, stream, &tiles)) return s;
     if (tiles.max > CR_SEL_BLOCKS) return CR_OK;       // no list is longer

@@ -171,10 +171,11 @@ def test_step_marks_dense_rows(starts, R):
 
 
 # Which kernel serves a part: one wave row-wise; then all tiles one way by their lists together (75 rows, a ragged part, as many tiles as
-# have an SM each); then tile by tile, a ragged last tile with the one before it.  Tiles that share their blocks, tiles that do not, and
-# both in turn, against the row-wise kernel (tolerance of the fp16 queries and probabilities of the tiled one).
+# have an SM each); then tile by tile, a ragged last tile with the one before it, unless it has too many entries per row (129 and 1,185
+# rows: a tile of one).  Tiles that share their blocks, tiles that do not, and both in turn, against the row-wise kernel (tolerance of
+# the fp16 queries and probabilities of the tiled one).
 @pytest.mark.parametrize("Hq", [16, 24])
-@pytest.mark.parametrize("R", [16, 17, 74, 75, 148, 1184, 1185, 1204])
+@pytest.mark.parametrize("R", [16, 17, 74, 75, 129, 148, 1184, 1185, 1204])
 @pytest.mark.parametrize("pattern", ["shared", "scattered", "mixed", "mixed last shared"])
 def test_prefill_kernel_choice(Hq, R, pattern):
     capi, layers, g, w = _weights(Hq)
