@@ -23,8 +23,7 @@ constexpr int kTileMost = 298;
 // may hold fewer than tile_rows.
 __device__ __forceinline__ bool qsa_tile_shares(const int* count, int tile, int tile_rows, int rows, int per_row, int mixed) {
   if (per_row >= CR_SEL_BLOCKS + 1) return true;         // no list is longer
-  const int here = min(tile_rows, rows - tile * tile_rows);
-  if (count[tile] > kTileMost * here) return false;
+  const int here = min(tile_rows, rows - tile * tile_rows), entries = count[tile];
   if (mixed >= 0) {
     int sum = 0;
     bool over = false;
@@ -34,10 +33,12 @@ __device__ __forceinline__ bool qsa_tile_shares(const int* count, int tile, int 
       over |= n > kTileMost * min(tile_rows, rows - i * tile_rows);
     }
     const int line = __any_sync(0xffffffffu, over) ? mixed : per_row;
-    return (int)__reduce_add_sync(0xffffffffu, sum) <= line * rows;
+    return ((int)__reduce_add_sync(0xffffffffu, sum) <= line * rows) & (entries <= kTileMost * here);
   }
   // A last tile of few rows has few entries and many per row: it follows the tile before it.
-  return count[here < tile_rows && tile > 0 ? tile - 1 : tile] <= per_row * (tile > 0 ? tile_rows : here);
+  const bool ragged = here < tile_rows && tile > 0;
+  const int decides = ragged ? count[tile - 1] : entries;
+  return (entries <= kTileMost * here) & (decides <= per_row * (tile > 0 ? tile_rows : here));
 }
 __device__ __forceinline__ bool qsa_row_is_tiled(const QsaParams& P, int r) {
   return P.tile_count && qsa_tile_shares(P.tile_count, r / P.tile_rows, P.tile_rows, P.span[0].R, P.tile_max, P.tile_mixed);
