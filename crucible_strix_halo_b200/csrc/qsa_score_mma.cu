@@ -10,11 +10,11 @@
 // One warp owns whole tiles and walks them in steps of 16 dims x 16 blocks; the loads of three steps are in flight
 // ahead of the one that multiplies.
 #include "qsa.cuh"
+#include "umma.cuh"
 
 namespace cr {
 
 constexpr int kSmLd = 136;                   // halves per query row in shared memory (272 bytes: conflict-free ldmatrix)
-constexpr int kSmTilesPerWarp = 4;
 
 __device__ __forceinline__ void sm_ldsm_x4(unsigned (&r)[4], const void* p) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(p);
@@ -34,14 +34,21 @@ __device__ __forceinline__ void split_pair(float x, float y, unsigned& hi, unsig
   lo = *reinterpret_cast<const unsigned*>(&r);
 }
 
-// grid (tile groups, 1, spans), 128 threads; MT = ceil(rows / 4) m-tiles of 16 (row, head) pairs.
+// grid (tile groups, 1, spans), 128 threads; MT = ceil(rows / 4) m-tiles of 16 (row, head) pairs; a warp walks `per_warp` tiles.
 template <int MT>
-__global__ void __launch_bounds__(128, 4) qsa_score_mma_kernel(const __grid_constant__ QsaParams P) {
+__global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_constant__ QsaParams P, int per_warp) {
   const cr_qsa_args& a = P.span[blockIdx.z];
+  pdl_release();
   const int nb_all = (a.pos0 + a.R) / 4;              // blocks complete for the last row
-  if (nb_all <= CR_SEL_BLOCKS || a.R > 4 * MT) return;
   __shared__ __align__(16) __half qh[16 * MT][kSmLd], ql[16 * MT][kSmLd];
   const int t = threadIdx.x, w = t >> 5, l = t & 31, g = l >> 2, tq = l & 3;
+  const int tiles = (nb_all + 31) / 32;
+  const int first = (blockIdx.x * 4 + w) * per_warp, last = min(first + per_warp, tiles);
+  const bool scored = nb_all > CR_SEL_BLOCKS && a.R <= 4 * MT;
+  // The first tile is asked into L2 while the kernel ahead still runs: a prefetch reads nothing that could be stale later.
+  if (scored && l == 0 && first < last) umma::bulk_prefetch_l2(a.c.ik_pool + (size_t)first * 4096, 16384);
+  pdl_wait();
+  if (!scored) return;
   for (int i = t; i < 16 * MT * 64; i += 128) {        // pairs of dims: row m = 4 r + h of the span's normalised indexer queries
     const int m = i >> 6, d = (i & 63) * 2, r = m >> 2, h = m & 3;
     float2 v = make_float2(0.f, 0.f);
@@ -52,94 +59,86 @@ __global__ void __launch_bounds__(128, 4) qsa_score_mma_kernel(const __grid_cons
     *reinterpret_cast<unsigned*>(&ql[m][d]) = lo;
   }
   __syncthreads();
-  const int tiles = (nb_all + 31) / 32;
-  const int first = (blockIdx.x * 4 + w) * kSmTilesPerWarp;
-  if (first >= tiles) return;
-  const int last = min(first + kSmTilesPerWarp, tiles);
-  // A step is one k-step (16 dims) of one half tile (16 blocks): this thread's 8 values are the dims
-  // 16 ks + 2 tq + {0, 1, 8, 9} of the blocks 16 half + 8 nt + g.  Three steps are in flight ahead of the one in use.
-  const int total = (last - first) * 16;
-  auto fetch = [&](float (&v)[8], int step) {
-    const int tile = first + (step >> 4), half = (step >> 3) & 1, ks = step & 7;
-    const float* pt = a.c.ik_pool + (size_t)tile * 4096 + (16 * ks + 2 * tq) * 32 + 16 * half + g;
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      v[4 * nt] = __ldg(pt + 8 * nt); v[4 * nt + 1] = __ldg(pt + 32 + 8 * nt);
-      v[4 * nt + 2] = __ldg(pt + 256 + 8 * nt); v[4 * nt + 3] = __ldg(pt + 288 + 8 * nt);
-    }
+  if (first >= last) return;
+  // A step is 16 dims of a whole tile: this thread's four 16-byte loads are the dims 16 ks + 2 tq + {0, 1, 8, 9} of the blocks
+  // 4 g .. 4 g + 3, and block 4 g + nt is column g of product nt.  Three steps are in flight ahead of the one in use.
+  const int total = (last - first) * 8;
+  const float* pt = a.c.ik_pool + (size_t)first * 4096 + 2 * tq * 32 + 4 * g;
+  auto fetch = [&](float4 (&v)[4], int step) {
+    const float* p = pt + (size_t)step * 512;          // tiles lie back to back
+    v[0] = __ldcg(reinterpret_cast<const float4*>(p)); v[1] = __ldcg(reinterpret_cast<const float4*>(p + 32));
+    v[2] = __ldcg(reinterpret_cast<const float4*>(p + 256)); v[3] = __ldcg(reinterpret_cast<const float4*>(p + 288));
   };
-  float ring[4][8];
-  fetch(ring[0], 0); fetch(ring[1], 1); fetch(ring[2], 2);          // total >= 16
-  float acc[MT][2][4];
-  for (int s0 = 0; s0 < total; s0 += 4) {
+  float4 ring[4][4];
+  fetch(ring[0], 0); fetch(ring[1], 1); fetch(ring[2], 2);          // total >= 8
+  for (int s0 = 0; s0 < total; s0 += 8) {
+    float acc[MT][4][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int step = s0 + j, ks = step & 7;
-      if (step + 3 < total) fetch(ring[(j + 3) & 3], step + 3);
-      if (ks == 0) {
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
+      for (int nt = 0; nt < 4; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.f;
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.f;
-      }
-      unsigned bh[2][2], bl[2][2];
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        split_pair(ring[j][4 * nt], ring[j][4 * nt + 1], bh[nt][0], bl[nt][0]);
-        split_pair(ring[j][4 * nt + 2], ring[j][4 * nt + 3], bh[nt][1], bl[nt][1]);
-      }
+    for (int ks = 0; ks < 8; ++ks) {
+      if (s0 + ks + 3 < total) fetch(ring[(ks + 3) & 3], s0 + ks + 3);
+      const float4 (&v)[4] = ring[ks & 3];
+      unsigned bh[4][2], bl[4][2];
+      split_pair(v[0].x, v[1].x, bh[0][0], bl[0][0]); split_pair(v[2].x, v[3].x, bh[0][1], bl[0][1]);
+      split_pair(v[0].y, v[1].y, bh[1][0], bl[1][0]); split_pair(v[2].y, v[3].y, bh[1][1], bl[1][1]);
+      split_pair(v[0].z, v[1].z, bh[2][0], bl[2][0]); split_pair(v[2].z, v[3].z, bh[2][1], bl[2][1]);
+      split_pair(v[0].w, v[1].w, bh[3][0], bl[3][0]); split_pair(v[2].w, v[3].w, bh[3][1], bl[3][1]);
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         unsigned ah[4], al[4];
         sm_ldsm_x4(ah, &qh[16 * m + (l & 15)][16 * ks + (l >> 4) * 8]);
         sm_ldsm_x4(al, &ql[16 * m + (l & 15)][16 * ks + (l >> 4) * 8]);
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          sm_mma(acc[m][nt], ah, bh[nt][0], bh[nt][1]);
-          sm_mma(acc[m][nt], al, bh[nt][0], bh[nt][1]);
-          sm_mma(acc[m][nt], ah, bl[nt][0], bl[nt][1]);
-        }
+        for (int nt = 0; nt < 4; ++nt) sm_mma(acc[m][nt], ah, bh[nt][0], bh[nt][1]);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) sm_mma(acc[m][nt], al, bh[nt][0], bh[nt][1]);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) sm_mma(acc[m][nt], ah, bl[nt][0], bl[nt][1]);
       }
-      if (ks != 7) continue;
-      // relu per head, sum over the four heads of a row (lanes g, g ^ 1, g ^ 2, g ^ 3 of the same row quartet), scale, store
-      const int blk0 = (first + (step >> 4)) * 32 + 16 * ((step >> 3) & 1);
+    }
+    // relu per head and the sum over the four heads of a row: lanes g, g ^ 1, g ^ 2, g ^ 3 hold the heads of the span rows
+    // 4 m + g / 4 (accumulator row g) and + 2 (row g + 8), columns 2 tq and 2 tq + 1.  Every exchange gives away half of what a
+    // lane holds, so that in the end lane g has the four blocks of column 2 tq + (g & 1) of row 4 m + 2 (g >> 1 & 1) + g / 4.
+    const bool odd = g & 1, lower = g & 2;
+    const int blk = (first + (s0 >> 3)) * 32 + 8 * tq + (odd ? 4 : 0);
 #pragma unroll
-      for (int m = 0; m < MT; ++m)
+    for (int m = 0; m < MT; ++m) {
+      float sc[4];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          float sc[4];
+      for (int nt = 0; nt < 4; ++nt) {
+        float half[2];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            sc[i] = fmaxf(acc[m][nt][i], 0.f);
-            sc[i] += __shfl_xor_sync(0xffffffffu, sc[i], 4);
-            sc[i] += __shfl_xor_sync(0xffffffffu, sc[i], 8);
-          }
-          if ((g & 3) == 0) {
-            const int blk = blk0 + 8 * nt + 2 * tq;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {                   // accumulator rows g and g + 8: span rows 4 m + g / 4 and + 2
-              const int r = 4 * m + 2 * half + (g >> 2);
-              if (r >= a.R) continue;
-              const int nb = (a.pos0 + r + 1) / 4;
-              if (nb <= CR_SEL_BLOCKS) continue;
-              float* dst = a.scores + (size_t)r * a.sstride + blk;
-              if (blk < nb) dst[0] = sc[2 * half] * kInvSqrt128;
-              if (blk + 1 < nb) dst[1] = sc[2 * half + 1] * kInvSqrt128;
-            }
-          }
+        for (int k = 0; k < 2; ++k) {
+          const float c0 = fmaxf(acc[m][nt][2 * k], 0.f), c1 = fmaxf(acc[m][nt][2 * k + 1], 0.f);
+          half[k] = (odd ? c1 : c0) + __shfl_xor_sync(0xffffffffu, odd ? c0 : c1, 4);
         }
+        sc[nt] = ((lower ? half[1] : half[0]) + __shfl_xor_sync(0xffffffffu, lower ? half[0] : half[1], 8)) * kInvSqrt128;
+      }
+      const int r = 4 * m + (lower ? 2 : 0) + (g >> 2);
+      const int nb = (a.pos0 + r + 1) / 4;
+      if (r >= a.R || nb <= CR_SEL_BLOCKS) continue;
+      float* dst = a.scores + (size_t)r * a.sstride + blk;
+      if (blk + 4 <= nb && ((uintptr_t)dst & 15) == 0) {
+        *reinterpret_cast<float4*>(dst) = make_float4(sc[0], sc[1], sc[2], sc[3]);
+      } else {
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+          if (blk + nt < nb) dst[nt] = sc[nt];
+      }
     }
   }
 }
 
-// Spans of 3..16 rows, every block of every row.
+// Spans of 3..16 rows, every block of every row.  Three CTAs of four warps fit an SM; the tiles are dealt in one wave of them.
 cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream) {
-  const dim3 grid((tiles + 4 * kSmTilesPerWarp - 1) / (4 * kSmTilesPerWarp), 1, n);
+  const int warps = sm_count() * 12, per_warp = (int)(((long long)tiles * n + warps - 1) / warps);
+  const dim3 grid((tiles + 4 * per_warp - 1) / (4 * per_warp), 1, n);
   const int mt = (Rmax + 3) / 4;
-  if (mt <= 1) qsa_score_mma_kernel<1><<<grid, 128, 0, stream>>>(P);
-  else if (mt == 2) qsa_score_mma_kernel<2><<<grid, 128, 0, stream>>>(P);
-  else if (mt == 3) qsa_score_mma_kernel<3><<<grid, 128, 0, stream>>>(P);
-  else qsa_score_mma_kernel<4><<<grid, 128, 0, stream>>>(P);
+  auto kernel = mt <= 1 ? qsa_score_mma_kernel<1> : mt == 2 ? qsa_score_mma_kernel<2> : mt == 3 ? qsa_score_mma_kernel<3> : qsa_score_mma_kernel<4>;
+  CR_CUDA(launch_pdl(kernel, grid, dim3(128), 0, stream, P, per_warp));
   CR_LAUNCH_CHECK("qsa_score_mma_kernel");
   return CR_OK;
 }
