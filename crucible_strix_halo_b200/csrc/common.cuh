@@ -197,6 +197,27 @@ __device__ __forceinline__ float load_in(const void* p, long long i) {
   else return reinterpret_cast<const float*>(p)[i];
 }
 
+// Brings kernel parameters into the constant cache: called before pdl_wait, while the kernel ahead still runs.
+template <typename T>
+__device__ __forceinline__ void touch_params(const T& p) {
+  const int* w = reinterpret_cast<const int*>(&p);
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(T) / 4); i += 16) asm volatile("" ::"r"(w[i]));
+}
+
+// Loads of what is read once per step and is larger than L2 together (the pooled keys of a scan): first to be evicted, so that the
+// scan leaves in L2 what the kernels around it read, their code among it.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ float4 load_stream4(const float* p, uint64_t policy) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(policy));
+  return v;
+}
+
 // Split-half partial RoPE angle terms for pair j (< 32) at position p with a 64-float table.
 __device__ __forceinline__ void rope_cs(const float* rope, int j, int p, float& c, float& s) {
   const float ang = (float)p * rope[j], m = rope[32];

@@ -20,8 +20,11 @@
 // a second kernel) was held by shared-memory reads and barriers: 2,048 rows at 262,144 positions took 1,875 us plus
 // 180 us of merge, 700 us now (12 TB/s of gathers: the rows walk their ascending positions side by side, so the rows in
 // flight share a region of the cache that L2 holds; from L2 alone 666 us, where every byte's way into and out of shared
-// memory takes three quarters of its bandwidth); 72 verify rows at 131,072 105 + 12 us, 53 us now; four decode rows at
-// 262,144 17 + 9 us, 13 us now.
+// memory takes three quarters of its bandwidth); 72 verify rows at 131,072 105 + 12 us, 53 us now.
+// Steps of few rows are a chain of round trips (parameters, selection, K, V, merge over the CTA, over the cluster): 10.8 us for a
+// row at 1,501 positions, 13 for four at 262,144, 16.4 for four of 24 heads at 32,003 while every warp fetched its query fragments
+// itself (256 line look-ups each), the count of a selection came before its ids, gates were asked for at the end and the
+// parts of a merge one by one; 8.3, 9.0 and 14.1 us now.
 #include <climits>
 #include <cooperative_groups.h>
 #include "qsa.cuh"
@@ -90,11 +93,12 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
                                                                        int p0, int p1, int fmt) {
   extern __shared__ __align__(1024) unsigned char ring_raw[];
   __shared__ float ml_s[kMaxWarps][8][2];              // (m, l) of every stream's heads
-  __shared__ float cta_ml[16][2];                      // of the CTA's merged unit, read by the cluster
+  __shared__ float2 cta_ml[16];                        // (m, l) of the CTA's merged unit, read by the cluster
   pdl_release();
-  pdl_wait();
   constexpr int W = kStreams<NG>;
   const cr_qsa_args& a = P.span[blockIdx.z];
+  touch_params(a);
+  pdl_wait();
   const int t = threadIdx.x, warp = t >> 5, l = t & 31, g8 = l >> 2, tq = l & 3;
   const int stream = warp / NG, hg = warp % NG;
   const int upc = W / shape.spu, crank = shape.cluster > 1 ? (int)(blockIdx.x % shape.cluster) : 0;
@@ -114,33 +118,52 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
   unsigned char* ring = ring_raw + (size_t)stream * kRingBytes;
 
   if (live) {
-    const int p = a.pos0 + r, ns = a.nsel[r], nb = (p + 1) / 4;
+    const int p = a.pos0 + r, nb = (p + 1) / 4;
     const int* sel = a.sel + (size_t)r * CR_SEL_BLOCKS;
-    // Entries: the selected blocks (all complete blocks when dense), then the open block.  They ascend, so those that reach
-    // into a rank's window [p0, p1) are one contiguous range.
-    const int full = ns < 0 ? nb : ns;
-    int e_lo = 0, e_hi = full + ((p + 1) % 4 != 0 ? 1 : 0);
-    if (p0 > 0 || p1 <= p) {
-      auto entry_at_least = [&](int blk) {               // first entry whose block is >= blk
-        if (ns < 0) return min(blk, e_hi);
-        int lo = 0, hi = full;
-        while (lo < hi) { const int mid = (lo + hi) >> 1; if (sel[mid] < blk) lo = mid + 1; else hi = mid; }
-        return lo == full && nb < blk ? e_hi : lo;
-      };
-      const int lo = entry_at_least(p0 / 4), hi = p1 > p ? e_hi : entry_at_least((p1 + 3) / 4);
-      e_lo = lo; e_hi = min(hi, e_hi);
+    // Where the CTA has one unit its query heads come in once, beside the selection: [head][256] with the 32-byte pieces of a row
+    // XORed by the head, so that the fragment reads meet no bank twice.  (Every warp loading them as fragments cost 256 line
+    // look-ups a warp: 2 us of a step's 9 to 16.)
+    float* qs = reinterpret_cast<float*>(ring_raw + (size_t)W * kRingBytes);
+    if (upc == 1) {
+      const float* q = a.q + ((size_t)r * P.Hq + g * gqa) * 512;
+      for (int i = t; i < gqa * 64; i += kAttnThreads<NG>) {
+        const int hd = i >> 6, pc = i & 63;
+        attn_cp16((unsigned)__cvta_generic_to_shared(qs) + hd * 1024 + (pc ^ ((hd & 7) << 1)) * 16, q + (size_t)hd * 512 + pc * 4);
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
-    const int tiles_all = max(e_hi - e_lo + 3, 0) / 4, streams = shape.spu * shape.cluster, s_idx = crank * shape.spu + sub;
-    const int tb = tiles_all / streams, trem = tiles_all % streams;
-    const int tile0 = s_idx * tb + min(s_idx, trem), tiles = tb + (s_idx < trem ? 1 : 0);
-    const int e0 = e_lo + 4 * tile0;                     // first entry of this stream
-
-    // Block ids: lane l of `ids` holds entry e0 + 32 k + l of the current group of eight tiles, `ids_next` the next group.
-    auto load_ids = [&](int k) {
+    // The selection holds all or 512 blocks, as the row's length says: its ids are asked for in that belief, beside the count.
+    const int counted = __ldcg(a.nsel + r);
+    int ns = nb <= CR_SEL_BLOCKS ? -1 : CR_SEL_BLOCKS;
+    int full, e_hi, e0, tiles, ids, ids_next;
+    auto load_ids = [&](int k) {                           // lane l: entry e0 + 32 k + l of this stream
       const int e = e0 + 32 * k + l;
       return e < e_hi ? (ns < 0 || e >= full ? (e >= full ? nb : e) : sel[e]) : -1;
     };
-    int ids = load_ids(0), ids_next = load_ids(1);
+    for (;; ns = counted) {
+      // Entries: the selected blocks (all complete blocks when dense), then the open block.  They ascend, so those that reach
+      // into a rank's window [p0, p1) are one contiguous range.
+      full = ns < 0 ? nb : ns;
+      int e_lo = 0;
+      e_hi = full + ((p + 1) % 4 != 0 ? 1 : 0);
+      if (p0 > 0 || p1 <= p) {
+        auto entry_at_least = [&](int blk) {               // first entry whose block is >= blk
+          if (ns < 0) return min(blk, e_hi);
+          int lo = 0, hi = full;
+          while (lo < hi) { const int mid = (lo + hi) >> 1; if (sel[mid] < blk) lo = mid + 1; else hi = mid; }
+          return lo == full && nb < blk ? e_hi : lo;
+        };
+        const int lo = entry_at_least(p0 / 4), hi = p1 > p ? e_hi : entry_at_least((p1 + 3) / 4);
+        e_lo = lo; e_hi = min(hi, e_hi);
+      }
+      const int tiles_all = max(e_hi - e_lo + 3, 0) / 4, streams = shape.spu * shape.cluster, s_idx = crank * shape.spu + sub;
+      const int tb = tiles_all / streams, trem = tiles_all % streams;
+      tiles = tb + (s_idx < trem ? 1 : 0);
+      e0 = e_lo + 4 * (s_idx * tb + min(s_idx, trem));     // first entry of this stream
+      // Block ids: lane l of `ids` holds entry e0 + 32 k + l of the current group of eight tiles, `ids_next` the next group.
+      ids = load_ids(0); ids_next = load_ids(1);
+      if (counted == ns) break;
+    }
     const size_t row_bytes = HKV ? (size_t)HKV * 512 : (size_t)P.Hkv * 512;
     const char* kc = reinterpret_cast<const char*>(a.c.k) + (size_t)g * 512 + l * 16;
     const char* vc = reinterpret_cast<const char*>(a.c.v) + (size_t)g * 512 + l * 16;
@@ -195,16 +218,27 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     // Query heads of the group as column fragments, fp16 head and remainder, while the first halves are in flight.
     unsigned qh[16][2], ql[16][2];
     {
-      const float* q = a.q + ((size_t)r * P.Hq + g * gqa + hg * gh + min(g8, heads - 1)) * 512 + 2 * tq;
       const bool have = g8 < heads;
+      const int hd = hg * gh + min(g8, heads - 1);
+      auto take = [&](int ks, int j, float2 v) {
+        if (!have) v = make_float2(0.f, 0.f);
+        split2(v.x, v.y, qh[ks][j], ql[ks][j]);
+      };
+      if (upc == 1) {
+        asm volatile("cp.async.wait_group 3;\n" ::: "memory");
+        __syncthreads();
+        const float* q = qs + hd * 256 + 2 * tq;
 #pragma unroll
-      for (int ks = 0; ks < 16; ++ks)
+        for (int ks = 0; ks < 16; ++ks)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          float2 v = *reinterpret_cast<const float2*>(q + 16 * ks + 8 * j);
-          if (!have) v = make_float2(0.f, 0.f);
-          split2(v.x, v.y, qh[ks][j], ql[ks][j]);
-        }
+          for (int j = 0; j < 2; ++j) take(ks, j, *reinterpret_cast<const float2*>(q + ((2 * ks + j) ^ (hd & 7)) * 8));
+      } else {
+        const float* q = a.q + ((size_t)r * P.Hq + g * gqa + hd) * 512 + 2 * tq;
+#pragma unroll
+        for (int ks = 0; ks < 16; ++ks)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) take(ks, j, *reinterpret_cast<const float2*>(q + (2 * ks + j) * 8));
+      }
     }
     constexpr float kScale = 0.0625f * 1.4426950408889634f;           // logits / 16, in powers of two
     // this lane's ldmatrix rows: K: matrices (positions 0-7 | 8-15) x (first | second 8 channels); V: the transpose of that
@@ -301,7 +335,8 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     __syncthreads();
   }
   if (shape.cluster == 1 && !live) return;
-  // This CTA's merged (m, l, acc) of head hd, channels c .. c + 3.
+  // This CTA's merged (m, l, acc) of head hd, channels c .. c + 3.  (One part at a time and the gate at the end: long parts, where a
+  // stream has its unit to itself, lose 1.5 % to eight parts or the gate in flight.)
   const int first_stream = stream - sub;
   auto merged = [&](int hd, int c, float& m, float& lsum) {
     const int hg_ = hd / gh, hl = hd % gh;
@@ -317,7 +352,10 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     }
     return o;
   };
-  auto finish = [&](int hd, int c, float m, float lsum, float4 o) {
+  auto gate_of = [&](int hd, int c) {
+    return partials ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(a.q + ((size_t)r * P.Hq + g * gqa + hd) * 512 + 256 + c);
+  };
+  auto finish = [&](int hd, int c, float m, float lsum, float4 o, float4 gate) {
     const int h = g * gqa + hd;
     if (partials) {                                      // a rank's partial: (m, l, acc) with m as a natural logarithm
       float* dst = partials + ((size_t)(P.base[blockIdx.z] + r) * P.Hq + h) * CR_QSA_PART;
@@ -326,7 +364,6 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
       *reinterpret_cast<float2*>(dst + 4 + c) = make_float2(o.z, o.w);
       return;
     }
-    const float4 gate = *reinterpret_cast<const float4*>(a.q + ((size_t)r * P.Hq + h) * 512 + 256 + c);
     const float inv = 1.f / lsum;
     emit_group(a, P.Hq, r, h, c, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv), gate, fmt);
   };
@@ -336,42 +373,74 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
       float m, lsum;
       const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
       const float4 o = merged(hd, c, m, lsum);
-      finish(hd, c, m, lsum, o);
+      finish(hd, c, m, lsum, o, gate_of(hd, c));
     }
     return;
   }
-  // cluster: the CTA's merged unit goes to shared memory behind the ring images of the first stream, then every CTA takes a
-  // share of the groups over all CTAs
-  cg::cluster_group cluster = cg::this_cluster();
-  float* mine = reinterpret_cast<float*>(ring_raw + (size_t)W * kRingBytes);
-  for (int gi = warp; gi < 2 * gqa; gi += W * NG) {
-    float m, lsum;
-    const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
-    const float4 o = merged(hd, c, m, lsum);
-    *reinterpret_cast<float4*>(mine + hd * 256 + c) = o;
-    if (c == 0) { cta_ml[hd][0] = m; cta_ml[hd][1] = lsum; }
-  }
-  cluster.sync();
-  for (int gi = crank + shape.cluster * warp; gi < 2 * gqa; gi += shape.cluster * W * NG) {
-    const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
-    float ms[8], m = -INFINITY, lsum = 0.f;
+  // (m, l) of `n` parts (at most 8), lane k & 7 holding those of part k: the factor of that part's accumulator; m and l become those of
+  // the whole.
+  auto weigh = [&](int n, float& m, float& lsum) {
+    const bool have = (l & 7) < n;
+    const float mk = have ? m : -INFINITY;
+    m = mk;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      ms[k] = k < shape.cluster ? cluster.map_shared_rank(&cta_ml[0][0], k)[2 * hd] : -INFINITY;
-      m = fmaxf(m, ms[k]);
-    }
+    for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float f = mk > -INFINITY ? ex2(mk - m) : 0.f;
+    lsum = have ? lsum * f : 0.f;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    return f;
+  };
+  auto weighted = [&](const float4 (&x)[8], int n, float f) {
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      if (k >= shape.cluster) break;
-      const float f = ms[k] > -INFINITY ? ex2(ms[k] - m) : 0.f;
-      lsum = fmaf(cluster.map_shared_rank(&cta_ml[0][0], k)[2 * hd + 1], f, lsum);
-      const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(mine, k) + hd * 256 + c);
-      o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
+      const float fk = __shfl_sync(0xffffffffu, f, k);
+      if (k < n) { o.x = fmaf(x[k].x, fk, o.x); o.y = fmaf(x[k].y, fk, o.y); o.z = fmaf(x[k].z, fk, o.z); o.w = fmaf(x[k].w, fk, o.w); }
     }
-    finish(hd, c, m, lsum, o);
+    return o;
+  };
+  // cluster: the CTA's merged unit goes to shared memory behind the ring images of the first stream, then every CTA takes a
+  // share of the groups over all CTAs: at most one group per warp (two CTAs have 16 or 24 warps, as many as there are groups)
+  cg::cluster_group cluster = cg::this_cluster();
+  float* mine = reinterpret_cast<float*>(ring_raw + (size_t)W * kRingBytes);
+  const int gi_out = crank + shape.cluster * warp, hd_out = gi_out >> 1, c_out = (gi_out & 1) * 128 + 4 * l;
+  const bool emits = gi_out < 2 * gqa;
+  float4 gate = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (emits) gate = gate_of(hd_out, c_out);                           // in flight through the merge
+  for (int hd = warp; hd < gqa; hd += W * NG) {                        // a head per warp: both halves share their weights
+    const int hg_ = hd / gh, hl = hd % gh;
+    const float* img = reinterpret_cast<const float*>(ring_raw) + (size_t)(hg_ * 8 + hl) * kAccLd + 4 * l;
+    float4 x[2][8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < W) {
+        x[0][k] = *reinterpret_cast<const float4*>(img + (size_t)k * (kRingBytes / 4));
+        x[1][k] = *reinterpret_cast<const float4*>(img + (size_t)k * (kRingBytes / 4) + 128);
+      }
+    const float* ml = ml_s[min(l & 7, W - 1) * NG + hg_][hl];
+    float m = ml[0], lsum = ml[1];
+    const float f = weigh(W, m, lsum);
+    *reinterpret_cast<float4*>(mine + hd * 256 + 4 * l) = weighted(x[0], W, f);
+    *reinterpret_cast<float4*>(mine + hd * 256 + 128 + 4 * l) = weighted(x[1], W, f);
+    if (l == 0) cta_ml[hd] = make_float2(m, lsum);
   }
-  cluster.sync();                                        // the images stay until every CTA has read them
+  cluster.sync();
+  float m = -INFINITY, lsum = 0.f;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (emits) {
+    float4 x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < shape.cluster) x[k] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(mine, k) + hd_out * 256 + c_out);
+    const float2 ml = cluster.map_shared_rank(&cta_ml[0], min(l & 7, shape.cluster - 1))[hd_out];
+    m = ml.x; lsum = ml.y;
+    const float f = weigh(shape.cluster, m, lsum);
+    o = weighted(x, shape.cluster, f);
+  }
+  cluster.barrier_arrive();                              // this CTA has read the others' images
+  if (emits) finish(hd_out, c_out, m, lsum, o, gate);
+  cluster.barrier_wait();                                // the own images stay until every CTA has read them
 }
 
 // Merge of the partial records of several ranks or of a tile's splits (QsaMergeKernel, engine/layers/qsa_long.h:458-499), gate and output

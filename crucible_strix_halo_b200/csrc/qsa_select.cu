@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(256) qsa_score_kernel(const __grid_constant__ 
 // Same scores for one or two rows with 128-bit loads: lane l reads blocks 4(l%8)..+3 of dims l/8, l/8+4, ...,
 // so a warp load covers four 128-byte lines and the tile costs 32 load instructions per lane instead of 128.
 // The four lanes that share a block group add their partial dots with two shuffles.
+// The pool passes through L2 as the first thing to be evicted: four sessions of 262,144 positions (134 MB, more than L2) had pushed
+// out the states, the rows and the code of the kernels around the scan: a step 75.4 -> 66.1 us, of which 4 in the attention.
 // RANGED: only the blocks [P.b_lo, P.b_hi) are scored (a rank's own blocks).  A separate instantiation: with the range
 // tests in it the whole-row kernel measured 40 us instead of 29 for four 262,144-token rows.
 template <int RT, bool RANGED>
@@ -102,7 +104,8 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
   const int tile = (RANGED ? P.b_lo / 32 : 0) + blockIdx.x * 8 + w;
   if (tile * 32 >= nb_hi) return;
   const int bq = (l & 7) * 4, dl = l >> 3;
-  const float4* pt = reinterpret_cast<const float4*>(a.c.ik_pool + (size_t)tile * 4096 + dl * 32 + bq);
+  const float* pt = a.c.ik_pool + (size_t)tile * 4096 + dl * 32 + bq;
+  const uint64_t policy = evict_first_policy();
   float acc[RT][4][4];                        // [row][block][head]
 #pragma unroll
   for (int r = 0; r < RT; ++r)
@@ -112,7 +115,7 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
   for (int it0 = 0; it0 < 32; it0 += 8) {
     float4 key[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) key[j] = __ldg(pt + (it0 + j) * 32);
+    for (int j = 0; j < 8; ++j) key[j] = load_stream4(pt + (it0 + j) * 128, policy);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float kb[4] = {key[j].x, key[j].y, key[j].z, key[j].w};
@@ -177,7 +180,11 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
     const bool ranged = b_lo > 0 || b_hi < INT_MAX;
     const int Rmax = qsa_max_rows(spans + s0, n);
     int nb_max = 0;
-    for (int s = 0; s < n; ++s) nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
+    bool wide = true;                               // pools at 16-byte boundaries
+    for (int s = 0; s < n; ++s) {
+      nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
+      wide &= ((uintptr_t)spans[s0 + s].c.ik_pool & 15) == 0;
+    }
     if (nb_max <= CR_SEL_BLOCKS) continue;
     const int hi = nb_max < b_hi ? nb_max : b_hi;
     if (hi <= b_lo) continue;                       // the range holds no complete block of these rows
@@ -195,7 +202,7 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
       CR_LAUNCH_CHECK("qsa_score_kernel");
       st = CR_OK;
     }
-    else if (Rmax <= 16 && !ranged && !options().qsa_score_simt) st = qsa_score_mma_launch(P, tiles, Rmax, n, stream);   // verify spans
+    else if (Rmax <= 16 && !ranged && wide && !options().qsa_score_simt) st = qsa_score_mma_launch(P, tiles, Rmax, n, stream);   // verify spans
     else if (Rmax >= 8 && !options().qsa_score_simt) st = qsa_score_tc_launch(P, n, stream);   // prefill parts (and a rank's range of a span)
     else if (Rmax <= 4) st = score_launch_t<4>(P, tiles, Rmax, n, ranged, stream);
     else st = score_launch_t<8>(P, tiles, Rmax, n, ranged, stream);
