@@ -34,6 +34,8 @@ namespace cr {
 constexpr int kSelThreads = 1024;
 constexpr int kMaxSelectCount = 262144;   // elements of one selection: the tie bitmap of the slow path shares the 32 KB of the candidate list
 constexpr int kSortCap = 4096;            // entries of the candidate list (32 KB)
+constexpr int kShortCap = 3072;           // of the list of 256 threads, which take rows of many
+constexpr int kShortRow = 14336;          // up to this many blocks (above, 512 threads are the quicker ones)
 
 // ---- element sources ---------------------------------------------------------------------------------------
 // A source maps an element index i in [0, count) to (bit pattern, block id, valid).  Index order is block-id order.
@@ -67,6 +69,7 @@ __device__ __forceinline__ RowSource row_source(const cr_qsa_args& a, int r, int
 }
 
 // ---- block-wide helpers ------------------------------------------------------------------------------------
+template <int T>
 __device__ __forceinline__ unsigned block_sum_u32(unsigned v, unsigned* red) {   // red: 33 words
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
@@ -74,7 +77,7 @@ __device__ __forceinline__ unsigned block_sum_u32(unsigned v, unsigned* red) {  
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x < 32) {
-    unsigned t = red[threadIdx.x];
+    unsigned t = threadIdx.x < T / 32 ? red[threadIdx.x] : 0u;
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
     if (threadIdx.x == 0) red[32] = t;
@@ -83,13 +86,14 @@ __device__ __forceinline__ unsigned block_sum_u32(unsigned v, unsigned* red) {  
   return red[32];
 }
 // Largest of one value per thread; one barrier (red: 32 words, free again after the caller's next barrier).
+template <int T>
 __device__ __forceinline__ unsigned block_max_u32(unsigned v, unsigned* red) {
   const unsigned m = __reduce_max_sync(0xffffffffu, v);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  return __reduce_max_sync(0xffffffffu, red[threadIdx.x & 31]);
+  return __reduce_max_sync(0xffffffffu, (threadIdx.x & 31) < T / 32 ? red[threadIdx.x & 31] : 0u);
 }
-// Exclusive prefix sum of one value per thread over the block (1024 threads); one barrier before red is written, one after.
+// Exclusive prefix sum of one value per thread over the block; one barrier before red is written, one after.
 __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* red) {
   const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned inc = v;
@@ -105,34 +109,35 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* r
 }
 // Shared memory of one CTA: candidate list (32 KB), bitmap over the row's elements (count bits), small arrays.
 struct SelectSmem {
-  uint2* cand;                 // kSortCap (key, index) pairs; the slow path keeps its tie bitmap here instead
+  uint2* cand;                 // cap (key, index) pairs; the slow path keeps its tie bitmap here instead
+  int cap;
   unsigned* bitmap;            // ceil(count / 32) words
   unsigned* red;               // 33 words
   unsigned* counter;           // 1 word
   int* hist;                   // kBins counters, zero between uses
   int* found;                  // 3 words
-  uint2* ties;                 // kRankCap entries
+  uint2* ties;                 // kRankCap entries, in the place of the histogram once that has done its work
 };
 
 constexpr int kBatch = 8;      // loads a thread issues before it uses any of them
 
-// Calls f(i, key) for the elements i = t, t + 1024, ... < count of this thread, key = bit pattern + 1 (0: no element).
+// Calls f(i, key) for the elements i = t, t + T, ... < count of this thread, key = bit pattern + 1 (0: no element).
 // Loads are issued kBatch at a time.  WARP_UNIFORM: f is also called with key 0 for indices past the end, so that all
 // lanes of a warp make the same number of calls (f may use warp-collective operations).
-template <bool WARP_UNIFORM, typename Src, typename F>
+template <int T, bool WARP_UNIFORM, typename Src, typename F>
 __device__ __forceinline__ void for_each_key(const Src& src, int count, F&& f) {
   const int lane = threadIdx.x & 31;
-  for (int i0 = threadIdx.x; i0 - lane < count; i0 += kSelThreads * kBatch) {   // the same trip count for a whole warp
+  for (int i0 = threadIdx.x; i0 - lane < count; i0 += T * kBatch) {   // the same trip count for a whole warp
     unsigned key[kBatch];
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) {
-      const int i = i0 + k * kSelThreads;
+      const int i = i0 + k * T;
       unsigned bits = 0u;
       key[k] = (i < count && src.get(i, bits)) ? bits + 1u : 0u;
     }
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) {
-      const int i = i0 + k * kSelThreads;
+      const int i = i0 + k * T;
       if (WARP_UNIFORM ? (i - lane < count) : (i < count)) f(i, key[k]);
     }
   }
@@ -140,20 +145,20 @@ __device__ __forceinline__ void for_each_key(const Src& src, int count, F&& f) {
 
 // The same four elements at a time (src.quads): f(i, keys) for the elements i .. i + 3, keys past the end 0.  All lanes of a
 // warp make the same number of calls.
-template <typename Src, typename F>
+template <int T, typename Src, typename F>
 __device__ __forceinline__ void for_each_quad(const Src& src, int count, F&& f) {
   const int lane = threadIdx.x & 31, quads = (count + 3) >> 2;
-  constexpr int kDeep = 2;
-  for (int q0 = threadIdx.x; q0 - lane < quads; q0 += kSelThreads * kDeep) {
+  constexpr int kDeep = T >= 1024 ? 2 : 4;
+  for (int q0 = threadIdx.x; q0 - lane < quads; q0 += T * kDeep) {
     uint4 v[kDeep];
 #pragma unroll
     for (int k = 0; k < kDeep; ++k) {
-      const int q = q0 + k * kSelThreads;
+      const int q = q0 + k * T;
       v[k] = q < quads ? src.get4(q) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int k = 0; k < kDeep; ++k) {
-      const int q = q0 + k * kSelThreads, i = 4 * q;
+      const int q = q0 + k * T, i = 4 * q;
       if (q - lane >= quads) break;                                 // warp uniform
       f(i, make_uint4(i < count ? v[k].x + 1u : 0u, i + 1 < count ? v[k].y + 1u : 0u, i + 2 < count ? v[k].z + 1u : 0u, i + 3 < count ? v[k].w + 1u : 0u));
     }
@@ -167,8 +172,9 @@ constexpr int kRankCap = 512;              // elements of the threshold bin that
 struct Threshold { int bin, above, in_bin; };   // the bin that holds the want-th largest; elements in higher bins; in it
 // sm.hist filled and visible.  The bin of the want-th largest counted element; bin = -1 when fewer were counted.  Two
 // barriers; the histogram is zero again afterwards (visible after the caller's next barrier).
+template <int T>
 __device__ __forceinline__ Threshold find_threshold(const SelectSmem& sm, int want) {
-  constexpr int PER = kBins / kSelThreads;
+  constexpr int PER = kBins / T;
   const int t = threadIdx.x, l = t & 31, w = t >> 5, first = kBins - 1 - t * PER;   // this thread's bins, descending
   int c[PER], sum = 0;
 #pragma unroll
@@ -199,30 +205,30 @@ __device__ __forceinline__ int bin_shift(unsigned lo, unsigned hi) {
   return span < (unsigned)kBins ? 0 : 21 - __clz(span);
 }
 
-// A lower bound of the want-th largest of one key per thread (0: none), such that at least `want` keys are >= it; 1 when
+// A lower bound of the want-th largest of G keys per thread (0: none), such that at least `want` keys are >= it; 1 when
 // there are fewer.  largest: the largest of all keys.  sm.hist zero on entry.
-__device__ __forceinline__ unsigned pivot_of(unsigned mine, unsigned largest, int want, const SelectSmem& sm) {
+template <int T, int G>
+__device__ __forceinline__ unsigned pivot_of(const unsigned (&mine)[G], unsigned largest, int want, const SelectSmem& sm) {
   unsigned shift = 14;                                             // the four octaves below the largest key
 #pragma unroll 1
   for (int round = 0; round < 2; ++round, shift = 20) {            // then everything
     const unsigned width = (unsigned)kBins << shift, lo = largest >= width ? largest - width + 1u : 1u;
-    if (mine >= lo) atomicAdd(&sm.hist[(mine - lo) >> shift], 1);
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+      if (mine[k] >= lo) atomicAdd(&sm.hist[(mine[k] - lo) >> shift], 1);
     __syncthreads();
-    const Threshold th = find_threshold(sm, want);
+    const Threshold th = find_threshold<T>(sm, want);
     __syncthreads();
     if (th.bin >= 0) return lo + ((unsigned)th.bin << shift);
   }
   return 1u;
 }
 
-// The list sm.cand[0, m) holds (key, index) pairs that include the `want` best elements of the row (want <= m <= kSortCap),
+// The list sm.cand[0, m) holds (key, index) pairs that include the `want` best elements of the row (want <= m <= sm.cap),
 // keys in [lo, hi]: marks those in sm.bitmap.  sm.hist zero and the list visible on entry; ends with a barrier.
+template <int T>
 __device__ __forceinline__ void select_from_list(int m, int want, const SelectSmem& sm, unsigned lo, unsigned hi) {
   const int t = threadIdx.x;
-  constexpr int PER = kSortCap / kSelThreads;
-  uint2 c[PER];
-#pragma unroll
-  for (int q = 0; q < PER; ++q) { const int i = t + q * kSelThreads; c[q] = i < m ? sm.cand[i] : make_uint2(0u, 0u); }
   // The first division covers the four octaves below the largest key (or less, if the list does); should they hold too few,
   // the whole range.
   const int full = bin_shift(lo, hi);
@@ -231,13 +237,12 @@ __device__ __forceinline__ void select_from_list(int m, int want, const SelectSm
   Threshold th;
   for (;;) {
     const unsigned width = (unsigned)kBins << shift;
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      const unsigned d = c[q].x - first;
-      if (c[q].x >= first && c[q].x != 0u && d < width) atomicAdd(&sm.hist[d >> shift], 1);
+    for (int i = t; i < m; i += T) {
+      const unsigned key = sm.cand[i].x, d = key - first;
+      if (key >= first && key != 0u && d < width) atomicAdd(&sm.hist[d >> shift], 1);
     }
     __syncthreads();
-    th = find_threshold(sm, need);
+    th = find_threshold<T>(sm, need);
     if (th.bin < 0) {
       shift = full; first = lo;
       __syncthreads();
@@ -254,44 +259,60 @@ __device__ __forceinline__ void select_from_list(int m, int want, const SelectSm
   if (ranked) {
     if (t == 0) *sm.counter = 0u;
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PER; ++q)
-      if (c[q].x >= first && c[q].x <= last && c[q].x != 0u) sm.ties[atomicAdd(sm.counter, 1u)] = c[q];
+    for (int i = t; i < m; i += T) {
+      const uint2 c = sm.cand[i];
+      if (c.x >= first && c.x <= last && c.x != 0u) sm.ties[atomicAdd(sm.counter, 1u)] = c;
+    }
     __syncthreads();
   }
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    if (c[q].x < first || c[q].x == 0u) continue;
-    bool take = c[q].x > last || all;
+  for (int i = t; i < m; i += T) {
+    const uint2 c = sm.cand[i];
+    if (c.x < first || c.x == 0u) continue;
+    bool take = c.x > last || all;
     if (!take) {                                                   // inside the bin: better keys, then lower indices first
       const uint2* list = ranked ? sm.ties : sm.cand;              // a bin too crowded to rank holds one key only
       const int n = ranked ? th.in_bin : m;
       int before = 0;
-      for (int j = 0; j < n; ++j) { const uint2 o = list[j]; before += (o.x > c[q].x && o.x <= last) || (o.x == c[q].x && o.y < c[q].y); }
+      for (int j = 0; j < n; ++j) { const uint2 o = list[j]; before += (o.x > c.x && o.x <= last) || (o.x == c.x && o.y < c.y); }
       take = before < need;
     }
-    if (take) atomicOr(&sm.bitmap[c[q].y >> 5], 1u << (c[q].y & 31));
+    if (take) atomicOr(&sm.bitmap[c.y >> 5], 1u << (c.y & 31));
   }
   __syncthreads();
 }
 
-template <typename Src>
+template <int T, typename Src>
 __device__ __forceinline__ void select_slow(const Src& src, int count, int want, const SelectSmem& sm);
 
 // Marks the `want` best elements of [0, count) in sm.bitmap (bit i = element i selected).  want <= valid elements.
-template <typename Src>
+template <int T, typename Src>
 __device__ __forceinline__ void select_mark(const Src& src, int count, int want, const SelectSmem& sm) {
   const int t = threadIdx.x, l = t & 31;
+  constexpr int G = 1024 / T;                                      // groups of a thread: 1024 in the block
   const int words = (count + 31) >> 5;
-  for (int i = t; i < words; i += kSelThreads) sm.bitmap[i] = 0u;
-  for (int i = t; i < kBins; i += kSelThreads) sm.hist[i] = 0;
+  for (int i = t; i < words; i += T) sm.bitmap[i] = 0u;
+  for (int i = t; i < kBins; i += T) sm.hist[i] = 0;
   if (t == 0) *sm.counter = 0u;
   unsigned pivot = 1u, mine = 0u, largest = 0u;                    // pivot 1: every element passes
-  if (count > kSortCap) {
-    if (src.quads) for_each_quad(src, count, [&](int, const uint4& k) { mine = max(max(max(mine, k.x), max(k.y, k.z)), k.w); });
-    else for_each_key<false>(src, count, [&](int, unsigned key) { mine = key > mine ? key : mine; });
-    largest = block_max_u32(mine, sm.red);
-    pivot = pivot_of(mine, largest, want, sm);
+  if (count > sm.cap) {
+    unsigned group[G];
+#pragma unroll
+    for (int k = 0; k < G; ++k) group[k] = 0u;
+    if (src.quads) {
+      for_each_quad<T>(src, count, [&](int, const uint4& k) {
+        group[0] = max(group[0], k.x); group[1 % G] = max(group[1 % G], k.y); group[2 % G] = max(group[2 % G], k.z); group[3 % G] = max(group[3 % G], k.w);
+      });
+    } else {
+      for_each_key<T, false>(src, count, [&](int i, unsigned key) {
+#pragma unroll
+        for (int k = 0; k < G; ++k)
+          if (G == 1 || ((i / T) & (G - 1)) == k) group[k] = max(group[k], key);
+      });
+    }
+#pragma unroll
+    for (int k = 0; k < G; ++k) mine = max(mine, group[k]);
+    largest = block_max_u32<T>(mine, sm.red);
+    pivot = pivot_of<T, G>(group, largest, want, sm);
   } else {
     __syncthreads();
   }
@@ -304,52 +325,52 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
       if (l == 0) base = atomicAdd(sm.counter, (unsigned)__popc(m));
       base = __shfl_sync(0xffffffffu, base, 0);
       const unsigned at = base + __popc(m & ((1u << l) - 1u));
-      if (pass && at < (unsigned)kSortCap) sm.cand[at] = make_uint2(key, (unsigned)i);
+      if (pass && at < (unsigned)sm.cap) sm.cand[at] = make_uint2(key, (unsigned)i);
     }
   };
   if (src.quads) {
-    for_each_quad(src, count, [&](int i, const uint4& k) {
+    for_each_quad<T>(src, count, [&](int i, const uint4& k) {
       const unsigned best = max(max(k.x, k.y), max(k.z, k.w));
       mine = max(mine, best);
       if (!__any_sync(0xffffffffu, best >= pivot)) return;         // most quads of a long row
       append(i, k.x); append(i + 1, k.y); append(i + 2, k.z); append(i + 3, k.w);
     });
   } else {
-    for_each_key<true>(src, count, [&](int i, unsigned key) {
+    for_each_key<T, true>(src, count, [&](int i, unsigned key) {
       mine = max(mine, key);
       append(i, key);
     });
   }
-  if (count > kSortCap) __syncthreads();
-  else largest = block_max_u32(mine, sm.red);
+  if (count > sm.cap) __syncthreads();
+  else largest = block_max_u32<T>(mine, sm.red);
   const int m = (int)*sm.counter;
-  if (m >= want && m <= kSortCap) { select_from_list(m, want, sm, pivot, largest); return; }
-  select_slow(src, count, want, sm);
+  if (m >= want && m <= sm.cap) { select_from_list<T>(m, want, sm, pivot, largest); return; }
+  select_slow<T>(src, count, want, sm);
 }
 
 // The slow exact path over the whole row; sm.bitmap zero on entry.
-template <typename Src>
+template <int T, typename Src>
 __device__ __forceinline__ void select_slow(const Src& src, int count, int want, const SelectSmem& sm) {
   const int t = threadIdx.x, l = t & 31;
   const int words = (count + 31) >> 5;
-  // ---- slow exact path: T = the largest key with at least `want` elements >= T
-  unsigned T = 0u;
+  // ---- slow exact path: limit = the largest key with at least `want` elements >= limit
+  unsigned limit = 0u;
   for (int bit = 30; bit >= 0; --bit) {
-    const unsigned trial = T | (1u << bit);
+    const unsigned trial = limit | (1u << bit);
     unsigned c = 0u;
-    for_each_key<false>(src, count, [&](int, unsigned key) { c += key >= trial; });
-    if (block_sum_u32(c, sm.red) >= (unsigned)want) T = trial;
+    for_each_key<T, false>(src, count, [&](int, unsigned key) { c += key >= trial; });
+    if (block_sum_u32<T>(c, sm.red) >= (unsigned)want) limit = trial;
   }
-  unsigned* ties = reinterpret_cast<unsigned*>(sm.cand);           // bitmap of the elements equal to T (<= 32 KB)
+  unsigned* ties = reinterpret_cast<unsigned*>(sm.cand);           // bitmap of the elements equal to limit (<= 32 KB)
   unsigned above = 0u;
-  for_each_key<true>(src, count, [&](int i, unsigned key) {        // a warp covers one bitmap word per call
-    const unsigned gt = __ballot_sync(0xffffffffu, key > T), eq = __ballot_sync(0xffffffffu, key == T);
+  for_each_key<T, true>(src, count, [&](int i, unsigned key) {        // a warp covers one bitmap word per call
+    const unsigned gt = __ballot_sync(0xffffffffu, key > limit), eq = __ballot_sync(0xffffffffu, key == limit);
     if (l == 0 && (i >> 5) < words) { sm.bitmap[i >> 5] = gt; ties[i >> 5] = eq; above += __popc(gt); }
   });
-  const unsigned n_above = block_sum_u32(above, sm.red);
+  const unsigned n_above = block_sum_u32<T>(above, sm.red);
   const unsigned need = (unsigned)want - n_above;                  // ties to take, lowest indices first
   // every thread owns a run of consecutive words: ties before the run decide how many of its own it takes
-  const int per = (words + kSelThreads - 1) / kSelThreads, w0 = t * per, w1 = min(w0 + per, words);
+  const int per = (words + T - 1) / T, w0 = t * per, w1 = min(w0 + per, words);
   unsigned mine = 0u;
   for (int w = w0; w < w1; ++w) mine += __popc(ties[w]);
   unsigned before = block_exclusive_scan(mine, sm.red);
@@ -368,11 +389,11 @@ __device__ __forceinline__ void select_slow(const Src& src, int count, int want,
 }
 
 // Writes the marked elements in index order: out_ids (and out_scores) get `want` entries.
-template <typename Src>
+template <int T, typename Src>
 __device__ __forceinline__ void select_emit(const Src& src, int count, const SelectSmem& sm, int* out_ids, float* out_scores) {
   const int t = threadIdx.x;
   const int words = (count + 31) >> 5;
-  const int per = (words + kSelThreads - 1) / kSelThreads, w0 = t * per, w1 = min(w0 + per, words);
+  const int per = (words + T - 1) / T, w0 = t * per, w1 = min(w0 + per, words);
   unsigned mine = 0u;
   for (int w = w0; w < w1; ++w) mine += __popc(sm.bitmap[w]);
   unsigned at = block_exclusive_scan(mine, sm.red);
@@ -388,21 +409,27 @@ __device__ __forceinline__ void select_emit(const Src& src, int count, const Sel
   }
 }
 
-__device__ __forceinline__ SelectSmem carve(unsigned char* raw, int max_count) {
+__device__ __forceinline__ SelectSmem carve(unsigned char* raw, int max_count, int cap = kSortCap) {
   SelectSmem sm;
   sm.cand = reinterpret_cast<uint2*>(raw);
-  sm.bitmap = reinterpret_cast<unsigned*>(raw + (size_t)kSortCap * 8);
+  sm.cap = cap;
+  sm.hist = reinterpret_cast<int*>(raw + (size_t)cap * 8);
+  sm.ties = reinterpret_cast<uint2*>(sm.hist);
+  sm.bitmap = reinterpret_cast<unsigned*>(sm.hist + kBins);
   sm.red = sm.bitmap + ((max_count + 31) >> 5);
   sm.counter = sm.red + 33;
   sm.found = reinterpret_cast<int*>(sm.counter + 1);
-  sm.hist = sm.found + 3;
-  sm.ties = reinterpret_cast<uint2*>(raw + (size_t)kSortCap * 8 + (((size_t)((max_count + 31) / 32) + 33 + 1 + 3 + kBins) * 4 + 7) / 8 * 8);
   return sm;
 }
-static size_t select_smem_bytes(int max_count) { return (size_t)kSortCap * 8 + ((size_t)((max_count + 31) / 32) + 37 + kBins) * 4 + 8 + (size_t)kRankCap * 8; }
+static size_t select_smem_bytes(int max_count, int cap = kSortCap) { return (size_t)cap * 8 + ((size_t)((max_count + 31) / 32) + 37 + kBins) * 4; }
 
-// grid (rows, spans): the selection of one row.
-__global__ void __launch_bounds__(kSelThreads, 2) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
+// grid (rows, spans): the selection of one row.  Few rows: 1,024 threads each, what counts is the time of one.  In many a row is a chain
+// of some sixteen short phases between barriers, and rows side by side on an SM are what fills it: five or six CTAs of 256 threads
+// (40 registers, a list of 3,072 entries) or, where the rows are long, three of 512, so that the rows in flight are still in L2 when
+// they are read again.  2,048 rows (two CTAs of 1,024 | 512 | 256 threads, us): 2,500 blocks 48 | 36 | 28, 8,192 blocks 69 | 51 | 47,
+// 15,500 94 | 77 | 79, 25,500 123 | 105 | 117, 65,536 198 | 189 | 234.
+template <int T>
+__global__ void __launch_bounds__(T, T == 1024 ? 2 : T == 512 ? 3 : 6) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
   extern __shared__ __align__(16) unsigned char raw[];
   pdl_release();
   pdl_wait();
@@ -411,10 +438,10 @@ __global__ void __launch_bounds__(kSelThreads, 2) qsa_topk_kernel(const __grid_c
   if (r >= a.R) return;
   const int nb = (a.pos0 + r + 1) / 4;
   if (nb <= CR_SEL_BLOCKS) { if (threadIdx.x == 0) a.nsel[r] = -1; return; }
-  const SelectSmem sm = carve(raw, max_count);
+  const SelectSmem sm = carve(raw, max_count, T == 1024 ? kSortCap : kShortCap);
   const RowSource src = row_source(a, r, 0);
-  select_mark(src, nb, CR_SEL_BLOCKS, sm);
-  select_emit(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
+  select_mark<T>(src, nb, CR_SEL_BLOCKS, sm);
+  select_emit<T>(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
   if (threadIdx.x == 0) a.nsel[r] = CR_SEL_BLOCKS;
 }
 
@@ -536,9 +563,9 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
     }
     __syncthreads();
     const RowSource src = row_source(a, r, 0);
-    if (total >= CR_SEL_BLOCKS && total <= kSortCap) select_from_list(total, CR_SEL_BLOCKS, sm, pivot, largest);
-    else select_slow(src, nb, CR_SEL_BLOCKS, sm);
-    select_emit(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
+    if (total >= CR_SEL_BLOCKS && total <= kSortCap) select_from_list<kSelThreads>(total, CR_SEL_BLOCKS, sm, pivot, largest);
+    else select_slow<kSelThreads>(src, nb, CR_SEL_BLOCKS, sm);
+    select_emit<kSelThreads>(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
     if (t == 0) a.nsel[r] = CR_SEL_BLOCKS;
   }
   cluster.sync();                                                  // the lists stay until CTA 0 has copied them
@@ -564,8 +591,8 @@ __global__ void __launch_bounds__(kSelThreads, 2) qsa_candidates_kernel(const __
   }
   const SelectSmem sm = carve(raw, max_count);
   const RowSource src = row_source(a, r, b0);
-  select_mark(src, count, CR_SEL_BLOCKS, sm);
-  select_emit(src, count, sm, ci, cs);
+  select_mark<kSelThreads>(src, count, CR_SEL_BLOCKS, sm);
+  select_emit<kSelThreads>(src, count, sm, ci, cs);
 }
 
 // Global selection from the gathered candidates [ranks][rows][512] of all ranks (ranks own ascending block ranges).
@@ -579,8 +606,8 @@ __global__ void __launch_bounds__(kSelThreads) qsa_merge_candidates_kernel(const
   const SelectSmem sm = carve(raw, max_count);
   const size_t off = (size_t)r * CR_SEL_BLOCKS;
   const GatheredSource src{cand_scores + off, cand_ids + off, (size_t)a.R * CR_SEL_BLOCKS};
-  select_mark(src, ranks * CR_SEL_BLOCKS, CR_SEL_BLOCKS, sm);
-  select_emit(src, ranks * CR_SEL_BLOCKS, sm, a.sel + off, nullptr);
+  select_mark<kSelThreads>(src, ranks * CR_SEL_BLOCKS, CR_SEL_BLOCKS, sm);
+  select_emit<kSelThreads>(src, ranks * CR_SEL_BLOCKS, sm, a.sel + off, nullptr);
   if (threadIdx.x == 0) a.nsel[r] = CR_SEL_BLOCKS;
 }
 
@@ -588,7 +615,9 @@ static cr_status select_configure() {
   static PerDeviceOnce configured;
   return once_per_device(configured, [] {
     const int most = (int)select_smem_bytes(kMaxSelectCount);
-    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<kSelThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)select_smem_bytes(kShortRow, kShortCap)));
+    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_cluster_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_cluster_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
@@ -615,7 +644,12 @@ cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
       CR_LAUNCH_CHECK("qsa_topk_cluster_kernel");
       continue;
     }
-    CR_CUDA(launch_pdl(qsa_topk_kernel, dim3(Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
+    if ((long long)Rmax * n <= 2 * sm_count())                      // all rows are on the chip at once
+      CR_CUDA(launch_pdl(qsa_topk_kernel<kSelThreads>, dim3(Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
+    else if (nb_max <= kShortRow)
+      CR_CUDA(launch_pdl(qsa_topk_kernel<256>, dim3(Rmax, n), dim3(256), select_smem_bytes(nb_max, kShortCap), stream, P, nb_max));
+    else
+      CR_CUDA(launch_pdl(qsa_topk_kernel<512>, dim3(Rmax, n), dim3(512), select_smem_bytes(nb_max), stream, P, nb_max));
     CR_LAUNCH_CHECK("qsa_topk_kernel");
   }
   return CR_OK;

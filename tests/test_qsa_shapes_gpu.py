@@ -129,6 +129,39 @@ def test_selection_threshold_patterns(nb, pattern):
             np.testing.assert_array_equal(cs[r].cpu().numpy(), sc[r].cpu().numpy()[want])
 
 
+# more rows than the chip holds at 1,024 threads each: 256 threads a row up to 14,336 blocks, 512 above; a full list, lists that
+# overflow (few distinct scores, mostly zeros), rows read four elements at a time and singly
+@pytest.mark.parametrize("last_nb", [700, 3072, 3073, 14336, 14337, 17000])
+@pytest.mark.parametrize("pattern,pad", [("random", 0), ("random", 1), ("seven", 0), ("zeros", 3)])
+def test_selection_of_many_rows(last_nb, pattern, pad):
+    capi, layers, g, w = _weights(16)
+    R = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 9
+    gen = torch.Generator(device="cuda").manual_seed(last_nb)
+    pos0 = 4 * last_nb - R
+    s = layers.QsaSession(g, pos0 + R, max_rows=R)
+    s.sstride = last_nb + pad
+    s.scores = torch.zeros(R, s.sstride, device="cuda")
+    tiles = torch.randn(s.ik_pool.numel() // 4096, 128, 32, device="cuda", generator=gen)
+    if pattern == "seven":
+        tiles = tiles[:1, :, :7].repeat(tiles.shape[0], 1, 5)[:, :, :32].contiguous()
+    if pattern == "zeros":
+        tiles *= (torch.rand(tiles.shape[0], 1, 32, device="cuda", generator=gen) < 300 / last_nb)
+    s.ik_pool.copy_(tiles.flatten())
+    idx = torch.randn(R, 640, device="cuda", generator=gen)
+    z = torch.zeros(R, 16, 512, device="cuda")
+    args = layers.qsa_args(w, s, z, z, z, idx, z, pos0)
+    capi.check(capi.lib.cr_qsa_select(C.byref(g), C.byref(args), 1, None, 0, None))
+    sc, sel, nsel = s.scores.cpu().numpy(), s.sel.cpu().numpy(), s.nsel.cpu().numpy()
+    for r in range(0, R, 3):
+        nb = (pos0 + r + 1) // 4
+        if nb <= capi.SEL_BLOCKS:
+            assert nsel[r] == -1
+            continue
+        assert nsel[r] == 512
+        want = np.sort(np.lexsort((np.arange(nb), -sc[r, :nb].astype(np.float64)))[:512])
+        np.testing.assert_array_equal(sel[r], want)
+
+
 # scores of prefill parts: dense rows in front of scored ones, ragged row tiles, fewer visits than CTA pairs, runs of a pair
 # that cross into the next row tile
 @pytest.mark.parametrize("start,R", [(2040, 70), (2100, 17), (9003, 117), (33000, 65), (6001, 257), (20000, 700)])
