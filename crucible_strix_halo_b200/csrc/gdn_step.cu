@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
   float* pk = vs + P.rows * 128;                               // staged pending rows: keys | values, then (decay, beta)
   float* pg = pk + min(P.replay, kReplayChunk) * 256;
   pdl_release();
+  touch_params(a);
   pdl_wait();
 
   // ---- everything the pass reads is asked for: state (L2), raw rows and pending rows (shared memory)

@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_cons
   const bool scored = nb_all > CR_SEL_BLOCKS && a.R <= 4 * MT;
   // The first tile is asked into L2 while the kernel ahead still runs: a prefetch reads nothing that could be stale later.
   if (scored && l == 0 && first < last) umma::bulk_prefetch_l2(a.c.ik_pool + (size_t)first * 4096, 16384);
+  touch_params(a);
   pdl_wait();
   if (!scored) return;
   for (int i = t; i < 16 * MT * 64; i += 128) {        // pairs of dims: row m = 4 r + h of the span's normalised indexer queries

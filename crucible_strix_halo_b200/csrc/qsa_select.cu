@@ -81,8 +81,9 @@ __global__ void __launch_bounds__(256) qsa_score_kernel(const __grid_constant__ 
 template <int RT, bool RANGED>
 __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__ QsaParams P) {
   pdl_release();
-  pdl_wait();
   const cr_qsa_args& a = P.span[blockIdx.z];
+  touch_params(a);
+  pdl_wait();
   const int rg0 = blockIdx.y * RT;
   if (rg0 >= a.R) return;
   const int nr = min(RT, a.R - rg0);

@@ -432,8 +432,9 @@ template <int T>
 __global__ void __launch_bounds__(T, T == 1024 ? 2 : T == 512 ? 3 : 6) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
   extern __shared__ __align__(16) unsigned char raw[];
   pdl_release();
-  pdl_wait();
   const cr_qsa_args& a = P.span[blockIdx.y];
+  touch_params(a);
+  pdl_wait();
   const int r = blockIdx.x;
   if (r >= a.R) return;
   const int nb = (a.pos0 + r + 1) / 4;
@@ -488,10 +489,11 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
   __shared__ unsigned offer_s, max_s, count_s;                     // read by the other CTAs of the cluster
   __shared__ unsigned top4[128];
   pdl_release();
+  const cr_qsa_args& a = P.span[blockIdx.y];
+  touch_params(a);
   pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  const cr_qsa_args& a = P.span[blockIdx.y];
   const int r = blockIdx.x / 8, t = threadIdx.x, l = t & 31;
   if (r >= a.R) return;                                            // the same for the whole cluster
   const int nb = (a.pos0 + r + 1) / 4;
