@@ -26,11 +26,13 @@
 //                      after the first steps), writes P as fp16 into a K-major shared-memory tile, sums it.
 //   epilogue           all warps: O through shared memory to a warp per (row, head), / sum, optional un-gated context,
 //                      sigmoid gate, output format.
-// Bound: latency around the two S accumulators (S product 1,000 cycles, softmax of a step 2,300, P V 520; the tensor pipe
-// alone would take 1,550 cycles per step, a step takes 2,350).  What it took to get there from 3,750: instruction fetches
-// were a third of all stalls while the roles had long unrolled bodies (rolled loops), the visibility words sat in the K
-// loaders' path (2,600 cycles), a thread wrote a row of its own at the end (20 us per CTA, now 12).  2,048 rows at 30,720,
-// 24 heads: 406 + 28 us of output transform before, 350 us now with it.
+// Bound: the tensor pipe beside the traffic of shared memory (a step takes 2,060 cycles; its 20 MMAs alone 1,550, and the 160 KB
+// that the gathers, P and the operands move through shared memory 1,280).  What it took to get there from 3,750: instruction
+// fetches were a third of all stalls while the roles had long unrolled bodies (rolled loops), the visibility words sat in the K
+// loaders' path (2,600 cycles), a thread wrote a row of its own at the end (20 us per CTA, now 12), and an S accumulator was held
+// until the step's exponentials were done, so that the next product into it waited 2,300 cycles for 64 logits that registers
+// hold (2,350 cycles a step; what had spilled there was the rescaling of O, 32 columns at a time).  2,048 rows at 30,720, 24
+// heads: 406 + 28 us of output transform, 353 us with it, 320 us now.
 // q and P are fp16 with fp32 accumulation, the reference's prefill numerics (prefill_qsa_union.h:680-684).
 // Every wait is bounded; a wait that gives up raises the status word and the CTA runs to its end.
 #include <climits>
@@ -171,6 +173,11 @@ __global__ void __launch_bounds__(kUbThreads) qsa_union_build_kernel(const __gri
 __device__ __forceinline__ void fl_cp_async16(unsigned d, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 __device__ __forceinline__ void fl_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(umma::smem_u32(bar)) : "memory");
@@ -384,22 +391,24 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
       const unsigned see0 = r < 16 ? seen_s[j % kFlSeen][r][0] : 0u, see1 = r < 16 ? seen_s[j % kFlSeen][r][1] : 0u;
       warp_wait(&sFull[s], (j >> 1) & 1);
       umma::fence_after_sync();
-      // S is read from tensor memory twice, 32 keys at a time in rolled loops: for the maximum, then for the exponentials.
-      // The roles of this kernel run different code on the same schedulers and evict each other's instructions; with 64
-      // keys unrolled (and unrolled loaders) a third of all stalls were instruction fetches.
-      float tmax = -INFINITY;
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        const unsigned see = h ? see1 : see0;
-        float sv[32], t1 = -INFINITY;
-        umma::tmem_ld32(umma::tmem_addr(tm, w, kColS + 64 * s + 32 * h), sv);
+      // The step's 64 logits are read at once and the accumulator is free again: the product of step j + 2 runs beside the rest.
+      float sv[kFlKeys];
+      umma::tmem_ld64(umma::tmem_addr(tm, w, kColS + 64 * s), sv);
+      umma::fence_before_sync();
+      __syncwarp();
+      if (l == 0) umma::mbar_arrive_relaxed(&sEmpty[s]);
+      float tmax = -INFINITY, t1 = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          tmax = fmaxf(tmax, (see >> c) & 1u ? sv[c] : -INFINITY);
-          t1 = fmaxf(t1, (see >> (c + 1)) & 1u ? sv[c + 1] : -INFINITY);
-        }
-        tmax = fmaxf(tmax, t1);
+      for (int c = 0; c < 32; ++c) {                                    // keys that the row does not see drop out
+        sv[c] = (see0 >> c) & 1u ? sv[c] : -INFINITY;
+        sv[32 + c] = (see1 >> c) & 1u ? sv[32 + c] : -INFINITY;
       }
+#pragma unroll
+      for (int c = 0; c < kFlKeys; c += 4) {
+        tmax = max3(tmax, sv[c], sv[c + 1]);
+        t1 = max3(t1, sv[c + 2], sv[c + 3]);
+      }
+      tmax = fmaxf(tmax, t1);
       tmax *= kScale;
       float ref = -INFINITY;                                            // the lane's reference after step j - 1
       if (j > 0) {
@@ -417,47 +426,34 @@ __global__ void __launch_bounds__(kFlThreads, 1) qsa_flash_tc_kernel(const __gri
         warp_wait(&pvDone[(j - 1) % kFlStages], ((j - 1) / kFlStages) & 1);
         umma::fence_after_sync();
 #pragma unroll 1
-        for (int c8 = 0; c8 < 8; ++c8) {
-          float o[32];
-          umma::tmem_ld32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+        for (int c16 = 0; c16 < 16; ++c16) {                             // 16 columns at a time beside the 64 logits
+          float o[16];
+          umma::tmem_ld16(umma::tmem_addr(tm, w, kColO + 16 * c16), o);
 #pragma unroll
-          for (int c = 0; c < 32; ++c) o[c] *= factor;
-          umma::tmem_st32(umma::tmem_addr(tm, w, kColO + 32 * c8), o);
+          for (int c = 0; c < 16; ++c) o[c] *= factor;
+          umma::tmem_st16(umma::tmem_addr(tm, w, kColO + 16 * c16), o);
         }
         umma::tmem_st_wait();
       }
       if (j >= 2) warp_wait(&pvDone[(j - 2) % kFlStages], ((j - 2) / kFlStages) & 1);   // the MMAs of step j - 2 have read this P buffer
       unsigned char* pd = Ps + s * kFlPBytes;
       const float sub = m_ref == -INFINITY ? 0.f : m_ref;               // nothing visible yet: every key drops out
-      float add = 0.f;
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        const unsigned see = h ? see1 : see0;
-        float sv[32];
-        umma::tmem_ld32(umma::tmem_addr(tm, w, kColS + 64 * s + 32 * h), sv);
+      f2 add = 0ull;
 #pragma unroll
-        for (int kc8 = 0; kc8 < 4; ++kc8) {
-          unsigned pk[4];
+      for (int kc8 = 0; kc8 < kFlKeys / 8; ++kc8) {
+        unsigned pk[4];
 #pragma unroll
-          for (int q2 = 0; q2 < 4; ++q2) {
-            float p[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int c = kc8 * 8 + 2 * q2 + i;
-              asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p[i]) : "f"(fmaf(sv[c], kScale, -sub)));
-              p[i] = (see >> c) & 1u ? p[i] : 0.f;                     // keys the row does not see drop out
-            }
-            add += p[0] + p[1];
-            const __half2 hp = __floats2half2_rn(p[0], p[1]);
-            pk[q2] = *reinterpret_cast<const unsigned*>(&hp);
-          }
-          *reinterpret_cast<uint4*>(pd + ((size_t)(4 * h + kc8) * 128 + m) * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        for (int q2 = 0; q2 < 4; ++q2) {
+          const int c = kc8 * 8 + 2 * q2;
+          const float p0 = ex2_ftz(fmaf(sv[c], kScale, -sub)), p1 = ex2_ftz(fmaf(sv[c + 1], kScale, -sub));
+          add = add2(add, pack2(p0, p1));
+          const __half2 hp = __floats2half2_rn(p0, p1);
+          pk[q2] = *reinterpret_cast<const unsigned*>(&hp);
         }
+        *reinterpret_cast<uint4*>(pd + ((size_t)kc8 * 128 + m) * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
-      umma::fence_before_sync();
-      __syncwarp();
-      if (l == 0) umma::mbar_arrive_relaxed(&sEmpty[s]);
-      lsum += add;
+      const float2 both = unpack2(add);
+      lsum += both.x + both.y;
       umma::fence_async_smem();
       umma::fence_before_sync();
       __syncwarp();
