@@ -474,20 +474,24 @@ __global__ void __launch_bounds__(64) qsa_merge_kernel(const __grid_constant__ Q
   emit_group(a, P.Hq, r, h, c, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv), gate, fmt);
 }
 
-// Streams of a unit.  The pass holds SMs x kStreams streams at a time; with s streams per unit it takes
-// ceil(units x s / that) waves of (longest unit's tiles / s + the set-up and merge of a stream, worth about four tiles).
+// Streams of a unit.  The pass holds `fits[k]` clusters of 2^k CTAs at a time (an SM each); with s streams per unit it takes
+// that many waves of (longest unit's tiles / s + the set-up and merge of a stream, worth about four tiles).
 // One stream per unit is the cheapest form but leaves SMs idle when units are few and ends in a ragged wave when they
-// are not many; a cluster (s above one CTA's streams) pays only while SMs would idle otherwise.
-static AttnShape attn_shape(int streams, long long units, int tiles, int sms) {
+// are not many; a cluster (s above one CTA's streams) pays only while SMs would idle otherwise.  A cluster lies in one
+// group of SMs, so that fewer fit than the SMs would hold (15 of eight CTAs where 148 SMs count 18), and one cluster too many doubles
+// the time of a step: 16 units (eight sessions of one row) 18.5 us of 16 heads and 26.6 of 24 by the count of SMs, 12.5 and 20.6 by
+// what fits; 36 units 23.7 and 40.2, now 17.8 and 32.8.
+static AttnShape attn_shape(int streams, long long units, int tiles, const int (&fits)[4]) {
   AttnShape best{1, 1};
   double best_cost = 1e30;
   for (int spu = 1; spu <= streams; ++spu) {
     if (streams % spu) continue;
-    for (int cl = 1; cl <= 8; cl <<= 1) {
-      if (cl > 1 && (spu != streams || units * cl > sms)) break;
+    for (int k = 0; k < 4; ++k) {
+      const int cl = 1 << k;
+      if (cl > 1 && (spu != streams || units > fits[k])) break;
       if (spu * cl > 1 && spu * cl > tiles) break;
-      const long long ctas = cl > 1 ? units * cl : (units * spu + streams - 1) / streams;
-      const long long waves = (ctas + sms - 1) / sms;
+      const long long clusters = cl > 1 ? units : (units * spu + streams - 1) / streams;
+      const long long waves = (clusters + fits[k] - 1) / fits[k];
       const double cost = (double)waves * ((tiles + spu * cl - 1) / (spu * cl) + 4);
       if (cost < best_cost - 1e-9) { best_cost = cost; best = AttnShape{spu, cl}; }
     }
@@ -498,12 +502,26 @@ static AttnShape attn_shape(int streams, long long units, int tiles, int sms) {
 template <int NG, int HKV>
 static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long units, int tiles, float* partials, int p0, int p1, int fmt, cudaStream_t stream) {
   static PerDeviceOnce configured;
-  constexpr size_t smem = kAttnSmem<NG> + 12 * 256 * sizeof(float);   // + the merged unit of a cluster's CTA
-  if (cr_status st = once_per_device(configured, [] {
+  static int fits_on[64][4];                            // per device: clusters of 1, 2, 4 and 8 CTAs that run at once
+  constexpr size_t smem = kAttnSmem<NG> + 12 * 256 * sizeof(float);   // + the query heads of a CTA's unit, then its merged unit
+  int dev = 0;
+  CR_CUDA(cudaGetDevice(&dev));
+  CR_REQUIRE(dev >= 0 && dev < 64, "qsa attention: device %d is out of range", dev);
+  if (cr_status st = once_per_device(configured, [dev] {
         CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG, HKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        fits_on[dev][0] = sm_count();
+        for (int k = 1; k < 4; ++k) {
+          cudaLaunchConfig_t cfg = {};
+          cfg.gridDim = dim3(sm_count() >> k << k); cfg.blockDim = dim3(kAttnThreads<NG>); cfg.dynamicSmemBytes = smem;
+          cudaLaunchAttribute attr;
+          attr.id = cudaLaunchAttributeClusterDimension;
+          attr.val.clusterDim.x = 1 << k; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+          cfg.attrs = &attr; cfg.numAttrs = 1;
+          CR_CUDA(cudaOccupancyMaxActiveClusters(&fits_on[dev][k], qsa_attn_kernel<NG, HKV>, &cfg));
+        }
         return CR_OK;
       })) return st;
-  const AttnShape shape = attn_shape(kStreams<NG>, units, tiles, sm_count());
+  const AttnShape shape = attn_shape(kStreams<NG>, units, tiles, fits_on[dev]);
   const int upc = kStreams<NG> / shape.spu;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(shape.cluster * ((Rmax * P.Hkv + upc - 1) / upc), 1, n);

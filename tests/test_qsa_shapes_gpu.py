@@ -43,7 +43,7 @@ def _attend(q, k, v, sel, nsel, pos):
 # units = sessions x rows x 2 KV heads; 8 streams a CTA (16 heads) or 6 (18 and 24 heads): one position, fewer tiles than
 # streams, clusters of 8 / 4 / 2, one CTA per unit, several units per CTA, ragged last CTA
 @pytest.mark.parametrize("Hq,sessions,rows,ctx", [(16, 1, 1, 1), (16, 1, 1, 37), (16, 1, 1, 1501), (16, 1, 2, 2052), (16, 4, 1, 9003), (16, 7, 2, 2600),
-                                                   (16, 8, 9, 3001), (16, 17, 13, 2301), (24, 1, 4, 2051), (24, 3, 1, 700), (18, 5, 5, 2301), (24, 9, 13, 2301)])
+                                                   (16, 8, 9, 3001), (16, 17, 13, 2301), (24, 1, 4, 2051), (24, 3, 1, 700), (18, 5, 5, 2301), (24, 9, 13, 2301), (16, 8, 1, 9003), (24, 2, 4, 9003), (16, 15, 1, 9003), (24, 9, 2, 9003), (16, 18, 1, 9003)])
 def test_attention_work_splits(Hq, sessions, rows, ctx):
     capi, layers, g, w = _weights(Hq)
     gen = torch.Generator(device="cuda").manual_seed(ctx + Hq)
