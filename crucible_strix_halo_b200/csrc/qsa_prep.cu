@@ -89,7 +89,7 @@ __device__ __forceinline__ bool raw_kept(const cr_qsa_args& a, int r) { return a
 __device__ __forceinline__ bool raw_after_pool(const cr_qsa_args& a, int r) {
   if (a.c.raw_slots == 0 || a.pos0 % 4 == 0 || (a.pos0 + a.R) / 4 == a.pos0 / 4) return false;
   for (int p = a.pos0 / 4 * 4; p < a.pos0; ++p)
-    if (p % a.c.raw_slots == (a.pos0 + r) % a.c.raw_slots) return true;
+    if ((a.pos0 + r - p) % a.c.raw_slots == 0) return true;
   return false;
 }
 
@@ -116,9 +116,13 @@ __device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
   for (int i = 0; i < 4; ++i) a.c.ik_pool[pool_offset(b, 32 * i + l)] = x[i];
   if (b == a.pos0 / 4 && a.c.raw_slots != 0) {            // the ring rows that had to wait for the reads above
     __syncwarp();
-    for (int r = max(0, a.R - a.c.raw_slots); r < a.R; ++r)
-      if (raw_after_pool(a, r))
+    for (int r0 = max(0, a.R - a.c.raw_slots); r0 < a.R; r0 += 32) {       // a lane looks at a row: at most three have to be written
+      unsigned rows = __ballot_sync(0xffffffffu, r0 + l < a.R && raw_after_pool(a, r0 + l));
+      for (; rows; rows &= rows - 1) {
+        const int r = r0 + __ffs(rows) - 1;
         st4<VEC>(a.c.ik_raw + raw_offset(a.c.raw_slots, a.pos0 + r, 4 * l), ld4<VEC>(a.idx + (size_t)r * 640 + 512 + 4 * l));
+      }
+    }
   }
 }
 
@@ -134,7 +138,8 @@ __device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
 // (128-bit loads, shuffle reduction, no barrier but the one behind the row's 32 cosines and sines, which every unit of the
 // row shares: angles past 105,615 take cosf's long reduction).  A step gives every unit a warp of its own (UPW = 1); a part
 // takes a row per CTA with all loads of a warp issued first (UPW = 5).  2,048 rows at 262,144 positions: 98.8 us as one
-// CTA per (row, unit), 28 us now (4.9 TB/s).
+// CTA per (row, unit), 28 us now (4.9 TB/s).  With a compact ring the warp that pools a call's first block looked at sixteen rows one by
+// one, two divisions for each of three positions: 10.0 us for 117 rows where a full raw cache took 3.9; a lane per row now.
 template <int UPW, bool VEC>
 __global__ void __launch_bounds__(256) qsa_prep_kernel(const __grid_constant__ QsaParams P, int u0, __half* q_hi, int q_skip, int queries_only, int mark_dense) {
   pdl_release();
