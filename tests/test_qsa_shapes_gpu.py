@@ -162,6 +162,32 @@ def test_selection_of_many_rows(last_nb, pattern, pad):
         np.testing.assert_array_equal(sel[r], want)
 
 
+# A compact raw ring beside a full raw cache: calls that start inside a block, whose pooled mean reads ring slots that the call's own
+# rows take, fewer and more rows than slots.  The pooled keys and the newest raw keys are the same, bit for bit.
+@pytest.mark.parametrize("slots", [16, 37])
+@pytest.mark.parametrize("start,R", [(0, 1), (1, 3), (5, 15), (6, 14), (7, 1), (7, 16), (30, 17), (35, 33), (1501, 117), (2047, 38)])
+def test_compact_ring_matches_full_cache(slots, start, R):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(start)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    full, ring = layers.QsaSession(g, start + R, max_rows=R), layers.QsaSession(g, start + R, max_rows=R, raw_slots=slots)
+    raw = rn(start + R, 128)
+    old = full.ik_raw.view(-1, 128)
+    old[:start] = raw[:start]
+    for p in range(max(0, start - slots), start):
+        ring.ik_raw.view(-1, 128)[p % slots] = raw[p]
+    q, k, v, idx = rn(R, g.q_heads, 512), rn(R, 512), rn(R, 512), rn(R, 640)
+    idx[:, 512:] = raw[start:]
+    outs = [layers.QsaPrefillPlan(w, R).run(s, q.clone(), k.clone(), v.clone(), idx.clone(), start) for s in (full, ring)]
+    done = torch.arange(start // 4, (start + R) // 4, device="cuda")                # blocks this call completes
+    for s in (full, ring):
+        assert torch.equal(s.ik_pool.view(-1, 128, 32)[done // 32, :, done % 32], full.ik_pool.view(-1, 128, 32)[done // 32, :, done % 32])
+    for p in range(max(start, start + R - slots), start + R):
+        assert torch.equal(ring.ik_raw.view(-1, 128)[p % slots], raw[p]) and torch.equal(old[p], raw[p])
+    if start == 0:
+        assert torch.equal(outs[0], outs[1])
+
+
 # scores of prefill parts: dense rows in front of scored ones, ragged row tiles, fewer visits than CTA pairs, runs of a pair
 # that cross into the next row tile
 @pytest.mark.parametrize("start,R", [(2040, 70), (2100, 17), (9003, 117), (33000, 65), (6001, 257), (20000, 700)])
