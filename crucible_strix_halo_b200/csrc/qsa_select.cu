@@ -76,6 +76,8 @@ __global__ void __launch_bounds__(256) qsa_score_kernel(const __grid_constant__ 
 // The four lanes that share a block group add their partial dots with two shuffles.
 // The pool passes through L2 as the first thing to be evicted: four sessions of 262,144 positions (134 MB, more than L2) had pushed
 // out the states, the rows and the code of the kernels around the scan: a step 75.4 -> 66.1 us, of which 4 in the attention.
+// Half a tile is asked for before the queries are staged and stays in flight: 60.0 -> 58.6 us for passes back to back.  (Asking the
+// tiles into L2 before the wait for the kernel ahead was slower: the prefetches come in with the ordinary policy.)
 // RANGED: only the blocks [P.b_lo, P.b_hi) are scored (a rank's own blocks).  A separate instantiation: with the range
 // tests in it the whole-row kernel measured 40 us instead of 29 for four 262,144-token rows.
 template <int RT, bool RANGED>
@@ -92,6 +94,17 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
   const int nb_hi = RANGED ? min(nb_all, P.b_hi) : nb_all;
   const int t = threadIdx.x, w = t >> 5, l = t & 31;
   __shared__ float4 iqs[128][RT];
+  const int tile = (RANGED ? P.b_lo / 32 : 0) + blockIdx.x * 8 + w;
+  const bool live = tile * 32 < nb_hi;
+  const int bq = (l & 7) * 4, dl = l >> 3;
+  const float* pt = a.c.ik_pool + (size_t)tile * 4096 + dl * 32 + bq;
+  const uint64_t policy = evict_first_policy();
+  float4 key[2][8];                           // a quarter of the tile; the first two are in flight while the queries are staged
+  auto fetch = [&](float4 (&k)[8], int it0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = load_stream4(pt + (it0 + j) * 128, policy);
+  };
+  if (live) { fetch(key[0], 0); fetch(key[1], 8); }
   for (int i = t; i < 128 * RT; i += 256) {
     const int d = i / RT, r = i % RT;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -102,11 +115,7 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
     iqs[d][r] = v;
   }
   __syncthreads();
-  const int tile = (RANGED ? P.b_lo / 32 : 0) + blockIdx.x * 8 + w;
-  if (tile * 32 >= nb_hi) return;
-  const int bq = (l & 7) * 4, dl = l >> 3;
-  const float* pt = a.c.ik_pool + (size_t)tile * 4096 + dl * 32 + bq;
-  const uint64_t policy = evict_first_policy();
+  if (!live) return;
   float acc[RT][4][4];                        // [row][block][head]
 #pragma unroll
   for (int r = 0; r < RT; ++r)
@@ -114,12 +123,10 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
     for (int b = 0; b < 4; ++b) acc[r][b][0] = acc[r][b][1] = acc[r][b][2] = acc[r][b][3] = 0.f;
 #pragma unroll
   for (int it0 = 0; it0 < 32; it0 += 8) {
-    float4 key[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) key[j] = load_stream4(pt + (it0 + j) * 128, policy);
+    float4 (&k)[8] = key[(it0 >> 3) & 1];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float kb[4] = {key[j].x, key[j].y, key[j].z, key[j].w};
+      const float kb[4] = {k[j].x, k[j].y, k[j].z, k[j].w};
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
         const float4 q = iqs[(it0 + j) * 4 + dl][r];
@@ -132,6 +139,7 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
         }
       }
     }
+    if (it0 + 16 < 32) fetch(k, it0 + 16);
   }
 #pragma unroll
   for (int r = 0; r < RT; ++r)
