@@ -3,14 +3,17 @@
 // (qsa_score4_kernel) and too short to fill the 128-row tiles of the tcgen05 kernel (qsa_score_tc.cu).
 //
 // The pool tile [128 dims][32 blocks] fp32 is, as it lies in HBM, the "column" operand of m16n8k16: a thread's B
-// fragment is pool[d][b] for four dims and one block, so every load instruction of a warp is four full 32-byte sectors
-// and nothing is transposed or staged.  Rows of the product are (row, indexer head) pairs, m = 4 r + h, so the four
-// heads of a row sit in four neighbouring lanes and relu + sum is two shuffles.  Queries and pool values are split
+// fragments are pool[d][b] for four dims and, as columns of four products, four blocks, so every load instruction of a warp is
+// four full lines and nothing is transposed or staged.  Rows of the product are (row, indexer head) pairs, m = 4 r + h, so the
+// four heads of a row sit in four neighbouring lanes and relu + sum is two exchanges.  Queries and pool values are split
 // into fp16 head + remainder (hi hi + lo hi + hi lo, fp32 accumulation): scores agree with fp32 dot products to 1e-5.
-// One warp owns whole tiles and walks them in steps of 16 dims x 16 blocks; the loads of three steps are in flight
-// ahead of the one that multiplies.
+// One warp owns whole tiles and walks them in steps of 16 dims; the loads of three steps are in flight ahead of the one
+// that multiplies, the first ones while the queries are staged.
+//
+// Bound: latency with ten to twelve warps on an SM (tensor pipe 49 %, shared memory and L1 56 % busy).  With half a tile a step in
+// 4-byte loads (128 of four lines and 96 ldmatrix a tile) and four tiles to a warp whatever their number, 8 sessions x 9 rows
+// at 131,072 took 52 us and one session x 4 rows at 32,003 (16 CTAs) 14.4; 37 and 5.5 us now.
 #include "qsa.cuh"
-#include "umma.cuh"
 
 namespace cr {
 
@@ -45,11 +48,20 @@ __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_cons
   const int tiles = (nb_all + 31) / 32;
   const int first = (blockIdx.x * 4 + w) * per_warp, last = min(first + per_warp, tiles);
   const bool scored = nb_all > CR_SEL_BLOCKS && a.R <= 4 * MT;
-  // The first tile is asked into L2 while the kernel ahead still runs: a prefetch reads nothing that could be stale later.
-  if (scored && l == 0 && first < last) umma::bulk_prefetch_l2(a.c.ik_pool + (size_t)first * 4096, 16384);
   touch_params(a);
   pdl_wait();
   if (!scored) return;
+  // A step is 16 dims of a whole tile: this thread's four 16-byte loads are the dims 16 ks + 2 tq + {0, 1, 8, 9} of the blocks
+  // 4 g .. 4 g + 3, and block 4 g + nt is column g of product nt.  Three steps are in flight ahead of the one in use.
+  const int total = (last - first) * 8;
+  const float* pt = a.c.ik_pool + (size_t)first * 4096 + 2 * tq * 32 + 4 * g;
+  auto fetch = [&](float4 (&v)[4], int step) {
+    const float* p = pt + (size_t)step * 512;          // tiles lie back to back
+    v[0] = __ldcg(reinterpret_cast<const float4*>(p)); v[1] = __ldcg(reinterpret_cast<const float4*>(p + 32));
+    v[2] = __ldcg(reinterpret_cast<const float4*>(p + 256)); v[3] = __ldcg(reinterpret_cast<const float4*>(p + 288));
+  };
+  float4 ring[4][4];
+  if (first < last) { fetch(ring[0], 0); fetch(ring[1], 1); fetch(ring[2], 2); }   // in flight while the queries are staged; total >= 8
   for (int i = t; i < 16 * MT * 64; i += 128) {        // pairs of dims: row m = 4 r + h of the span's normalised indexer queries
     const int m = i >> 6, d = (i & 63) * 2, r = m >> 2, h = m & 3;
     float2 v = make_float2(0.f, 0.f);
@@ -61,17 +73,6 @@ __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_cons
   }
   __syncthreads();
   if (first >= last) return;
-  // A step is 16 dims of a whole tile: this thread's four 16-byte loads are the dims 16 ks + 2 tq + {0, 1, 8, 9} of the blocks
-  // 4 g .. 4 g + 3, and block 4 g + nt is column g of product nt.  Three steps are in flight ahead of the one in use.
-  const int total = (last - first) * 8;
-  const float* pt = a.c.ik_pool + (size_t)first * 4096 + 2 * tq * 32 + 4 * g;
-  auto fetch = [&](float4 (&v)[4], int step) {
-    const float* p = pt + (size_t)step * 512;          // tiles lie back to back
-    v[0] = __ldcg(reinterpret_cast<const float4*>(p)); v[1] = __ldcg(reinterpret_cast<const float4*>(p + 32));
-    v[2] = __ldcg(reinterpret_cast<const float4*>(p + 256)); v[3] = __ldcg(reinterpret_cast<const float4*>(p + 288));
-  };
-  float4 ring[4][4];
-  fetch(ring[0], 0); fetch(ring[1], 1); fetch(ring[2], 2);          // total >= 8
   for (int s0 = 0; s0 < total; s0 += 8) {
     float acc[MT][4][4];
 #pragma unroll

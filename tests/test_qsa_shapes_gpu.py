@@ -162,6 +162,37 @@ def test_selection_of_many_rows(last_nb, pattern, pad):
         np.testing.assert_array_equal(sel[r], want)
 
 
+# scores of spans of 3 to 16 rows: every number of row quartets, ragged last tiles, several tiles to a warp (the longest), spans of
+# different length in a launch, a pool off the 16-byte boundary (scalar loads), score rows off it
+@pytest.mark.parametrize("starts,R,pad,shift", [([2050, 9003], 3, 0, 0), ([4096], 4, 1, 0), ([2300, 2041], 5, 0, 0), ([9003], 9, 2, 0), ([33001], 13, 0, 0),
+                                                ([6000], 16, 3, 0), ([262100, 200001], 4, 0, 0), ([9003], 6, 0, 1), ([9003], 12, 1, 3)])
+def test_span_scores(starts, R, pad, shift):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    spans, args, keep = [], (capi.QsaArgs * len(starts))(), []
+    for i, start in enumerate(starts):
+        s = layers.QsaSession(g, start + R, max_rows=R)
+        s.ik_pool = rn(s.ik_pool.numel() + 4)[shift:]
+        s.sstride = (start + R) // 4 + pad
+        s.scores = torch.full((R, s.sstride), -7.0, device="cuda")
+        idx, z = rn(R, 640), torch.zeros(R, 16, 512, device="cuda")
+        args[i] = layers.qsa_args(w, s, z, z, z, idx, z, start)
+        spans.append((s, idx, start))
+        keep.append(z)
+    capi.check(capi.lib.cr_qsa_select(C.byref(g), args, len(starts), None, 0, None))
+    for s, idx, start in spans:
+        nb_all = (start + R) // 4
+        tiles = s.ik_pool[:s.ik_pool.numel() // 4096 * 4096].view(-1, 128, 32).double()
+        pool = tiles.transpose(1, 2).reshape(-1, 128)[:nb_all]
+        want = torch.relu(torch.einsum("rhd,bd->rhb", idx[:, :512].view(R, 4, 128).double(), pool)).sum(1) / 128 ** 0.5
+        for r in range(R):
+            nb = (start + r + 1) // 4
+            if nb > capi.SEL_BLOCKS:
+                assert (s.scores[r, :nb].double() - want[r, :nb]).abs().max().item() < 2e-4, r
+                assert (s.scores[r, nb:] == -7.0).all(), r                          # nothing past a row's blocks
+
+
 # A compact raw ring beside a full raw cache: calls that start inside a block, whose pooled mean reads ring slots that the call's own
 # rows take, fewer and more rows than slots.  The pooled keys and the newest raw keys are the same, bit for bit.
 @pytest.mark.parametrize("slots", [16, 37])
