@@ -18,7 +18,7 @@
 // heads, state in L2 / in HBM: 6.8 / 9.2 us in that first form, 8.6 / 9.1 on a CTA per head, which pulls 64 KB of state, 6.6 / 7.1
 // as clusters of four.  4 sessions x 1 row: 9.8 / 12.9, now 8.8 / 10.1.  (Plain launches; chained ones take 0.5 to 0.8 less.)
 #include <cooperative_groups.h>
-#include "common.cuh"
+#include "gdn_prefill.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -33,7 +33,11 @@ struct GdnStepParams {
   cr_gdn_args span[kMaxSpans];
   int Hv, Hk, hidden, pend_rows, fmt;
   int rows, replay;                                    // most of any span: the shared-memory layout
+  const void* logits;                                  // rows of a prefill call: [R][2 Hv] a and b logits in the place of x and ab
 };
+// What a pass reads: the rows of a step (fp32 projections, a and b from dot products with x), or those of a short prefill call
+// (projections and logits in fp32 or bf16).
+enum StepInput { kStepRowsIn, kPrefillF32, kPrefillBf16 };
 
 // Floats of dynamic shared memory: raw rows with halo, q, k and v rows (the readout replaces v), staged pending rows.
 __host__ __device__ constexpr int step_smem_floats(int rows, int replay) {
@@ -48,7 +52,7 @@ __device__ __forceinline__ void step_cp(float* dst, const float* src, bool valid
 }
 
 // A head is a cluster of CL CTAs (grid x: CL per head); CTA k has 128 / CL of its value columns, NC of them per lane.
-template <int CL>
+template <int CL, int IN>
 __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_constant__ GdnStepParams P) {
   constexpr int NC = CL == 1 ? 4 : 2, kWarpCols = 4 * NC, kOwners = 128 / CL / kWarpCols;   // columns of a lane, of a warp; warps that own columns
   extern __shared__ __align__(16) float step_sm[];
@@ -67,6 +71,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
   float* vs = ks + P.rows * 128;                               // a column's y replaces its v once that has been read
   float* pk = vs + P.rows * 128;                               // staged pending rows: keys | values, then (decay, beta)
   float* pg = pk + min(P.replay, kReplayChunk) * 256;
+  constexpr bool BF = IN == kPrefillBf16;
   pdl_release();
   touch_params(a);
   pdl_wait();
@@ -86,6 +91,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
     const int per = vec ? kRawCols / 4 : kRawCols;
     for (int rr = w; rr < R + 3; rr += kStepWarps) {
       const int p = a.pos0 + rr - 3;
+      if (BF && rr >= 3) {
+        for (int c = l; c < kRawCols; c += 32)
+          raw[rr * kRawCols + c] = load_in<BF>(a.qkv, (long long)(rr - 3) * C + (c < 128 ? kh * 128 + c : (c < 256 ? KW + kh * 128 + c - 128 : 2 * KW + h * 128 + c - 256)));
+        continue;
+      }
       const float* row = rr >= 3 ? qkv + (size_t)(rr - 3) * C : a.hist + (size_t)(p & 15) * C;
       for (int i = l; i < per; i += 32) {
         const int c = vec ? 4 * i : i;
@@ -106,7 +116,10 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
 
   // ---- a / b dot products: all threads on one row, or four groups of 64 threads on every fourth row
   const int groups = R == 1 ? 1 : 4, lanes = kStepThreads / groups, grp = t / lanes;
-  {
+  float la = 0.f, lb = 0.f;                                    // a prefill call brings them along: row t
+  if (IN != kStepRowsIn) {
+    if (t < R) { la = load_in<BF>(P.logits, (long long)t * 2 * P.Hv + h); lb = load_in<BF>(P.logits, (long long)t * 2 * P.Hv + P.Hv + h); }
+  } else {
     constexpr int kMost = (kStepRows + 3) / 4;                 // rows of a group
     f2 pa[kMost], pb[kMost];
 #pragma unroll
@@ -271,9 +284,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
     *row = make_float4(x.x * sc, x.y * sc, x.z * sc, x.w * sc);
   }
   if (t < R) {
-    float pa = 0.f, pb = 0.f;
-    const int per = kStepWarps / groups, w0 = R == 1 ? 0 : (t & 3) * per;
-    for (int k = w0; k < w0 + per; ++k) { pa += ab_warp[k][t][0]; pb += ab_warp[k][t][1]; }
+    float pa = la, pb = lb;
+    if (IN == kStepRowsIn) {
+      const int per = kStepWarps / groups, w0 = R == 1 ? 0 : (t & 3) * per;
+      for (int k = w0; k < w0 + per; ++k) { pa += ab_warp[k][t][0]; pb += ab_warp[k][t][1]; }
+    }
     const float sp = pa + a.dt_bias[h];
     const float softplus = sp > 20.f ? sp : log1pf(expf(sp));
     dec[t] = expf(-__expf(a.A_log[h]) * softplus);
@@ -285,7 +300,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
   for (int k = 0; k < kGateRows; ++k) {
     const int r = rank + CL * (w + kStepWarps * k);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) z[k][i] = r < R ? reinterpret_cast<const float*>(a.z)[(size_t)r * VW + h * 128 + 4 * l + i] : 0.f;
+    for (int i = 0; i < 4; ++i) z[k][i] = r < R ? load_in<BF>(a.z, (long long)r * VW + h * 128 + 4 * l + i) : 0.f;
   }
   __syncthreads();
 
@@ -387,31 +402,56 @@ static cudaLaunchConfig_t step_config(dim3 grid, size_t smem, cudaStream_t strea
   return cfg;
 }
 // Heads whose clusters of CL CTAs, an SM to each, the device holds at once (looked up once per device).
-template <int CL>
+template <int CL, int IN>
 static cr_status step_heads(int& heads) {
   static PerDeviceOnce looked_up;
   static int table[64];
   int dev = 0;
   CR_CUDA(cudaGetDevice(&dev));
   if (cr_status st = once_per_device(looked_up, [dev] {
-        CR_CUDA(cudaFuncSetAttribute(gdn_step_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAloneSmem));
+        CR_CUDA(cudaFuncSetAttribute(gdn_step_kernel<CL, IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAloneSmem));
         cudaLaunchAttribute attr[2];
         cudaLaunchConfig_t cfg = step_config<CL>(dim3(CL), kAloneSmem, nullptr, attr);
-        if (CL > 1) CR_CUDA(cudaOccupancyMaxActiveClusters(&table[dev & 63], gdn_step_kernel<CL>, &cfg));
+        if (CL > 1) CR_CUDA(cudaOccupancyMaxActiveClusters(&table[dev & 63], gdn_step_kernel<CL, IN>, &cfg));
         else table[dev & 63] = sm_count();
         return CR_OK;
       })) return st;
   heads = table[dev & 63];
   return CR_OK;
 }
-template <int CL>
+template <int CL, int IN>
 static cr_status step_launch(const GdnStepParams& P, int n, bool alone, cudaStream_t stream) {
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = step_config<CL>(dim3(P.Hv * CL, n), alone ? kAloneSmem : step_smem_floats(P.rows, P.replay) * sizeof(float), stream, attr);
   if (pdl_enabled()) { attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1; }
-  CR_CUDA(cudaLaunchKernelEx(&cfg, gdn_step_kernel<CL>, P));
+  CR_CUDA(cudaLaunchKernelEx(&cfg, gdn_step_kernel<CL, IN>, P));
   CR_LAUNCH_CHECK("gdn_step_kernel");
   return CR_OK;
+}
+
+// Few heads leave SMs idle: a head is spread over as many CTAs as there are SMs for, all clusters at once.  States in HBM, 1 / 9
+// rows: 32 heads 9.1 / 21.2 us on one CTA each, 8.0 / 18.3 on two, 7.1 / 17.3 on four; 64 heads 9.3 / 21.7, 8.4 / 18.9, 8.6 / 19.8;
+// 96 heads 9.7 / 22.1, 10.8 / 22.5: once two CTAs share an SM the work that a head's CTAs repeat (rows, dot products) costs more.
+template <int IN>
+static cr_status step_dispatch(const GdnStepParams& P, int n, cudaStream_t stream) {
+  int fit4, fit2, fit1;
+  if (cr_status st = step_heads<4, IN>(fit4)) return st;
+  if (cr_status st = step_heads<2, IN>(fit2)) return st;
+  if (cr_status st = step_heads<1, IN>(fit1)) return st;
+  const int heads = n * P.Hv;
+  const auto launch = heads <= fit4 ? step_launch<4, IN> : (heads <= fit2 ? step_launch<2, IN> : step_launch<1, IN>);
+  return launch(P, n, heads <= fit1, stream);
+}
+
+// The rows of a prefill call of at most CR_MAX_STEP_ROWS rows through the recurrence: what bounds a call of one chunk is the chain of
+// its phases, whatever its rows.
+cr_status gdn_few_rows(const cr_geometry* g, const cr_gdn_args& a, const void* logits, bool bf16_in, cr_out_format fmt, cudaStream_t stream) {
+  GdnStepParams P;
+  P.span[0] = a;
+  P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.hidden = g->hidden; P.pend_rows = 1; P.fmt = (int)fmt;
+  P.rows = a.R; P.replay = 0;
+  P.logits = logits;
+  return bf16_in ? step_dispatch<kPrefillBf16>(P, 1, stream) : step_dispatch<kPrefillF32>(P, 1, stream);
 }
 
 }  // namespace cr
@@ -443,20 +483,12 @@ extern "C" cr_status cr_gdn_step(const cr_geometry* g, const cr_gdn_args* spans,
     for (int s = 0; s < n; ++s) P.span[s] = spans[s0 + s];
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.hidden = g->hidden; P.pend_rows = pend_rows; P.fmt = (int)fmt;
     P.rows = P.replay = 0;
+    P.logits = nullptr;
     for (int s = 0; s < n; ++s) {
       P.rows = P.rows > P.span[s].R ? P.rows : P.span[s].R;
       P.replay = P.replay > P.span[s].replay ? P.replay : P.span[s].replay;
     }
-    // Few heads leave SMs idle: a head is spread over as many CTAs as there are SMs for, all clusters at once.  States in HBM, 1 / 9
-    // rows: 32 heads 9.1 / 21.2 us on one CTA each, 8.0 / 18.3 on two, 7.1 / 17.3 on four; 64 heads 9.3 / 21.7, 8.4 / 18.9, 8.6 / 19.8;
-    // 96 heads 9.7 / 22.1, 10.8 / 22.5: once two CTAs share an SM the work that a head's CTAs repeat (rows, dot products) costs more.
-    int fit4, fit2, fit1;
-    if (cr_status st = step_heads<4>(fit4)) return st;
-    if (cr_status st = step_heads<2>(fit2)) return st;
-    if (cr_status st = step_heads<1>(fit1)) return st;
-    const int heads = n * P.Hv;
-    const auto launch = heads <= fit4 ? step_launch<4> : (heads <= fit2 ? step_launch<2> : step_launch<1>);
-    if (cr_status st = launch(P, n, heads <= fit1, (cudaStream_t)stream)) return st;
+    if (cr_status st = step_dispatch<kStepRowsIn>(P, n, (cudaStream_t)stream)) return st;
   }
   return CR_OK;
 }

@@ -1,4 +1,6 @@
 """Kernels outside the QSA path at the sizes where their work split changes."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -69,6 +71,50 @@ def test_gdn_chunk_prefill_splits(geometry, bf16, R):
         ring[(pos0 + r) % 16] = qkv[r].float()
     assert torch.equal(h0, ring) and torch.equal(h1, ring)
     assert (o1 - o0).abs().max() < 4e-3 * o0.abs().max() and (s1 - s0).abs().max() < 4e-3 * s0.abs().max()
+
+
+# Calls of a few rows run through the step's recurrence, 14 to 26 rows in two launches: the serial fp32 scan over the same rows differs
+# by the order of fp32 additions only (128 terms, 26 rows: a few 1e-6), which the output format then rounds.  Positions without a
+# full halo, every row format, the packed layout, states off the 16-byte boundary (which take the chunked scan, tf32).
+@pytest.mark.parametrize("heads", [(16, 32), (16, 48), (4, 4)])
+@pytest.mark.parametrize("R,pos0", [(1, 0), (1, 3), (2, 1), (4, 100), (12, 5), (13, 2), (14, 0), (17, 100), (25, 1), (26, 77), (27, 9)])
+@pytest.mark.parametrize("bf16,fmt,offset", [(False, "f32", 0), (True, "bf16", 0), (True, "exl3", 0), (False, "packed", 0), (False, "f32", 1)])
+def test_gdn_prefill_of_few_rows(heads, R, pos0, bf16, fmt, offset):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, heads[1], heads[0])
+    gen = torch.Generator(device="cuda").manual_seed(100 * R + pos0)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    width, Hv = g.gdn_channels, g.gdn_vheads
+    dt = torch.bfloat16 if bf16 else torch.float32
+    w = layers.GdnWeights(g, rn(width, 4, std=0.5), rn(Hv) - 1, rn(Hv, std=0.5), 1 + rn(128, std=0.1), suh=1 + rn(Hv * 128, std=0.1))
+    qkv, z, ab = rn(R, width).to(dt), rn(R, Hv * 128).to(dt), rn(R, 2 * Hv).to(dt)
+    hist, state = rn(16, width).bfloat16().float(), rn(Hv * 16384, std=0.1)
+    code = {"f32": capi.OUT_RAW_F32, "bf16": capi.OUT_RAW_BF16}.get(fmt, capi.OUT_EXL3_WHT)
+    got = []
+    for algo in (capi.GDN_SERIAL_F32, capi.GDN_CHUNK_TC):
+        s = layers.GdnSession(g)
+        s.state = torch.zeros(s.state.numel() + 4, device="cuda")[offset:offset + s.state.numel()]
+        s.state[:Hv * 16384] = state
+        s.hist.copy_(hist)
+        plan = layers.GdnPrefillPlan(w, max(R, 27), in_dtype=capi.IN_BF16 if bf16 else capi.IN_F32, fmt=code)
+        out = torch.zeros((R + 5) * Hv * 128, device="cuda", dtype=plan.out.dtype) if fmt == "packed" else plan.out
+        d = capi.dptr
+        args = capi.GdnPrefillArgs(capi.GdnArgs(d(qkv), d(z), None, None, d(w.conv), d(w.A_log), d(w.dt_bias), d(w.gamma), d(s.hist), d(s.state), d(w.suh), d(out),
+                                                None, pos0, R, 0, R, R + 5 if fmt == "packed" else 0, 3 if fmt == "packed" else 0),
+                                   d(ab), plan.in_dtype, d(plan.workspace), plan.workspace.numel(), None)
+        capi.check(capi.lib.cr_gdn_prefill(C.byref(g), C.byref(args), algo, code, None))
+        got.append(((out if fmt == "packed" else plan.out[:R]).float().clone(), s.state[:Hv * 16384].clone(), s.hist.clone()))
+    assert capi.lib.cr_device_check() == 0
+    (o0, s0, h0), (o1, s1, h1) = got
+    ring = hist.clone()
+    for r in range(max(0, R - 16), R):
+        ring[(pos0 + r) % 16] = qkv[r].float()
+    assert torch.equal(h0, ring) and torch.equal(h1, ring)
+    chunked = R > 26 or offset
+    tol = 4e-3 if chunked else 2e-5
+    assert (s1 - s0).abs().max() < tol * s0.abs().max()
+    step = {"f32": 0.0, "bf16": 2.0 ** -8}.get(fmt, 3e-3)                  # one step of the format (fp16 is rounded twice before its transform)
+    assert (o1 - o0).abs().max() < (tol + step) * o0.abs().max()
 
 
 # Calls in a row on one plan, with nothing between them: every call writes its operands where the one before had its own, and its
