@@ -34,6 +34,8 @@ namespace cr {
 constexpr int kSelThreads = 1024;
 constexpr int kMaxSelectCount = 262144;   // elements of one selection: the tie bitmap of the slow path shares the 32 KB of the candidate list
 constexpr int kSortCap = 4096;            // entries of the candidate list (32 KB)
+constexpr int kClusterRow = 20480;        // rows of at least this many blocks may take a cluster
+constexpr int kHeldFrom = 14336, kHeldRow = 32 * kSelThreads;   // rows of one CTA that stay in registers: more blocks than the first, at most the second
 constexpr int kShortCap = 3072;           // of the list of 256 threads, which take rows of many
 constexpr int kShortRow = 14336;          // up to this many blocks (above, 512 threads are the quicker ones)
 
@@ -285,7 +287,8 @@ template <int T, typename Src>
 __device__ __forceinline__ void select_slow(const Src& src, int count, int want, const SelectSmem& sm);
 
 // Marks the `want` best elements of [0, count) in sm.bitmap (bit i = element i selected).  want <= valid elements.
-template <int T, typename Src>
+// HELD > 0: up to HELD quads of a thread stay in registers between the two passes over the row, all of them in flight at once.
+template <int T, int HELD = 0, typename Src>
 __device__ __forceinline__ void select_mark(const Src& src, int count, int want, const SelectSmem& sm) {
   const int t = threadIdx.x, l = t & 31;
   constexpr int G = 1024 / T;                                      // groups of a thread: 1024 in the block
@@ -294,11 +297,30 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
   for (int i = t; i < kBins; i += T) sm.hist[i] = 0;
   if (t == 0) *sm.counter = 0u;
   unsigned pivot = 1u, mine = 0u, largest = 0u;                    // pivot 1: every element passes
+  const bool held = HELD > 0 && src.quads && count <= 4 * HELD * T;
+  uint4 row[HELD > 0 ? HELD : 1];
+  // f(i, keys) for the quads of this thread, all lanes of a warp alike
+  auto held_quads = [&](auto&& f) {
+#pragma unroll
+    for (int k = 0; k < HELD; ++k)
+      if (4 * k * T < count) f(4 * (t + k * T), row[k]);           // uniform
+  };
+  if (held) {
+#pragma unroll
+    for (int k = 0; k < HELD; ++k) {
+      const int q = t + k * T, i = 4 * q;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (i < count) v = src.get4(q);
+      row[k] = make_uint4(i < count ? v.x + 1u : 0u, i + 1 < count ? v.y + 1u : 0u, i + 2 < count ? v.z + 1u : 0u, i + 3 < count ? v.w + 1u : 0u);
+    }
+  }
   if (count > sm.cap) {
     unsigned group[G];
 #pragma unroll
     for (int k = 0; k < G; ++k) group[k] = 0u;
-    if (src.quads) {
+    if (held) {
+      held_quads([&](int, const uint4& k) { group[0] = max(max(max(group[0], k.x), max(k.y, k.z)), k.w); });
+    } else if (src.quads) {
       for_each_quad<T>(src, count, [&](int, const uint4& k) {
         group[0] = max(group[0], k.x); group[1 % G] = max(group[1 % G], k.y); group[2 % G] = max(group[2 % G], k.z); group[3 % G] = max(group[3 % G], k.w);
       });
@@ -328,13 +350,16 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
       if (pass && at < (unsigned)sm.cap) sm.cand[at] = make_uint2(key, (unsigned)i);
     }
   };
-  if (src.quads) {
-    for_each_quad<T>(src, count, [&](int i, const uint4& k) {
-      const unsigned best = max(max(k.x, k.y), max(k.z, k.w));
-      mine = max(mine, best);
-      if (!__any_sync(0xffffffffu, best >= pivot)) return;         // most quads of a long row
-      append(i, k.x); append(i + 1, k.y); append(i + 2, k.z); append(i + 3, k.w);
-    });
+  auto append4 = [&](int i, const uint4& k) {
+    const unsigned best = max(max(k.x, k.y), max(k.z, k.w));
+    mine = max(mine, best);
+    if (!__any_sync(0xffffffffu, best >= pivot)) return;           // most quads of a long row
+    append(i, k.x); append(i + 1, k.y); append(i + 2, k.z); append(i + 3, k.w);
+  };
+  if (held) {
+    held_quads(append4);
+  } else if (src.quads) {
+    for_each_quad<T>(src, count, append4);
   } else {
     for_each_key<T, true>(src, count, [&](int i, unsigned key) {
       mine = max(mine, key);
@@ -428,8 +453,9 @@ static size_t select_smem_bytes(int max_count, int cap = kSortCap) { return (siz
 // (40 registers, a list of 3,072 entries) or, where the rows are long, three of 512, so that the rows in flight are still in L2 when
 // they are read again.  2,048 rows (two CTAs of 1,024 | 512 | 256 threads, us): 2,500 blocks 48 | 36 | 28, 8,192 blocks 69 | 51 | 47,
 // 15,500 94 | 77 | 79, 25,500 123 | 105 | 117, 65,536 198 | 189 | 234.
-template <int T>
-__global__ void __launch_bounds__(T, T == 1024 ? 2 : T == 512 ? 3 : 6) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
+// HELD (up to 32,768 blocks, a row to an SM): a thread's share of the row is loaded once, all at once, and stays in registers.
+template <int T, int HELD = 0>
+__global__ void __launch_bounds__(T, HELD > 0 ? 1 : T == 1024 ? 2 : T == 512 ? 3 : 6) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
   extern __shared__ __align__(16) unsigned char raw[];
   pdl_release();
   const cr_qsa_args& a = P.span[blockIdx.y];
@@ -441,7 +467,7 @@ __global__ void __launch_bounds__(T, T == 1024 ? 2 : T == 512 ? 3 : 6) qsa_topk_
   if (nb <= CR_SEL_BLOCKS) { if (threadIdx.x == 0) a.nsel[r] = -1; return; }
   const SelectSmem sm = carve(raw, max_count, T == 1024 ? kSortCap : kShortCap);
   const RowSource src = row_source(a, r, 0);
-  select_mark<T>(src, nb, CR_SEL_BLOCKS, sm);
+  select_mark<T, HELD>(src, nb, CR_SEL_BLOCKS, sm);
   select_emit<T>(src, nb, sm, a.sel + (size_t)r * CR_SEL_BLOCKS, nullptr);
   if (threadIdx.x == 0) a.nsel[r] = CR_SEL_BLOCKS;
 }
@@ -613,17 +639,24 @@ __global__ void __launch_bounds__(kSelThreads) qsa_merge_candidates_kernel(const
   if (threadIdx.x == 0) a.nsel[r] = CR_SEL_BLOCKS;
 }
 
+static int g_topk_clusters[64];                          // per device: clusters of 8 CTAs that run at once
 static cr_status select_configure() {
   static PerDeviceOnce configured;
   return once_per_device(configured, [] {
     const int most = (int)select_smem_bytes(kMaxSelectCount);
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<kSelThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<kSelThreads, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)select_smem_bytes(kShortRow, kShortCap)));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_cluster_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_cluster_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_merge_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    int dev = 0;
+    CR_CUDA(cudaGetDevice(&dev));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(8 * 64); cfg.blockDim = dim3(kSelThreads); cfg.dynamicSmemBytes = select_smem_bytes(65536);
+    CR_CUDA(cudaOccupancyMaxActiveClusters(&g_topk_clusters[dev & 63], qsa_topk_cluster_kernel<8>, &cfg));
     return CR_OK;
   });
 }
@@ -640,13 +673,22 @@ cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     for (int s = 0; s < n; ++s) nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
     CR_REQUIRE(nb_max <= kMaxSelectCount, "qsa select: %d blocks exceed the selectable range of %d", nb_max, kMaxSelectCount);
     if (dense_marked && nb_max <= CR_SEL_BLOCKS) continue;          // no row of these spans selects
-    if ((long long)Rmax * n <= 64 && nb_max >= 16384) {             // few long rows: 8 SMs per row
+    // Long rows take 8 SMs each while all clusters run at once (fifteen or so: 10.5 us at 16,384 to 65,536 blocks; 16 rows took 18 to 21, 36
+    // rows 28 to 31).  A CTA per row: 20 us at 65,536 blocks, 12 at 32,768 with the row held in registers (14.1 read twice), 10 at
+    // 16,384, and 9.4 against 8.8 at 12,288, so that shorter rows are read twice.
+    const long long rows = (long long)Rmax * n;
+    int dev = 0;
+    CR_CUDA(cudaGetDevice(&dev));
+    const int fit = g_topk_clusters[dev & 63];
+    if (nb_max >= kClusterRow && rows <= fit) {
       if (nb_max <= 65536) CR_CUDA(launch_pdl(qsa_topk_cluster_kernel<8>, dim3(8 * Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
       else CR_CUDA(launch_pdl(qsa_topk_cluster_kernel<32>, dim3(8 * Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
       CR_LAUNCH_CHECK("qsa_topk_cluster_kernel");
       continue;
     }
-    if ((long long)Rmax * n <= 2 * sm_count())                      // all rows are on the chip at once
+    if (rows <= sm_count() && nb_max > kHeldFrom && nb_max <= kHeldRow)
+      CR_CUDA(launch_pdl(qsa_topk_kernel<kSelThreads, 8>, dim3(Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
+    else if (rows <= 2 * sm_count())                 // all rows are on the chip at once
       CR_CUDA(launch_pdl(qsa_topk_kernel<kSelThreads>, dim3(Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
     else if (nb_max <= kShortRow)
       CR_CUDA(launch_pdl(qsa_topk_kernel<256>, dim3(Rmax, n), dim3(256), select_smem_bytes(nb_max, kShortCap), stream, P, nb_max));

@@ -162,6 +162,32 @@ def test_selection_of_many_rows(last_nb, pattern, pad):
         np.testing.assert_array_equal(sel[r], want)
 
 
+# rows of a step at the lines between a CTA per row (read twice, held in registers) and a cluster per row
+@pytest.mark.parametrize("nb,sessions", [(14336, 3), (14337, 3), (20479, 2), (20480, 2), (20481, 20), (32768, 20), (32769, 20), (32768, 3), (65537, 2), (65537, 20)])
+@pytest.mark.parametrize("pattern,pad", [("random", 0), ("random", 1), ("zeros", 0)])
+def test_selection_of_step_rows(nb, sessions, pattern, pad):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(nb + sessions)
+    pool = torch.randn((nb + 31) // 32, 128, 32, device="cuda", generator=gen)
+    if pattern == "zeros":
+        pool *= torch.rand(pool.shape[0], 1, 32, device="cuda", generator=gen) < 300 / nb
+    spans, args, z = [], (capi.QsaArgs * sessions)(), torch.zeros(1, 16, 512, device="cuda")
+    for i in range(sessions):
+        s = layers.QsaSession(g, 64)                                    # the spans share one pool and write no cache
+        s.ik_pool = pool.flatten()
+        s.sstride = nb + pad
+        s.scores = torch.zeros(1, s.sstride, device="cuda")
+        idx = torch.randn(1, 640, device="cuda", generator=gen)
+        args[i] = layers.qsa_args(w, s, z, z, z, idx, z, 4 * nb - 1)
+        spans.append((s, idx))
+    capi.check(capi.lib.cr_qsa_select(C.byref(g), args, sessions, None, 0, None))
+    for s, _ in spans:
+        v = s.scores[0, :nb].double().cpu().numpy()
+        want = np.sort(np.lexsort((np.arange(nb), -v))[:512])
+        np.testing.assert_array_equal(s.sel[0].cpu().numpy(), want)
+        assert int(s.nsel[0]) == 512
+
+
 # scores of spans of 3 to 16 rows: every number of row quartets, ragged last tiles, several tiles to a warp (the longest), spans of
 # different length in a launch, a pool off the 16-byte boundary (scalar loads), score rows off it
 @pytest.mark.parametrize("starts,R,pad,shift", [([2050, 9003], 3, 0, 0), ([4096], 4, 1, 0), ([2300, 2041], 5, 0, 0), ([9003], 9, 2, 0), ([33001], 13, 0, 0),
