@@ -675,12 +675,14 @@ cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     if (dense_marked && nb_max <= CR_SEL_BLOCKS) continue;          // no row of these spans selects
     // Long rows take 8 SMs each while all clusters run at once (fifteen or so: 10.5 us at 16,384 to 65,536 blocks; 16 rows took 18 to 21, 36
     // rows 28 to 31).  A CTA per row: 20 us at 65,536 blocks, 12 at 32,768 with the row held in registers (14.1 read twice), 10 at
-    // 16,384, and 9.4 against 8.8 at 12,288, so that shorter rows are read twice.
+    // 16,384, and 9.4 against 8.8 at 12,288, so that shorter rows are read twice.  Rows too long for the registers take up to two waves
+    // of clusters: as quick alone, and beside another kernel the few CTAs of the other form wait for their second reading (16 sessions
+    // at 262,144 with the GDN step on a stream of its own: 146 us a step, 161 with a CTA per row).
     const long long rows = (long long)Rmax * n;
     int dev = 0;
     CR_CUDA(cudaGetDevice(&dev));
     const int fit = g_topk_clusters[dev & 63];
-    if (nb_max >= kClusterRow && rows <= fit) {
+    if (nb_max >= kClusterRow && rows <= (nb_max > kHeldRow ? 2 * fit : fit)) {
       if (nb_max <= 65536) CR_CUDA(launch_pdl(qsa_topk_cluster_kernel<8>, dim3(8 * Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
       else CR_CUDA(launch_pdl(qsa_topk_cluster_kernel<32>, dim3(8 * Rmax, n), dim3(kSelThreads), select_smem_bytes(nb_max), stream, P, nb_max));
       CR_LAUNCH_CHECK("qsa_topk_cluster_kernel");
