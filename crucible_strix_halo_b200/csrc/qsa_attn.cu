@@ -88,7 +88,9 @@ __device__ __forceinline__ float ex2(float x) {
 
 // grid (cluster x ceil(Rmax * Hkv / units per CTA), 1, spans).  HKV: the cache's KV heads where they are two (row pitches
 // become constants), else 0.
-template <int NG, int HKV>
+// UNIT: a CTA, or a cluster of them, has one unit (steps); without it streams have units of their own (long parts).  Two kernels: what
+// the one form needs on its way from the selection to the output costs the other's loop 1 to 2 % in registers and instructions.
+template <int NG, int HKV, bool UNIT>
 __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __grid_constant__ QsaParams P, const AttnShape shape, float* partials,
                                                                        int p0, int p1, int fmt) {
   extern __shared__ __align__(1024) unsigned char ring_raw[];
@@ -101,8 +103,8 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
   pdl_wait();
   const int t = threadIdx.x, warp = t >> 5, l = t & 31, g8 = l >> 2, tq = l & 3;
   const int stream = warp / NG, hg = warp % NG;
-  const int upc = W / shape.spu, crank = shape.cluster > 1 ? (int)(blockIdx.x % shape.cluster) : 0;
-  const int unit = (int)(blockIdx.x / shape.cluster) * upc + stream / shape.spu, sub = stream % shape.spu;
+  const int upc = UNIT ? 1 : W / shape.spu, crank = UNIT && shape.cluster > 1 ? (int)(blockIdx.x % shape.cluster) : 0;
+  const int unit = UNIT ? (int)(blockIdx.x / shape.cluster) : (int)blockIdx.x * upc + stream / shape.spu, sub = UNIT ? stream : stream % shape.spu;
   const int r = unit / P.Hkv, g = unit % P.Hkv;
   const int gqa = P.Hq / P.Hkv, gh = (gqa + NG - 1) / NG;           // heads of a head group
   const int heads = min(gh, gqa - hg * gh);
@@ -124,7 +126,8 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     // XORed by the head, so that the fragment reads meet no bank twice.  (Every warp loading them as fragments cost 256 line
     // look-ups a warp: 2 us of a step's 9 to 16.)
     float* qs = reinterpret_cast<float*>(ring_raw + (size_t)W * kRingBytes);
-    if (upc == 1) {
+    const bool q_shared = UNIT && ((uintptr_t)a.q & 15) == 0;    // a rank's partials read no gates: its rows may lie at 8 bytes
+    if (q_shared) {
       const float* q = a.q + ((size_t)r * P.Hq + g * gqa) * 512;
       for (int i = t; i < gqa * 64; i += kAttnThreads<NG>) {
         const int hd = i >> 6, pc = i & 63;
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
         if (!have) v = make_float2(0.f, 0.f);
         split2(v.x, v.y, qh[ks][j], ql[ks][j]);
       };
-      if (upc == 1) {
+      if (q_shared) {
         asm volatile("cp.async.wait_group 3;\n" ::: "memory");
         __syncthreads();
         const float* q = qs + hd * 256 + 2 * tq;
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
   } else {
     __syncthreads();
   }
-  if (shape.cluster == 1 && !live) return;
+  if ((!UNIT || shape.cluster == 1) && !live) return;
   // This CTA's merged (m, l, acc) of head hd, channels c .. c + 3.  (One part at a time and the gate at the end: long parts, where a
   // stream has its unit to itself, lose 1.5 % to eight parts or the gate in flight.)
   const int first_stream = stream - sub;
@@ -368,7 +371,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     emit_group(a, P.Hq, r, h, c, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv), gate, fmt);
   };
   const int uw = sub * NG + hg, uwarps = shape.spu * NG;               // this warp among the warps of its unit in this CTA
-  if (shape.cluster == 1) {
+  if (!UNIT || shape.cluster == 1) {
     for (int gi = uw; gi < 2 * gqa; gi += uwarps) {                     // groups: (head, 128 channels)
       float m, lsum;
       const int hd = gi >> 1, c = (gi & 1) * 128 + 4 * l;
@@ -377,6 +380,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
     }
     return;
   }
+  if constexpr (UNIT) {
   // (m, l) of `n` parts (at most 8), lane k & 7 holding those of part k: the factor of that part's accumulator; m and l become those of
   // the whole.
   auto weigh = [&](int n, float& m, float& lsum) {
@@ -441,6 +445,7 @@ __global__ void __launch_bounds__(kAttnThreads<NG>, 1) qsa_attn_kernel(const __g
   cluster.barrier_arrive();                              // this CTA has read the others' images
   if (emits) finish(hd_out, c_out, m, lsum, o, gate);
   cluster.barrier_wait();                                // the own images stay until every CTA has read them
+  }
 }
 
 // Merge of the partial records of several ranks or of a tile's splits (QsaMergeKernel, engine/layers/qsa_long.h:458-499), gate and output
@@ -506,9 +511,10 @@ static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long un
   constexpr size_t smem = kAttnSmem<NG> + 12 * 256 * sizeof(float);   // + the query heads of a CTA's unit, then its merged unit
   int dev = 0;
   CR_CUDA(cudaGetDevice(&dev));
-  CR_REQUIRE(dev >= 0 && dev < 64, "qsa attention: device %d is out of range", dev);
+  dev &= 63;
   if (cr_status st = once_per_device(configured, [dev] {
-        CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG, HKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG, HKV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CR_CUDA(cudaFuncSetAttribute(qsa_attn_kernel<NG, HKV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         fits_on[dev][0] = sm_count();
         for (int k = 1; k < 4; ++k) {
           cudaLaunchConfig_t cfg = {};
@@ -517,7 +523,7 @@ static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long un
           attr.id = cudaLaunchAttributeClusterDimension;
           attr.val.clusterDim.x = 1 << k; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
           cfg.attrs = &attr; cfg.numAttrs = 1;
-          CR_CUDA(cudaOccupancyMaxActiveClusters(&fits_on[dev][k], qsa_attn_kernel<NG, HKV>, &cfg));
+          CR_CUDA(cudaOccupancyMaxActiveClusters(&fits_on[dev][k], qsa_attn_kernel<NG, HKV, true>, &cfg));
         }
         return CR_OK;
       })) return st;
@@ -536,7 +542,7 @@ static cr_status attn_launch_t(const QsaParams& P, int Rmax, int n, long long un
     attr[na].val.clusterDim.x = shape.cluster; attr[na].val.clusterDim.y = 1; attr[na++].val.clusterDim.z = 1;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
-  CR_CUDA(cudaLaunchKernelEx(&cfg, qsa_attn_kernel<NG, HKV>, P, shape, partials, p0, p1, fmt));
+  CR_CUDA(cudaLaunchKernelEx(&cfg, upc == 1 ? qsa_attn_kernel<NG, HKV, true> : qsa_attn_kernel<NG, HKV, false>, P, shape, partials, p0, p1, fmt));
   CR_LAUNCH_CHECK("qsa_attn_kernel");
   return CR_OK;
 }

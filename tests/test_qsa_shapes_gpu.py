@@ -162,6 +162,31 @@ def test_selection_of_many_rows(last_nb, pattern, pad):
         np.testing.assert_array_equal(sel[r], want)
 
 
+# a rank's partials from query rows off the 16-byte boundary (fragments from global memory) and on it (through shared memory)
+@pytest.mark.parametrize("Hq", [16, 24])
+@pytest.mark.parametrize("p0,p1", [(0, 4000), (1024, 2600)])
+def test_shard_attention_of_shifted_rows(Hq, p0, p1):
+    capi, layers, g, w = _weights(Hq)
+    gen = torch.Generator(device="cuda").manual_seed(Hq + p0)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    R, start = 3, 2997
+    s = layers.QsaSession(g, start + R, max_rows=R)
+    s.k.copy_(rn(*s.k.shape).half()); s.v.copy_(rn(*s.v.shape).half())
+    for r in range(R):
+        s.sel[r] = torch.randperm((start + r + 1) // 4, device="cuda", generator=gen)[:512].sort().values.int()
+    s.nsel.fill_(512)
+    q, z, got = rn(R, Hq, 512), torch.zeros(R, 640, device="cuda"), []
+    for shift in (0, 2):
+        buf = torch.zeros(q.numel() + 4, device="cuda")
+        rows = buf[shift:shift + q.numel()].view_as(q)
+        rows.copy_(q)
+        args = layers.qsa_args(w, s, rows, z, z, z, z, start)
+        part = torch.zeros(R, Hq, 258, device="cuda")
+        capi.check(capi.lib.cr_qsa_shard_attn(C.byref(g), C.byref(args), p0, p1, capi.dptr(part), None, 0, None))
+        got.append(part)
+    assert torch.equal(got[0], got[1]) and got[0][..., 1].min().item() > 0
+
+
 # rows of a step at the lines between a CTA per row (read twice, held in registers) and a cluster per row
 @pytest.mark.parametrize("nb,sessions", [(14336, 3), (14337, 3), (20479, 2), (20480, 2), (20481, 20), (32768, 20), (32769, 20), (32768, 3), (65537, 2), (65537, 20)])
 @pytest.mark.parametrize("pattern,pad", [("random", 0), ("random", 1), ("zeros", 0)])
