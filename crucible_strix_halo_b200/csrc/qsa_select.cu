@@ -189,7 +189,7 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
     const bool ranged = b_lo > 0 || b_hi < INT_MAX;
     const int Rmax = qsa_max_rows(spans + s0, n);
     int nb_max = 0;
-    bool wide = true;                               // pools at 16-byte boundaries
+    bool wide = true;                               // pools at 16-byte boundaries: the 128-bit kernels, else a 4-byte load for each block
     for (int s = 0; s < n; ++s) {
       nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
       wide &= ((uintptr_t)spans[s0 + s].c.ik_pool & 15) == 0;
@@ -199,7 +199,7 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
     if (hi <= b_lo) continue;                       // the range holds no complete block of these rows
     const int tiles = (hi + 31) / 32 - b_lo / 32;   // 32-block pool tiles that overlap the scored range
     cr_status st;
-    if (Rmax <= 2) {
+    if (Rmax <= 2 && wide) {
       const dim3 grid((tiles + 7) / 8, 1, n);
       if (ranged) {
         if (Rmax == 1) CR_CUDA(launch_pdl(qsa_score4_kernel<1, true>, grid, dim3(256), 0, stream, P));
@@ -211,7 +211,7 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
       CR_LAUNCH_CHECK("qsa_score_kernel");
       st = CR_OK;
     }
-    else if (Rmax <= 16 && !ranged && wide && !options().qsa_score_simt) st = qsa_score_mma_launch(P, tiles, Rmax, n, stream);   // verify spans
+    else if (Rmax > 2 && Rmax <= 16 && !ranged && wide && !options().qsa_score_simt) st = qsa_score_mma_launch(P, tiles, Rmax, n, stream);   // verify spans
     else if (Rmax >= 8 && (wide || ranged || Rmax > 16) && !options().qsa_score_simt) st = qsa_score_tc_launch(P, n, stream);   // prefill parts (and a rank's range of a span)
     else if (Rmax <= 4) st = score_launch_t<4>(P, tiles, Rmax, n, ranged, stream);
     else st = score_launch_t<8>(P, tiles, Rmax, n, ranged, stream);

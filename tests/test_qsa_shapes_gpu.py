@@ -244,6 +244,42 @@ def test_span_scores(starts, R, pad, shift):
                 assert (s.scores[r, nb:] == -7.0).all(), r                          # nothing past a row's blocks
 
 
+# scores of one and two rows, of every block and of a range, from pools on and off the 16-byte boundary (which the wide loads want):
+# the order of the 128 products of a dot differs, fp32 throughout
+@pytest.mark.parametrize("shift", [0, 1, 2])
+@pytest.mark.parametrize("starts,R,b0,b1", [([2051], 1, 0, 0), ([9003, 2300], 2, 0, 0), ([9003], 1, 700, 2200), ([9004], 2, 5, 2251)])
+def test_short_span_scores_of_shifted_pools(starts, R, b0, b1, shift):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(R + b0)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    spans, args, keep = [], (capi.QsaArgs * len(starts))(), []
+    for i, start in enumerate(starts):
+        s = layers.QsaSession(g, start + R, max_rows=R)
+        s.ik_pool = rn(s.ik_pool.numel() + 4)[shift:]
+        s.scores = torch.full((R, s.sstride), -7.0, device="cuda")
+        idx, z = rn(R, 640), torch.zeros(R, 16, 512, device="cuda")
+        args[i] = layers.qsa_args(w, s, z, z, z, idx, z, start)
+        spans.append((s, idx, start))
+        keep.append(z)
+    cs, ci = torch.zeros(R, 512, device="cuda"), torch.zeros(R, 512, device="cuda", dtype=torch.int32)
+    if b1:
+        capi.check(capi.lib.cr_qsa_shard_select(C.byref(g), args, b0, b1, capi.dptr(cs), capi.dptr(ci), None))
+    else:
+        capi.check(capi.lib.cr_qsa_select(C.byref(g), args, len(starts), None, 0, None))
+    for s, idx, start in spans:
+        tiles = s.ik_pool[:s.ik_pool.numel() // 4096 * 4096].view(-1, 128, 32).double()
+        pool = tiles.transpose(1, 2).reshape(-1, 128)[:(start + R) // 4]
+        want = torch.relu(torch.einsum("rhd,bd->rhb", idx[:, :512].view(R, 4, 128).double(), pool)).sum(1) / 128 ** 0.5
+        for r in range(R):
+            nb = (start + r + 1) // 4
+            lo, hi = (b0, min(b1, nb)) if b1 else (0, nb)
+            if nb > capi.SEL_BLOCKS:
+                assert (s.scores[r, lo:hi].double() - want[r, lo:hi]).abs().max().item() < 2e-4, r
+            else:
+                lo = hi = 0
+            assert (s.scores[r, :lo] == -7.0).all() and (s.scores[r, hi:] == -7.0).all(), r
+
+
 # A compact raw ring beside a full raw cache: calls that start inside a block, whose pooled mean reads ring slots that the call's own
 # rows take, fewer and more rows than slots.  The pooled keys and the newest raw keys are the same, bit for bit.
 @pytest.mark.parametrize("slots", [16, 37])
