@@ -55,7 +55,8 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
 // Prefill parts (many rows): the scores as four GEMMs on tcgen05 tensor cores.
 cr_status qsa_score_tc_launch(const QsaParams& P, int n, cudaStream_t stream);
 // Spans of 3..16 rows (verify passes): the scores as an HBM stream through mma.sync, every block of every row.
-cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream);
+// wide: every pool lies at a 16-byte boundary.
+cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, bool wide, cudaStream_t stream);
 cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
 cr_status qsa_select_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, bool dense_marked = false);
 struct QsaTileSplit { const int* count; int rows, max, mixed; };   // see QsaParams::tile_count

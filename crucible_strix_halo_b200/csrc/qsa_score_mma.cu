@@ -13,6 +13,7 @@
 // Bound: latency with ten to twelve warps on an SM (tensor pipe 49 %, shared memory and L1 56 % busy).  With half a tile a step in
 // 4-byte loads (128 of four lines and 96 ldmatrix a tile) and four tiles to a warp whatever their number, 8 sessions x 9 rows
 // at 131,072 took 52 us and one session x 4 rows at 32,003 (16 CTAs) 14.4; 37 and 5.5 us now.
+#include <type_traits>
 #include "qsa.cuh"
 
 namespace cr {
@@ -37,8 +38,15 @@ __device__ __forceinline__ void split_pair(float x, float y, unsigned& hi, unsig
   lo = *reinterpret_cast<const unsigned*>(&r);
 }
 
+// Four blocks' values of a dim.  Pools off the 16-byte boundary (!WIDE, some pool of the launch) are read a float at a time.
+template <bool WIDE>
+__device__ __forceinline__ float4 sm_load4(const float* p) {
+  if constexpr (WIDE) return __ldcg(reinterpret_cast<const float4*>(p));
+  else return make_float4(p[0], p[1], p[2], p[3]);
+}
+
 // grid (tile groups, 1, spans), 128 threads; MT = ceil(rows / 4) m-tiles of 16 (row, head) pairs; a warp walks `per_warp` tiles.
-template <int MT>
+template <int MT, bool WIDE>
 __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_constant__ QsaParams P, int per_warp) {
   const cr_qsa_args& a = P.span[blockIdx.z];
   pdl_release();
@@ -57,8 +65,7 @@ __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_cons
   const float* pt = a.c.ik_pool + (size_t)first * 4096 + 2 * tq * 32 + 4 * g;
   auto fetch = [&](float4 (&v)[4], int step) {
     const float* p = pt + (size_t)step * 512;          // tiles lie back to back
-    v[0] = __ldcg(reinterpret_cast<const float4*>(p)); v[1] = __ldcg(reinterpret_cast<const float4*>(p + 32));
-    v[2] = __ldcg(reinterpret_cast<const float4*>(p + 256)); v[3] = __ldcg(reinterpret_cast<const float4*>(p + 288));
+    v[0] = sm_load4<WIDE>(p); v[1] = sm_load4<WIDE>(p + 32); v[2] = sm_load4<WIDE>(p + 256); v[3] = sm_load4<WIDE>(p + 288);
   };
   float4 ring[4][4];
   if (first < last) { fetch(ring[0], 0); fetch(ring[1], 1); fetch(ring[2], 2); }   // in flight while the queries are staged; total >= 8
@@ -135,12 +142,15 @@ __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_cons
 }
 
 // Spans of 3..16 rows, every block of every row.  Three CTAs of four warps fit an SM; the tiles are dealt in one wave of them.
-cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, cudaStream_t stream) {
+cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, bool wide, cudaStream_t stream) {
   const int warps = sm_count() * 12, per_warp = (int)(((long long)tiles * n + warps - 1) / warps);
   const dim3 grid((tiles + 4 * per_warp - 1) / (4 * per_warp), 1, n);
   const int mt = (Rmax + 3) / 4;
-  auto kernel = mt <= 1 ? qsa_score_mma_kernel<1> : mt == 2 ? qsa_score_mma_kernel<2> : mt == 3 ? qsa_score_mma_kernel<3> : qsa_score_mma_kernel<4>;
-  CR_CUDA(launch_pdl(kernel, grid, dim3(128), 0, stream, P, per_warp));
+  auto pick = [&](auto w) {
+    constexpr bool W = decltype(w)::value;
+    return mt <= 1 ? qsa_score_mma_kernel<1, W> : mt == 2 ? qsa_score_mma_kernel<2, W> : mt == 3 ? qsa_score_mma_kernel<3, W> : qsa_score_mma_kernel<4, W>;
+  };
+  CR_CUDA(launch_pdl(wide ? pick(std::true_type{}) : pick(std::false_type{}), grid, dim3(128), 0, stream, P, per_warp));
   CR_LAUNCH_CHECK("qsa_score_mma_kernel");
   return CR_OK;
 }

@@ -189,7 +189,7 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
     const bool ranged = b_lo > 0 || b_hi < INT_MAX;
     const int Rmax = qsa_max_rows(spans + s0, n);
     int nb_max = 0;
-    bool wide = true;                               // pools at 16-byte boundaries: the 128-bit kernels, else a 4-byte load for each block
+    bool wide = true;                               // every pool at a 16-byte boundary: loads of four blocks, else of one
     for (int s = 0; s < n; ++s) {
       nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
       wide &= ((uintptr_t)spans[s0 + s].c.ik_pool & 15) == 0;
@@ -211,8 +211,8 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
       CR_LAUNCH_CHECK("qsa_score_kernel");
       st = CR_OK;
     }
-    else if (Rmax > 2 && Rmax <= 16 && !ranged && wide && !options().qsa_score_simt) st = qsa_score_mma_launch(P, tiles, Rmax, n, stream);   // verify spans
-    else if (Rmax >= 8 && (wide || ranged || Rmax > 16) && !options().qsa_score_simt) st = qsa_score_tc_launch(P, n, stream);   // prefill parts (and a rank's range of a span)
+    else if (Rmax > 2 && Rmax <= 16 && !ranged && !options().qsa_score_simt) st = qsa_score_mma_launch(P, tiles, Rmax, n, wide, stream);   // verify spans
+    else if (Rmax >= 8 && !options().qsa_score_simt) st = qsa_score_tc_launch(P, n, stream);   // prefill parts (and a rank's range of a span)
     else if (Rmax <= 4) st = score_launch_t<4>(P, tiles, Rmax, n, ranged, stream);
     else st = score_launch_t<8>(P, tiles, Rmax, n, ranged, stream);
     if (st) return st;

@@ -154,8 +154,8 @@ typedef struct {
   uint16_t* k;     /* fp16 [ctx][Hkv][256] */
   uint16_t* v;     /* fp16 [ctx][Hkv][256] */
   float* ik_raw;   /* fp32 [ctx][128], or a ring of raw_slots rows */
-  float* ik_pool;  /* fp32 tiles [ceil(ctx/128)][128][32]: offset(b,d) = (b/32)*4096 + d*32 + b%32; any float address will do,
-                      pools at 16-byte boundaries are scored with 16-byte loads */
+  float* ik_pool;  /* fp32 tiles [ceil(ctx/128)][128][32]: offset(b,d) = (b/32)*4096 + d*32 + b%32; any float address, though
+                      a launch with a pool off the 16-byte boundary is scored with 4-byte loads */
   int raw_slots;   /* 0 keeps the full-prefix layout */
 } cr_qsa_cache;
 

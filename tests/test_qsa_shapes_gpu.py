@@ -280,6 +280,34 @@ def test_short_span_scores_of_shifted_pools(starts, R, b0, b1, shift):
             assert (s.scores[r, :lo] == -7.0).all() and (s.scores[r, hi:] == -7.0).all(), r
 
 
+# Spans of 3 to 16 rows are scored on tensor cores whatever the address of a pool; one pool off the 16-byte boundary beside another on it
+@pytest.mark.parametrize("R", [3, 7, 9, 16])
+def test_shifted_pools_stay_on_tensor_cores(R):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    args, keep = (capi.QsaArgs * 2)(), []
+    for i, shift in enumerate((0, 3)):
+        s = layers.QsaSession(g, 6001 + R, max_rows=R)
+        s.ik_pool = rn(s.ik_pool.numel() + 4)[shift:]
+        idx, z = rn(R, 640), torch.zeros(R, 16, 512, device="cuda")
+        args[i] = layers.qsa_args(w, s, z, z, z, idx, z, 6001)
+        keep.append((s, idx, z))
+    capi.check(capi.lib.cr_profile_enable(1))
+    try:
+        capi.check(capi.lib.cr_qsa_select(C.byref(g), args, 2, None, 0, None))
+        names = capi.profile_collect()
+    finally:
+        capi.check(capi.lib.cr_profile_enable(0))
+    assert "qsa_score_mma_kernel" in names and "qsa_score_kernel" not in names, names
+    for s, idx, _ in keep:
+        pool = s.ik_pool[:s.ik_pool.numel() // 4096 * 4096].view(-1, 128, 32).transpose(1, 2).reshape(-1, 128)[:(6001 + R) // 4].double()
+        want = torch.relu(torch.einsum("rhd,bd->rhb", idx[:, :512].view(R, 4, 128).double(), pool)).sum(1) / 128 ** 0.5
+        for r in range(R):
+            nb = (6001 + r + 1) // 4
+            assert (s.scores[r, :nb].double() - want[r, :nb]).abs().max().item() < 2e-4, r
+
+
 # A compact raw ring beside a full raw cache: calls that start inside a block, whose pooled mean reads ring slots that the call's own
 # rows take, fewer and more rows than slots.  The pooled keys and the newest raw keys are the same, bit for bit.
 @pytest.mark.parametrize("slots", [16, 37])
