@@ -26,6 +26,7 @@
 #include <climits>
 #include <cooperative_groups.h>
 #include "qsa.cuh"
+#include "splits.h"
 
 namespace cg = cooperative_groups;
 
@@ -526,14 +527,17 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
   if (nb <= CR_SEL_BLOCKS) { if (rank == 0 && t == 0) a.nsel[r] = -1; return; }
   const SelectSmem sm = carve(raw, max_count);
   const float* sc = a.scores + (size_t)r * a.sstride;
-  const int chunk = (((nb + 7) / 8) + kSelThreads - 1) / kSelThreads * kSelThreads;   // elements per CTA, a multiple of 1024
-  const int base = rank * chunk;
+  // An eighth of the row to each, to within one element: a CTA that holds less than the others would offer less than its 64th
+  // largest, or nothing, and a pivot of nothing sends the row to the slow path.  (As multiples of 1,024 elements the eighths left the last
+  // CTA short at three lengths in ten: 57 us at 21,000 blocks and 125 at 57,500, 10 and
+  // 11 now.)
+  const int base = topk_share(nb, rank), end = topk_share(nb, rank + 1);
   unsigned u[PT];
   unsigned mine = 0u;
 #pragma unroll
   for (int k = 0; k < PT; ++k) {
     const int i = base + k * kSelThreads + t;
-    u[k] = (k * kSelThreads < chunk && i < nb) ? __float_as_uint(sc[i]) + 1u : 0u;
+    u[k] = (base + k * kSelThreads < end && i < end) ? __float_as_uint(sc[i]) + 1u : 0u;   // the first test is the same for the CTA
     mine = u[k] > mine ? u[k] : mine;
   }
   const int words = (nb + 31) >> 5;
@@ -563,7 +567,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSelThreads, 1) qsa_
   __syncthreads();
   unsigned pivot = sm.red[0];
   const unsigned largest = sm.red[1];
-  if (pivot == 0u) pivot = 1u;                                     // a CTA with fewer than 64 threads that hold an element: everything passes
+  if (pivot == 0u) pivot = 1u;                                     // rows of fewer than 4,096 blocks: everything passes, and the list holds it
 #pragma unroll
   for (int k = 0; k < PT; ++k) {
     const bool pass = u[k] >= pivot && u[k] != 0u;
@@ -673,11 +677,12 @@ cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     for (int s = 0; s < n; ++s) nb_max = max(nb_max, (spans[s0 + s].pos0 + spans[s0 + s].R) / 4);
     CR_REQUIRE(nb_max <= kMaxSelectCount, "qsa select: %d blocks exceed the selectable range of %d", nb_max, kMaxSelectCount);
     if (dense_marked && nb_max <= CR_SEL_BLOCKS) continue;          // no row of these spans selects
-    // Long rows take 8 SMs each while all clusters run at once (fifteen or so: 10.5 us at 16,384 to 65,536 blocks; 16 rows took 18 to 21, 36
-    // rows 28 to 31).  A CTA per row: 20 us at 65,536 blocks, 12 at 32,768 with the row held in registers (14.1 read twice), 10 at
-    // 16,384, and 9.4 against 8.8 at 12,288, so that shorter rows are read twice.  Rows too long for the registers take up to two waves
-    // of clusters: as quick alone, and beside another kernel the few CTAs of the other form wait for their second reading (16 sessions
-    // at 262,144 with the GDN step on a stream of its own: 146 us a step, 161 with a CTA per row).
+    // Long rows take 8 SMs each while all clusters run at once (fifteen or so: 10 to 11.7 us at 12,000 to 65,536 blocks, 12.6 to 15.2 at
+    // 70,000 to 262,144, whatever the length; 16 rows took 18 to 21, 36 rows 28 to 31).  A CTA per row: 20 us at 65,536 blocks, 12 at 32,768 with
+    // the row held in registers (14.1 read twice), 10.5 at 20,000, 10 at 16,384, and 9.4 against 8.8 at 12,288, so that shorter rows are read
+    // twice.  Rows too long for the registers take up to two waves of clusters: as quick alone, and beside another kernel the few CTAs
+    // of the other form wait for their second reading (16 sessions at 262,144 with the GDN step on a stream of its own: 146 us a step, 161
+    // with a CTA per row).
     const long long rows = (long long)Rmax * n;
     int dev = 0;
     CR_CUDA(cudaGetDevice(&dev));
