@@ -288,7 +288,7 @@ template <int T, typename Src>
 __device__ __forceinline__ void select_slow(const Src& src, int count, int want, const SelectSmem& sm);
 
 // Marks the `want` best elements of [0, count) in sm.bitmap (bit i = element i selected).  want <= valid elements.
-// HELD > 0: up to HELD quads of a thread stay in registers between the two passes over the row, all of them in flight at once.
+// HELD > 0: up to 4 HELD elements of a thread stay in registers between the two passes over the row, all of them in flight at once.
 template <int T, int HELD = 0, typename Src>
 __device__ __forceinline__ void select_mark(const Src& src, int count, int want, const SelectSmem& sm) {
   const int t = threadIdx.x, l = t & 31;
@@ -298,21 +298,37 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
   for (int i = t; i < kBins; i += T) sm.hist[i] = 0;
   if (t == 0) *sm.counter = 0u;
   unsigned pivot = 1u, mine = 0u, largest = 0u;                    // pivot 1: every element passes
-  const bool held = HELD > 0 && src.quads && count <= 4 * HELD * T;
+  const bool held = HELD > 0 && count <= 4 * HELD * T;
   uint4 row[HELD > 0 ? HELD : 1];
-  // f(i, keys) for the quads of this thread, all lanes of a warp alike
-  auto held_quads = [&](auto&& f) {
+  // The elements of row[k]: i, i + step, i + 2 step, i + 3 step, with i = held_at(k); quads, or where the row has none four that T lie between.
+  const int step = src.quads ? 1 : T;
+  auto held_at = [&](int k) { return (src.quads ? 4 * t : t) + 4 * k * T; };
+  // f(i, keys) for the fours of this thread, all lanes of a warp alike
+  auto held_fours = [&](auto&& f) {
 #pragma unroll
     for (int k = 0; k < HELD; ++k)
-      if (4 * k * T < count) f(4 * (t + k * T), row[k]);           // uniform
+      if (4 * k * T < count) f(held_at(k), row[k]);                // uniform
   };
   if (held) {
+    if (src.quads) {
+#pragma unroll
+      for (int k = 0; k < HELD; ++k) row[k] = held_at(k) < count ? src.get4(t + k * T) : make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+      for (int k = 0; k < HELD; ++k) {
+        const int i = held_at(k);
+        row[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (i < count) src.get(i, row[k].x);
+        if (i + T < count) src.get(i + T, row[k].y);
+        if (i + 2 * T < count) src.get(i + 2 * T, row[k].z);
+        if (i + 3 * T < count) src.get(i + 3 * T, row[k].w);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < HELD; ++k) {
-      const int q = t + k * T, i = 4 * q;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (i < count) v = src.get4(q);
-      row[k] = make_uint4(i < count ? v.x + 1u : 0u, i + 1 < count ? v.y + 1u : 0u, i + 2 < count ? v.z + 1u : 0u, i + 3 < count ? v.w + 1u : 0u);
+      const int i = held_at(k);
+      row[k] = make_uint4(i < count ? row[k].x + 1u : 0u, i + step < count ? row[k].y + 1u : 0u, i + 2 * step < count ? row[k].z + 1u : 0u,
+                          i + 3 * step < count ? row[k].w + 1u : 0u);
     }
   }
   if (count > sm.cap) {
@@ -320,7 +336,7 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
 #pragma unroll
     for (int k = 0; k < G; ++k) group[k] = 0u;
     if (held) {
-      held_quads([&](int, const uint4& k) { group[0] = max(max(max(group[0], k.x), max(k.y, k.z)), k.w); });
+      held_fours([&](int, const uint4& k) { group[0] = max(max(max(group[0], k.x), max(k.y, k.z)), k.w); });
     } else if (src.quads) {
       for_each_quad<T>(src, count, [&](int, const uint4& k) {
         group[0] = max(group[0], k.x); group[1 % G] = max(group[1 % G], k.y); group[2 % G] = max(group[2 % G], k.z); group[3 % G] = max(group[3 % G], k.w);
@@ -351,16 +367,16 @@ __device__ __forceinline__ void select_mark(const Src& src, int count, int want,
       if (pass && at < (unsigned)sm.cap) sm.cand[at] = make_uint2(key, (unsigned)i);
     }
   };
-  auto append4 = [&](int i, const uint4& k) {
+  auto append4 = [&](int i, const uint4& k, int by) {
     const unsigned best = max(max(k.x, k.y), max(k.z, k.w));
     mine = max(mine, best);
     if (!__any_sync(0xffffffffu, best >= pivot)) return;           // most quads of a long row
-    append(i, k.x); append(i + 1, k.y); append(i + 2, k.z); append(i + 3, k.w);
+    append(i, k.x); append(i + by, k.y); append(i + 2 * by, k.z); append(i + 3 * by, k.w);
   };
   if (held) {
-    held_quads(append4);
+    held_fours([&](int i, const uint4& k) { append4(i, k, step); });
   } else if (src.quads) {
-    for_each_quad<T>(src, count, append4);
+    for_each_quad<T>(src, count, [&](int i, const uint4& k) { append4(i, k, 1); });
   } else {
     for_each_key<T, true>(src, count, [&](int i, unsigned key) {
       mine = max(mine, key);
@@ -454,7 +470,9 @@ static size_t select_smem_bytes(int max_count, int cap = kSortCap) { return (siz
 // (40 registers, a list of 3,072 entries) or, where the rows are long, three of 512, so that the rows in flight are still in L2 when
 // they are read again.  2,048 rows (two CTAs of 1,024 | 512 | 256 threads, us): 2,500 blocks 48 | 36 | 28, 8,192 blocks 69 | 51 | 47,
 // 15,500 94 | 77 | 79, 25,500 123 | 105 | 117, 65,536 198 | 189 | 234.
-// HELD (up to 32,768 blocks, a row to an SM): a thread's share of the row is loaded once, all at once, and stays in registers.
+// HELD (up to 32,768 blocks, a row to an SM): a thread's share of the row is loaded once, all at once, and stays in registers; by quads, or
+// singly where the row does not lie at 16 bytes (three pitches in four): 15 rows of 20,479 blocks 10.8 and 11.2 us, 12.4 while the
+// latter were read twice.
 template <int T, int HELD = 0>
 __global__ void __launch_bounds__(T, HELD > 0 ? 1 : T == 1024 ? 2 : T == 512 ? 3 : 6) qsa_topk_kernel(const __grid_constant__ QsaParams P, int max_count) {
   extern __shared__ __align__(16) unsigned char raw[];
