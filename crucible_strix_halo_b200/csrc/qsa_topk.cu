@@ -33,11 +33,11 @@ namespace cg = cooperative_groups;
 namespace cr {
 
 constexpr int kSelThreads = 1024;
-constexpr int kMaxSelectCount = 262144;   // elements of one selection: the tie bitmap of the slow path shares the 32 KB of the candidate list
+constexpr int kMaxSelectCount = 262144;   // elements of one selection: the tie bitmap of the slow path takes the place of list and histogram
 constexpr int kSortCap = 4096;            // entries of the candidate list (32 KB)
 constexpr int kClusterRow = 20480;        // rows of at least this many blocks may take a cluster
 constexpr int kHeldFrom = 14336, kHeldRow = 32 * kSelThreads;   // rows of one CTA that stay in registers: more blocks than the first, at most the second
-constexpr int kShortCap = 3072;           // of the list of 256 threads, which take rows of many
+constexpr int kShortCap = 3072;           // of the list of 256 and 512 threads, which take rows of many
 constexpr int kShortRow = 14336;          // up to this many blocks (above, 512 threads are the quicker ones)
 
 // ---- element sources ---------------------------------------------------------------------------------------
@@ -172,6 +172,8 @@ __device__ __forceinline__ void for_each_quad(const Src& src, int count, F&& f) 
 constexpr int kBins = 2048;
 constexpr int kRankCap = 512;              // elements of the threshold bin that are ranked against each other
 
+static_assert(kShortCap <= kSortCap && kShortCap * 8 + kBins * 4 >= kMaxSelectCount / 8, "the tie bitmap of the longest row ends where the selection's begins");
+static_assert(kRankCap * 8 <= kBins * 4, "the ranked elements fit the histogram's place");
 struct Threshold { int bin, above, in_bin; };   // the bin that holds the want-th largest; elements in higher bins; in it
 // sm.hist filled and visible.  The bin of the want-th largest counted element; bin = -1 when fewer were counted.  Two
 // barriers; the histogram is zero again afterwards (visible after the caller's next barrier).
@@ -403,7 +405,7 @@ __device__ __forceinline__ void select_slow(const Src& src, int count, int want,
     for_each_key<T, false>(src, count, [&](int, unsigned key) { c += key >= trial; });
     if (block_sum_u32<T>(c, sm.red) >= (unsigned)want) limit = trial;
   }
-  unsigned* ties = reinterpret_cast<unsigned*>(sm.cand);           // bitmap of the elements equal to limit (<= 32 KB)
+  unsigned* ties = reinterpret_cast<unsigned*>(sm.cand);           // bitmap of the elements equal to limit: at most 32 KB, over the list and, past a short one, the histogram
   unsigned above = 0u;
   for_each_key<T, true>(src, count, [&](int i, unsigned key) {        // a warp covers one bitmap word per call
     const unsigned gt = __ballot_sync(0xffffffffu, key > limit), eq = __ballot_sync(0xffffffffu, key == limit);
@@ -669,7 +671,7 @@ static cr_status select_configure() {
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<kSelThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<kSelThreads, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)select_smem_bytes(kShortRow, kShortCap)));
-    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CR_CUDA(cudaFuncSetAttribute(qsa_topk_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)select_smem_bytes(kMaxSelectCount, kShortCap)));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_cluster_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_topk_cluster_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CR_CUDA(cudaFuncSetAttribute(qsa_candidates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
@@ -718,7 +720,7 @@ cr_status qsa_topk_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_
     else if (nb_max <= kShortRow)
       CR_CUDA(launch_pdl(qsa_topk_kernel<256>, dim3(Rmax, n), dim3(256), select_smem_bytes(nb_max, kShortCap), stream, P, nb_max));
     else
-      CR_CUDA(launch_pdl(qsa_topk_kernel<512>, dim3(Rmax, n), dim3(512), select_smem_bytes(nb_max), stream, P, nb_max));
+      CR_CUDA(launch_pdl(qsa_topk_kernel<512>, dim3(Rmax, n), dim3(512), select_smem_bytes(nb_max, kShortCap), stream, P, nb_max));
     CR_LAUNCH_CHECK("qsa_topk_kernel");
   }
   return CR_OK;

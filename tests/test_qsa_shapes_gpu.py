@@ -162,6 +162,33 @@ def test_selection_of_many_rows(last_nb, pattern, pad):
         np.testing.assert_array_equal(sel[r], want)
 
 
+# many rows of equal scores past 196,608 blocks: the bitmap of the ties runs past the short list over the histogram's place and ends where the
+# selection's own begins
+@pytest.mark.parametrize("last_nb", [196608, 200003, 262144])
+def test_selection_of_many_long_rows_of_ties(last_nb):
+    capi, layers, g, w = _weights(16)
+    R = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 9
+    gen = torch.Generator(device="cuda").manual_seed(last_nb)
+    s = layers.QsaSession(g, 64, max_rows=R)                            # no cache row is written
+    s.ik_pool = torch.zeros((last_nb + 31) // 32, 128, 32, device="cuda")
+    some = torch.randperm(last_nb, device="cuda", generator=gen)[:300]
+    s.ik_pool[some // 32, :, some % 32] = torch.randn(300, 128, device="cuda", generator=gen)
+    s.ik_pool = s.ik_pool.flatten()
+    s.sstride = last_nb
+    s.scores = torch.zeros(R, s.sstride, device="cuda")
+    idx, z = torch.randn(R, 640, device="cuda", generator=gen), torch.zeros(R, 16, 512, device="cuda")
+    pos0 = 4 * last_nb - R
+    args = layers.qsa_args(w, s, z, z, z, idx, z, pos0)
+    capi.check(capi.lib.cr_qsa_select(C.byref(g), C.byref(args), 1, None, 0, None))
+    for r in range(0, R, 38):
+        nb = (pos0 + r + 1) // 4
+        v = s.scores[r, :nb].cpu().numpy()
+        assert (v > 0).sum() < 512 and int(s.nsel[r]) == 512
+        best = np.nonzero(v > 0)[0]
+        want = np.sort(np.concatenate([best, np.nonzero(v == 0)[0][:512 - len(best)]]))
+        np.testing.assert_array_equal(s.sel[r].cpu().numpy(), want)
+
+
 # a rank's partials from query rows off the 16-byte boundary (fragments from global memory) and on it (through shared memory)
 @pytest.mark.parametrize("Hq", [16, 24])
 @pytest.mark.parametrize("p0,p1", [(0, 4000), (1024, 2600)])
