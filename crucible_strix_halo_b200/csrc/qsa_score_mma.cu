@@ -15,6 +15,7 @@
 // at 131,072 took 52 us and one session x 4 rows at 32,003 (16 CTAs) 14.4; 37 and 5.5 us now.
 #include <type_traits>
 #include "qsa.cuh"
+#include "splits.h"
 
 namespace cr {
 
@@ -141,9 +142,12 @@ __global__ void __launch_bounds__(128, 3) qsa_score_mma_kernel(const __grid_cons
   }
 }
 
-// Spans of 3..16 rows, every block of every row.  Three CTAs of four warps fit an SM; the tiles are dealt in one wave of them.
+// Spans of 3..16 rows, every block of every row.  Three CTAs of four warps fit an SM; the tiles are dealt in one wave of them.  (Dealt over
+// all warps, whatever the spans' last CTAs held, 16 spans of 111 tiles came to 448 CTAs for 444 places: 11.2 us for 4 rows, 9.8
+// now; 8 of 1,110 tiles 38.0 and 30.5, of 9 rows 50.8 and 44.6.)  13 to 16 rows, 168 registers a thread with 24 bytes spilled: 8 sessions at 131,072
+// positions 50.5 us, 66 to 68 in the form of half a tile a step with four CTAs to an SM.
 cr_status qsa_score_mma_launch(const QsaParams& P, int tiles, int Rmax, int n, bool wide, cudaStream_t stream) {
-  const int warps = sm_count() * 12, per_warp = (int)(((long long)tiles * n + warps - 1) / warps);
+  const int per_warp = score_tiles_per_warp(tiles, n, sm_count());
   const dim3 grid((tiles + 4 * per_warp - 1) / (4 * per_warp), 1, n);
   const int mt = (Rmax + 3) / 4;
   auto pick = [&](auto w) {

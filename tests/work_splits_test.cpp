@@ -20,8 +20,21 @@ static int topk_shares() {
   return 0;
 }
 
+// The tiles of a launch of span scores: no CTA is left for a second wave, and no warp walks more tiles than that takes.
+static int score_tiles() {
+  for (int sms = 132; sms <= 160; sms += 16)
+    for (int n = 1; n <= 32; ++n)
+      for (int tiles = 16; tiles <= 8192; ++tiles) {
+        const int per = cr::score_tiles_per_warp(tiles, n, sms);
+        auto ctas = [&](int p) { return n * ((tiles + 4 * p - 1) / (4 * p)); };
+        if (per < 1 || ctas(per) > 3 * sms) return fail("score_tiles_per_warp: a second wave", tiles, n);
+        if (per > 1 && ctas(per - 1) <= 3 * sms) return fail("score_tiles_per_warp: more than needed", tiles, n);
+      }
+  return 0;
+}
+
 int main() {
-  if (topk_shares()) return 1;
+  if (topk_shares() || score_tiles()) return 1;
   std::puts("work_splits_test: ok");
   return 0;
 }
