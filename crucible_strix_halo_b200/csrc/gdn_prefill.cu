@@ -371,9 +371,8 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
   const size_t in_elt = bf ? 2 : 4, out_elt = fmt == CR_OUT_RAW_F32 ? 4 : 2;
   const size_t Cw = 2 * (size_t)g->gdn_kheads * 128 + (size_t)g->gdn_vheads * 128, VWs = (size_t)g->gdn_vheads * 128;
   // A handful of rows: the step's recurrence over the rows, in fp32.  A call of one chunk takes 28 to 30 us whatever its rows (a chain of
-  // latencies), the step kernel 6.5 to 13.7 for 1 to 13 of them and twice that for 26.  (Its 128-bit accesses want an aligned state, and it
-  // keeps the un-gated readout to itself.)
-  if (algo == CR_GDN_CHUNK_TC && a.R <= 2 * CR_MAX_STEP_ROWS && !args->raw_y && ((uintptr_t)a.state & 15) == 0) {
+  // latencies), the step kernel 6.5 to 13.7 for 1 to 13 of them and twice that for 26.  (Its 128-bit accesses want an aligned state.)
+  if (algo == CR_GDN_CHUNK_TC && a.R <= 2 * CR_MAX_STEP_ROWS && ((uintptr_t)a.state & 15) == 0) {
     for (int p0 = 0, n; p0 < a.R; p0 += n) {
       n = a.R <= CR_MAX_STEP_ROWS || p0 > 0 ? a.R - p0 : (a.R + 1) / 2;
       cr_gdn_args part = a;
@@ -382,7 +381,8 @@ extern "C" cr_status cr_gdn_prefill(const cr_geometry* g, const cr_gdn_prefill_a
       if (a.pack_rows) part.pack_off = a.pack_off + p0; else part.out = (char*)a.out + (size_t)p0 * VWs * out_elt;
       part.pos0 = a.pos0 + p0;
       part.R = part.commit = n;
-      if (cr_status s = gdn_few_rows(g, part, (const char*)args->ab_logits + (size_t)p0 * 2 * g->gdn_vheads * in_elt, bf, fmt, stream)) return s;
+      const char* logits = (const char*)args->ab_logits + (size_t)p0 * 2 * g->gdn_vheads * in_elt;
+      if (cr_status s = gdn_few_rows(g, part, logits, args->raw_y ? args->raw_y + (size_t)p0 * VWs : nullptr, bf, fmt, stream)) return s;
     }
     return CR_OK;
   }

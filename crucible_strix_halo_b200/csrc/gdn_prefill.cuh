@@ -27,7 +27,7 @@ struct GdnPrefillParams {
 };
 
 // A call of at most CR_MAX_STEP_ROWS rows through the step's recurrence (gdn_step.cu).
-cr_status gdn_few_rows(const cr_geometry* g, const cr_gdn_args& a, const void* logits, bool bf16_in, cr_out_format fmt, cudaStream_t stream);
+cr_status gdn_few_rows(const cr_geometry* g, const cr_gdn_args& a, const void* logits, float* raw_y, bool bf16_in, cr_out_format fmt, cudaStream_t stream);
 bool gdn_chunk_available();
 size_t gdn_chunk_workspace_bytes(const cr_geometry* g, int rows);
 cr_status gdn_chunk_scan(const cr_geometry* g, const GdnPrefillParams& P, bool bf16_in, cudaStream_t stream);

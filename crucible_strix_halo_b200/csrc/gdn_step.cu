@@ -17,6 +17,9 @@
 // of the columns per CTA and two barriers a row, 52 us with 8 columns per warp and none, 32 us now.  One session x 1 row, 32
 // heads, state in L2 / in HBM: 6.8 / 9.2 us in that first form, 8.6 / 9.1 on a CTA per head, which pulls 64 KB of state, 6.6 / 7.1
 // as clusters of four.  4 sessions x 1 row: 9.8 / 12.9, now 8.8 / 10.1.  (Plain launches; chained ones take 0.5 to 0.8 less.)
+//
+// Prefill calls of up to 26 rows run here as well, 13 at most to a launch: their rows come in fp32 or bf16 with a and b as logits, all of
+// them are committed, and nothing is replayed.
 #include <cooperative_groups.h>
 #include "gdn_prefill.cuh"
 
@@ -34,6 +37,7 @@ struct GdnStepParams {
   int Hv, Hk, hidden, pend_rows, fmt;
   int rows, replay;                                    // most of any span: the shared-memory layout
   const void* logits;                                  // rows of a prefill call: [R][2 Hv] a and b logits in the place of x and ab
+  float* raw_y;                                        // and, where it is asked for, [R][Hv * 128] of un-gated readout
 };
 // What a pass reads: the rows of a step (fp32 projections, a and b from dot products with x), or those of a short prefill call
 // (projections and logits in fp32 or bf16).
@@ -360,6 +364,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) gdn_step_kernel(const __grid_
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[i] = yv[i] * rs * a.gamma[4 * l + i] * sigmoidf_(z[k][i]);
     const size_t at = (size_t)r * VW + h * 128 + 4 * l;
+    if (IN != kStepRowsIn && P.raw_y) *reinterpret_cast<float4*>(P.raw_y + at) = y;
     if (P.fmt == CR_OUT_RAW_F32) {
       float* dst = reinterpret_cast<float*>(a.out) + at;
       if (((uintptr_t)dst & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
@@ -445,12 +450,12 @@ static cr_status step_dispatch(const GdnStepParams& P, int n, cudaStream_t strea
 
 // The rows of a prefill call of at most CR_MAX_STEP_ROWS rows through the recurrence: what bounds a call of one chunk is the chain of
 // its phases, whatever its rows.
-cr_status gdn_few_rows(const cr_geometry* g, const cr_gdn_args& a, const void* logits, bool bf16_in, cr_out_format fmt, cudaStream_t stream) {
+cr_status gdn_few_rows(const cr_geometry* g, const cr_gdn_args& a, const void* logits, float* raw_y, bool bf16_in, cr_out_format fmt, cudaStream_t stream) {
   GdnStepParams P;
   P.span[0] = a;
   P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.hidden = g->hidden; P.pend_rows = 1; P.fmt = (int)fmt;
   P.rows = a.R; P.replay = 0;
-  P.logits = logits;
+  P.logits = logits; P.raw_y = raw_y;
   return bf16_in ? step_dispatch<kPrefillBf16>(P, 1, stream) : step_dispatch<kPrefillF32>(P, 1, stream);
 }
 
@@ -483,7 +488,7 @@ extern "C" cr_status cr_gdn_step(const cr_geometry* g, const cr_gdn_args* spans,
     for (int s = 0; s < n; ++s) P.span[s] = spans[s0 + s];
     P.Hv = g->gdn_vheads; P.Hk = g->gdn_kheads; P.hidden = g->hidden; P.pend_rows = pend_rows; P.fmt = (int)fmt;
     P.rows = P.replay = 0;
-    P.logits = nullptr;
+    P.logits = nullptr; P.raw_y = nullptr;
     for (int s = 0; s < n; ++s) {
       P.rows = P.rows > P.span[s].R ? P.rows : P.span[s].R;
       P.replay = P.replay > P.span[s].replay ? P.replay : P.span[s].replay;

@@ -132,9 +132,10 @@ int cr_gdn_prefill_parts(int rows, int* first_row, int* n_rows, int max_parts);
  * (engine/layers/kernels/prefill_gdn.h:1206-1216, :1161, :1229-1279, :274-282): rows pos0..pos0+R-1 of one
  * layer from the carried state; writes the gated output, the new state and the raw-row ring.
  * Any R >= 1 is accepted (the engine calls it with parts of <= 2048 rows).
- * With CR_GDN_CHUNK_TC a call of up to 2 CR_MAX_STEP_ROWS rows runs through the step's fp32 recurrence (one or two launches; not
- * with raw_y, nor with a state off a 16-byte boundary), one of one internal part is three chained launches on `stream`; a longer one runs its
- * kernels on three library-owned streams
+ * With CR_GDN_CHUNK_TC a call of up to 2 CR_MAX_STEP_ROWS rows runs through the step's fp32 recurrence (one or two launches).  A state off
+ * a 16-byte boundary keeps such a call on the chunked scan, whose products are tf32: output and state then differ in their last bits from
+ * those of an aligned state (about 1e-3 of their size against about 1e-6).  A call of one internal part is three chained launches on
+ * `stream`; a longer one runs its kernels on three library-owned streams
  * (created on first use, one set per device) that fork from `stream` and join it again with events before the
  * call returns: to the caller the work is still asynchronous on `stream`, and it can be captured into a graph.
  * Calls on one device are serialised while they enqueue.  With stage timing on everything stays on `stream`. */

@@ -117,6 +117,35 @@ def test_gdn_prefill_of_few_rows(heads, R, pos0, bf16, fmt, offset):
     assert (o1 - o0).abs().max() < (tol + step) * o0.abs().max()
 
 
+# The un-gated readout is an output like the others: asking for it changes neither the route of a call nor a bit of its results.
+@pytest.mark.parametrize("R", [1, 13, 14, 26, 27])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_raw_readout_changes_nothing_else(R, bf16):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, 32, 16)
+    gen = torch.Generator(device="cuda").manual_seed(R)
+    rn = lambda *s, std=1.0: torch.randn(*s, device="cuda", generator=gen) * std
+    width, Hv = g.gdn_channels, g.gdn_vheads
+    dt = torch.bfloat16 if bf16 else torch.float32
+    w = layers.GdnWeights(g, rn(width, 4, std=0.5), rn(Hv) - 1, rn(Hv, std=0.5), 1 + rn(128, std=0.1))
+    qkv, z, ab = rn(R, width).to(dt), rn(R, Hv * 128).to(dt), rn(R, 2 * Hv).to(dt)
+    hist, state = rn(16, width), rn(Hv * 16384, std=0.1)
+    got = []
+    for algo, raw in ((capi.GDN_CHUNK_TC, False), (capi.GDN_CHUNK_TC, True), (capi.GDN_SERIAL_F32, True)):
+        s = layers.GdnSession(g)
+        s.state[:Hv * 16384] = state
+        s.hist.copy_(hist)
+        plan = layers.GdnPrefillPlan(w, R, in_dtype=capi.IN_BF16 if bf16 else capi.IN_F32, raw_y=raw)
+        if raw:
+            plan.raw_y.fill_(float("nan"))
+        out = plan.run(s, qkv, z, ab, 1000, algo).clone()
+        got.append((out, s.state.clone(), s.hist.clone(), plan.raw_y))
+    for x, y in zip(got[0][:3], got[1][:3]):
+        assert torch.equal(x, y)
+    y, want = got[1][3], got[2][3]
+    assert (y - want).abs().max() < (4e-3 if R > 26 else 2e-5) * want.abs().max()
+
+
 # Calls in a row on one plan, with nothing between them: every call writes its operands where the one before had its own, and its
 # scan must not take those for new.  The workspace of the first call holds marks that say everything is written.  Rows: a CTA
 # with a unit for one half, units for both, several per half; more chunks than the scan's loader looks at in one go (32).
