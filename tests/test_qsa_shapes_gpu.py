@@ -335,6 +335,45 @@ def test_shifted_pools_stay_on_tensor_cores(R):
             assert (s.scores[r, :nb].double() - want[r, :nb]).abs().max().item() < 2e-4, r
 
 
+# Rotations of far positions against 64 bits: text positions, and multimodal ones with an axis each, around the angle past which the
+# reduction changes (105,615), up to 4 M and at the end of the integers that a float holds; the plain table and a YaRN one, whose
+# multiplier scales both.  A head of ones in the first 32 channels comes out as cosines and sines times one factor.  Bound: cosf and
+# sinf 2 ulp (2^-23 below one), the remainder's first-order term 2^-24, the norm's factor and the products 5 roundings of 2^-24.
+@pytest.mark.parametrize("factor", [1, 4])
+@pytest.mark.parametrize("first", [0, 105000, 105600, 262144, 1048576, 4000000, 16775000])
+@pytest.mark.parametrize("axes", [1, 3])
+def test_rotation_of_far_positions(first, axes, factor):
+    from crucible_strix_halo_b200 import capi, layers
+    g = capi.Geometry(256, 16, 2, 4, 2)
+    one = [torch.ones(n) for n in (256, 256, 128, 128)]
+    w = layers.QsaWeights(g, *one, rope_factor=factor)
+    rng = np.random.default_rng(first + axes)
+    R = 2048
+    pos = np.arange(first, first + R, dtype=np.int32)[:, None].repeat(3, 1)
+    if axes == 3:
+        pos = np.stack([pos[:, 0], rng.integers(0, first + R, R), rng.integers(0, 4194304, R)], 1).astype(np.int32)
+    q = torch.zeros(R, 16, 512, device="cuda")
+    q[:, :, :32] = 1.0
+    q[:, 1::2, :32], q[:, 1::2, 32:64] = 0.0, 1.0
+    s, z = layers.QsaSession(g, 64, max_rows=1), torch.zeros(R, 640, device="cuda")
+    table = torch.zeros(R, 4, device="cuda", dtype=torch.int32)
+    table[:, :3] = torch.from_numpy(pos)
+    args = layers.qsa_args(w, s, q, z, z, z, z, first if axes == 1 else 0, mrope=table if axes == 3 else None)
+    args.sstride = (first + R) // 4                              # the query half touches neither scores nor cache
+    capi.check(capi.lib.cr_qsa_prep_queries(C.byref(g), C.byref(args), 1, None))
+    rope = w.rope.cpu().numpy()
+    j = np.arange(32)
+    axis = np.where(j % 3 == 1, 1, np.where((j % 3 == 2) & (j < 30), 2, 0))
+    ang = (pos[:, axis].astype(np.float32) * rope[:32]).astype(np.float64)              # the fp32 angle is the rotation's definition
+    scale = float(rope[32]) / np.sqrt(32 / 256 + 1e-6)
+    got = q[:, :, :64].cpu().numpy().astype(np.float64) / scale
+    want = np.cos(ang), np.sin(ang)
+    for h in range(16):
+        c, sn = (want[0], want[1]) if h % 2 == 0 else (-want[1], want[0])
+        err = max(np.abs(got[:, h, :32] - c).max(), np.abs(got[:, h, 32:] - sn).max())
+        assert err < 8 * 2.0 ** -24, (h, err * 2.0 ** 24)
+
+
 # A compact raw ring beside a full raw cache: calls that start inside a block, whose pooled mean reads ring slots that the call's own
 # rows take, fewer and more rows than slots.  The pooled keys and the newest raw keys are the same, bit for bit.
 @pytest.mark.parametrize("slots", [16, 37])
