@@ -80,8 +80,10 @@ __global__ void __launch_bounds__(256) qsa_score_kernel(const __grid_constant__ 
 // tiles into L2 before the wait for the kernel ahead was slower: the prefetches come in with the ordinary policy.)
 // RANGED: only the blocks [P.b_lo, P.b_hi) are scored (a rank's own blocks).  A separate instantiation: with the range
 // tests in it the whole-row kernel measured 40 us instead of 29 for four 262,144-token rows.
-template <int RT, bool RANGED>
-__global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__ QsaParams P) {
+// AHEAD: with half a tile in flight from the start two CTAs of 101 or 123 registers a thread fit an SM; without it four of two rows, a
+// quarter of a tile at a time.  score4_ahead() has the line.
+template <int RT, bool RANGED, bool AHEAD>
+__global__ void __launch_bounds__(256, AHEAD ? 0 : 4) qsa_score4_kernel(const __grid_constant__ QsaParams P) {
   pdl_release();
   const cr_qsa_args& a = P.span[blockIdx.z];
   touch_params(a);
@@ -99,12 +101,14 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
   const int bq = (l & 7) * 4, dl = l >> 3;
   const float* pt = a.c.ik_pool + (size_t)tile * 4096 + dl * 32 + bq;
   const uint64_t policy = evict_first_policy();
-  float4 key[2][8];                           // a quarter of the tile; the first two are in flight while the queries are staged
+  float4 key[AHEAD ? 2 : 1][8];               // a quarter of the tile each
   auto fetch = [&](float4 (&k)[8], int it0) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) k[j] = load_stream4(pt + (it0 + j) * 128, policy);
   };
-  if (live) { fetch(key[0], 0); fetch(key[1], 8); }
+  if constexpr (AHEAD) {
+    if (live) { fetch(key[0], 0); fetch(key[1], 8); }             // in flight while the queries are staged
+  }
   for (int i = t; i < 128 * RT; i += 256) {
     const int d = i / RT, r = i % RT;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -123,7 +127,8 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
     for (int b = 0; b < 4; ++b) acc[r][b][0] = acc[r][b][1] = acc[r][b][2] = acc[r][b][3] = 0.f;
 #pragma unroll
   for (int it0 = 0; it0 < 32; it0 += 8) {
-    float4 (&k)[8] = key[(it0 >> 3) & 1];
+    float4 (&k)[8] = key[AHEAD ? (it0 >> 3) & 1 : 0];
+    if constexpr (!AHEAD) fetch(k, it0);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float kb[4] = {k[j].x, k[j].y, k[j].z, k[j].w};
@@ -139,7 +144,9 @@ __global__ void __launch_bounds__(256) qsa_score4_kernel(const __grid_constant__
         }
       }
     }
-    if (it0 + 16 < 32) fetch(k, it0 + 16);
+    if constexpr (AHEAD) {
+      if (it0 + 16 < 32) fetch(k, it0 + 16);
+    }
   }
 #pragma unroll
   for (int r = 0; r < RT; ++r)
@@ -179,6 +186,13 @@ static cr_status score_launch_t(const QsaParams& P, int tiles, int Rmax, int n, 
   return CR_OK;
 }
 
+// Whether a launch of `ctas` CTAs of qsa_score4_kernel has the loads of half a tile in flight from the start: all but whole rows in pairs
+// where that form's CTAs need a second wave and those of the other do not.  Two rows each, us in the one form | the other: pool in L2, 4 sessions
+// of 20,000 blocks 10.9 | 9.3, 8 of 14,000 11.6 | 9.8, 4 of 32,768 12.1 | 11.8; from HBM 13.5 | 11.7, 14.7 | 13.6, 15.6 | 15.2; on either side of
+// the range 4 of 8,001 5.2 | 5.5, 8 of 32,768 24.9 | 26.1.  One row: L2 7.6 | 6.4 and 9.2 | 7.9 for 4 sessions of 20,000 and 32,768 blocks, but HBM
+// 10.3 | 10.5 and 13.5 | 14.3, where the pools of a model with several layers are.  A range of 131,072 blocks: 12.3 | 12.0.
+static bool score4_ahead(int rows, bool ranged, long long ctas) { return rows == 1 || ranged || ctas <= 2 * sm_count() || ctas > 4 * sm_count(); }
+
 cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n_spans, cudaStream_t stream, int b_lo, int b_hi) {
   use_stream(stream);
   for (int s0 = 0; s0 < n_spans; s0 += kMaxSpans) {
@@ -201,13 +215,11 @@ cr_status qsa_score_launch(const cr_geometry* g, const cr_qsa_args* spans, int n
     cr_status st;
     if (Rmax <= 2 && wide) {
       const dim3 grid((tiles + 7) / 8, 1, n);
-      if (ranged) {
-        if (Rmax == 1) CR_CUDA(launch_pdl(qsa_score4_kernel<1, true>, grid, dim3(256), 0, stream, P));
-        else CR_CUDA(launch_pdl(qsa_score4_kernel<2, true>, grid, dim3(256), 0, stream, P));
-      } else {
-        if (Rmax == 1) CR_CUDA(launch_pdl(qsa_score4_kernel<1, false>, grid, dim3(256), 0, stream, P));
-        else CR_CUDA(launch_pdl(qsa_score4_kernel<2, false>, grid, dim3(256), 0, stream, P));
-      }
+      const bool ahead = score4_ahead(Rmax, ranged, (long long)grid.x * n);
+      auto kernel = Rmax == 1 ? (ranged ? qsa_score4_kernel<1, true, true> : qsa_score4_kernel<1, false, true>)
+                    : ranged  ? qsa_score4_kernel<2, true, true>
+                              : (ahead ? qsa_score4_kernel<2, false, true> : qsa_score4_kernel<2, false, false>);
+      CR_CUDA(launch_pdl(kernel, grid, dim3(256), 0, stream, P));
       CR_LAUNCH_CHECK("qsa_score_kernel");
       st = CR_OK;
     }

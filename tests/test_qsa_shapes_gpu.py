@@ -272,9 +272,9 @@ def test_span_scores(starts, R, pad, shift):
 
 
 # scores of one and two rows, of every block and of a range, from pools on and off the 16-byte boundary (which the wide loads want):
-# the order of the 128 products of a dot differs, fp32 throughout
+# the order of the 128 products of a dot differs, fp32 throughout; pairs of rows in more CTAs than the form with half a tile in flight has places
 @pytest.mark.parametrize("shift", [0, 1, 2])
-@pytest.mark.parametrize("starts,R,b0,b1", [([2051], 1, 0, 0), ([9003, 2300], 2, 0, 0), ([9003], 1, 700, 2200), ([9004], 2, 5, 2251)])
+@pytest.mark.parametrize("starts,R,b0,b1", [([2051], 1, 0, 0), ([9003, 2300], 2, 0, 0), ([79997] * 4, 2, 0, 0), ([9003], 1, 700, 2200), ([9004], 2, 5, 2251)])
 def test_short_span_scores_of_shifted_pools(starts, R, b0, b1, shift):
     capi, layers, g, w = _weights(16)
     gen = torch.Generator(device="cuda").manual_seed(R + b0)
