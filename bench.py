@@ -47,11 +47,11 @@ NCU_TRAFFIC = {
     "gdn_prefill_32k": {"gdn_chunk_scan_tc_kernel": ("token", (526.38e6 + 99.4e6) / 7104),
                         "gdn_chunk_local_kernel": ("token", (75.55e6 + 282.96e6) / 4544),
                         "gdn_gate_kernel": ("token", (174.89e6 + 34.3e6) / 7104)},
-    "decode_262k": {"qsa_score_kernel": ("step", 134.24e6 + 2.98e6), "qsa_attn_kernel": ("step", 16.98e6),
+    "decode_262k": {"qsa_score_kernel": ("step", 134.24e6 + 0.94e6), "qsa_attn_kernel": ("step", 16.98e6),
                     "qsa_topk_cluster_kernel": ("step", 1.11e6), "qsa_prep_kernel": ("step", 0.13e6),
                     "gdn_step_kernel": ("step", 9.47e6)},
-    "qsa_prefill_262k": {"qsa_attn_kernel": ("step", 3500e6 + 14.7e6), "qsa_score_tc_kernel": ("step", 141.3e6 + 483.3e6),
-                         "qsa_topk_kernel": ("step", 831.7e6 + 6.3e6)},
+    "qsa_prefill_262k": {"qsa_attn_kernel": ("step", 3434e6 + 14.7e6), "qsa_score_tc_kernel": ("step", 149.9e6 + 483.8e6),
+                         "qsa_topk_kernel": ("step", 834.9e6 + 3.6e6)},
     "qsa_attend_262k_drift": {"qsa_flash_tc_kernel": ("step", 1005.9e6 + 12.8e6)},
     "verify_131k": {"qsa_attn_kernel": ("step", 288.1e6 + 0.1e6), "gdn_step_kernel": ("step", 23.3e6)},
 }

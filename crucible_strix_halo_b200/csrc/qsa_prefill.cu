@@ -35,17 +35,21 @@ static size_t partial_bytes(const cr_geometry* g, int rows) {
 static size_t list_ints(int rows) { return (size_t)((rows + 7) / 8) * qsa_union_cap(8) * 2; }
 // Which of the two kernels serves a part, or a tile of it.  Measured on parts of 2 to 2,048 rows at 8 K to 262 K positions, where the
 // position hardly matters (sparse rows, us of the attention stage):
-//   row-wise, up to 8 heads per KV head   5 + 24 for each wave of one (row, KV head) per SM: 29 to 74 rows, 50 to 148, 190 at 512,
-//                                         664 at 2,048;
-//   row-wise, 9 to 12 heads (two warps)   23 to 16 rows, 34 to 37, then 4 + 52.5 per wave: 57 to 74 rows, 110 to 148, 1,470 at 2,048;
-//   tiled                                 24 + 1.3 for each entry of a row and wave of CTAs, divided by the splits of a list: 128
-//                                         rows of 16 heads 33 at 42 entries and 70 at 264, 1,024 rows 78 and 340, 2,048 rows 150 and 700.
-// Two warps: the tiled kernel from 17 rows on, whatever the rows share (at 513 entries, the most there are, the lines cross between
-// 80 and 512 rows).
+//   row-wise, up to 8 heads per KV head   4 + 24 for each wave of one (row, KV head) per SM: 28 to 74 rows, 50 to 54 to 148, 188 at 512,
+//                                         660 at 2,048;
+//   row-wise, 9 to 12 heads (two warps)   19.5 to 16 rows, 31 to 37, then 53 per wave: 53 to 74 rows, 112 to 148, 1,490 at 2,048;
+//   tiled                                 29 + 1.1 for each entry of a row (of 16 in a tile) and wave of CTAs, divided by the splits of a list:
+//                                         128 rows of 16 heads 30 at 42 entries and 64 at 264, 1,024 rows 76 and 318, 2,048 rows 142
+//                                         and 626.
+// The lines below stand where the kernels crossed while the tiled one took 24 + 1.3 (2,048 rows 150 and 700).  Since then they cross later, at 283
+// entries for 243 at 2,048 rows and at 250 for 213 at 768; the tiles between the two stay row-wise, with the bits that it keeps of queries and
+// probabilities.
+// Two warps: the tiled kernel from 17 rows on, whatever the rows share.  (Rows that share little cross later, 17 to 37 rows at 200 entries a
+// row, where they take 31 us row-wise and 33 to 40 tiled above that, 64 to 74 rows at 340, 128 rows beyond 513.)
 // One warp: a part of one wave row-wise (64 rows at 42 entries, nearly the fewest: 27 to 29 tiled).  Above that the lists decide.
 // While every tile has an SM of its own, a tile left out makes the tiled kernel no quicker and the row-wise launch beside it costs
 // its whole waves (192 rows about the line, tile by tile: 108 us, either kernel alone 81 to 86), so the part goes one way; lists
-// built in vain cost 15 us at 128 rows and 27 at 512, and a wave of row-wise CTAs for a tile past kTileMost 30.  With the lists paid for
+// built in vain cost 12 us at 117 rows and 23 at 512, and a wave of row-wise CTAs for a tile past kTileMost 30.  With the lists paid for
 // the lines cross at 263 entries per row for 128 and 512 rows, 213 for 768 (one CTA per tile).  Longer parts decide tile by tile:
 // 165 entries for 1,204 rows, 243 for 2,048, two waves of CTAs either way.
 static bool one_warp_streams(const cr_geometry* g) { return g->q_heads / g->kv_heads <= 8; }

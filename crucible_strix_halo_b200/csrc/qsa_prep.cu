@@ -136,7 +136,7 @@ __device__ __forceinline__ void pool_block(const cr_qsa_args& a, int b) {
 //
 // Bound: HBM for a part (query rows in and out, fp16 copies, cache rows), latency for a step.  A head lives in one warp
 // (128-bit loads, shuffle reduction, no barrier but the one behind the row's 32 cosines and sines, which every unit of the
-// row shares: angles past 105,615 take cosf's long reduction).  A step gives every unit a warp of its own (UPW = 1); a part
+// row shares).  A step gives every unit a warp of its own (UPW = 1); a part
 // takes a row per CTA with all loads of a warp issued first (UPW = 5).  2,048 rows at 262,144 positions: 98.8 us as one
 // CTA per (row, unit), 28 us now (4.9 TB/s).  With a compact ring the warp that pools a call's first block looked at sixteen rows one by
 // one, two divisions for each of three positions: 10.0 us for 117 rows where a full raw cache took 3.9; a lane per row now.

@@ -1,24 +1,27 @@
 // Exact top-512 of a row of indexer scores for sm_100a (the job of LaunchQsaTop, engine/layers/qsa_long.h:111-380):
 // the 512 best blocks in the total order (score descending, block id ascending), emitted in ascending block id.
 //
-// Method: group maxima, pivot, filter, histogram, mark, compact.  One CTA of 1024 threads per row.
+// Method: group maxima, pivot, filter, histogram, mark, compact.  One CTA of T = 1,024, 512 or 256 threads per row (many rows take the
+// smaller ones), or a cluster of eight of 1,024 (long rows of steps; its own pivot, below).
 //   1. Scores are >= +0, so their fp32 bit patterns order like unsigned integers (key = pattern + 1; 0 = no element).
-//      Thread t reads the elements t, t + 1024, ... (its group) and keeps their maximum.
+//      The row falls into 1,024 groups: a thread reads every T-th element, or four where the row lies at 16 bytes, and keeps the maxima of
+//      its 1,024 / T groups.
 //   2. The pivot is a lower bound of the 512th largest of the 1024 group maxima: they are counted in 2,048 bins of the key
 //      range below the largest, and a suffix scan finds the bin that holds the 512th.  At least 512 elements are >= the
 //      bin's lower edge (those maxima themselves), so every element that can be among the best 512, ties included, is; with
 //      unrelated scores about 700 are.
-//   3. A second pass gathers the elements >= the pivot into a shared-memory list (warp-aggregated appends).
+//   3. A second pass gathers the elements >= the pivot into a shared-memory list (warp-aggregated appends); the form for few rows of 14,337 to
+//      32,768 blocks holds its elements in registers and reads the row once.
 //   4. The same histogram over the list, between its known bounds, finds the bin of the 512th key: everything above is
 //      taken, and the few elements inside the bin are ranked against each other (key, then index).  A crowded bin is
 //      divided again, down to single keys; of equal keys the lowest indices are taken.
 //   5. The taken elements set their bit in a bitmap over the row, which is compacted in index order: a prefix sum over
 //      word popcounts gives every thread its output offset.
-//   Rows of at most 4096 elements skip 1-3: every element goes into the list.
+//   Rows that fit the list (4,096 elements; 3,072 with 512 or 256 threads) skip 1-3: every element goes into it.
 //   Bound: block barriers of a latency chain (the row itself is read at L2 speed).  As 31-step bisections with a
 //   block-wide count per bit, a row of 2,300 blocks took 16 us, 7 now; 2,048 rows of 65,536 blocks 268 -> 203 us (long
 //   rows are read four elements at a time), of 8,192 blocks 125 -> 68 us.
-//   When more than 4096 elements pass the pivot (long runs of equal scores), the row takes the slow exact path: the
+//   When more elements pass the pivot than the list holds (long runs of equal scores), the row takes the slow exact path: the
 //   same bisection over the whole row, counting with plain reductions, then the values above the 512th best pattern
 //   plus its first ties in index order from a second bitmap.
 // The same routine serves a whole row, a rank's block range (candidates with their scores, for split-KV across
