@@ -240,6 +240,32 @@ def test_selection_of_step_rows(nb, sessions, pattern, pad):
         assert int(s.nsel[0]) == 512
 
 
+# rows of every length beside a long one, by clusters: shares of a few dozen elements, all of which pass, up to the first that has 64 to
+# offer in each; rows that attend everything in between
+@pytest.mark.parametrize("long_nb", [21000, 57501, 70001])
+def test_selection_of_mixed_rows_by_clusters(long_nb):
+    capi, layers, g, w = _weights(16)
+    gen = torch.Generator(device="cuda").manual_seed(long_nb)
+    lengths = [513, 519, 300, 2051, 4095, 4096, 4097, 4103, 7651, 9001, long_nb]
+    pool = torch.randn((long_nb + 31) // 32, 128, 32, device="cuda", generator=gen).flatten()
+    spans, args, z = [], (capi.QsaArgs * len(lengths))(), torch.zeros(1, 16, 512, device="cuda")
+    for i, nb in enumerate(lengths):
+        s = layers.QsaSession(g, 64)                                    # the spans share one pool and write no cache
+        s.ik_pool, s.sstride = pool, nb
+        s.scores = torch.zeros(1, nb, device="cuda")
+        idx = torch.randn(1, 640, device="cuda", generator=gen)
+        args[i] = layers.qsa_args(w, s, z, z, z, idx, z, 4 * nb - 1)
+        spans.append((s, idx))
+    capi.check(capi.lib.cr_qsa_select(C.byref(g), args, len(lengths), None, 0, None))
+    for (s, _), nb in zip(spans, lengths):
+        if nb <= capi.SEL_BLOCKS:
+            assert int(s.nsel[0]) == -1
+            continue
+        v = s.scores[0].double().cpu().numpy()
+        np.testing.assert_array_equal(s.sel[0].cpu().numpy(), np.sort(np.lexsort((np.arange(nb), -v))[:512]))
+        assert int(s.nsel[0]) == 512
+
+
 # scores of spans of 3 to 16 rows: every number of row quartets, ragged last tiles, several tiles to a warp (the longest), spans of
 # different length in a launch, a pool off the 16-byte boundary (scalar loads), score rows off it
 @pytest.mark.parametrize("starts,R,pad,shift", [([2050, 9003], 3, 0, 0), ([4096], 4, 1, 0), ([2300, 2041], 5, 0, 0), ([9003], 9, 2, 0), ([33001], 13, 0, 0),
